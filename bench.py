@@ -406,7 +406,7 @@ def batched_build(threads: int, count: int) -> dict:
     reb_tuned = rebuilds()
     check()
     # label construction alone: one forest fill against the per-graph fills
-    # (our dataflow fill, and the reference's level-by-level mapping)
+    # (our block fill, and the reference's level-by-level mapping)
     plain_ms, plain_bad = 0.0, 0
     for gs in seq:
         ms, bad = gs.fill_labels_plain("pair")
@@ -466,7 +466,7 @@ def small_graph_run(name: str, threads: int, steps: int, build_reps: int, plain_
     fill_bytes = 8 * info["label_size"] + 8 * info["pos_size"] + 4 * info["label_updates"]
     plain_fill_ms, plain_fill_bad = g.fill_labels_plain("pair")
     assert plain_fill_bad == 0, "the plain fill mapping disagrees with the labels"
-    fill = {"kernel": "fill_flow_kernel", "updates": info["label_updates"], "seconds": fill_s,
+    fill = {"kernel": "block_fill_kernel", "updates": info["label_updates"], "seconds": fill_s,
             "plain_gpu_seconds": plain_fill_ms / 1e3,
             "plain_gpu": "the reference's mapping: one thread per (v,u) pair, one launch + sync per tree level",
             "updates_per_s": info["label_updates"] / fill_s if fill_s > 0 else None,
@@ -827,7 +827,7 @@ def main():
         assert parity["mismatches_lca"] == 0 and parity["mismatches_nolca"] == 0, "answers differ from Dijkstra"
     fill_s = info["t_fill_gpu_us"] / 1e6
     fill_bytes = 8 * info["label_size"] + 8 * info["pos_size"] + 4 * info["label_updates"]
-    fill = {"kernel": "fill_flow_kernel", "updates": info["label_updates"], "seconds": fill_s,
+    fill = {"kernel": "block_fill_kernel", "updates": info["label_updates"], "seconds": fill_s,
             "updates_per_s": info["label_updates"] / fill_s if fill_s > 0 else None,
             "algorithmic_bytes": fill_bytes, "achieved_gbs": fill_bytes / fill_s / 1e9 if fill_s > 0 else None,
             "frac_of_hbm": fill_bytes / fill_s / 1e9 / peak if fill_s > 0 else None}

@@ -6,7 +6,7 @@
 // A batch of small graphs therefore spends its time on launches that fill a
 // few SMs.  Here the graphs' vertices share one numbering: ElimPlan runs
 // level H_i - s of every graph in launch s and every graph's global order in
-// one last launch; FillPlan fills the forest of all trees in one dataflow
+// one last launch; FillPlan fills the forest of all trees in one
 // launch.  Host phases between them (elimination sets, tree, Euler tour,
 // sparse table, label layout) run per graph on a thread pool.
 //
@@ -175,9 +175,7 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch 
                    (long long)b->info.t_tree_us, sum, mx);
     }
     clk.reset();
-    int height = 0;
-    for (const gh::Graph *g : b->gs) height = std::max(height, g->tree_height);
-    gh::TilePolicy pol = gh::TilePolicy::for_height(height);
+    gh::TilePolicy pol;
     if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
       GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
     b->fill = std::make_unique<gh::FillPlan>(b->gs, pol, b->elim->lists);

@@ -1,0 +1,920 @@
+// fill_blocks.cu -- the no-hub L4 label fill (the work of
+// makeH2HLabel_noHub_noComm_3 / makeH2HLabel_noCommunication_D_noHub_3,
+// tanslate.cu:511-617, kernel_functions.cu:717-796, with the L4 block
+// :738-743 enabled) as min-plus products over blocks of the tree.
+//
+// Row v holds dis[v][j] = D(v, a_j), the distance to the ancestor a_j at depth
+// j + 1, and
+//   D(v, a) = min over u in X(v)\{v} of sc(v, u) + E(u, a),
+//   E(u, a) = dis[u][j] (u below a), 0 (u = a), dis[a][p_u] (u above a).
+// Node by node that is a load per (v, u, j) and a dependency per tree level.
+// Here the tree is cut into blocks of at most 32 nodes, each a connected piece
+// with one top t.  Every node i of a block has its upper neighbours among the
+// block's own nodes and X(t) (the lists nest: X(v) without v's father lies in
+// X(father)), so replacing a neighbour inside the block by that neighbour's
+// own recursion leaves, for every ancestor a above the block,
+//   D(i, a) = min over u in X(t) of S(i, u) + E(u, a),
+//   S(i, u) = min(sc(i, u), min over w in X(i) inside the block of sc(i, w) + S(w, u)).
+// S needs no label (closure_kernel computes it for all blocks at once), and
+// the columns above the block become one min-plus product [32 x |X(t)|] by
+// [|X(t)| x depth(t)] whose second factor is loaded once for 32 rows.  The
+// columns inside the block follow from a second, 32 x 32 product with the
+// direct weights and a short sequential pass.  Sums are those of the
+// recursion, regrouped; they are taken in unsigned 32-bit arithmetic, where
+// two values below 2^31 cannot wrap, with INT_MAX for "no entry".
+//
+// A fill that takes a warp per (node, column block, separator chunk) tile is
+// bound by one L2 load per update and 13 us per tree level of the narrow top.
+// On one GB300 the blocks took the fill of a 264k-vertex road graph (4.5e9
+// updates) from 28.4 to 4.7 ms and of a 1M-vertex one (3.8e10) from 104 to
+// 18.9 ms.
+#include <algorithm>
+#include <climits>
+#include <cstdio>
+#include <cstdlib>
+
+#include "graph.h"
+#include "scan.h"
+
+namespace gh {
+
+namespace {
+
+constexpr int kRows = 32;     // nodes of a block (rows of its product)
+constexpr int kSmall = 16;    // largest light subtree that joins its father's block whole
+constexpr int kCols = 64;     // columns of one step of the product
+constexpr int kMembers = 32;  // separator members of one step
+constexpr int kEStride = 72;  // row stride of the staged second factor: 16-byte stores of four rows hit all banks
+constexpr unsigned kInf = 0x7fffffffu;
+
+constexpr int kErrWait = 4;    // a dependency wait ran out
+constexpr int kErrNested = 6;  // an upper neighbour is missing from the block top's separator
+
+template <typename T>
+T *dalloc(size_t n, int64_t &bytes) {
+  T *p = nullptr;
+  if (n == 0) n = 1;
+  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  bytes += (int64_t)(n * sizeof(T));
+  return p;
+}
+
+__device__ __forceinline__ int ld_acquire(const int *p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int *p, int v) {
+  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int ld_relaxed(const int *p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned add_min(unsigned a, unsigned b, unsigned c) { return __viaddmin_u32(a, b, c); }
+
+// ------------------------------------------------------------ the plan
+//
+// Blocks from the heavy-path layout (hld: a depth-first order that visits the
+// heavy child first, so a subtree is a range of it).  A light subtree of at
+// most kSmall nodes joins its father's block; the nodes left are paths, cut
+// greedily from the top so that a path node with its small subtrees stays in
+// one block and a block holds at most kRows nodes.  A path node whose small
+// subtrees alone exceed a block leaves each of them a block of its own.  On a
+// 264k-vertex road graph: 11.2k blocks of 23.5 nodes on average, 67 blocks
+// from the root to the deepest leaf (1,347 nodes), 9e9 product terms for
+// 4.6e9 updates of the recursion, and 3e8 loads of E in place of 4.6e9.  With
+// kSmall 8 the blocks average 19 nodes; blocks of 64 nodes would halve the
+// loads again but add 15% terms and double the top's in-block pass.
+
+// size of the subtree at every position, if at most kSmall (else kSmall + 1)
+__global__ void small_size_kernel(const int *hld, const int *depth, int *size, int *weight, int n) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int d = depth[hld[k]];
+    int s = 1;
+    while (s <= kSmall && k + s < n && depth[hld[k + s]] > d) s++;
+    size[k] = s;
+    weight[k] = 1;
+  }
+}
+
+// weight of a path node: itself and its small light subtrees
+__global__ void hang_weight_kernel(const int *father, const int *htop, const int *hpos, const int *size, int *weight,
+                                   int n) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const int f = father[v];
+    if (f < 0 || htop[v] != v) continue;
+    const int s = size[hpos[v]];
+    if (s <= kSmall) atomicAdd(weight + hpos[f], s);
+  }
+}
+
+// Greedy cut of every long path, one warp per path: lanes load 32 path nodes,
+// the running weight goes through them by shuffles.
+__global__ void cut_paths_kernel(const int *father, const int *htop, const int *hpos, const int *hld, const int *size,
+                                 const int *weight, int *block_top, int n) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < n;
+       base += ((gridDim.x * (int64_t)blockDim.x) >> 5) * 32) {
+    const int v = (int)base + lane;
+    const bool path = v < n && htop[v] == v && (father[v] < 0 || size[hpos[v]] > kSmall);
+    unsigned todo = __ballot_sync(0xffffffffu, path);
+    while (todo) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int top = (int)base + l;
+      int cur = kRows, bt = top;  // the first node opens a block
+      for (int64_t k0 = hpos[top]; k0 < n; k0 += 32) {
+        const int64_t k = k0 + lane;
+        const int u = k < n ? hld[k] : -1;
+        const bool on = u >= 0 && htop[u] == top;
+        int w = on ? weight[k] : 0;
+        if (w > kRows) w = 1;
+        const unsigned live = __ballot_sync(0xffffffffu, on);
+        const int cnt = live == 0xffffffffu ? 32 : __ffs(~live) - 1;  // the path's nodes are contiguous
+        int mine = 0;
+        for (int s = 0; s < cnt; s++) {
+          const int ws = __shfl_sync(0xffffffffu, w, s), us = __shfl_sync(0xffffffffu, u, s);
+          if (cur + ws > kRows) {
+            cur = 0;
+            bt = us;
+          }
+          cur += ws;
+          if (s == lane) mine = bt;
+        }
+        if (lane < cnt) block_top[k] = mine;
+        if (cnt < 32) break;
+      }
+    }
+  }
+}
+
+// Every node's block top; nodes and separator work per block top and level.
+__global__ void node_block_kernel(const int *father, const int *htop, const int *hpos, const int *depth,
+                                  const int64_t *pos_hash, const int *size, const int *weight, const int *block_top,
+                                  int *top_of, int *count, int *lvl_tops, int *lvl_width, unsigned long long *lvl_work,
+                                  int n) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    int u = v, c = -1;
+    for (;;) {
+      const int t = htop[u], f = father[t];
+      if (f < 0 || size[hpos[t]] > kSmall) break;
+      c = t;
+      u = f;
+    }
+    const int bt = c >= 0 && weight[hpos[u]] > kRows ? c : block_top[hpos[u]];
+    const int d = depth[v];
+    top_of[v] = bt;
+    atomicAdd(count + bt, 1);
+    if (bt == v) atomicAdd(lvl_tops + d - 1, 1);
+    atomicAdd(lvl_width + d - 1, 1);
+    atomicAdd(lvl_work + d - 1, (unsigned long long)(pos_hash[v + 1] - pos_hash[v] - 1) * (unsigned long long)d);
+  }
+}
+
+// Blocks in the order of their tops' depths: a block's father block (the
+// block of its top's father) comes before it.
+__global__ void order_blocks_kernel(const int *top_of, const int *depth, const int64_t *lvl_first, int *lvl_next,
+                                    int *blk_top, int *blk_of_top, int n) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    if (top_of[v] != v) continue;
+    const int d = depth[v] - 1;
+    const int b = (int)lvl_first[d] + atomicAdd(lvl_next + d, 1);
+    blk_top[b] = v;
+    blk_of_top[v] = b;
+  }
+}
+
+// Level classes of TilePolicy: 0 narrow (fewer nodes than SMs), 2 heavy
+// (wider, its nodes averaging at least per_node updates), 1 the others.
+__global__ void level_class_kernel(const int *width, const unsigned long long *work, int nlev, int nsm,
+                                   unsigned long long per_node, int *cls) {
+  for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nlev; l += gridDim.x * blockDim.x)
+    cls[l] = width[l] < nsm ? 0 : work[l] >= per_node * (unsigned long long)width[l] ? 2 : 1;
+}
+
+__global__ void block_sizes_kernel(const int *blk_top, const int *count, const int64_t *pos_hash, int *rows, int *mem,
+                                   int *cells, int nblk) {
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nblk; b += gridDim.x * blockDim.x) {
+    int r = 0, m = 0;
+    if (b < nblk) {
+      const int t = blk_top[b];
+      r = count[t];
+      m = (int)(pos_hash[t + 1] - pos_hash[t]) - 1;
+    }
+    rows[b] = r;
+    mem[b] = m;
+    cells[b] = m * ((r + 3) & ~3);
+  }
+}
+
+// Tasks of every block: the columns above it in one task, or cut into
+// policy.col_block columns each.
+__global__ void block_tasks_kernel(const int *blk_top, const int *depth, const int *mem, const int64_t *boff,
+                                   const int *lvl_cls, TilePolicy pol, int *ntask, int *pieces, int *tcols, int nblk) {
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nblk; b += gridDim.x * blockDim.x) {
+    int nt = 0, tc = kCols;
+    if (b < nblk) {
+      const int d = depth[blk_top[b]], m = mem[b];
+      const int wb = lvl_cls[d - 1], sb = m <= 16 ? 0 : m <= 64 ? 1 : m <= 256 ? 2 : 3;
+      const int cols = d - 1;
+      tc = (pol.col_block[wb][sb] + kCols - 1) / kCols * kCols;
+      if ((int64_t)m * d <= pol.small_work[wb][sb]) tc = max(kCols, (cols + kCols - 1) / kCols * kCols);
+      nt = max(1, (cols + tc - 1) / tc);
+    }
+    ntask[b] = nt;
+    pieces[b] = b < nblk ? nt * (int)(boff[b + 1] - boff[b]) : 0;
+    tcols[b] = tc;
+  }
+}
+
+__global__ void scatter_nodes_kernel(const int *top_of, const int *blk_of_top, const int64_t *boff, int *fill, int *bnode,
+                                     int n) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const int b = blk_of_top[top_of[v]];
+    const int64_t at = boff[b] + atomicAdd(fill + b, 1);
+    if (at < boff[b + 1]) bnode[at] = v;
+  }
+}
+
+// A block's nodes in depth-first order (ancestors first), every node's block
+// and place in it, and the top's members (positions, row offsets).  One warp
+// per block.
+__global__ void block_nodes_kernel(const int *blk_top, const int64_t *boff, const int64_t *moff, const int *hpos,
+                                   const int64_t *pos_hash, const int *pos_pos, const int *pos_id, const int64_t *drow,
+                                   int *bnode, int *blk_of, unsigned char *loc_of, int *bm_p, int64_t *bm_row,
+                                   int nblk) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; b < nblk;
+       b += (gridDim.x * (int64_t)blockDim.x) >> 5) {
+    const int64_t o = boff[b];
+    const int R = (int)(boff[b + 1] - o);
+    const int v = lane < R ? bnode[o + lane] : -1;
+    const int k = lane < R ? hpos[v] : INT_MAX;
+    int r = 0;
+    for (int s = 0; s < R; s++) r += __shfl_sync(0xffffffffu, k, s) < k;
+    __syncwarp();
+    if (lane < R) {
+      bnode[o + r] = v;
+      blk_of[v] = (int)b;
+      loc_of[v] = (unsigned char)r;
+    }
+    const int64_t pb = pos_hash[blk_top[b]], m0 = moff[b];
+    const int m = (int)(moff[b + 1] - m0);
+    for (int i = lane; i < m; i += 32) {
+      bm_p[m0 + i] = pos_pos[pb + i];
+      bm_row[m0 + i] = drow[pos_id[pb + i]];
+    }
+  }
+}
+
+__global__ void expand_tasks_kernel(const int64_t *task0, int *task_blk, int nblk) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; b < nblk;
+       b += (gridDim.x * (int64_t)blockDim.x) >> 5)
+    for (int64_t t = task0[b] + lane; t < task0[b + 1]; t += 32) task_blk[t] = (int)b;
+}
+
+// ------------------------------------------------------------ the closure
+
+struct BlockArgs {
+  const int *blk_top;
+  const int64_t *boff, *moff, *soff;  // first node, first member, first cell of S and of the direct weights
+  const int *bnode;
+  const int *blk_of;
+  const unsigned char *loc_of;
+  const int *bm_p;
+  const int64_t *bm_row;
+  const int *father, *depth;
+  const int64_t *drow, *pos_hash;
+  const int *pos_pos, *pos_id, *pos_w;
+  unsigned *direct, *closed;  // per block [member][row], rows padded to a multiple of four
+  int nblk;
+  int *err;
+};
+
+// Members of X(v) inside the block (the end of v's position list, v itself
+// excluded: positions at or below the top's), one per lane: place and weight
+// into tl / tw; returns their number in every lane.
+__device__ __forceinline__ int stage_inner(const BlockArgs &A, int v, int dt, unsigned char *tl, int *tw, int lane) {
+  const int64_t pb = A.pos_hash[v], e = A.pos_hash[v + 1] - 2 - lane;
+  const bool in = e >= pb && __ldg(A.pos_pos + e) >= dt;
+  if (in) {
+    tl[lane] = A.loc_of[__ldg(A.pos_id + e)];
+    tw[lane] = __ldg(A.pos_w + e);
+  }
+  return __popc(__ballot_sync(0xffffffffu, in));
+}
+
+constexpr int kClosureWarps = 4;
+
+// S and the direct weights of every block, 32 members at a time: a warp
+// scatters its block's list entries into a 32 x 32 tile (row i, member), writes
+// it out as the direct weights, then lane k carries member k's column through
+// the block's nodes in depth-first order.  Columns are independent, so the
+// chunks of a wide separator run in different warps (blockIdx.y).  Bound:
+// latency of the scattered list reads; 0.1 ms beside the product's 2 ms on
+// the 264k-vertex graph.
+__global__ void __launch_bounds__(32 * kClosureWarps) closure_kernel(BlockArgs A) {
+  __shared__ unsigned s_row[kClosureWarps][kRows * 33];
+  __shared__ int s_tw[kClosureWarps][kRows * 32];
+  __shared__ unsigned char s_tl[kClosureWarps][kRows * 32];
+  __shared__ int s_p[kClosureWarps][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int b = blockIdx.x * kClosureWarps + wid;
+  if (b >= A.nblk) return;
+  const int64_t m0 = A.moff[b];
+  const int m = (int)(A.moff[b + 1] - m0);
+  if ((int)blockIdx.y * 32 >= m) return;
+  unsigned *row = s_row[wid];
+  int *tw = s_tw[wid], *sp = s_p[wid];
+  unsigned char *tl = s_tl[wid];
+  const int64_t o = A.boff[b];
+  const int R = (int)(A.boff[b + 1] - o), Rp = (R + 3) & ~3;
+  const int dt = A.depth[A.blk_top[b]] - 1;
+  int tc = 0;  // lane i: inner members of node i
+  for (int i = 0; i < R; i++) {
+    const int c = stage_inner(A, A.bnode[o + i], dt, tl + 32 * i, tw + 32 * i, lane);
+    if (lane == i) tc = c;
+  }
+  int64_t lb = 0, le = 0;  // lane i: node i's list entries above the block
+  if (lane < R) {
+    const int v = A.bnode[o + lane];
+    lb = A.pos_hash[v];
+    le = A.pos_hash[v + 1] - 1 - tc;
+  }
+  __syncwarp();
+  for (int k0 = blockIdx.y * 32; k0 < m; k0 += gridDim.y * 32) {
+    const int kn = min(32, m - k0);
+    const int p = k0 + lane < m ? A.bm_p[m0 + k0 + lane] : INT_MAX;
+    sp[lane] = p;
+    const int pfirst = __shfl_sync(0xffffffffu, p, 0), plast = __shfl_sync(0xffffffffu, p, kn - 1);
+    for (int64_t a = lb, z = le; lane < R;) {  // first entry of node `lane` at or after the chunk
+      if (a >= z) {
+        lb = a;
+        break;
+      }
+      const int64_t mid = (a + z) >> 1;
+      if (__ldg(A.pos_pos + mid) < pfirst) a = mid + 1; else z = mid;
+    }
+    for (int i = 0; i < R; i++) row[i * 33 + lane] = kInf;
+    __syncwarp();
+    for (int i = 0; i < R; i++) {
+      const int64_t e = __shfl_sync(0xffffffffu, lb, i) + lane;
+      if (e >= __shfl_sync(0xffffffffu, le, i)) continue;
+      const int q = __ldg(A.pos_pos + e);
+      if (q > plast) continue;
+      int x = 0, y = kn - 1;
+      while (x < y) {
+        const int mid = (x + y) >> 1;
+        if (sp[mid] < q) x = mid + 1; else y = mid;
+      }
+      if (sp[x] == q) row[i * 33 + x] = (unsigned)__ldg(A.pos_w + e);
+      else atomicCAS(A.err, 0, kErrNested);
+    }
+    __syncwarp();
+    const int64_t out = A.soff[b] + (int64_t)k0 * Rp;
+    for (int k = 0; k < kn; k++)
+      if (lane < Rp) A.direct[out + k * Rp + lane] = lane < R ? row[lane * 33 + k] : kInf;
+    __syncwarp();
+    for (int i = 1; i < R; i++) {
+      unsigned r = row[i * 33 + lane];
+      const int c = __shfl_sync(0xffffffffu, tc, i);
+      for (int x = 0; x < c; x++) r = add_min((unsigned)tw[32 * i + x], row[tl[32 * i + x] * 33 + lane], r);
+      row[i * 33 + lane] = r;
+    }
+    __syncwarp();
+    for (int k = 0; k < kn; k++)
+      if (lane < Rp) A.closed[out + k * Rp + lane] = lane < R ? row[lane * 33 + k] : kInf;
+    __syncwarp();
+  }
+}
+
+// ------------------------------------------------------------ the product
+
+struct FillKernelArgs {
+  BlockArgs B;
+  int *dis;
+  const int64_t *hld_row;  // heavy paths, top to bottom: the row offset of the node at each position
+  const int64_t *seg_off;  // root-path segments per node
+  const int *seg_top, *seg_pos;
+  const int *task_blk;
+  const int64_t *task0;
+  const int *tcols;
+  int ntasks;
+  int *done, *count, *next;
+  long long spin_limit;
+  int max_segs;
+  unsigned long long *trace_t;  // non-null (GPUH2H_TRACE): each node's publish time, ns
+};
+
+// A CTA of four warps takes tasks (a block, a range of columns) in the order
+// of the blocks' depths, waits for the father block's flag, and sweeps its
+// columns 64 at a time and the top's members 32 at a time: the second factor
+// E goes through registers into shared memory one step ahead (so a step's
+// loads overlap the product before it), every thread owns a 4 x 4 patch of
+// the 32 x 64 result.  The last task of a block to finish fills in the
+// columns inside the block and publishes it.  Rows produced in the launch are
+// read through L2 (ld.global.cg).  A quad of four columns that lies above a
+// member (p_u >= J + 4) is one 128-bit load of u's row; below it, four
+// ancestors' entries at p_u, 16 members of consecutive positions per warp
+// request.
+__global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
+  extern __shared__ __align__(16) int s_seg[];
+  __shared__ __align__(16) unsigned s_E[kMembers * kEStride];
+  __shared__ __align__(16) unsigned s_S[kMembers * kRows];
+  __shared__ __align__(16) int64_t s_arow[2][kCols];
+  __shared__ int64_t s_rowoff[kRows];
+  __shared__ unsigned s_M[kRows * 33];
+  __shared__ int s_tw[kRows * 32];
+  __shared__ unsigned char s_tl[kRows * 32];
+  __shared__ int s_tc[kRows], s_dcol[kRows], s_par[kRows];
+  __shared__ unsigned s_anc[kRows];
+  __shared__ int s_t, s_flag;
+  const BlockArgs &B = A.B;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  int *const s_top = s_seg, *const s_pos = s_seg + A.max_segs;
+  const int hk = (wid >> 1) * 16 + (lane >> 1);         // the member of a step this thread loads
+  const int q0 = (wid & 1) * 8 + (lane & 1);            // its quads of columns: q0, q0 + 2, q0 + 4, q0 + 6
+  const int ry = tid >> 4, cx = tid & 15;               // its patch of the result
+  for (;;) {
+    __syncthreads();  // the last task's shared memory is free
+    if (tid == 0) s_t = atomicAdd(A.next, 1);
+    __syncthreads();
+    const int t = s_t;
+    if (t >= A.ntasks) return;
+    const int b = __ldg(A.task_blk + t);
+    const int64_t task0 = __ldg(A.task0 + b);
+    const int ntask = (int)(__ldg(A.task0 + b + 1) - task0);
+    const int tc = __ldg(A.tcols + b);
+    const int top = __ldg(B.blk_top + b);
+    const int dt = __ldg(B.depth + top) - 1;  // columns above the block
+    const int64_t bo = __ldg(B.boff + b), m0 = __ldg(B.moff + b), so = __ldg(B.soff + b);
+    const int R = (int)(__ldg(B.boff + b + 1) - bo), Rp = (R + 3) & ~3;
+    const int m = (int)(__ldg(B.moff + b + 1) - m0);
+    const int c0 = (int)(t - task0) * tc, c1 = min(dt, c0 + tc);
+    const int64_t sb = __ldg(A.seg_off + top);
+    const int ns = (int)(__ldg(A.seg_off + top + 1) - sb);
+    for (int i = tid; i < ns; i += 128) {
+      s_top[i] = __ldg(A.seg_top + sb + i);
+      s_pos[i] = __ldg(A.seg_pos + sb + i);
+    }
+    if (tid < R) s_rowoff[tid] = __ldg(B.drow + __ldg(B.bnode + bo + tid));
+    __syncthreads();
+    auto ancestor_row = [&](int j) -> int64_t {  // row offset of the ancestor at depth j + 1
+      if (j >= c1) return 0;
+      int lo = 0, hi = ns - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (s_top[mid] <= j + 1) lo = mid; else hi = mid - 1;
+      }
+      return __ldg(A.hld_row + s_pos[lo] + (j + 1 - s_top[lo]));
+    };
+    s_arow[tid >> 6][tid & 63] = ancestor_row(c0 + tid);
+    const int nchunk = (m + kMembers - 1) / kMembers, ntile = (c1 - c0 + kCols - 1) / kCols;
+    const int nsteps = c1 > c0 ? nchunk * ntile : 0;
+    uint4 eb[4], sbuf[2];
+    auto issue_s = [&](const unsigned *src, int k0) {
+      const int nq = min(kMembers, m - k0) * (Rp >> 2);
+      const uint4 *p = reinterpret_cast<const uint4 *>(src + so + (int64_t)k0 * Rp);
+      sbuf[0] = tid < nq ? __ldg(p + tid) : make_uint4(kInf, kInf, kInf, kInf);
+      sbuf[1] = tid + 128 < nq ? __ldg(p + tid + 128) : make_uint4(kInf, kInf, kInf, kInf);
+    };
+    auto store_s = [&]() {
+      reinterpret_cast<uint4 *>(s_S)[tid] = sbuf[0];
+      reinterpret_cast<uint4 *>(s_S)[tid + 128] = sbuf[1];
+    };
+    auto issue_e = [&](int T, int k0) {
+      const int k = k0 + hk;
+      const bool kv = k < m;
+      const int p = kv ? __ldg(B.bm_p + m0 + k) : -1;
+      const int64_t row = kv ? __ldg(B.bm_row + m0 + k) : 0;
+      const int64_t *ar = s_arow[T & 1];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int q = q0 + 2 * i, J = c0 + T * kCols + 4 * q;
+        uint4 e = make_uint4(kInf, kInf, kInf, kInf);
+        if (kv && J < c1) {
+          if (p >= J + 4) {
+            e = __ldcg(reinterpret_cast<const uint4 *>(A.dis + row + J));
+          } else {
+            unsigned x[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              const int j = J + c;
+              x[c] = j < p    ? (unsigned)__ldcg(A.dis + row + j)
+                     : j == p ? 0u
+                     : j < c1 ? (unsigned)__ldcg(A.dis + ar[4 * q + c] + p)
+                              : kInf;
+            }
+            e = make_uint4(x[0], x[1], x[2], x[3]);
+          }
+        }
+        eb[i] = e;
+      }
+    };
+    if (nsteps > 0) issue_s(B.closed, 0);
+    if (tid == 0) {
+      int ok = 1;
+      const int f = __ldg(B.father + top);
+      if (f >= 0) {
+        const int *flag = A.done + __ldg(B.blk_of + f);
+        const long long t0 = clock64();
+        while (ld_acquire(flag) == 0) {
+          if (ld_relaxed(B.err) != 0 || clock64() - t0 > A.spin_limit) {
+            atomicCAS(B.err, 0, kErrWait);
+            ok = 0;
+            break;
+          }
+          __nanosleep(32);
+        }
+      }
+      s_flag = ok;
+    }
+    __syncthreads();
+    if (!s_flag) return;
+    if (nsteps > 0) issue_e(0, 0);
+    unsigned acc[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[r][c] = kInf;
+    int64_t arow_next = 0;  // threads below 64: the column's ancestor row two tiles ahead
+    for (int s = 0, T = 0, ch = 0; s < nsteps; s++) {
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        *reinterpret_cast<uint4 *>(s_E + hk * kEStride + 4 * (q0 + 2 * i)) = eb[i];
+      if (nchunk > 1 || s == 0) store_s();
+      if (ch == 0 && T > 0 && tid < kCols) s_arow[(T + 1) & 1][tid] = arow_next;
+      __syncthreads();
+      const int kn = min(kMembers, m - ch * kMembers);
+      int nT = T, nch = ch + 1;
+      if (nch == nchunk) {
+        nch = 0;
+        nT++;
+      }
+      if (s + 1 < nsteps) {
+        if (nchunk > 1) issue_s(B.closed, nch * kMembers);
+        issue_e(nT, nch * kMembers);
+      }
+      if (ch == 0 && tid < kCols) arow_next = ancestor_row(c0 + (T + 2) * kCols + tid);
+      if (4 * ry < Rp) {
+        const unsigned *pe = s_E + 4 * cx, *ps = s_S + 4 * ry;
+#pragma unroll 4
+        for (int k = 0; k < kn; k++) {
+          const uint4 e = *reinterpret_cast<const uint4 *>(pe + k * kEStride);
+          const uint4 w = *reinterpret_cast<const uint4 *>(ps + k * Rp);
+          const unsigned wr[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int r = 0; r < 4; r++) {
+            acc[r][0] = add_min(wr[r], e.x, acc[r][0]);
+            acc[r][1] = add_min(wr[r], e.y, acc[r][1]);
+            acc[r][2] = add_min(wr[r], e.z, acc[r][2]);
+            acc[r][3] = add_min(wr[r], e.w, acc[r][3]);
+          }
+        }
+      }
+      if (nch == 0) {  // the tile is complete
+        const int j = c0 + T * kCols + 4 * cx;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const int i = 4 * ry + r;
+          if (i < R && j < c1) {
+            int *out = A.dis + s_rowoff[i] + j;
+            if (j + 4 <= c1) {
+              *reinterpret_cast<uint4 *>(out) = make_uint4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            } else {
+#pragma unroll
+              for (int c = 0; c < 4; c++)
+                if (j + c < c1) out[c] = (int)acc[r][c];
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 4; c++) acc[r][c] = kInf;
+        }
+      }
+      T = nT;
+      ch = nch;
+      __syncthreads();
+    }
+    // ---- the last task of the block finishes it
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      s_flag = ntask == 1 || atomicAdd(A.count + b, 1) == ntask - 1;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!s_flag) continue;
+    // columns inside the block.  For nodes i below a (both in the block):
+    //   M(i, a) = min over u in X(i) of sc(i, u) + E(u, a); the part over u
+    // above the block is a product of the direct weights with column p_u of
+    // row a, just completed
+    unsigned mm[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) mm[r][c] = kInf;
+    if (R > 1 && m > 0) {
+      unsigned gb[8];
+      auto issue_g = [&](int k0) {
+        const bool kv = k0 + lane < m;
+        const int p = kv ? __ldg(B.bm_p + m0 + k0 + lane) : 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int a = wid + 4 * i;
+          gb[i] = kv && a < R ? (unsigned)__ldcg(A.dis + s_rowoff[a] + p) : kInf;
+        }
+      };
+      issue_s(B.direct, 0);
+      issue_g(0);
+      const int my = tid >> 3, mx = tid & 7;
+      for (int ch = 0; ch < nchunk; ch++) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) s_E[lane * 36 + wid + 4 * i] = gb[i];
+        store_s();
+        __syncthreads();
+        const int kn = min(kMembers, m - ch * kMembers);
+        if (ch + 1 < nchunk) {
+          issue_s(B.direct, (ch + 1) * kMembers);
+          issue_g((ch + 1) * kMembers);
+        }
+        if (2 * my < Rp) {
+#pragma unroll 4
+          for (int k = 0; k < kn; k++) {
+            const uint4 e = *reinterpret_cast<const uint4 *>(s_E + k * 36 + 4 * mx);
+            const uint2 w = *reinterpret_cast<const uint2 *>(s_S + k * Rp + 2 * my);
+            const unsigned wr[2] = {w.x, w.y};
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+              mm[r][0] = add_min(wr[r], e.x, mm[r][0]);
+              mm[r][1] = add_min(wr[r], e.y, mm[r][1]);
+              mm[r][2] = add_min(wr[r], e.z, mm[r][2]);
+              mm[r][3] = add_min(wr[r], e.w, mm[r][3]);
+            }
+          }
+        }
+        __syncthreads();
+      }
+    }
+    {
+      const int my = tid >> 3, mx = tid & 7;
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) s_M[(2 * my + r) * 33 + 4 * mx + c] = mm[r][c];
+    }
+    for (int i = wid; i < R; i += 4) {
+      const int v = __ldg(B.bnode + bo + i);
+      const int c = stage_inner(B, v, dt, s_tl + 32 * i, s_tw + 32 * i, lane);
+      if (lane == 0) {
+        s_tc[i] = c;
+        s_dcol[i] = __ldg(B.depth + v) - 1;
+        s_par[i] = i > 0 ? B.loc_of[__ldg(B.father + v)] : 0;
+      }
+    }
+    __syncthreads();
+    if (wid == 0) {
+      // nodes in depth-first order; lane a holds the entry for the node at
+      // place a.  M stays symmetric over finished pairs, so E(w, a) is one
+      // read whichever of w and a lies deeper.
+      unsigned anc = 0;
+      for (int i = 1; i < R; i++) {
+        const int par = s_par[i];
+        const unsigned ai = __shfl_sync(0xffffffffu, anc, par) | (1u << par);
+        if (lane == i) anc = ai;
+        unsigned r = s_M[i * 33 + lane];
+        const int c = s_tc[i];
+#pragma unroll 4
+        for (int x = 0; x < c; x++) {
+          const int w = s_tl[32 * i + x];
+          r = add_min((unsigned)s_tw[32 * i + x], w == lane ? 0u : s_M[w * 33 + lane], r);
+        }
+        __syncwarp();
+        if ((ai >> lane) & 1u) {
+          s_M[i * 33 + lane] = r;
+          s_M[lane * 33 + i] = r;
+        }
+        __syncwarp();
+      }
+      s_anc[lane] = anc;
+    }
+    __syncthreads();
+    for (int i = wid; i < R; i += 4) {
+      int *row = A.dis + s_rowoff[i];
+      const int own = s_dcol[i];
+      if ((s_anc[i] >> lane) & 1u) row[s_dcol[lane]] = (int)s_M[i * 33 + lane];
+      if (lane < 4) {  // 0 for the node itself, INT_MAX in the row's padding
+        const int j = own + lane;
+        if (lane == 0) row[j] = 0;
+        else if (j < ((own + 4) & ~3)) row[j] = INT_MAX;
+      }
+    }
+    __syncthreads();
+    if (A.trace_t && tid < R) {
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      A.trace_t[__ldg(B.bnode + bo + tid)] = now;
+    }
+    if (tid == 0) {
+      __threadfence();
+      st_release(A.done + b, 1);
+    }
+  }
+}
+
+// Shortcut weights of every pos entry, read from the contraction's lists:
+// entry k of v takes list index pos_src[k] of v's list, or 0 for v itself.
+// One warp per vertex.
+__global__ void gather_pos_weights_kernel(const int64_t *pos_hash, const int *pos_src, const int64_t *list_off,
+                                          const int *list_w, int *pos_w, int n) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
+       v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
+    const int64_t b = pos_hash[v], e = pos_hash[v + 1], so = list_off[v];
+    for (int64_t k = b + lane; k < e; k += 32) {
+      const int src = pos_src[k];
+      pos_w[k] = src < 0 ? 0 : list_w[so + src];
+    }
+  }
+}
+
+int grid_for(int64_t n, int nsm) { return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * 16, (n + 255) / 256)); }
+
+template <typename T>
+T read_one(const T *p) {
+  T x{};
+  GH_CUDA(cudaMemcpy(&x, p, sizeof(T), cudaMemcpyDeviceToHost));
+  return x;
+}
+
+}  // namespace
+
+// Cuts the forest into blocks and lays out their tables (weights come later,
+// with enqueue).
+void FillPlan::build_blocks() {
+  int height = 0;
+  for (const Graph *g : gs) height = std::max(height, (int)g->tree_hash.size() - 1);
+  nlev = height;
+  const int grid = grid_for(N, nsm);
+  Workspace ws;
+  int *size = ws.get<int>(N), *weight = ws.get<int>(N), *block_top = ws.get<int>(N), *top_of = ws.get<int>(N);
+  int *count = ws.get<int>(N), *blk_of_top = ws.get<int>(N);
+  int *lvl = ws.get<int>(3 * (int64_t)nlev + 1);  // block tops, width, next free per level
+  int *lvl_tops = lvl, *lvl_width = lvl + nlev + 1, *lvl_next = lvl_width + nlev;
+  unsigned long long *lvl_work = ws.get<unsigned long long>(nlev);
+  int64_t *lvl_first = ws.get<int64_t>(nlev + 1);
+  GH_CUDA(cudaMemset(count, 0, sizeof(int) * N));
+  GH_CUDA(cudaMemset(lvl, 0, sizeof(int) * (3 * (int64_t)nlev + 1)));
+  GH_CUDA(cudaMemset(lvl_work, 0, sizeof(unsigned long long) * nlev));
+  GH_CUDA(cudaMemset(block_top, 0, sizeof(int) * N));
+  small_size_kernel<<<grid, 256>>>(hld, depth, size, weight, N);
+  hang_weight_kernel<<<grid, 256>>>(father, htop, hpos, size, weight, N);
+  cut_paths_kernel<<<grid, 256>>>(father, htop, hpos, hld, size, weight, block_top, N);
+  node_block_kernel<<<grid, 256>>>(father, htop, hpos, depth, pos_hash, size, weight, block_top, top_of, count,
+                                   lvl_tops, lvl_width, lvl_work, N);
+  GH_CUDA(cudaGetLastError());
+  exclusive_scan<int>(lvl_tops, lvl_first, nlev + 1, ws, 0);
+  nblk = (int)read_one(lvl_first + nlev);
+  GH_CHECK(nblk >= 1 && nblk <= N, H2H_ERR_STATE, "fill blocks do not cover the tree");
+  blk_top = dalloc<int>(nblk, work_bytes);
+  blk_mem = dalloc<int>(nblk + 1, work_bytes);
+  blk_boff = dalloc<int64_t>(nblk + 1, work_bytes);
+  blk_moff = dalloc<int64_t>(nblk + 1, work_bytes);
+  blk_soff = dalloc<int64_t>(nblk + 1, work_bytes);
+  bnode = dalloc<int>(N, work_bytes);
+  blk_of = dalloc<int>(N, work_bytes);
+  loc_of = dalloc<unsigned char>(N, work_bytes);
+  lvl_cls = dalloc<int>(nlev, work_bytes);
+  done = dalloc<int>(2 * (int64_t)nblk, work_bytes);  // done flags, then finished tasks per block
+  unsigned long long per_node = 1ull << 18;
+  if (const char *e = std::getenv("GPUH2H_HEAVY_LEVEL_WORK")) per_node = (unsigned long long)std::max(1LL, std::atoll(e));
+  level_class_kernel<<<grid_for(nlev, nsm), 256>>>(lvl_width, lvl_work, nlev, nsm, per_node, lvl_cls);
+  order_blocks_kernel<<<grid, 256>>>(top_of, depth, lvl_first, lvl_next, blk_top, blk_of_top, N);
+  int *rows = ws.get<int>(nblk + 1), *cells = ws.get<int>(nblk + 1), *filled = ws.get<int>(nblk);
+  GH_CUDA(cudaMemset(filled, 0, sizeof(int) * nblk));
+  block_sizes_kernel<<<grid_for(nblk + 1, nsm), 256>>>(blk_top, count, pos_hash, rows, blk_mem, cells, nblk);
+  GH_CUDA(cudaGetLastError());
+  exclusive_scan<int>(rows, blk_boff, nblk + 1, ws, 0);
+  exclusive_scan<int>(blk_mem, blk_moff, nblk + 1, ws, 0);
+  exclusive_scan<int>(cells, blk_soff, nblk + 1, ws, 0);
+  GH_CHECK(read_one(blk_boff + nblk) == N, H2H_ERR_STATE, "fill blocks do not cover the tree");
+  const int64_t members = read_one(blk_moff + nblk), cell_total = read_one(blk_soff + nblk);
+  bm_p = dalloc<int>(members, work_bytes);
+  bm_row = dalloc<int64_t>(members, work_bytes);
+  direct = dalloc<unsigned>(cell_total, work_bytes);
+  closed = dalloc<unsigned>(cell_total, work_bytes);
+  scatter_nodes_kernel<<<grid, 256>>>(top_of, blk_of_top, blk_boff, filled, bnode, N);
+  block_nodes_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(blk_top, blk_boff, blk_moff, hpos, pos_hash, pos_pos,
+                                                                 pos_id, drow, bnode, blk_of, loc_of, bm_p, bm_row,
+                                                                 nblk);
+  GH_CUDA(cudaGetLastError());
+}
+
+std::vector<int> FillPlan::level_classes() const {
+  std::vector<int> cls(nlev);
+  GH_CUDA(cudaMemcpy(cls.data(), lvl_cls, sizeof(int) * nlev, cudaMemcpyDeviceToHost));
+  return cls;
+}
+
+// Tasks in block order, cut as the policy says.
+void FillPlan::build_tiles(const TilePolicy &pol) {
+  policy = pol;
+  Workspace ws;
+  int *ntask = ws.get<int>(nblk + 1), *pieces = ws.get<int>(nblk + 1);
+  int64_t *piece0 = ws.get<int64_t>(nblk + 1);
+  if (!task0) {
+    task0 = dalloc<int64_t>(nblk + 1, work_bytes);
+    tcols = dalloc<int>(nblk + 1, work_bytes);
+  }
+  block_tasks_kernel<<<grid_for(nblk + 1, nsm), 256>>>(blk_top, depth, blk_mem, blk_boff, lvl_cls, pol, ntask, pieces,
+                                                            tcols, nblk);
+  GH_CUDA(cudaGetLastError());
+  exclusive_scan<int>(ntask, task0, nblk + 1, ws, 0);
+  exclusive_scan<int>(pieces, piece0, nblk + 1, ws, 0);
+  ntasks = read_one(task0 + nblk);
+  ntiles = read_one(piece0 + nblk);
+  GH_CHECK(ntasks >= nblk && ntasks < INT32_MAX, H2H_ERR_ARG, "too many fill tasks");
+  if (ntasks > tasks_cap) {
+    cudaFree(tasks);
+    tasks = nullptr;
+    tasks_cap = 0;
+    tasks = dalloc<int>(ntasks, work_bytes);
+    tasks_cap = ntasks;
+  }
+  expand_tasks_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(task0, tasks, nblk);
+  GH_CUDA(cudaGetLastError());
+  const int smem_dyn = enable_max_dynamic_smem(block_fill_kernel);
+  smem = 2 * sizeof(int) * (size_t)std::max(max_segs, 1);
+  GH_CHECK(smem <= (size_t)smem_dyn, H2H_ERR_DEVICE, "tree too large for the fill staging");
+  int per_sm = 0;
+  GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_fill_kernel, 128, smem));
+  blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * std::max(1, per_sm), ntasks));
+}
+
+void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
+  gather_pos_weights_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256, 0, s>>>(
+      pos_hash, pos_src, lists.off, lists.w, pos_w, N);
+  GH_CUDA(cudaGetLastError());
+  GH_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * 2 * (int64_t)nblk, s));
+  GH_CUDA(cudaMemsetAsync(next, 0, sizeof(int), s));
+  GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  FillKernelArgs A{};
+  BlockArgs &B = A.B;
+  B.blk_top = blk_top;
+  B.boff = blk_boff;
+  B.moff = blk_moff;
+  B.soff = blk_soff;
+  B.bnode = bnode;
+  B.blk_of = blk_of;
+  B.loc_of = loc_of;
+  B.bm_p = bm_p;
+  B.bm_row = bm_row;
+  B.father = father;
+  B.depth = depth;
+  B.drow = drow;
+  B.pos_hash = pos_hash;
+  B.pos_pos = pos_pos;
+  B.pos_id = pos_id;
+  B.pos_w = pos_w;
+  B.direct = direct;
+  B.closed = closed;
+  B.nblk = nblk;
+  B.err = err;
+  A.dis = dis;
+  A.hld_row = hld_row;
+  A.seg_off = seg_off;
+  A.seg_top = seg_top;
+  A.seg_pos = seg_pos;
+  A.task_blk = tasks;
+  A.task0 = task0;
+  A.tcols = tcols;
+  A.ntasks = (int)ntasks;
+  A.done = done;
+  A.count = done + nblk;
+  A.next = next;
+  A.spin_limit = spin_limit_cycles();
+  A.max_segs = std::max(max_segs, 1);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  GH_CUDA(cudaStreamIsCapturing(s, &cs));
+  const bool capturing = cs != cudaStreamCaptureStatusNone;
+  if (std::getenv("GPUH2H_TRACE") && !capturing) {
+    if (!trace_t) GH_CUDA(cudaMalloc(&trace_t, sizeof(unsigned long long) * std::max(N, 1)));
+    GH_CUDA(cudaMemsetAsync(trace_t, 0, sizeof(unsigned long long) * std::max(N, 1), s));
+    A.trace_t = trace_t;
+  }
+  // inside a capture an event record becomes a graph node only when external
+  auto record = [&](cudaEvent_t e) {
+    GH_CUDA(capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s));
+  };
+  if (fill_ev) record(fill_ev[0]);
+  closure_kernel<<<dim3((nblk + kClosureWarps - 1) / kClosureWarps, 4), 32 * kClosureWarps, 0, s>>>(B);
+  GH_CUDA(cudaGetLastError());
+  block_fill_kernel<<<blocks, 128, smem, s>>>(A);
+  GH_CUDA(cudaGetLastError());
+  if (fill_ev) record(fill_ev[1]);
+}
+
+}  // namespace gh

@@ -194,19 +194,17 @@ struct ElimPlan {
   void set_weights(int gi, const int *w, cudaStream_t s);  // arc weights in the graph's file order
 };
 
-// Tile shapes of the L4 dataflow fill, keyed on the node's tree level --
+// Task shapes of the L4 fill, keyed on a block's top: its tree level --
 // class 0: fewer nodes than SMs (the chain-like top, on the critical path);
 // class 1: wider; class 2: wider and heavy (its nodes average at least 2^18
-// min-plus updates m*d) -- and on its separator size m (buckets m <= 16, <= 64,
-// <= 256, > 256).  A node whose m * d is at most small_work is one tile; a
-// larger one is cut into col_block columns x sep_chunk separator members.
+// min-plus updates m*d) -- and its separator size m (buckets m <= 16, <= 64,
+// <= 256, > 256).  A block whose m * d is at most small_work is one task; a
+// larger one is cut into tasks of col_block columns (rounded up to 64).
+// sep_chunk belongs to the text form and shapes nothing.
 struct TilePolicy {
   static constexpr int kWidth = 3, kSep = 4;
   int small_work[kWidth][kSep], col_block[kWidth][kSep], sep_chunk[kWidth][kSep];
-  TilePolicy();  // the shallow preset
-  // the default for a forest whose deepest tree has `height` levels: the
-  // shallow preset up to 2048 levels, the deep one beyond
-  static TilePolicy for_height(int height);
+  TilePolicy();
   static int sep_bucket(int m) { return m <= 16 ? 0 : m <= 64 ? 1 : m <= 256 ? 2 : 3; }
   std::string str() const;
   bool parse(const std::string &s);
@@ -214,7 +212,7 @@ struct TilePolicy {
 
 // The L4 label fill over one or more graphs as one forest (labels.cu): the
 // graphs' trees are laid side by side (graph i's vertex v is forest vertex
-// vbase[i] + v) and filled by one dataflow launch.  Each graph's DeviceIndex
+// vbase[i] + v) and filled by one launch.  Each graph's DeviceIndex
 // becomes a view into the forest arrays.
 struct FillPlan {
   std::vector<Graph *> gs;
@@ -231,11 +229,21 @@ struct FillPlan {
   int *hld = nullptr, *htop = nullptr, *hpos = nullptr, *seg_top = nullptr, *seg_pos = nullptr;
   int64_t *hld_row = nullptr;
   int64_t *seg_off = nullptr;
-  int *done = nullptr, *next = nullptr, *err = nullptr, *tiles = nullptr;
+  int *done = nullptr, *next = nullptr, *err = nullptr, *tasks = nullptr;  // tasks: task -> block
+  // the blocks (fill_blocks.cu): top, separator size, first node / member /
+  // cell of the weight tables per block; node lists and places; members'
+  // positions and row offsets; direct and closed weights; first task and
+  // columns per task
+  int nblk = 0, nlev = 0;
+  int *blk_top = nullptr, *blk_mem = nullptr, *bnode = nullptr, *blk_of = nullptr, *lvl_cls = nullptr, *bm_p = nullptr,
+      *tcols = nullptr;
+  int64_t *blk_boff = nullptr, *blk_moff = nullptr, *blk_soff = nullptr, *bm_row = nullptr, *task0 = nullptr;
+  unsigned char *loc_of = nullptr;
+  unsigned *direct = nullptr, *closed = nullptr;
   unsigned long long *trace_t = nullptr;  // publish time per node (GPUH2H_TRACE)
-  int64_t ntiles = 0, tiles_cap = 0, nchunks = 0;
-  int max_u = 1, max_c = 1, max_segs = 1, blocks = 1, threads = 128;
-  int scalar_cols = 32;  // tiles this narrow sweep one column per lane (labels.cu)
+  int64_t ntasks = 0, tasks_cap = 0;
+  int64_t ntiles = 0;  // row pieces: every node of a block once per task of the block
+  int max_segs = 1, blocks = 1;
   size_t smem = 0;
   int nsm = 0;
   int64_t work_bytes = 0;
@@ -245,10 +253,11 @@ struct FillPlan {
   void release_work();
   FillPlan(const FillPlan &) = delete;
   FillPlan &operator=(const FillPlan &) = delete;
+  void build_blocks();
   void build_tiles(const TilePolicy &pol);
   std::vector<int> level_classes() const;  // TilePolicy class per forest level
   // Gathers the shortcut weights of the pos entries from the lists, resets
-  // rows and flags and runs the fill on s.
+  // the flags, closes the blocks' weights and runs the fill on s.
   void enqueue(cudaStream_t s, cudaEvent_t *fill_ev = nullptr);
   void check_error();            // synchronises; throws if a dependency wait ran out
   void trace_report();           // GPUH2H_TRACE: the last fill's time per level class
@@ -278,7 +287,7 @@ inline void build_tree_and_rmq(Graph &g) {
 void allocate_labels_and_bfs(Graph &g);                // tree.cpp
 void fill_labels_gpu(Graph &g);                        // labels.cu
 // The level-synchronous fill (L3 labels, or L4 with GPUH2H_LEVEL_FILL set)
-// runs from host position lists; the L4 dataflow fill builds them on the GPU.
+// runs from host position lists; the L4 block fill builds them on the GPU.
 inline bool uses_level_fill(const Graph &g) {
   return g.label_mode == H2H_LABEL_L3 || std::getenv("GPUH2H_LEVEL_FILL") != nullptr;
 }

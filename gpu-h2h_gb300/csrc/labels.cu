@@ -9,9 +9,8 @@
 //   dis[v][j] = min(dis[v][j], t + dis[u][j])            j < p   (ancestors above u)
 //   dis[v][j] = min(dis[v][j], t + dis[anc_j(v)][p])     p < j < d-1 (L4: below u)
 //
-// Three fills live here:
-//   * fill_flow_kernel, the L4 fill: a dataflow over tiles of the forest of
-//     one or more graphs, one warp per tile (FillPlan, further down);
+// The L4 fill is in fill_blocks.cu; here are its plan's forest arrays and
+// position lists, the exports, and two more fills:
 //   * fill_level_kernel, level-synchronous, one warp per node in the
 //     reference's update order: L3 rows (order-dependent) and L4 on request;
 //     the node's row stays in shared memory, and its ancestors' row offsets
@@ -174,295 +173,6 @@ __global__ void fill_level_kernel(FillArgs A) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// L4 fill as a dataflow over the tree (the fast path for label_mode L4).
-//
-// L4 rows are exact: dis[v][j] = D(v, a_j) for the ancestor a_j at depth
-// j+1, and D(v, a) = min over u in X(v)\{v} of sc(v,u) + D(u, a), where
-// D(u, a) is dis[u][j] when u is below a (p_u > j), 0 when u = a, and
-// dis[a][p_u] when u is above a.  The reference reaches the same values with
-// its in-place descending-position updates, so every column can be computed
-// independently from shortcut weights and finished ancestor rows.
-//
-// A node needs only its ancestors' rows, and its father finishes after all
-// of them, so CTAs take nodes in BFS order from a device counter and wait
-// for the father's flag alone: no level barriers, so the thin top of the
-// tree pipelines with the wide middle.  A CTA spins on the flag with an
-// acquire load, a nanosleep back-off and a clock limit (on expiry it records
-// an error and stops); rows produced in this launch are read through L2
-// (ld.global.cg) so no stale L1 line is used.
-//
-// The ancestor a_j of a column comes from the tree's heavy-path layout: the
-// node's root path is a handful of heavy-path segments (at most one more
-// than the light edges above it, so O(log n)), staged in shared memory; a
-// short search finds the segment holding depth j+1 and the path array gives
-// the node.  No per-node ancestor list is stored.
-
-struct FlowArgs {
-  // tiles in forest BFS order: ticket t belongs to node tile_node[t]; the
-  // node's tiles are tickets node_first .. + node_ntiles, its column blocks
-  // (node_cb columns) outer and separator chunks (node_sc members) inner
-  const int *tile_node;
-  int ntiles;
-  const int *node_first, *node_ntiles, *node_cb, *node_sc;
-  // the counter hands out chunks of consecutive tickets: one tile on the
-  // narrow levels, several on the wide ones (fewer atomics)
-  const int *chunk_start;  // [nchunks + 1]; nullptr: chunk k is tile k
-  int nchunks;
-  int *node_cnt;           // finished tiles per node
-  const int *father;
-  const int *depth;
-  const int64_t *drow;
-  int *dis;
-  const int64_t *pos_hash;
-  const int *pos_id;
-  const int *pos_pos;
-  const int *pos_w;
-  const int64_t *hld_row;  // heavy paths, top to bottom: the row offset of the node at each position
-  const int64_t *seg_off;  // root-path segments per node
-  const int *seg_top, *seg_pos;
-  int *done;          // per vertex: 1 once its row is visible
-  int *next;          // work counter
-  int *err;           // 0 = ok, 4 = a wait ran out
-  long long spin_limit;
-  int max_u;          // max separator members in one tile (staging size)
-  int max_segs;       // max root-path segments of a node (staging size)
-  int scalar_cols;    // tiles of at most this many columns sweep one column per lane
-  unsigned long long *trace_t;  // non-null (GPUH2H_TRACE): each node's publish time, ns
-};
-
-__device__ __forceinline__ int ld_acquire(const int *p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(int *p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ int ld_relaxed(const int *p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Every warp is an independent worker: it takes a ticket, stages the tile's
-// separator entries and the node's root-path segments in its own slice of
-// shared memory while lane 0 waits for the father, sweeps the columns (lane
-// per column) and publishes; only warp-level barriers, so a thin tile or a
-// dependency wait stalls one warp, not a CTA.
-// Ten 4-warp blocks per SM (48 registers, 8 bytes of spill) instead of eight
-// at 64 registers: the 6.26M-vertex fill 1,003 -> 928 ms, the 264k-vertex
-// fill 28.9 -> 28.2 ms.
-__global__ void __launch_bounds__(128, 10) fill_flow_kernel(FlowArgs A) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int ual = (A.max_u + 1) & ~1, sal = (A.max_segs + 1) & ~1;
-  unsigned char *mine = smem + (size_t)wid * ((size_t)ual * 16 + (size_t)sal * 8);
-  int64_t *xs_row = (int64_t *)mine;                 // [max_u]
-  int *xs_p = (int *)(xs_row + ual);                 // [max_u]
-  int *xs_w = xs_p + ual;                            // [max_u]
-  int *s_top = xs_w + ual;                           // [max_segs]
-  int *s_pos = s_top + sal;                          // [max_segs]
-  for (;;) {
-    int k = 0;
-    if (lane == 0) k = atomicAdd(A.next, 1);
-    k = __shfl_sync(0xffffffffu, k, 0);
-    if (k >= A.nchunks) return;
-    const int t_beg = A.chunk_start ? max(__ldg(A.chunk_start + k), 0) : k;
-    const int t_end = A.chunk_start ? min(__ldg(A.chunk_start + k + 1), A.ntiles) : k + 1;
-    for (int t = t_beg; t < t_end; t++) {
-    const int v = __ldg(A.tile_node + t);
-    const int d = __ldg(A.depth + v);
-    const int f = __ldg(A.father + v);
-    const int64_t base = __ldg(A.drow + v);
-    const int64_t pb = __ldg(A.pos_hash + v);
-    const int m = (int)(__ldg(A.pos_hash + v + 1) - pb) - 1;   // X(v)\{v}
-    const int sub = t - __ldg(A.node_first + v);
-    const int cb = __ldg(A.node_cb + v), sc = __ldg(A.node_sc + v);
-    const int nuc = (max(m, 1) + sc - 1) / sc;
-    const int ci = sub / nuc, ui = sub - ci * nuc;
-    const int c0 = ci * cb, c1 = min(d, c0 + cb);
-    const int u0 = ui * sc, u1 = min(m, u0 + sc);
-    const bool whole_sep = u0 == 0 && u1 == m;                  // this tile sees every member
-    const int nu = u1 - u0;
-    // separator entries and root-path segments need no finished row
-#pragma unroll 4
-    for (int i = lane; i < nu; i += 32) {
-      xs_p[i] = __ldg(A.pos_pos + pb + u0 + i);
-      xs_w[i] = __ldg(A.pos_w + pb + u0 + i);
-      xs_row[i] = __ldg(A.drow + __ldg(A.pos_id + pb + u0 + i));
-    }
-    const int64_t sb = __ldg(A.seg_off + v);
-    const int ns = (int)(__ldg(A.seg_off + v + 1) - sb);
-    for (int i = lane; i < ns; i += 32) {
-      s_top[i] = __ldg(A.seg_top + sb + i);
-      s_pos[i] = __ldg(A.seg_pos + sb + i);
-    }
-    int stop = 0;
-    if (lane == 0) {
-      if (f >= 0) {
-        long long t0 = clock64();
-        while (ld_acquire(A.done + f) == 0) {
-          if (ld_relaxed(A.err) != 0 || clock64() - t0 > A.spin_limit) {
-            atomicCAS(A.err, 0, 4);
-            stop = 1;
-            break;
-          }
-          __nanosleep(64);
-        }
-      }
-      if (c1 == d && u0 == 0) A.dis[base + d - 1] = 0;
-    }
-    stop = __shfl_sync(0xffffffffu, stop, 0);
-    __syncwarp();
-    if (stop) return;
-    // Column sweep, four consecutive columns [J, J + 4) per lane (rows start
-    // on 16-byte boundaries and column blocks are multiples of four, so J is
-    // a multiple of four inside every row).  The tile's members are sorted by
-    // position, so for a lane's columns they fall into three runs:
-    //   i >= hi  (p >= J + 4): every column lies above u_i -- one 128-bit
-    //            load of u_i's row gives all four candidates;
-    //   i <  lo  (p <  J):     every column lies below u_i -- the candidate
-    //            of column j is the ancestor a_j's entry at p (L4);
-    //   lo <= i < hi:          at most four members with p inside the quad,
-    //            resolved column by column.
-    // No per-member branch, and a quarter of the iterations of a
-    // column-per-lane sweep.  A tile of 33 to 127 columns spreads its
-    // members over 2 or 4 lane groups (every group takes every G-th member)
-    // and combines the groups' minima with shuffles, so all 32 lanes work.
-    const int cend = min(c1, d - 1);
-    if (cend - c0 <= A.scalar_cols) {
-      // a tile of at most scalar_cols columns (32 on trees of up to 2,048
-      // levels, whose narrow levels are a latency chain): one column per
-      // lane, one ancestor lookup each -- the shortest chain of dependent
-      // loads per tile
-      const int j = c0 + lane;
-      if (j < cend) {
-        int lo = 0, hi = ns - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (s_top[mid] <= j + 1) lo = mid; else hi = mid - 1;
-        }
-        const int64_t arow = __ldg(A.hld_row + s_pos[lo] + (j + 1 - s_top[lo]));
-        int r = INT_MAX;
-#pragma unroll 8
-        for (int i = 0; i < nu; i++) {
-          const int p = xs_p[i];
-          const int val = p > j ? __ldcg(A.dis + xs_row[i] + j) : p == j ? 0 : __ldcg(A.dis + arow + p);
-          r = min(r, xs_w[i] + val);
-        }
-        if (whole_sep) A.dis[base + j] = r;
-        else atomicMin(A.dis + base + j, r);
-      }
-    }
-    const int nquad = cend - c0 <= A.scalar_cols ? 0 : (cend - c0 + 3) >> 2;
-    const int QW = nquad > 16 ? 32 : nquad > 8 ? 16 : 8;  // lanes along the columns
-    const int G = 32 / QW;                                 // member groups
-    const int qi = lane & (QW - 1), grp = lane / QW;
-    for (int Jb = c0; nquad > 0 && Jb < cend; Jb += 4 * QW) {  // the same trip count in every lane
-      const int J = Jb + 4 * qi;
-      const bool active = J < cend;
-      const int nvalid = active ? min(4, cend - J) : 0;
-      int r0 = INT_MAX, r1 = INT_MAX, r2 = INT_MAX, r3 = INT_MAX;
-      if (active) {
-        int64_t arow[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          // ancestor at depth j + 1 (a column past cend reuses column J's
-          // ancestor: its reads stay inside that row or its padding and its
-          // result is discarded)
-          const int j = J + (k < nvalid ? k : 0);
-          int lo = 0, hi = ns - 1;
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_top[mid] <= j + 1) lo = mid; else hi = mid - 1;
-          }
-          arow[k] = __ldg(A.hld_row + s_pos[lo] + (j + 1 - s_top[lo]));
-        }
-        int ilo = 0, ihi = nu;  // first member with p >= J
-        while (ilo < ihi) {
-          const int mid = (ilo + ihi) >> 1;
-          if (xs_p[mid] < J) ilo = mid + 1; else ihi = mid;
-        }
-        const int mlo = ilo;
-        ihi = nu;               // first member with p >= J + 4
-        while (ilo < ihi) {
-          const int mid = (ilo + ihi) >> 1;
-          if (xs_p[mid] < J + 4) ilo = mid + 1; else ihi = mid;
-        }
-        const int mhi = ilo;
-#pragma unroll 4
-        for (int i = mhi + grp; i < nu; i += G) {
-          const int4 x = __ldcg(reinterpret_cast<const int4 *>(A.dis + xs_row[i] + J));
-          const int w = xs_w[i];
-          r0 = min(r0, w + x.x);
-          r1 = min(r1, w + x.y);
-          r2 = min(r2, w + x.z);
-          r3 = min(r3, w + x.w);
-        }
-#pragma unroll 4
-        for (int i = grp; i < mlo; i += G) {
-          const int p = xs_p[i], w = xs_w[i];
-          r0 = min(r0, w + __ldcg(A.dis + arow[0] + p));
-          r1 = min(r1, w + __ldcg(A.dis + arow[1] + p));
-          r2 = min(r2, w + __ldcg(A.dis + arow[2] + p));
-          r3 = min(r3, w + __ldcg(A.dis + arow[3] + p));
-        }
-        for (int i = mlo + grp; i < mhi; i += G) {
-          const int p = xs_p[i], w = xs_w[i];
-          const int64_t ur = xs_row[i];
-          int c[4];
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const int j = J + k;
-            c[k] = p > j ? __ldcg(A.dis + ur + j) : p == j ? 0 : __ldcg(A.dis + arow[k] + p);
-          }
-          r0 = min(r0, w + c[0]);
-          r1 = min(r1, w + c[1]);
-          r2 = min(r2, w + c[2]);
-          r3 = min(r3, w + c[3]);
-        }
-      }
-      for (int o = QW; o < 32; o <<= 1) {  // combine the member groups (lanes qi, qi + QW, ...)
-        r0 = min(r0, __shfl_xor_sync(0xffffffffu, r0, o));
-        r1 = min(r1, __shfl_xor_sync(0xffffffffu, r1, o));
-        r2 = min(r2, __shfl_xor_sync(0xffffffffu, r2, o));
-        r3 = min(r3, __shfl_xor_sync(0xffffffffu, r3, o));
-      }
-      if (active && grp == 0) {
-        int *out = A.dis + base + J;
-        if (whole_sep && nvalid == 4) {
-          *reinterpret_cast<int4 *>(out) = make_int4(r0, r1, r2, r3);
-        } else {
-          const int r[4] = {r0, r1, r2, r3};
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            if (k < nvalid) {
-              if (whole_sep) out[k] = r[k];
-              else atomicMin(out + k, r[k]);
-            }
-        }
-      }
-    }
-    __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      const int nt = __ldg(A.node_ntiles + v);
-      if (nt == 1 || atomicAdd(A.node_cnt + v, 1) == nt - 1) {
-        __threadfence();
-        st_release(A.done + v, 1);
-        if (A.trace_t) {
-          unsigned long long now;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-          A.trace_t[v] = now;
-        }
-      }
-    }
-    __syncwarp();  // the slice is restaged only after every lane left the sweep
-    }
-  }
-}
-
 // The reference's GPU label fill mapping, kept as a measurement baseline
 // (makeH2HLabel_noCommunication_D_noHub_3, kernel_functions.cu:717-744, with
 // the L4 block :738-743 enabled): one thread per (v, u) pair of one tree
@@ -525,35 +235,6 @@ __global__ void count_mismatch_kernel(const int *a, const int *b, int64_t n, uns
   if (c) atomicAdd(bad, c);
 }
 
-// Chunk k's first ticket, from per-level rows (first chunk, first ticket,
-// step): the level holding k by binary search, then an arithmetic step;
-// entry nchunks closes the table.
-__global__ void chunk_table_kernel(const int64_t *ltab, int nlev, int64_t nchunks, int64_t ntiles, int *chunks) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= nchunks;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    if (k == nchunks) {
-      chunks[k] = (int)ntiles;
-      continue;
-    }
-    int lo = 0, hi = nlev - 1;  // last level whose first chunk is <= k
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (ltab[3 * mid] <= k) lo = mid; else hi = mid - 1;
-    }
-    chunks[k] = (int)(ltab[3 * lo + 1] + (k - ltab[3 * lo]) * ltab[3 * lo + 2]);
-  }
-}
-
-// tile_node[t] = v for the tickets of every node v.  One warp per node.
-__global__ void expand_tiles_kernel(const int *node_first, const int *node_ntiles, int *tile_node, int n) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
-       v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
-    const int f = node_first[v], c = node_ntiles[v];
-    for (int k = lane; k < c; k += 32) tile_node[f + k] = (int)v;
-  }
-}
-
 // Row offset of the node at every heavy-path position (the fill reads an
 // ancestor's row offset with one load instead of two dependent ones).
 __global__ void hld_row_kernel(const int *hld, const int64_t *drow, int64_t *hld_row, int n) {
@@ -578,11 +259,6 @@ __global__ void root_path_segments_kernel(const int *father, const int *depth, c
   }
 }
 
-__global__ void fill_int_kernel(int *p, int64_t n, int value) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = value;
-}
-
 __global__ void max_label_kernel(const int *dis, int64_t n, int *out) {
   int m = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -591,22 +267,6 @@ __global__ void max_label_kernel(const int *dis, int64_t n, int *out) {
   }
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
-// Shortcut weights of every pos entry, read from the contraction's lists:
-// entry k of v takes list index pos_src[k] of v's list, or 0 for v itself.
-// One warp per vertex.
-__global__ void gather_pos_weights_kernel(const int64_t *pos_hash, const int *pos_src, const int64_t *list_off,
-                                          const int *list_w, int *pos_w, int n) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
-       v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
-    const int64_t b = pos_hash[v], e = pos_hash[v + 1], so = list_off[v];
-    for (int64_t k = b + lane; k < e; k += 32) {
-      const int src = pos_src[k];
-      pos_w[k] = src < 0 ? 0 : list_w[so + src];
-    }
-  }
 }
 
 // Position lists (mallocH2HLabel_noHub, H2HConsturction.cu:656-700): X(v)
@@ -649,43 +309,17 @@ __global__ void build_positions_kernel(const int64_t *list_off, const int *list_
 
 }  // namespace
 
-// Defaults measured on road graphs (one warp per tile): narrow levels cut a
-// node into 32-column x 4-member tiles once m*d exceeds 1,024 (the 264k-
-// vertex graph's fill is a latency chain through 1,343 such levels); wider
-// levels 32 x 16 above 4,096; heavy levels (the 6.26M-vertex graph's middle)
-// 128 x 256 above 16,384 -- whole separators, so no atomicMin combining.
-// Separators above 256 members always split.
-// Two measured presets.  Shallow trees (the 264k-vertex graph, tree height
-// 1,343; batches of road graphs) fill as a latency chain through the narrow
-// levels and want small tiles.  Deep trees have rows several thousand
-// columns long, so the same tiles are too many: the autotuner on the
-// 3.6M-vertex graph (height 4,180) moved the wide levels to 64-column x
-// 32-member tiles and the narrow levels' widest separators to 16-member
-// chunks, fill 1,080 -> 788 ms; on the 264k-vertex graph those shapes cost
-// 29 -> 40 ms.
+// A narrow level's blocks are cut as finely as the kernel's step (64 columns):
+// they are the chain the fill waits for.  Elsewhere a task is about 16k
+// (member, column) pairs, so a block of the bottom (m <= 16) is one task.
 TilePolicy::TilePolicy() {
-  static const int sw[kWidth] = {1024, 4096, 16384}, cb[kWidth] = {32, 32, 128}, sc[kWidth] = {4, 16, 256};
+  static const int cb[kWidth][kSep] = {{64, 64, 64, 64}, {1024, 256, 64, 64}, {1024, 256, 64, 64}};
   for (int w = 0; w < kWidth; w++)
     for (int b = 0; b < kSep; b++) {
-      small_work[w][b] = b == kSep - 1 ? 0 : sw[w];
-      col_block[w][b] = cb[w];
-      sep_chunk[w][b] = sc[w];
+      small_work[w][b] = 1024;
+      col_block[w][b] = cb[w][b];
+      sep_chunk[w][b] = 32;
     }
-}
-
-TilePolicy TilePolicy::for_height(int height) {
-  TilePolicy t;
-  if (height <= 2048) return t;
-  static const int sw[kWidth][kSep] = {{1024, 1024, 1024, 0}, {16384, 4096, 4096, 0}, {16384, 16384, 16384, 0}};
-  static const int cb[kWidth][kSep] = {{32, 32, 32, 32}, {32, 64, 64, 64}, {128, 128, 128, 128}};
-  static const int sc[kWidth][kSep] = {{4, 4, 4, 16}, {16, 32, 32, 32}, {256, 256, 256, 256}};
-  for (int w = 0; w < kWidth; w++)
-    for (int b = 0; b < kSep; b++) {
-      t.small_work[w][b] = sw[w][b];
-      t.col_block[w][b] = cb[w][b];
-      t.sep_chunk[w][b] = sc[w][b];
-    }
-  return t;
 }
 
 std::string TilePolicy::str() const {
@@ -809,20 +443,8 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
   });
   f_drow[N] = dis_total;
   f_pos_hash[N] = pos_total;
-  // Narrow tiles sweep one column per lane on trees of up to 2,048 levels,
-  // whose narrow levels fill as a latency chain (264k-vertex graph: 29 ms
-  // against 34 ms with four columns per lane); deeper trees cut their long
-  // rows into many more tiles per level and take four columns per lane
-  // throughout (6.26M-vertex graph: narrow levels 500 -> 300 ms).
-  {
-    int height = 0;
-    for (const Graph *g : gs) height = std::max(height, g->tree_height);
-    scalar_cols = height <= 2048 ? 32 : 0;
-    if (const char *e = std::getenv("GPUH2H_FILL_SCALAR_COLS")) scalar_cols = std::max(0, std::atoi(e));
-  }
   f_seg_off[N] = seg_total;
   mark("host assembly");
-  threads = 128;
   int dev = 0;
   GH_CUDA(cudaGetDevice(&dev));
   GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -844,7 +466,6 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
     seg_off = dalloc<int64_t>(N + 1, work_bytes);
     seg_top = dalloc<int>(std::max<int64_t>(seg_total, 1), work_bytes);
     seg_pos = dalloc<int>(std::max<int64_t>(seg_total, 1), work_bytes);
-    done = dalloc<int>(2 * (int64_t)N, work_bytes);  // done flags, then per-node tile counters
     next = dalloc<int>(1, work_bytes);
     err = dalloc<int>(1, work_bytes);
     GH_CUDA(cudaMemcpy(drow, f_drow.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
@@ -876,8 +497,10 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
                                                                                      seg_off, seg_top, seg_pos, N);
     GH_CUDA(cudaGetLastError());
     mark("root-path segments");
+    build_blocks();
+    mark("blocks");
     build_tiles(pol);
-    mark("tiles");
+    mark("tasks");
   } catch (...) {
     release_work();
     throw;
@@ -887,315 +510,21 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
 FillPlan::~FillPlan() { release_work(); }
 
 void FillPlan::release_work() {
-  void *ps[] = {pos_w, pos_src, hld, htop, hpos, seg_off, seg_top, seg_pos, done, next, err, tiles, trace_t, hld_row};
+  void *ps[] = {pos_w,    pos_src,  hld,      htop,  hpos,   seg_off, seg_top, seg_pos, done,   next,   err,    tasks,   trace_t,
+                hld_row,  blk_top,  blk_mem,  blk_boff, blk_moff, blk_soff, bnode, blk_of, loc_of, lvl_cls, bm_p, bm_row,
+                direct,   closed,   task0,    tcols};
   for (void *p : ps) cudaFree(p);
   trace_t = nullptr;
-  pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = tiles = nullptr;
-  hld_row = nullptr;
-  seg_off = nullptr;
-}
-
-// Work items of the host passes over the forest: (graph, level, BFS range
-// of at most kItemNodes nodes), graph by graph, levels in order.
-namespace {
-constexpr int kItemNodes = 32768;
-struct LevelItem {
-  int g, l, q0, q1;
-};
-std::vector<LevelItem> level_items(const std::vector<Graph *> &gs) {
-  std::vector<LevelItem> items;
-  for (int i = 0; i < (int)gs.size(); i++) {
-    const Graph &g = *gs[i];
-    for (int l = 0; l + 1 < (int)g.tree_hash.size(); l++)
-      for (int q = g.tree_hash[l]; q < g.tree_hash[l + 1]; q += kItemNodes)
-        items.push_back({i, l, q, std::min(q + kItemNodes, g.tree_hash[l + 1])});
-  }
-  return items;
-}
-int host_threads_of(const std::vector<Graph *> &gs) {
-  int t = 1;
-  for (const Graph *g : gs) t = std::max(t, g->threads);
-  return t;
-}
-}  // namespace
-
-std::vector<int> FillPlan::level_classes() const {
-  int nlev = 0;
-  for (const Graph *g : gs) nlev = std::max(nlev, (int)g->tree_hash.size() - 1);
-  // nodes and min-plus updates per forest level, summed over items computed in parallel
-  const std::vector<LevelItem> items = level_items(gs);
-  std::vector<int64_t> iwork(items.size(), 0);
-  {
-    Pool pool(host_threads_of(gs));
-    pool.parallel_for((int64_t)items.size(), 1, [&](int64_t lo, int64_t hi, int) {
-      for (int64_t t = lo; t < hi; t++) {
-        const LevelItem &it = items[t];
-        const Graph &g = *gs[it.g];
-        int64_t w = 0;
-        for (int q = it.q0; q < it.q1; q++) {
-          const int v = g.tree_bfs[q];
-          w += (g.pos_hash[v + 1] - g.pos_hash[v] - 1) * (int64_t)g.depth[v];
-        }
-        iwork[t] = w;
-      }
-    });
-  }
-  std::vector<int64_t> width(nlev, 0), work(nlev, 0);
-  for (size_t t = 0; t < items.size(); t++) {
-    width[items[t].l] += items[t].q1 - items[t].q0;
-    work[items[t].l] += iwork[t];
-  }
-  // narrow: fewer nodes than SMs, whatever their work (the critical path);
-  // heavy: a wider level whose nodes average at least 2^18 min-plus updates
-  // (GPUH2H_HEAVY_LEVEL_WORK overrides the figure)
-  int64_t per_node = int64_t(1) << 18;
-  if (const char *e = std::getenv("GPUH2H_HEAVY_LEVEL_WORK")) per_node = std::max(1LL, std::atoll(e));
-  std::vector<int> cls(nlev, 0);
-  for (int l = 0; l < nlev; l++)
-    cls[l] = width[l] < nsm ? 0 : work[l] >= per_node * width[l] ? 2 : 1;
-  return cls;
-}
-
-// Tiles in forest BFS order (level l of every graph, then level l + 1): a
-// node's father always holds an earlier ticket, so the dataflow cannot wait
-// on work no CTA has taken.  Two passes over the graphs in parallel: tile
-// counts per (level, graph), then each graph writes its tiles at the
-// offsets the counts give.
-void FillPlan::build_tiles(const TilePolicy &pol) {
-  const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
-  Clock tclk;
-  auto mark = [&](const char *what) {
-    if (!trace) return;
-    cudaDeviceSynchronize();
-    std::fprintf(stderr, "[gpuh2h] tiles: %s %.3f ms\n", what, tclk.us() / 1e3);
-    tclk.reset();
-  };
-  policy = pol;
-  const int K = (int)gs.size();
-  int nlev = 0;
-  for (const Graph *g : gs) nlev = std::max(nlev, (int)g->tree_hash.size() - 1);
-  const std::vector<int> lcls = level_classes();
-  mark("level classes");
-  auto tiles_of = [&](int wb, int m, int d, int &nt_node, int &cb, int &sc) {
-    const int sb = TilePolicy::sep_bucket(m);
-    if ((int64_t)m * d <= pol.small_work[wb][sb]) {
-      nt_node = 1;
-      cb = d;
-      sc = std::max(m, 1);
-      return true;  // one tile
-    }
-    cb = (pol.col_block[wb][sb] + 3) & ~3;  // the sweep takes columns four at a time
-    sc = pol.sep_chunk[wb][sb];
-    nt_node = ((d + cb - 1) / cb) * ((std::max(m, 1) + sc - 1) / sc);
-    return false;
-  };
-  Pool pool(host_threads_of(gs));
-  // pass 1 (items in parallel): every node's tile count and shape, tiles
-  // per item, staging bounds
-  const std::vector<LevelItem> items = level_items(gs);
-  const int64_t nitems = (int64_t)items.size();
-  std::vector<int, NoInit<int>> host((size_t)4 * N);  // every node's four entries are written below
-  int *nfirst = host.data(), *nt = nfirst + N, *ncb = nfirst + 2 * N, *nsc = nfirst + 3 * N;
-  std::vector<int64_t> icnt(nitems, 0);
-  std::vector<int> imu(nitems, 1), imc(nitems, 1);
-  pool.parallel_for(nitems, 1, [&](int64_t lo, int64_t hi, int) {
-    for (int64_t t = lo; t < hi; t++) {
-      const LevelItem &it = items[t];
-      const Graph &g = *gs[it.g];
-      const int vb = vbase[it.g], wb = lcls[it.l];
-      int64_t c = 0;
-      int mu = 1, mc = 1;
-      for (int q = it.q0; q < it.q1; q++) {
-        const int v = g.tree_bfs[q], V = vb + v, d = g.depth[v];
-        const int m = (int)(g.pos_hash[v + 1] - g.pos_hash[v]) - 1;
-        int nt_node, cb, sc;
-        const bool one = tiles_of(wb, m, d, nt_node, cb, sc);
-        nt[V] = nt_node;
-        ncb[V] = cb;
-        nsc[V] = sc;
-        c += nt_node;
-        mu = std::max(mu, one ? m : std::min(m, sc));
-        mc = std::max(mc, one ? d : std::min(d, cb));
-      }
-      icnt[t] = c;
-      imu[t] = mu;
-      imc[t] = mc;
-    }
-  });
-  // tickets: forest level by forest level, graphs in order inside a level,
-  // BFS order inside a graph's level; the items of a (graph, level) are
-  // consecutive in BFS order
-  std::vector<std::vector<int64_t>> cnt(K);
-  for (int i = 0; i < K; i++) cnt[i].assign(std::max(0, (int)gs[i]->tree_hash.size() - 1), 0);
-  for (int64_t t = 0; t < nitems; t++) cnt[items[t].g][items[t].l] += icnt[t];
-  std::vector<std::vector<int64_t>> off(K);
-  int64_t total = 0;
-  for (int i = 0; i < K; i++) off[i].assign(cnt[i].size(), 0);
-  for (int l = 0; l < nlev; l++)
-    for (int i = 0; i < K; i++)
-      if (l < (int)cnt[i].size()) {
-        off[i][l] = total;
-        total += cnt[i][l];
-      }
-  ntiles = total;
-  GH_CHECK(ntiles < INT32_MAX, H2H_ERR_ARG, "too many fill tiles");
-  max_u = *std::max_element(imu.begin(), imu.end());
-  max_c = *std::max_element(imc.begin(), imc.end());
-  std::vector<int64_t> ibase(nitems, 0);
-  for (int64_t t = 0; t < nitems; t++) {
-    const bool first = t == 0 || items[t - 1].g != items[t].g || items[t - 1].l != items[t].l;
-    ibase[t] = first ? off[items[t].g][items[t].l] : ibase[t - 1] + icnt[t - 1];
-  }
-  mark("pass 1");
-  // pass 2 (items in parallel): every node's first ticket; the ticket ->
-  // node array is expanded on the device
-  pool.parallel_for(nitems, 1, [&](int64_t lo, int64_t hi, int) {
-    for (int64_t t = lo; t < hi; t++) {
-      const LevelItem &it = items[t];
-      const Graph &g = *gs[it.g];
-      const int vb = vbase[it.g];
-      int64_t tk = ibase[t];
-      for (int q = it.q0; q < it.q1; q++) {
-        const int V = vb + g.tree_bfs[q];
-        nfirst[V] = (int)tk;
-        tk += nt[V];
-      }
-    }
-  });
-  const int64_t need = ntiles + 4 * (int64_t)N + (int64_t)(ntiles + nlev + 1);  // + chunk table bound
-  if (need > tiles_cap) {
-    cudaFree(tiles);
-    tiles = nullptr;
-    tiles_cap = 0;
-    tiles = dalloc<int>(need, work_bytes);
-    tiles_cap = need;
-  }
-  mark("pass 2 and allocation");
-  // chunks: forest levels in ticket order.  A level with many times more
-  // tiles than resident warps hands them out in groups (fewer atomics on the
-  // counter); any other level one by one, so its tiles spread over warps.
-  // When every level goes one by one there is no table (chunk k = tile k).
-  // the table is built on the device from one (first chunk, first ticket,
-  // step) row per level
-  std::vector<int64_t> ltab;  // per level: first chunk, first ticket, step
-  {
-    const int64_t warps = (int64_t)nsm * 64;
-    std::vector<int64_t> lt(nlev, 0);
-    std::vector<int> step(nlev, 1);
-    int64_t nc = 0;
-    bool grouped = false;
-    for (int l = 0; l < nlev; l++) {
-      for (int i = 0; i < K; i++)
-        if (l < (int)cnt[i].size()) lt[l] += cnt[i][l];
-      step[l] = (int)std::max<int64_t>(1, std::min<int64_t>(8, lt[l] / (8 * warps)));
-      grouped |= step[l] > 1;
-      nc += (lt[l] + step[l] - 1) / step[l];
-    }
-    nchunks = grouped ? nc : ntiles;
-    if (grouped) {
-      ltab.resize(3 * (size_t)nlev);
-      int64_t t = 0, k = 0;
-      for (int l = 0; l < nlev; l++) {
-        ltab[3 * l] = k;
-        ltab[3 * l + 1] = t;
-        ltab[3 * l + 2] = step[l];
-        k += (lt[l] + step[l] - 1) / step[l];
-        t += lt[l];
-      }
-      GH_CHECK(t == ntiles && k == nc, H2H_ERR_STATE, "fill chunks do not cover the tiles");
-    }
-  }
-  mark("chunks");
-  GH_CUDA(cudaMemcpy(tiles + ntiles, host.data(), sizeof(int) * 4 * (int64_t)N, cudaMemcpyHostToDevice));
-  if (!ltab.empty()) {
-    int64_t *d_ltab = nullptr;
-    GH_CUDA(cudaMalloc(&d_ltab, sizeof(int64_t) * ltab.size()));
-    cudaError_t e = cudaMemcpy(d_ltab, ltab.data(), sizeof(int64_t) * ltab.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) {
-      chunk_table_kernel<<<std::max(1, std::min<int>(nsm * 8, (int)((nchunks + 255) / 256))), 256>>>(
-          d_ltab, nlev, nchunks, ntiles, tiles + ntiles + 4 * (int64_t)N);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    cudaFree(d_ltab);
-    GH_CUDA(e);
-  }
-  expand_tiles_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256>>>(tiles + ntiles, tiles + ntiles + N,
-                                                                                  tiles, N);
-  GH_CUDA(cudaGetLastError());
-  mark("uploads and expansion");
-  const int smem_dyn = enable_max_dynamic_smem(fill_flow_kernel);
-  // one staging slice per warp (4 warps per 128-thread block)
-  smem = 4 * ((size_t)((max_u + 1) & ~1) * 16 + (size_t)((std::max(max_segs, 1) + 1) & ~1) * 8);
-  GH_CHECK(smem <= (size_t)smem_dyn, H2H_ERR_DEVICE, "separator or tree too large for the fill staging");
-  int per_sm = 0;
-  GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fill_flow_kernel, threads, smem));
-  per_sm = std::max(1, per_sm);
-  blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * per_sm, ntiles));
-}
-
-void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
-  gather_pos_weights_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256, 0, s>>>(
-      pos_hash, pos_src, lists.off, lists.w, pos_w, N);
-  GH_CUDA(cudaGetLastError());
-  // rows start at INT_MAX: split tiles combine with atomicMin; padding stays defined
-  fill_int_kernel<<<1024, 256, 0, s>>>(dis, dis_total, INT_MAX);
-  GH_CUDA(cudaGetLastError());
-  GH_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * 2 * (int64_t)N, s));
-  GH_CUDA(cudaMemsetAsync(next, 0, sizeof(int), s));
-  GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-  FlowArgs A;
-  A.tile_node = tiles;
-  A.ntiles = (int)ntiles;
-  A.node_first = tiles + ntiles;
-  A.node_ntiles = tiles + ntiles + N;
-  A.node_cb = tiles + ntiles + 2 * (int64_t)N;
-  A.node_sc = tiles + ntiles + 3 * (int64_t)N;
-  A.chunk_start = nchunks == ntiles ? nullptr : tiles + ntiles + 4 * (int64_t)N;
-  A.nchunks = (int)nchunks;
-  A.node_cnt = done + N;
-  A.father = father;
-  A.depth = depth;
-  A.drow = drow;
-  A.dis = dis;
-  A.pos_hash = pos_hash;
-  A.pos_id = pos_id;
-  A.pos_pos = pos_pos;
-  A.pos_w = pos_w;
-  A.hld_row = hld_row;
-  A.seg_off = seg_off;
-  A.seg_top = seg_top;
-  A.seg_pos = seg_pos;
-  A.done = done;
-  A.next = next;
-  A.err = err;
-  A.spin_limit = spin_limit_cycles();
-  A.max_u = max_u;
-  A.max_segs = std::max(max_segs, 1);
-  A.scalar_cols = scalar_cols;
-  A.trace_t = nullptr;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  GH_CUDA(cudaStreamIsCapturing(s, &cs));
-  const bool capturing = cs != cudaStreamCaptureStatusNone;
-  if (std::getenv("GPUH2H_TRACE") && !capturing) {
-    if (!trace_t) GH_CUDA(cudaMalloc(&trace_t, sizeof(unsigned long long) * std::max(N, 1)));
-    GH_CUDA(cudaMemsetAsync(trace_t, 0, sizeof(unsigned long long) * std::max(N, 1), s));
-    A.trace_t = trace_t;
-  }
-  // inside a capture an event record becomes a graph node only when external
-  auto record = [&](cudaEvent_t e) {
-    GH_CUDA(capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s));
-  };
-  if (fill_ev) record(fill_ev[0]);
-  fill_flow_kernel<<<blocks, threads, smem, s>>>(A);
-  GH_CUDA(cudaGetLastError());
-  if (fill_ev) record(fill_ev[1]);
+  pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = tasks = nullptr;
+  blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;
+  hld_row = seg_off = blk_boff = blk_moff = blk_soff = bm_row = task0 = nullptr;
+  loc_of = nullptr;
+  direct = closed = nullptr;
 }
 
 // With GPUH2H_TRACE: where the last fill's time went, from the nodes'
 // publish times -- per forest level the time from the previous level's last
-// publish to its own (levels overlap in the dataflow; the spans add up to
-// the fill), summed per tile class, and the ten longest levels.
+// publish to its own (levels overlap; the spans add up to the fill), summed per tile class, and the ten longest levels.
 void FillPlan::trace_report() {
   if (!trace_t) return;
   GH_CUDA(cudaDeviceSynchronize());
@@ -1301,8 +630,8 @@ int64_t label_max(const Graph &gc) {
 
 // Autotuner of the forest fill's tile shapes.  Coordinate descent over the
 // (level width x separator size) buckets that hold nodes: for each bucket in
-// turn, first the one-tile threshold, then the column-block x separator-chunk
-// split, each candidate timed as a whole fill (best of two runs) with the
+// turn, first the one-task threshold, then the columns of a task, each
+// candidate timed as a whole fill (best of two runs) with the
 // other buckets held; a candidate replaces the incumbent only when it is 2%
 // faster.  Any policy gives the same labels: only the schedule changes.
 std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
@@ -1335,8 +664,8 @@ std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
     }
     return best;
   };
-  static const int kSmall[] = {0, 1 << 8, 1 << 10, 1 << 12, 1 << 14, 1 << 16};
-  static const int kShape[][2] = {{32, 4}, {32, 8}, {32, 16}, {32, 32}, {64, 32}, {128, 256}};
+  static const int kSmall[] = {0, 1 << 10, 1 << 12, 1 << 14, 1 << 16, 1 << 20};
+  static const int kCols[] = {64, 128, 256, 512, 1024, 4096};
   TilePolicy best = plan.policy;
   float best_ms = 0;
   try {
@@ -1352,11 +681,10 @@ std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
             const float t = time_policy(p);
             if (t < best_ms * 0.98f) { best = p; best_ms = t; }
           }
-          for (const auto &sh : kShape) {
-            if (sh[0] == best.col_block[wb][sb] && sh[1] == best.sep_chunk[wb][sb]) continue;
+          for (int cols : kCols) {
+            if (cols == best.col_block[wb][sb]) continue;
             TilePolicy p = best;
-            p.col_block[wb][sb] = sh[0];
-            p.sep_chunk[wb][sb] = sh[1];
+            p.col_block[wb][sb] = cols;
             const float t = time_policy(p);
             if (t < best_ms * 0.98f) { best = p; best_ms = t; }
           }
@@ -1376,11 +704,11 @@ void fill_labels_gpu(Graph &g) {
   Clock clk;
   const int n = g.n;
   DeviceIndex &D = g.dev;
-  // L4 runs as a dataflow over the tree; L3 (order-dependent, as shipped)
+  // L4 runs over blocks of the tree; L3 (order-dependent, as shipped)
   // keeps the level-synchronous kernel that applies the reference's order.
   const bool flow = !uses_level_fill(g);
   if (flow) {
-    TilePolicy pol = TilePolicy::for_height(g.tree_height);
+    TilePolicy pol = TilePolicy();
     if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
       GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
     FillPlan plan({&g}, pol, D.lists);

@@ -112,7 +112,7 @@ void allocate_labels_and_bfs(Graph &g) {
   Pool pool(g.threads);
   if (!g.tree_layout) prefix_sums(pool, n, g.dis_hash, [&](int64_t v) { return (int64_t)g.depth[v]; });
   prefix_sums(pool, n, g.pos_hash, [&](int64_t v) { return (int64_t)(g.x_off[v + 1] - g.x_off[v]) + 1; });
-  // host position lists only for the level-synchronous fill; the dataflow
+  // host position lists only for the level-synchronous fill; the block
   // fill builds them on the GPU from the device lists
   if (uses_level_fill(g)) {
     if ((int64_t)g.x_id.size() != g.x_off[n]) download_lists(g);

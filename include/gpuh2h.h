@@ -174,7 +174,7 @@ int h2h_fill_labels_l4_noalloc(int n, const int *order, const int *father, const
  * one graph per process (main.cu:84-147).  Many loaded graphs are contracted
  * together (one elimination launch per level step across every graph, one
  * launch for every graph's global order over levels <= C) and labelled (L4)
- * by one dataflow launch over the forest of their trees.  Each graph ends in
+ * by one launch over the forest of their trees.  Each graph ends in
  * the state h2h_contract(g, 1) + h2h_build_labels(g, 2, 1, H2H_LABEL_L4)
  * leaves, with bit-identical order, tree and labels, and answers queries on
  * its own handle.  The graphs must outlive the batch. */
@@ -204,10 +204,13 @@ int h2h_batch_rebuild(h2h_batch *b);
 /* Waits for the batch's stream.  Accessors (h2h_copy_adj, h2h_copy_labels)
  * read the device arrays, so they see the last rebuild once it returned. */
 int h2h_batch_sync_host(h2h_batch *b);
-/* Tile shapes of the forest label fill.  policy is 12 entries
+/* Task shapes of the forest label fill.  policy is 12 entries
  * "small_work/col_block/sep_chunk" separated by spaces: level class (fewer
  * nodes than SMs / wider / heavy: nodes averaging 2^18+ min-plus updates),
- * times separator size m <= 16, <= 64, <= 256, > 256.
+ * times separator size m <= 16, <= 64, <= 256, > 256 of a tree block's top.
+ * A block with m * depth <= small_work is one task, a larger one is cut into
+ * tasks of col_block columns (rounded up to 64); sep_chunk shapes nothing.
+ * fill_tiles counts every node once per task of its block.
  * h2h_batch_tune times candidate shapes on this batch (coordinate descent,
  * `rounds` passes), keeps the fastest and writes it to policy_out. */
 int h2h_batch_set_policy(h2h_batch *b, const char *policy);
