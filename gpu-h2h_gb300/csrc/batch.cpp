@@ -54,7 +54,7 @@ struct h2h_batch {
   void fill_info() {
     info.graphs = (int)gs.size();
     info.vertices = elim->N;
-    info.elim_launches = (int)elim->launches.size();
+    info.elim_launches = elim->launch_count();
     info.fill_tiles = fill->ntiles;
     int64_t db = elim->bytes + fill->work_bytes;
     int64_t upd = 0;
@@ -135,65 +135,77 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch 
     clk.reset();
     GH_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     for (auto &e : b->ev) GH_CUDA(cudaEventCreate(&e));
-    b->elim = std::make_unique<gh::ElimPlan>(b->gs);
-    GH_CUDA(cudaDeviceSynchronize());
-    b->info.t_plan_us = clk.us();
-    clk.reset();
-    GH_CUDA(cudaEventRecord(b->ev[0], b->stream));
-    cudaEvent_t hev[2] = {b->ev[1], b->ev[2]};
-    b->elim->enqueue(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr);
-    b->elim->check_error();
-    b->info.t_contract_us = event_us(b->ev[0], b->ev[1]);
-    b->info.t_global_us = event_us(b->ev[1], b->ev[2]);
-    clk.reset();
-    b->elim->build_lists();
-    for (gh::Graph *g : b->gs) {
-      g->contract_device = 1;
-      g->t.td_gpu = 0;
-      g->t.td_cpu = 0;
-    }
-    b->info.t_download_us = clk.us();
-    clk.reset();
-    per_graph([](gh::Graph &g) {
-      gh::build_tree(g);
-      g.contracted = true;
-      g.parallel_fine = 2;
-      g.construct_device = 1;
-      g.label_mode = H2H_LABEL_L4;
-      gh::allocate_labels_and_bfs(g);
-    });
-    gh::build_rmq_gpu(b->gs);
-    b->info.t_tree_us = clk.us();
-    if (std::getenv("GPUH2H_TRACE")) {
-      long long sum = 0, mx = 0;
+    for (bool allow_bits = true;; allow_bits = false) {
+      b->elim = std::make_unique<gh::ElimPlan>(b->gs, allow_bits);
+      GH_CUDA(cudaDeviceSynchronize());
+      b->info.t_plan_us = clk.us();
+      clk.reset();
+      GH_CUDA(cudaEventRecord(b->ev[0], b->stream));
+      cudaEvent_t hev[2] = {b->ev[1], b->ev[2]};
+      b->elim->enqueue(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr);
+      b->elim->check_error();
+      b->info.t_contract_us = event_us(b->ev[0], b->ev[1]);
+      b->info.t_global_us = event_us(b->ev[1], b->ev[2]);
+      clk.reset();
+      b->elim->build_lists();
       for (gh::Graph *g : b->gs) {
-        const long long t = g->t.tree + g->t.malloc_labels + g->t.bfs;
-        sum += t;
-        mx = std::max(mx, t);
+        g->contract_device = 1;
+        g->t.td_gpu = 0;
+        g->t.td_cpu = 0;
       }
-      std::fprintf(stderr, "[gpuh2h] batch tree phase: %lld us wall, per-graph sum %lld us, max %lld us\n",
-                   (long long)b->info.t_tree_us, sum, mx);
+      b->info.t_download_us = clk.us();
+      clk.reset();
+      per_graph([](gh::Graph &g) {
+        gh::build_tree(g);
+        g.contracted = true;
+        g.parallel_fine = 2;
+        g.construct_device = 1;
+        g.label_mode = H2H_LABEL_L4;
+        gh::allocate_labels_and_bfs(g);
+      });
+      gh::build_rmq_gpu(b->gs);
+      b->info.t_tree_us = clk.us();
+      if (std::getenv("GPUH2H_TRACE")) {
+        long long sum = 0, mx = 0;
+        for (gh::Graph *g : b->gs) {
+          const long long t = g->t.tree + g->t.malloc_labels + g->t.bfs;
+          sum += t;
+          mx = std::max(mx, t);
+        }
+        std::fprintf(stderr, "[gpuh2h] batch tree phase: %lld us wall, per-graph sum %lld us, max %lld us\n",
+                     (long long)b->info.t_tree_us, sum, mx);
+      }
+      clk.reset();
+      gh::TilePolicy pol;
+      if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
+        GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
+      b->fill = std::make_unique<gh::FillPlan>(b->gs, b->elim->lists, b->elim.get());
+      if (!b->fill->weights_fit) {  // very wide separators: the list kernels, which need no update triangles
+        b->fill.reset();
+        continue;
+      }
+      b->fill->prepare(pol);
+      GH_CUDA(cudaDeviceSynchronize());
+      b->info.t_fill_plan_us = clk.us();
+      clk.reset();
+      b->fill->enqueue_weights(b->stream);
+      b->fill->check_error();
+      b->info.t_contract_us += clk.us();  // the weights are the contraction's
+      clk.reset();
+      cudaEvent_t fev[2] = {b->ev[0], b->ev[3]};
+      b->fill->enqueue(b->stream, fev);
+      b->fill->check_error();
+      b->info.t_fill_us = event_us(b->ev[0], b->ev[3]);
+      b->fill->trace_report();
+      clk.reset();
+      b->fill->attach(true);
+      for (gh::Graph *g : b->gs) {
+        gh::upload_query_index(*g);
+        g->labelled = true;
+      }
+      b->info.t_attach_us = clk.us();
+      break;
     }
-    clk.reset();
-    gh::TilePolicy pol;
-    if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
-      GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
-    b->fill = std::make_unique<gh::FillPlan>(b->gs, pol, b->elim->lists);
-    GH_CUDA(cudaDeviceSynchronize());
-    b->info.t_fill_plan_us = clk.us();
-    clk.reset();
-    cudaEvent_t fev[2] = {b->ev[0], b->ev[3]};
-    b->fill->enqueue(b->stream, fev);
-    b->fill->check_error();
-    b->info.t_fill_us = event_us(b->ev[0], b->ev[3]);
-    b->fill->trace_report();
-    clk.reset();
-    b->fill->attach(true);
-    for (gh::Graph *g : b->gs) {
-      gh::upload_query_index(*g);
-      g->labelled = true;
-    }
-    b->info.t_attach_us = clk.us();
     b->info.t_total_us = total.us();
     b->fill_info();
     *out = b.release();
@@ -218,8 +230,11 @@ int h2h_batch_rebuild(h2h_batch *b) {
       cudaGraph_t graph = nullptr;
       GH_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
       try {
-        b->elim->enqueue(b->stream);
-        b->elim->enqueue_gather(b->stream);
+        if (!b->elim->bits) {  // on bit rows the order and the lists stand: only weights change
+          b->elim->enqueue(b->stream);
+          b->elim->enqueue_gather(b->stream);
+        }
+        b->fill->enqueue_weights(b->stream);
         cudaEvent_t fev[2] = {b->ev[1], b->ev[2]};  // recorded by the graph around the fill kernel
         b->fill->enqueue(b->stream, fev);
       } catch (...) {

@@ -1,4 +1,7 @@
-// contract.cu -- vertex elimination on the GPU: the partition levels of
+// contract.cu -- vertex elimination on the GPU on weighted neighbour lists, for
+// graphs whose cells hold more members than a bit row (symbolic.cu takes the
+// others), and what both have in common: the input lists, the final lists and
+// the fathers.  The list kernels run the partition levels of
 // makeCHPerHeight_2 / makeCHPerHeight_D_2 (kernel_functions.cu:309-553) and
 // the global minimum-degree heap of TDInCPU / uploadCHset / CHUsingHeap_2
 // (Traditional_H2H.cu:6-118, :216-351), both as one elimination kernel.
@@ -1253,12 +1256,6 @@ T *dalloc(size_t n) {
 
 namespace {
 
-// Where a graph's global order starts: the vertices of the cells at levels
-// C..1 (the tail of elim).
-struct GraphLevels {
-  int heap_start = 0, heap_n = 0;
-};
-
 GraphLevels graph_levels(const Graph &g) {
   GraphLevels L;
   int64_t heap_start = INT32_MAX;
@@ -1281,19 +1278,9 @@ T *palloc(size_t n, int64_t &bytes) {
 
 }  // namespace
 
-ElimPlan::ElimPlan(const std::vector<Graph *> &graphs) : gs(graphs) {
+ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(graphs) {
   const int K = (int)gs.size();
   GH_CHECK(K >= 1, H2H_ERR_ARG, "no graph to contract");
-  const bool force_global_stage = std::getenv("GPUH2H_GLOBAL_STAGING") != nullptr;
-  // with global staging, the shared memory left over is an arena of merge
-  // buffers (GPUH2H_GRID_ARENA: 0 = every merge stages in global memory,
-  // 1 = partition levels only, 2 = the global order too)
-  int grid_arena = 2;
-  if (const char *e = std::getenv("GPUH2H_GRID_ARENA")) grid_arena = std::max(0, std::min(2, std::atoi(e)));
-  // cooperative steps: split each pick's merges over the cell's blocks by
-  // work (GPUH2H_ELIM_BALANCE=0: each block merges the neighbours it owns)
-  if (const char *e = std::getenv("GPUH2H_ELIM_BALANCE")) elim_balance = std::atoi(e) != 0;
-
   // cell list bounds come with the elimination sets (build_elimination_sets)
   std::vector<GraphLevels> L(K);
   int threads = 1;
@@ -1372,13 +1359,91 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs) : gs(graphs) {
     }
   }
   f_adj_off[N] = (int)M;
-  // ---- launches.  Step s takes level H_i - s of every graph still above
-  // C_i; the last step takes every graph's global order as one cell per
-  // graph.  Within a step, cells are grouped by size class, each group is a
-  // launch with its own cluster size (a large cell spreads its merges over up
-  // to 16 CTAs), and the groups of a step run side by side on forked streams.
-  // A step with few cells (or the global orders) instead runs as one
-  // cooperative launch of cell_grid_kernel over all SMs.
+  ListLaunches LL;
+  bits = allow_bits && plan_bits();
+  if (!bits) plan_lists(f_elim.data(), L, LL);
+  const std::vector<int> &fcs = LL.fcs, &fcc = LL.fcc, &gmap = LL.gmap;
+  const int64_t pstage_ints = LL.pstage_ints, partial_max = LL.partial_max;
+  // ---- device state
+  try {
+    slot_nbr = palloc<int>(pool_size + 4, bytes);  // + 4: a list's last 128-bit load stays inside
+    slot_w = palloc<int>(pool_size + 4, bytes);
+    pool_next = palloc<unsigned long long>(1, bytes);
+    pool_first = palloc<unsigned long long>(1, bytes);
+    slot_off = palloc<int64_t>(N, bytes);
+    slot_off_init = palloc<int64_t>(N, bytes);
+    lsize = palloc<int>(N, bytes);
+    cap = palloc<int>(N, bytes);
+    cap_init = palloc<int>(N, bytes);
+    height = palloc<int>(N, bytes);
+    elim = palloc<int>(N, bytes);
+    elim_init = palloc<int>(N, bytes);
+    deg0 = palloc<int>(N, bytes);
+    deg_init = palloc<int>(N, bytes);
+    h0 = palloc<int>(N, bytes);
+    cpos = palloc<int>(N, bytes);
+    err = palloc<int>(1, bytes);
+    ljunk = palloc<int>(N, bytes);
+    cell_start = palloc<int>(fcs.size(), bytes);
+    cell_count = palloc<int>(fcc.size(), bytes);
+    adj_off = palloc<int>(N + 1, bytes);
+    adj_v = palloc<int>(std::max<int64_t>(M, 1), bytes);
+    adj_w = palloc<int>(std::max<int64_t>(M, 1), bytes);
+    heap_verts = palloc<int>(std::max(heap_total, 1), bytes);
+    if (pstage_ints) pstage = palloc<int>(pstage_ints, bytes);
+    if (!gmap.empty()) {
+      hg_partial = palloc<int4>(2 * partial_max, bytes);  // per block: argmin, then (first word) merge count
+      partial_cap = partial_max;
+      grid_map = palloc<int>(gmap.size(), bytes);
+      grid_bar = palloc<unsigned>(grid_bar_words, bytes);
+      GH_CUDA(cudaMemcpy(grid_map, gmap.data(), sizeof(int) * gmap.size(), cudaMemcpyHostToDevice));
+    }
+    for (int k = 1; k < max_group; k++) {
+      cudaStream_t st = nullptr;
+      cudaEvent_t e = nullptr;
+      GH_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      side.push_back(st);
+      GH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      ev_join.push_back(e);
+    }
+    GH_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+    GH_CUDA(cudaMemcpy(slot_off_init, f_slot_off.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(deg_init, f_deg.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(cap_init, f_cap.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(elim_init, f_elim.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(cell_start, fcs.data(), sizeof(int) * fcs.size(), cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(cell_count, fcc.data(), sizeof(int) * fcc.size(), cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(adj_off, f_adj_off.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(adj_v, f_adj_v.data(), sizeof(int) * f_adj_v.size(), cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(adj_w, f_adj_w.data(), sizeof(int) * f_adj_w.size(), cudaMemcpyHostToDevice));
+    if (heap_total)
+      GH_CUDA(cudaMemcpy(heap_verts, f_heap.data(), sizeof(int) * heap_total, cudaMemcpyHostToDevice));
+    const unsigned long long first_free = (unsigned long long)lub;
+    GH_CUDA(cudaMemcpy(pool_first, &first_free, sizeof(first_free), cudaMemcpyHostToDevice));
+  } catch (...) {
+    release();
+    throw;
+  }
+}
+
+// The launches of the list kernels.  Step s takes level H_i - s of every graph still above
+// C_i; the last step takes every graph's global order as one cell per
+// graph.  Within a step, cells are grouped by size class, each group is a
+// launch with its own cluster size (a large cell spreads its merges over up
+// to 16 CTAs), and the groups of a step run side by side on forked streams.
+// A step with few cells (or the global orders) instead runs as one
+// cooperative launch of cell_grid_kernel over all SMs.
+void ElimPlan::plan_lists(const int *f_elim, const std::vector<GraphLevels> &L, ListLaunches &LL) {
+  const int K = (int)gs.size();
+  const bool force_global_stage = std::getenv("GPUH2H_GLOBAL_STAGING") != nullptr;
+  // with global staging, the shared memory left over is an arena of merge
+  // buffers (GPUH2H_GRID_ARENA: 0 = every merge stages in global memory,
+  // 1 = partition levels only, 2 = the global order too)
+  int grid_arena = 2;
+  if (const char *e = std::getenv("GPUH2H_GRID_ARENA")) grid_arena = std::max(0, std::min(2, std::atoi(e)));
+  // cooperative steps: split each pick's merges over the cell's blocks by
+  // work (GPUH2H_ELIM_BALANCE=0: each block merges the neighbours it owns)
+  if (const char *e = std::getenv("GPUH2H_ELIM_BALANCE")) elim_balance = std::atoi(e) != 0;
   const int smem_dyn = enable_max_dynamic_smem(elim_kernel);
   const int smem_dyn_g = enable_max_dynamic_smem(cell_grid_kernel);
   const bool force_cluster = std::getenv("GPUH2H_CLUSTER_HEAP") != nullptr;
@@ -1423,10 +1488,9 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs) : gs(graphs) {
     step_level.push_back(0);
   }
   const int nsteps = (int)step_cells.size();
-  std::vector<int> fcs, fcc;
+  std::vector<int> &fcs = LL.fcs, &fcc = LL.fcc, &gmap = LL.gmap;
   auto al = [](int64_t bb) { return (bb + 15) & ~int64_t(15); };
-  int64_t pstage_ints = 0, partial_max = 0;
-  std::vector<int> gmap;
+  int64_t &pstage_ints = LL.pstage_ints, &partial_max = LL.partial_max;
   // Whole-step cooperative launch: one block per SM, for steps of at most
   // nsm / 2 cells (GPUH2H_GRID_CELLS overrides), where a cell gets two SMs
   // or more -- the cluster kernel caps a cell at 16 CTAs, and long lists
@@ -1625,66 +1689,6 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs) : gs(graphs) {
     }
     max_group = most;
   }
-  // ---- device state
-  try {
-    slot_nbr = palloc<int>(pool_size + 4, bytes);  // + 4: a list's last 128-bit load stays inside
-    slot_w = palloc<int>(pool_size + 4, bytes);
-    pool_next = palloc<unsigned long long>(1, bytes);
-    pool_first = palloc<unsigned long long>(1, bytes);
-    slot_off = palloc<int64_t>(N, bytes);
-    slot_off_init = palloc<int64_t>(N, bytes);
-    lsize = palloc<int>(N, bytes);
-    cap = palloc<int>(N, bytes);
-    cap_init = palloc<int>(N, bytes);
-    height = palloc<int>(N, bytes);
-    elim = palloc<int>(N, bytes);
-    elim_init = palloc<int>(N, bytes);
-    deg0 = palloc<int>(N, bytes);
-    deg_init = palloc<int>(N, bytes);
-    h0 = palloc<int>(N, bytes);
-    cpos = palloc<int>(N, bytes);
-    err = palloc<int>(1, bytes);
-    ljunk = palloc<int>(N, bytes);
-    cell_start = palloc<int>(fcs.size(), bytes);
-    cell_count = palloc<int>(fcc.size(), bytes);
-    adj_off = palloc<int>(N + 1, bytes);
-    adj_v = palloc<int>(std::max<int64_t>(M, 1), bytes);
-    adj_w = palloc<int>(std::max<int64_t>(M, 1), bytes);
-    heap_verts = palloc<int>(std::max(heap_total, 1), bytes);
-    if (pstage_ints) pstage = palloc<int>(pstage_ints, bytes);
-    if (!gmap.empty()) {
-      hg_partial = palloc<int4>(2 * partial_max, bytes);  // per block: argmin, then (first word) merge count
-      partial_cap = partial_max;
-      grid_map = palloc<int>(gmap.size(), bytes);
-      grid_bar = palloc<unsigned>(grid_bar_words, bytes);
-      GH_CUDA(cudaMemcpy(grid_map, gmap.data(), sizeof(int) * gmap.size(), cudaMemcpyHostToDevice));
-    }
-    for (int k = 1; k < max_group; k++) {
-      cudaStream_t st = nullptr;
-      cudaEvent_t e = nullptr;
-      GH_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-      side.push_back(st);
-      GH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      ev_join.push_back(e);
-    }
-    GH_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    GH_CUDA(cudaMemcpy(slot_off_init, f_slot_off.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(deg_init, f_deg.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(cap_init, f_cap.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(elim_init, f_elim.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(cell_start, fcs.data(), sizeof(int) * fcs.size(), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(cell_count, fcc.data(), sizeof(int) * fcc.size(), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(adj_off, f_adj_off.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(adj_v, f_adj_v.data(), sizeof(int) * f_adj_v.size(), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(adj_w, f_adj_w.data(), sizeof(int) * f_adj_w.size(), cudaMemcpyHostToDevice));
-    if (heap_total)
-      GH_CUDA(cudaMemcpy(heap_verts, f_heap.data(), sizeof(int) * heap_total, cudaMemcpyHostToDevice));
-    const unsigned long long first_free = (unsigned long long)lub;
-    GH_CUDA(cudaMemcpy(pool_first, &first_free, sizeof(first_free), cudaMemcpyHostToDevice));
-  } catch (...) {
-    release();
-    throw;
-  }
 }
 
 ElimPlan::~ElimPlan() { release(); }
@@ -1694,6 +1698,10 @@ void ElimPlan::release() {
                 elim_init, deg0, deg_init, h0, cpos, err, ljunk, cell_start, cell_count, adj_off, adj_v, adj_w,
                 heap_verts, pstage};
   for (void *p : ps) cudaFree(p);
+  for (void *p : {(void *)members, (void *)extra, (void *)fin, (void *)sym_cells, (void *)grows}) cudaFree(p);
+  members = extra = nullptr;
+  fin = sym_cells = nullptr;
+  grows = nullptr;
   cudaFree(hg_partial);
   cudaFree(grid_map);
   cudaFree(grid_bar);
@@ -1790,6 +1798,10 @@ void ElimPlan::launch_one(const Launch &Lc, cudaStream_t s, bool trace) {
 }
 
 void ElimPlan::enqueue(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
+  if (bits) {
+    enqueue_bits(s, heap_ev, trace);
+    return;
+  }
   // ---- reset to the input lists (relocation in the global order moves
   // lists and grows their capacity)
   GH_CUDA(cudaMemcpyAsync(slot_off, slot_off_init, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice, s));
@@ -1873,6 +1885,11 @@ void ElimPlan::build_lists() {
   GH_CUDA(cudaGetLastError());
   father_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256>>>(lists.off, lists.id, rank, father_dev, N);
   GH_CUDA(cudaGetLastError());
+  if (bits) {  // the lists never run again: only their weights are replayed
+    GH_CUDA(cudaFree(slot_nbr));
+    GH_CUDA(cudaFree(slot_w));
+    slot_nbr = slot_w = nullptr;
+  }
   GH_CUDA(cudaMemcpy(f_elim.data(), elim, sizeof(int) * N, cudaMemcpyDeviceToHost));
   GH_CUDA(cudaMemcpy(f_father.data(), father_dev, sizeof(int) * N, cudaMemcpyDeviceToHost));
   for (size_t i = 0; i < gs.size(); i++) {
@@ -1898,6 +1915,10 @@ void ElimPlan::build_lists() {
 }
 
 void ElimPlan::enqueue_gather(cudaStream_t s) {
+  if (bits) {
+    gather_bits(s);
+    return;
+  }
   gather_lists_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256, 0, s>>>(
       slot_off, lsize, lists.off, slot_nbr, slot_w, lists.id, lists.w, N);
   GH_CUDA(cudaGetLastError());
@@ -1937,41 +1958,63 @@ void download_lists(Graph &g) {
     for (int64_t k = 0; k < t; k++) g.x_id[k] -= g.dev.id_base;
 }
 
-// Whole elimination of one graph on the GPU: partition levels H..C+1, then
-// the global order over the vertices of levels <= C.  Fills g.elim
-// (elimination order), g.father, g.x_off and g.gpu_vertices; the lists
-// X(v)\{v} (sorted by id, the lists at elimination time) stay on the device.
+// Whole contraction of one graph on the GPU: partition levels H..C+1, then
+// the global order over the vertices of levels <= C, the tree and the sparse
+// table.  Fills g.elim (elimination order), g.father, g.x_off and
+// g.gpu_vertices; the lists X(v)\{v} (sorted by id, the lists at elimination
+// time) stay on the device.  On bit rows the lists' weights follow from the
+// tree's blocks, which g.plan keeps for the label fill.
 void contract_gpu(Graph &g) {
   Clock clk;
   const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
-  auto owned = std::make_unique<ElimPlan>(std::vector<Graph *>{&g});
-  ElimPlan &plan = *owned;
-  GH_CUDA(cudaDeviceSynchronize());
-  g.t.translate_lub = clk.us();
-  clk.reset();
-  cudaEvent_t ev[2];
-  GH_CUDA(cudaEventCreate(&ev[0]));
-  GH_CUDA(cudaEventCreate(&ev[1]));
-  long long heap_us = 0;
-  try {
-    plan.enqueue(0, ev, trace);
-    plan.check_error();
-    float hms = 0;
-    GH_CUDA(cudaEventElapsedTime(&hms, ev[0], ev[1]));
-    heap_us = (long long)(hms * 1000.0f);
-  } catch (...) {
+  for (bool allow_bits = true;; allow_bits = false) {
+    auto owned = std::make_unique<ElimPlan>(std::vector<Graph *>{&g}, allow_bits);
+    ElimPlan &plan = *owned;
+    GH_CUDA(cudaDeviceSynchronize());
+    g.t.translate_lub = clk.us();
+    clk.reset();
+    cudaEvent_t ev[2];
+    GH_CUDA(cudaEventCreate(&ev[0]));
+    GH_CUDA(cudaEventCreate(&ev[1]));
+    long long heap_us = 0;
+    try {
+      plan.enqueue(0, ev, trace);
+      plan.check_error();
+      float hms = 0;
+      GH_CUDA(cudaEventElapsedTime(&hms, ev[0], ev[1]));
+      heap_us = (long long)(hms * 1000.0f);
+    } catch (...) {
+      cudaEventDestroy(ev[0]);
+      cudaEventDestroy(ev[1]);
+      throw;
+    }
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
-    throw;
+    g.t.td_gpu = clk.us() - heap_us;  // partition levels
+    g.t.td_cpu = heap_us;             // global order over levels <= C (TDInCPUTime in the reference, on the GPU here)
+    clk.reset();
+    plan.build_lists();
+    g.t.translate_back = clk.us();
+    build_tree_and_rmq(g);
+    clk.reset();
+    if (plan.bits) {
+      position_offsets(g);
+      g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, plan.lists, &plan);
+      if (!g.plan->weights_fit) {  // very wide separators: the list kernels, which need no update triangles
+        g.plan.reset();
+        continue;
+      }
+      g.plan->enqueue_weights(0);
+      g.plan->check_error();
+      g.plan->arcs = nullptr;
+      if (trace) std::fprintf(stderr, "[gpuh2h] weights plan and weights: %.3f ms\n", clk.us() / 1e3);
+      g.t.td_gpu += clk.us();  // the weights
+      clk.reset();
+    }
+    owned.reset();  // the elimination's device state is freed here, inside the timed phase
+    g.t.translate_back += clk.us();
+    return;
   }
-  cudaEventDestroy(ev[0]);
-  cudaEventDestroy(ev[1]);
-  g.t.td_gpu = clk.us() - heap_us;  // partition levels
-  g.t.td_cpu = heap_us;             // global order over levels <= C (TDInCPUTime in the reference, on the GPU here)
-  clk.reset();
-  plan.build_lists();
-  owned.reset();  // the elimination's device state is freed here, inside the timed phase
-  g.t.translate_back = clk.us();
 }
 
 }  // namespace gh

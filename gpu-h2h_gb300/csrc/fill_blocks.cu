@@ -204,9 +204,10 @@ __global__ void block_sizes_kernel(const int *blk_top, const int *count, const i
       r = count[t];
       m = (int)(pos_hash[t + 1] - pos_hash[t]) - 1;
     }
+    const int rp = (r + 3) & ~3;
     rows[b] = r;
     mem[b] = m;
-    cells[b] = m * ((r + 3) & ~3);
+    cells[b] = (m + rp) * rp;
   }
 }
 
@@ -290,7 +291,9 @@ struct BlockArgs {
   const int *father, *depth;
   const int64_t *drow, *pos_hash;
   const int *pos_pos, *pos_id, *pos_w;
-  unsigned *direct, *closed;  // per block [member][row], rows padded to a multiple of four
+  // per block [column][row], rows padded to a multiple of four: the columns
+  // are the top's members, then (direct only) the block's own nodes
+  unsigned *direct, *closed;
   int nblk;
   int *err;
 };
@@ -389,6 +392,360 @@ __global__ void __launch_bounds__(32 * kClosureWarps) closure_kernel(BlockArgs A
     for (int k = 0; k < kn; k++)
       if (lane < Rp) A.closed[out + k * Rp + lane] = lane < R ? row[lane * 33 + k] : kInf;
     __syncwarp();
+  }
+}
+
+// ------------------------------------------------------------ the weights
+//
+// With the order and the lists known (symbolic.cu), the shortcut weights are
+// an elimination over the blocks, leaves to root: a block's rows hold the
+// weights between its nodes and its nodes' upper neighbours, first the input
+// arcs and what the blocks below add; eliminating the nodes deepest first
+// gives row(u)[x] = min(row(u)[x], row(i)[u] + row(i)[x]) for u, x upper
+// neighbours of i.  Inside the block that is a 32 x 32 triangle; each further
+// column is a triangular solve of its own; and what the block adds between
+// two of its top's members x, y -- min over its nodes i of row(i)[x] +
+// row(i)[y] -- is a min-plus product that goes to the parent block by
+// atomicMin.  Every sum is one the list kernels take, with the row of the
+// vertex eliminated first (arcs' weights may differ by direction).
+//
+// Repeated arcs: a row takes the smallest, except in the global order, whose
+// lists keep the first of equal ids (unordered_map::emplace).
+
+// Each member's column in the parent block (its place there, encoded ~place,
+// or its index among the parent's members), and how many tasks a parent waits
+// for.  One warp per block.
+__global__ void parent_columns_kernel(BlockArgs B, const int64_t *wtask0, int *blk_up, int *bm_up, int *pend) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; b < B.nblk;
+       b += (gridDim.x * (int64_t)blockDim.x) >> 5) {
+    const int top = B.blk_top[b], f = B.father[top];
+    const int p = f < 0 ? -1 : B.blk_of[f];
+    if (lane == 0) {
+      blk_up[b] = p;
+      if (p >= 0) atomicAdd(pend + p, (int)(wtask0[b + 1] - wtask0[b]));
+    }
+    if (p < 0) continue;
+    const int64_t pb = B.pos_hash[top], m0 = B.moff[b], pm0 = B.moff[p];
+    const int m = (int)(B.moff[b + 1] - m0), pm = (int)(B.moff[p + 1] - pm0);
+    const int pdt = B.depth[B.blk_top[p]] - 1;
+    for (int k = lane; k < m; k += 32) {
+      const int q = B.pos_pos[pb + k];
+      int code;
+      if (q >= pdt) {
+        code = ~(int)B.loc_of[B.pos_id[pb + k]];
+      } else {
+        int lo = 0, hi = pm;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (B.bm_p[pm0 + mid] < q) lo = mid + 1; else hi = mid;
+        }
+        if (lo >= pm || B.bm_p[pm0 + lo] != q) {
+          atomicCAS(B.err, 0, kErrNested);
+          lo = 0;
+        }
+        code = lo;
+      }
+      bm_up[m0 + k] = code;
+    }
+  }
+}
+
+__global__ void weight_tasks_kernel(const int *mem, int *ntask, int nblk) {
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nblk; b += gridDim.x * blockDim.x) {
+    const int nt = b < nblk ? max(1, (mem[b] + 63) / 64) : 0;
+    ntask[b] = nt * (nt + 1) / 2;
+  }
+}
+
+// Entries of a block's update triangle: none where no block lies below.
+__global__ void update_sizes_kernel(const int *mem, const int *pend, int64_t *cells, int nblk) {
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nblk; b += gridDim.x * blockDim.x)
+    cells[b] = b < nblk && pend[b] > 0 ? (int64_t)mem[b] * (mem[b] - 1) / 2 : 0;
+}
+
+__global__ void mark_kernel(const int *verts, int n, unsigned char *flag) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) flag[verts[i]] = 1;
+}
+
+// The cell every arc v -> x with x an upper neighbour of v starts from; -1
+// for the other direction and for repeated arcs of the global order.
+__global__ void arc_cells_kernel(BlockArgs B, const int *adj_off, const int *adj_v, const unsigned char *global,
+                                 int64_t *arc_cell, int n) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const int d = B.depth[v], b = B.blk_of[v], i = B.loc_of[v];
+    const int64_t m0 = B.moff[b], so = B.soff[b];
+    const int m = (int)(B.moff[b + 1] - m0), Rp = ((int)(B.boff[b + 1] - B.boff[b]) + 3) & ~3;
+    const int dt = B.depth[B.blk_top[b]] - 1;
+    const int a0 = adj_off[v], a1 = adj_off[v + 1];
+    for (int e = a0; e < a1; e++) {
+      const int x = adj_v[e];
+      int64_t cell = -1;
+      const int p = B.depth[x] - 1;
+      bool use = p < d - 1;
+      if (use && global[v])
+        for (int q = a0; q < e && use; q++) use = adj_v[q] != x;
+      if (use) {
+        int c;
+        if (p >= dt) {
+          c = m + B.loc_of[x];
+        } else {
+          int lo = 0, hi = m;
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (B.bm_p[m0 + mid] < p) lo = mid + 1; else hi = mid;
+          }
+          c = lo;
+          if (lo >= m || B.bm_p[m0 + lo] != p) {
+            atomicCAS(B.err, 0, kErrNested);
+            c = -1;
+          }
+        }
+        if (c >= 0) cell = so + (int64_t)c * Rp + i;
+      }
+      arc_cell[e] = cell;
+    }
+  }
+}
+
+__global__ void fill_inf_kernel(unsigned *p, int64_t n) {
+  const int64_t q = n >> 2;
+  uint4 *p4 = reinterpret_cast<uint4 *>(p);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < q; i += (int64_t)gridDim.x * blockDim.x)
+    p4[i] = make_uint4(kInf, kInf, kInf, kInf);
+  if (blockIdx.x == 0 && threadIdx.x < (n & 3)) p[4 * q + threadIdx.x] = kInf;
+}
+
+__global__ void scatter_arcs_kernel(const int64_t *arc_cell, const int *w, unsigned *cells, int64_t m) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = arc_cell[e];
+    if (c >= 0) atomicMin(cells + c, (unsigned)w[e]);
+  }
+}
+
+struct WeightArgs {
+  BlockArgs B;
+  const int *blk_up, *bm_up;
+  const int64_t *uoff;
+  unsigned *upd;  // per block with blocks below it: pairs (x < y) of members at y (y - 1) / 2 + x
+  const int *task_blk;
+  const int64_t *task0;
+  int ntasks;
+  int *pending, *next;
+  long long spin_limit;
+};
+
+// A CTA takes a 64 x 64 tile of a block's update triangle, blocks from the
+// deepest up (a block's tasks wait for the tasks of the blocks below it).  It
+// eliminates the block's triangle, solves the tile's (at most 128) columns,
+// one per lane in registers, and forms the tile.  The diagonal tiles write
+// their columns back, direct and closed (see the closure); a tile may read
+// columns another has already written back, which solves to the same values.
+__global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
+  __shared__ __align__(16) unsigned s_L[kRows * 36];
+  __shared__ __align__(16) unsigned s_P[2][kRows * 68];
+  __shared__ int s_up[2][64];
+  __shared__ int s_t, s_flag;
+  const BlockArgs &B = A.B;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) s_t = atomicAdd(A.next, 1);
+    __syncthreads();
+    if (s_t >= A.ntasks) return;
+    const int t = A.ntasks - 1 - s_t;  // deepest blocks first
+    const int b = __ldg(A.task_blk + t);
+    int sub = t - (int)__ldg(A.task0 + b);
+    const int64_t bo = __ldg(B.boff + b), m0 = __ldg(B.moff + b), so = __ldg(B.soff + b);
+    const int R = (int)(__ldg(B.boff + b + 1) - bo), Rp = (R + 3) & ~3;
+    const int m = (int)(__ldg(B.moff + b + 1) - m0);
+    int X = 0, Y = 0;  // tile (X, Y), X <= Y, numbered Y (Y + 1) / 2 + X
+    Y = (int)((sqrtf(8.0f * (float)sub + 1.0f) - 1.0f) * 0.5f);
+    while ((Y + 1) * (Y + 2) / 2 <= sub) Y++;
+    while (Y * (Y + 1) / 2 > sub) Y--;
+    X = sub - Y * (Y + 1) / 2;
+    const int p = __ldg(A.blk_up + b);
+    const bool diag = X == Y;
+    if (p >= 0) {
+      const int k = 64 * (tid < 64 ? X : Y) + (tid & 63);
+      s_up[tid >> 6][tid & 63] = k < m ? __ldg(A.bm_up + m0 + k) : 0;
+    }
+    if (tid == 0) {
+      int ok = 1;
+      const int *flag = A.pending + b;
+      const long long t0 = clock64();
+      while (ld_acquire(flag) != 0) {
+        if (ld_relaxed(B.err) != 0 || clock64() - t0 > A.spin_limit) {
+          atomicCAS(B.err, 0, kErrWait);
+          ok = 0;
+          break;
+        }
+        __nanosleep(32);
+      }
+      s_flag = ok;
+    }
+    __syncthreads();
+    if (!s_flag) return;
+    unsigned *const cells = B.direct + so;
+    // the block's own triangle
+    for (int i = tid; i < kRows * 36; i += 128) s_L[i] = kInf;
+    __syncthreads();
+    for (int i = tid; i < R * Rp; i += 128) {
+      const int c = i / Rp, r = i - c * Rp;
+      if (r > c && r < R) s_L[r * 36 + c] = __ldcg(cells + (int64_t)(m + c) * Rp + r);
+    }
+    __syncthreads();
+    for (int i = R - 1; i > 1; i--) {
+      const unsigned li = s_L[i * 36 + lane];
+      unsigned ups = __ballot_sync(0xffffffffu, li != kInf && lane < i);
+      int turn = 0;
+      while (ups) {
+        const int u = __ffs(ups) - 1;
+        ups &= ups - 1;
+        if ((turn++ & 3) == wid && lane < u)
+          s_L[u * 36 + lane] = add_min(s_L[i * 36 + u], li, s_L[u * 36 + lane]);
+      }
+      __syncthreads();
+    }
+    if (sub == 0)
+      for (int i = tid; i < R * Rp; i += 128) {
+        const int c = i / Rp, r = i - c * Rp;
+        if (r > c && r < R) cells[(int64_t)(m + c) * Rp + r] = s_L[r * 36 + c];
+      }
+    // the tile's columns, one per lane
+    const int half = wid >> 1;  // warps 0, 1: X's columns; 2, 3: Y's
+    const int k = 64 * (half ? Y : X) + 32 * (wid & 1) + lane;
+    if (!(diag && half) && 64 * (half ? Y : X) + 32 * (wid & 1) < m) {
+      unsigned col[kRows];
+      const uint4 *src = reinterpret_cast<const uint4 *>(cells + (int64_t)min(k, m - 1) * Rp);
+#pragma unroll
+      for (int q = 0; q < kRows / 4; q++) {
+        const uint4 x = 4 * q < Rp && k < m ? __ldcg(src + q) : make_uint4(kInf, kInf, kInf, kInf);
+        col[4 * q] = x.x;
+        col[4 * q + 1] = x.y;
+        col[4 * q + 2] = x.z;
+        col[4 * q + 3] = x.w;
+      }
+#pragma unroll
+      for (int i = kRows - 1; i > 0; i--)
+        if (i < R) {
+#pragma unroll
+          for (int u = 0; u < i; u++) col[u] = add_min(s_L[i * 36 + u], col[i], col[u]);
+        }
+#pragma unroll
+      for (int i = 0; i < kRows; i++) s_P[half][i * 68 + 32 * (wid & 1) + lane] = col[i];
+      if (diag) {
+        uint4 *dst = reinterpret_cast<uint4 *>(cells + (int64_t)k * Rp);
+        uint4 *cls = reinterpret_cast<uint4 *>(B.closed + so + (int64_t)k * Rp);
+#pragma unroll
+        for (int q = 0; q < kRows / 4; q++)
+          if (4 * q < Rp && k < m) dst[q] = make_uint4(col[4 * q], col[4 * q + 1], col[4 * q + 2], col[4 * q + 3]);
+#pragma unroll
+        for (int i = 1; i < kRows; i++)
+          if (i < R) {
+#pragma unroll
+            for (int u = 0; u < i; u++) col[i] = add_min(s_L[i * 36 + u], col[u], col[i]);
+          }
+#pragma unroll
+        for (int q = 0; q < kRows / 4; q++)
+          if (4 * q < Rp && k < m) cls[q] = make_uint4(col[4 * q], col[4 * q + 1], col[4 * q + 2], col[4 * q + 3]);
+      }
+    }
+    if (p < 0) continue;
+    __syncthreads();
+    // the tile of the update: lanes along x, so an address run of the parent
+    const int xg = tid & 15, yg = tid >> 4;
+    const int x0 = 64 * X + 4 * xg, y0 = 64 * Y + 8 * yg;
+    if (x0 < m && y0 < m) {
+      unsigned acc[8][4];
+#pragma unroll
+      for (int y = 0; y < 8; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) acc[y][x] = kInf;
+      const unsigned *px = s_P[0] + 4 * xg, *py = s_P[diag ? 0 : 1] + 8 * yg;
+#pragma unroll 2
+      for (int i = 0; i < R; i++) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(px + i * 68);
+        const uint4 c = *reinterpret_cast<const uint4 *>(py + i * 68);
+        const uint4 d = *reinterpret_cast<const uint4 *>(py + i * 68 + 4);
+        const unsigned yv[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int y = 0; y < 8; y++) {
+          acc[y][0] = add_min(yv[y], a.x, acc[y][0]);
+          acc[y][1] = add_min(yv[y], a.y, acc[y][1]);
+          acc[y][2] = add_min(yv[y], a.z, acc[y][2]);
+          acc[y][3] = add_min(yv[y], a.w, acc[y][3]);
+        }
+      }
+      const int64_t uo = __ldg(A.uoff + b);
+      const bool below = __ldg(A.uoff + b + 1) > uo;
+      const int64_t pso = __ldg(B.soff + p), puo = __ldg(A.uoff + p);
+      const int pm = (int)(__ldg(B.moff + p + 1) - __ldg(B.moff + p));
+      const int pRp = ((int)(__ldg(B.boff + p + 1) - __ldg(B.boff + p)) + 3) & ~3;
+#pragma unroll
+      for (int y = 0; y < 8; y++) {
+        const int yy = y0 + y;
+        if (yy >= m) break;
+        const int cy = s_up[1][8 * yg + y];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          const int xx = x0 + x;
+          if (xx >= yy) break;
+          unsigned v = acc[y][x];
+          if (below) v = min(v, __ldcg(A.upd + uo + (int64_t)yy * (yy - 1) / 2 + xx));
+          if (v >= kInf) continue;
+          const int cx = s_up[0][4 * xg + x];
+          unsigned *dst;
+          if (cy < 0)  // y is the parent's own node, eliminated before x
+            dst = B.direct + pso + (int64_t)(cx < 0 ? pm + ~cx : cx) * pRp + ~cy;
+          else
+            dst = A.upd + puo + (int64_t)cy * (cy - 1) / 2 + cx;
+          atomicMin(dst, v);
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicSub(A.pending + p, 1);
+    }
+  }
+}
+
+// Every list entry's weight, in the lists and in the position arrays.  One
+// warp per vertex.
+__global__ void list_weights_kernel(BlockArgs B, const int *pos_src, const int64_t *list_off, int *list_w, int *pos_w,
+                                    int n) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
+       v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
+    const int b = B.blk_of[v], i = B.loc_of[v];
+    const int64_t m0 = B.moff[b], so = B.soff[b];
+    const int m = (int)(B.moff[b + 1] - m0), Rp = ((int)(B.boff[b + 1] - B.boff[b]) + 3) & ~3;
+    const int dt = B.depth[B.blk_top[b]] - 1;
+    const int64_t pb = B.pos_hash[v], pe = B.pos_hash[v + 1];
+    for (int64_t e = pb + lane; e < pe; e += 32) {
+      const int src = pos_src[e];
+      if (src < 0) {
+        pos_w[e] = 0;
+        continue;
+      }
+      const int p = B.pos_pos[e];
+      int c;
+      if (p >= dt) {
+        c = m + B.loc_of[B.pos_id[e]];
+      } else {
+        int lo = 0, hi = m - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (__ldg(B.bm_p + m0 + mid) < p) lo = mid + 1; else hi = mid;
+        }
+        c = lo;
+      }
+      const int w = (int)B.direct[so + (int64_t)c * Rp + i];
+      pos_w[e] = w;
+      list_w[list_off[v] + src] = w;
+    }
   }
 }
 
@@ -801,7 +1158,8 @@ void FillPlan::build_blocks() {
   exclusive_scan<int>(blk_mem, blk_moff, nblk + 1, ws, 0);
   exclusive_scan<int>(cells, blk_soff, nblk + 1, ws, 0);
   GH_CHECK(read_one(blk_boff + nblk) == N, H2H_ERR_STATE, "fill blocks do not cover the tree");
-  const int64_t members = read_one(blk_moff + nblk), cell_total = read_one(blk_soff + nblk);
+  const int64_t members = read_one(blk_moff + nblk);
+  cell_total = read_one(blk_soff + nblk);
   bm_p = dalloc<int>(members, work_bytes);
   bm_row = dalloc<int64_t>(members, work_bytes);
   direct = dalloc<unsigned>(cell_total, work_bytes);
@@ -810,6 +1168,132 @@ void FillPlan::build_blocks() {
   block_nodes_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(blk_top, blk_boff, blk_moff, hpos, pos_hash, pos_pos,
                                                                  pos_id, drow, bnode, blk_of, loc_of, bm_p, bm_row,
                                                                  nblk);
+  GH_CUDA(cudaGetLastError());
+}
+
+namespace {
+
+BlockArgs block_args(const FillPlan &P) {
+  BlockArgs B{};
+  B.blk_top = P.blk_top;
+  B.boff = P.blk_boff;
+  B.moff = P.blk_moff;
+  B.soff = P.blk_soff;
+  B.bnode = P.bnode;
+  B.blk_of = P.blk_of;
+  B.loc_of = P.loc_of;
+  B.bm_p = P.bm_p;
+  B.bm_row = P.bm_row;
+  B.father = P.father;
+  B.depth = P.depth;
+  B.drow = P.drow;
+  B.pos_hash = P.pos_hash;
+  B.pos_pos = P.pos_pos;
+  B.pos_id = P.pos_id;
+  B.pos_w = P.pos_w;
+  B.direct = P.direct;
+  B.closed = P.closed;
+  B.nblk = P.nblk;
+  B.err = P.err;
+  return B;
+}
+
+}  // namespace
+
+// Where the weights come from when the order was made on bit rows: every
+// arc's cell, the tasks of the block elimination and the blocks' places in
+// their parents.  The update triangles of very wide separators (a dense graph
+// of many thousand vertices) can outgrow the memory; weights_fit then tells
+// the caller to use the list kernels.
+void FillPlan::build_weights_plan(const ElimPlan &from) {
+  arcs = &from;
+  Workspace ws;
+  int *ntask = ws.get<int>(nblk + 1);
+  int64_t *ucells = ws.get<int64_t>(nblk + 1);
+  unsigned char *global = ws.get<unsigned char>(N);
+  wtask0 = dalloc<int64_t>(nblk + 1, work_bytes);
+  blk_up = dalloc<int>(nblk, work_bytes);
+  blk_uoff = dalloc<int64_t>(nblk + 1, work_bytes);
+  pending = dalloc<int>(nblk, work_bytes);
+  pend_init = dalloc<int>(nblk, work_bytes);
+  const int64_t members = read_one(blk_moff + nblk);
+  bm_up = dalloc<int>(members, work_bytes);
+  arc_cell = dalloc<int64_t>(from.M, work_bytes);
+  const BlockArgs B = block_args(*this);
+  const int gb = grid_for(nblk + 1, nsm), gw = grid_for((int64_t)nblk * 32, nsm);
+  weight_tasks_kernel<<<gb, 256>>>(blk_mem, ntask, nblk);
+  GH_CUDA(cudaGetLastError());
+  exclusive_scan<int>(ntask, wtask0, nblk + 1, ws, 0);
+  wtasks = read_one(wtask0 + nblk);
+  GH_CHECK(wtasks < INT32_MAX, H2H_ERR_ARG, "too many weight tasks");
+  wtask_blk = dalloc<int>(wtasks, work_bytes);
+  expand_tasks_kernel<<<gw, 256>>>(wtask0, wtask_blk, nblk);
+  GH_CUDA(cudaMemset(err, 0, sizeof(int)));
+  GH_CUDA(cudaMemset(pend_init, 0, sizeof(int) * nblk));
+  parent_columns_kernel<<<gw, 256>>>(B, wtask0, blk_up, bm_up, pend_init);
+  update_sizes_kernel<<<gb, 256>>>(blk_mem, pend_init, ucells, nblk);
+  GH_CUDA(cudaGetLastError());
+  exclusive_scan<int64_t>(ucells, blk_uoff, nblk + 1, ws, 0);
+  upd_total = read_one(blk_uoff + nblk);
+  size_t fr = 0, tot = 0;
+  GH_CUDA(cudaMemGetInfo(&fr, &tot));
+  weights_fit = (uint64_t)upd_total * 4 <= fr / 2;
+  if (!weights_fit) return;
+  upd = dalloc<unsigned>(upd_total, work_bytes);
+  GH_CUDA(cudaMemset(global, 0, N));
+  if (from.heap_total) {
+    mark_kernel<<<grid_for(from.heap_total, nsm), 256>>>(from.heap_verts, from.heap_total, global);
+    GH_CUDA(cudaGetLastError());
+  }
+  arc_cells_kernel<<<grid_for(N, nsm), 256>>>(B, from.adj_off, from.adj_v, global, arc_cell, N);
+  GH_CUDA(cudaGetLastError());
+  GH_CHECK(read_one(err) == 0, H2H_ERR_STATE, "an upper neighbour is missing from its block's separator");
+}
+
+void FillPlan::enqueue_weights(cudaStream_t s) {
+  const BlockArgs B = block_args(*this);
+  const int gn = std::max(1, std::min(8192, (N + 7) / 8));  // a warp per vertex
+  GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  if (!arcs) {  // the lists carry the weights
+    gather_pos_weights_kernel<<<gn, 256, 0, s>>>(pos_hash, pos_src, lists.off, lists.w, pos_w, N);
+    GH_CUDA(cudaGetLastError());
+    closure_kernel<<<dim3((nblk + kClosureWarps - 1) / kClosureWarps, 4), 32 * kClosureWarps, 0, s>>>(B);
+    GH_CUDA(cudaGetLastError());
+    return;
+  }
+  fill_inf_kernel<<<grid_for(cell_total >> 2, nsm), 256, 0, s>>>(direct, cell_total);
+  fill_inf_kernel<<<grid_for(upd_total >> 2, nsm), 256, 0, s>>>(upd, upd_total);
+  GH_CUDA(cudaMemcpyAsync(pending, pend_init, sizeof(int) * nblk, cudaMemcpyDeviceToDevice, s));
+  GH_CUDA(cudaMemsetAsync(next, 0, sizeof(int), s));
+  scatter_arcs_kernel<<<grid_for(arcs->M, nsm), 256, 0, s>>>(arc_cell, arcs->adj_w, direct, arcs->M);
+  GH_CUDA(cudaGetLastError());
+  WeightArgs A{};
+  A.B = B;
+  A.blk_up = blk_up;
+  A.bm_up = bm_up;
+  A.uoff = blk_uoff;
+  A.upd = upd;
+  A.task_blk = wtask_blk;
+  A.task0 = wtask0;
+  A.ntasks = (int)wtasks;
+  A.pending = pending;
+  A.next = next;
+  A.spin_limit = spin_limit_cycles();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  GH_CUDA(cudaStreamIsCapturing(s, &cs));
+  const bool trace = std::getenv("GPUH2H_TRACE") && cs == cudaStreamCaptureStatusNone;
+  if (trace) GH_CUDA(cudaStreamSynchronize(s));
+  Clock clk;
+  int per_sm = 0;
+  GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, weights_kernel, 128, 0));
+  weights_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * std::max(1, per_sm), wtasks)), 128, 0,
+                   s>>>(A);
+  if (trace) {
+    GH_CUDA(cudaStreamSynchronize(s));
+    std::fprintf(stderr, "[gpuh2h] weights: %d blocks, %lld tiles, %.1f MB of update triangles, %.3f ms\n", nblk,
+                 (long long)wtasks, upd_total * 4e-6, clk.us() / 1e3);
+  }
+  list_weights_kernel<<<gn, 256, 0, s>>>(B, pos_src, lists.off, lists.w, pos_w, N);
   GH_CUDA(cudaGetLastError());
 }
 
@@ -855,34 +1339,11 @@ void FillPlan::build_tiles(const TilePolicy &pol) {
 }
 
 void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
-  gather_pos_weights_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256, 0, s>>>(
-      pos_hash, pos_src, lists.off, lists.w, pos_w, N);
-  GH_CUDA(cudaGetLastError());
   GH_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * 2 * (int64_t)nblk, s));
   GH_CUDA(cudaMemsetAsync(next, 0, sizeof(int), s));
   GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   FillKernelArgs A{};
-  BlockArgs &B = A.B;
-  B.blk_top = blk_top;
-  B.boff = blk_boff;
-  B.moff = blk_moff;
-  B.soff = blk_soff;
-  B.bnode = bnode;
-  B.blk_of = blk_of;
-  B.loc_of = loc_of;
-  B.bm_p = bm_p;
-  B.bm_row = bm_row;
-  B.father = father;
-  B.depth = depth;
-  B.drow = drow;
-  B.pos_hash = pos_hash;
-  B.pos_pos = pos_pos;
-  B.pos_id = pos_id;
-  B.pos_w = pos_w;
-  B.direct = direct;
-  B.closed = closed;
-  B.nblk = nblk;
-  B.err = err;
+  A.B = block_args(*this);
   A.dis = dis;
   A.hld_row = hld_row;
   A.seg_off = seg_off;
@@ -910,8 +1371,6 @@ void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
     GH_CUDA(capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s));
   };
   if (fill_ev) record(fill_ev[0]);
-  closure_kernel<<<dim3((nblk + kClosureWarps - 1) / kClosureWarps, 4), 32 * kClosureWarps, 0, s>>>(B);
-  GH_CUDA(cudaGetLastError());
   block_fill_kernel<<<blocks, 128, smem, s>>>(A);
   GH_CUDA(cudaGetLastError());
   if (fill_ev) record(fill_ev[1]);

@@ -118,13 +118,20 @@ struct Graph {
   int64_t max_label = 0;  // -1: not computed yet (label_max computes it)
   // device
   DeviceIndex dev;
+  std::shared_ptr<struct FillPlan> plan;  // blocks and weights made by the contraction, until the labels are built
   Timings t;
 
   ~Graph() { dev.release(); }
 };
 
+// Where a graph's global order starts: the vertices of the cells at levels
+// C..1 (the tail of elim).
+struct GraphLevels {
+  int heap_start = 0, heap_n = 0;
+};
+
 // Vertex elimination over one or more graphs in one set of launches
-// (contract.cu).  The graphs' vertices are numbered consecutively (graph i
+// (symbolic.cu; contract.cu where the cells are too large for bit rows).  The graphs' vertices are numbered consecutively (graph i
 // starts at vbase[i]); launch s eliminates the cells of level H_i - s of
 // every graph i with H_i - s > C_i, and one last launch runs every graph's
 // global order (levels <= C_i) as one cell per graph.  The list structure
@@ -145,9 +152,28 @@ struct ElimPlan {
     int slice_max;
     int64_t map_off, bar_off;
   };
+  // A launch of symbolic_kernel: cells lo .. lo + ncell of sym_cells, clusters
+  // of cs CTAs with nw warps, rows of up to smax members
+  struct SymLaunch {
+    int step, level, ncell, kmax, smax, npow, cs, nw;
+    bool heap, global;
+    int64_t lo, smem, rows_off;
+  };
+  // What the list kernels' launches need on the device
+  struct ListLaunches {
+    std::vector<int> fcs, fcc, gmap;  // cell starts and counts, block maps
+    int64_t pstage_ints = 0, partial_max = 0;
+  };
   std::vector<Graph *> gs;
   std::vector<int> vbase;
   std::vector<int64_t> mbase;
+  // the order and the lists' ids come from bit rows, the weights from
+  // FillPlan::enqueue_weights; otherwise the list kernels make all three
+  bool bits = false;
+  std::vector<SymLaunch> sym;
+  int *members = nullptr, *extra = nullptr;
+  unsigned char *fin = nullptr, *sym_cells = nullptr;
+  unsigned *grows = nullptr;
   int N = 0, heap_total = 0;
   int64_t M = 0, lub = 0, pool_size = 0;
   std::vector<Launch> launches;  // in step order; launches of one step are independent
@@ -173,8 +199,13 @@ struct ElimPlan {
   unsigned *grid_bar = nullptr;
   int64_t grid_bar_words = 0;
   int64_t bytes = 0;
-  explicit ElimPlan(const std::vector<Graph *> &graphs);
+  explicit ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits = true);
   ~ElimPlan();
+  bool plan_bits();
+  void plan_lists(const int *f_elim, const std::vector<GraphLevels> &L, ListLaunches &LL);
+  void enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace);
+  void gather_bits(cudaStream_t s);
+  int launch_count() const { return (int)(bits ? sym.size() : launches.size()); }
   void release();
   ElimPlan(const ElimPlan &) = delete;
   ElimPlan &operator=(const ElimPlan &) = delete;
@@ -240,6 +271,15 @@ struct FillPlan {
   int64_t *blk_boff = nullptr, *blk_moff = nullptr, *blk_soff = nullptr, *bm_row = nullptr, *task0 = nullptr;
   unsigned char *loc_of = nullptr;
   unsigned *direct = nullptr, *closed = nullptr;
+  int64_t cell_total = 0;
+  // weights from arcs: parent block and the members' places in it, update
+  // triangles, task tables, arrivals a block waits for, each arc's cell
+  const ElimPlan *arcs = nullptr;
+  bool weights_fit = true;  // false: the update triangles would take over half of the free memory
+  int *blk_up = nullptr, *bm_up = nullptr, *wtask_blk = nullptr, *pending = nullptr, *pend_init = nullptr;
+  int64_t *blk_uoff = nullptr, *wtask0 = nullptr, *arc_cell = nullptr;
+  unsigned *upd = nullptr;
+  int64_t wtasks = 0, upd_total = 0;
   unsigned long long *trace_t = nullptr;  // publish time per node (GPUH2H_TRACE)
   int64_t ntasks = 0, tasks_cap = 0;
   int64_t ntiles = 0;  // row pieces: every node of a block once per task of the block
@@ -247,17 +287,23 @@ struct FillPlan {
   size_t smem = 0;
   int nsm = 0;
   int64_t work_bytes = 0;
-  // lists: the graphs' X lists in the same forest numbering.
-  FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, const ListStore &lists);
+  // The blocks and, when `arcs` made the order on bit rows, where each of its
+  // arcs enters the blocks' weights.  lists: the graphs' X lists in the same
+  // forest numbering.
+  FillPlan(const std::vector<Graph *> &graphs, const ListStore &lists, const ElimPlan *arcs);
   ~FillPlan();
   void release_work();
   FillPlan(const FillPlan &) = delete;
   FillPlan &operator=(const FillPlan &) = delete;
   void build_blocks();
+  void build_weights_plan(const ElimPlan &arcs);
+  void prepare(const TilePolicy &pol);  // label rows and tasks
   void build_tiles(const TilePolicy &pol);
   std::vector<int> level_classes() const;  // TilePolicy class per forest level
-  // Gathers the shortcut weights of the pos entries from the lists, resets
-  // the flags, closes the blocks' weights and runs the fill on s.
+  // The shortcut weights of every list and block on s: eliminated block by
+  // block from the arcs' current weights, or gathered from the lists.
+  void enqueue_weights(cudaStream_t s);
+  // Resets the flags and runs the fill on s.
   void enqueue(cudaStream_t s, cudaEvent_t *fill_ev = nullptr);
   void check_error();            // synchronises; throws if a dependency wait ran out
   void trace_report();           // GPUH2H_TRACE: the last fill's time per level class
@@ -271,7 +317,9 @@ void load_graph(Graph &g, const std::string &edge, const std::string &idf, const
 void build_elimination_sets(const std::vector<Graph *> &gs);
 // contract.cu: partition levels H..C+1 and the global heap over levels <= C;
 // fills g.elim (elimination order) and g.x_off / x_id / x_w
+// contraction (then the tree, sparse table and weights of one graph)
 void contract_gpu(Graph &g);
+void position_offsets(Graph &g);                       // tree.cpp: pos_hash
 void build_tree(Graph &g);                             // tree.cpp: father, children, Euler tour
 // tree_gpu.cu: the same on the GPU, plus the level order, heavy paths and
 // root-path segment offsets (sets g.tree_layout)

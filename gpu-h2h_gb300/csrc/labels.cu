@@ -349,8 +349,8 @@ bool TilePolicy::parse(const std::string &text) {
   return true;
 }
 
-FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, const ListStore &lst)
-    : gs(graphs), policy(pol), lists(lst) {
+FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, const ElimPlan *from)
+    : gs(graphs), lists(lst) {
   const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
   Clock tclk;
   auto mark = [&](const char *what) {
@@ -456,7 +456,6 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
   pos_id = st->alloc<int>(pos_total);
   father = st->alloc<int>(N);
   depth = st->alloc<int>(N);
-  dis = st->alloc<int>(dis_total);
   try {
     pos_w = dalloc<int>(pos_total, work_bytes);
     pos_src = dalloc<int>(pos_total, work_bytes);
@@ -499,8 +498,10 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
     mark("root-path segments");
     build_blocks();
     mark("blocks");
-    build_tiles(pol);
-    mark("tasks");
+    if (from && from->bits) {
+      build_weights_plan(*from);
+      mark("weights plan");
+    }
   } catch (...) {
     release_work();
     throw;
@@ -509,17 +510,25 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const TilePolicy &pol, co
 
 FillPlan::~FillPlan() { release_work(); }
 
+void FillPlan::prepare(const TilePolicy &pol) {
+  dis = static_cast<DevArrays *>(storage.get())->alloc<int>(dis_total);
+  build_tiles(pol);
+}
+
 void FillPlan::release_work() {
   void *ps[] = {pos_w,    pos_src,  hld,      htop,  hpos,   seg_off, seg_top, seg_pos, done,   next,   err,    tasks,   trace_t,
                 hld_row,  blk_top,  blk_mem,  blk_boff, blk_moff, blk_soff, bnode, blk_of, loc_of, lvl_cls, bm_p, bm_row,
-                direct,   closed,   task0,    tcols};
+                direct,   closed,   task0,    tcols,  blk_up, bm_up,   wtask_blk, pending, pend_init, blk_uoff, wtask0,
+                arc_cell, upd};
   for (void *p : ps) cudaFree(p);
   trace_t = nullptr;
   pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = tasks = nullptr;
   blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;
   hld_row = seg_off = blk_boff = blk_moff = blk_soff = bm_row = task0 = nullptr;
   loc_of = nullptr;
-  direct = closed = nullptr;
+  direct = closed = upd = nullptr;
+  blk_up = bm_up = wtask_blk = pending = pend_init = nullptr;
+  blk_uoff = wtask0 = arc_cell = nullptr;
 }
 
 // With GPUH2H_TRACE: where the last fill's time went, from the nodes'
@@ -711,7 +720,12 @@ void fill_labels_gpu(Graph &g) {
     TilePolicy pol = TilePolicy();
     if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
       GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
-    FillPlan plan({&g}, pol, D.lists);
+    if (!g.plan) {  // contracted by the list kernels
+      g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, D.lists, nullptr);
+      g.plan->enqueue_weights(0);
+    }
+    FillPlan &plan = *g.plan;
+    plan.prepare(pol);
     GH_CUDA(cudaDeviceSynchronize());
     g.t.translate_labels = clk.us();
     clk.reset();
@@ -734,10 +748,11 @@ void fill_labels_gpu(Graph &g) {
     g.t.fill_gpu = (long long)(ms * 1000.0f);
     Clock tail;  // the per-graph view and the plan's work buffers count with the plan's host time
     plan.attach(true);
-    plan.release_work();
+    g.plan.reset();
     g.t.translate_labels += tail.us();
     return;
   }
+  g.plan.reset();
   D.release_labels();
   D.n = n;
   D.pos_base = 0;

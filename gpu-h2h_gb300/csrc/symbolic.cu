@@ -1,0 +1,726 @@
+// symbolic.cu -- the elimination order and the upper neighbours X(v)\{v} of
+// every vertex, without weights: the same eliminations as contract.cu's list
+// kernels (makeCHPerHeight_2 / makeCHPerHeight_D_2, kernel_functions.cu:
+// 309-553, and TDInCPU / CHUsingHeap_2, Traditional_H2H.cu:6-118, :216-351),
+// on neighbour sets.
+//
+// Which vertex is eliminated next depends on degrees and heights alone, never
+// on weights, and a list's order and weights reach no later pick.  So a cell
+// keeps, for each of its alive members (candidates and the boundary that
+// stays), the set of its neighbours inside the cell as a bit row over the
+// members in id order, and what the reference's list lengths count besides:
+// entries outside the cell, repeated entries of parallel arcs, the junk
+// prefix a list keeps when every valid entry vanished (kernel_functions.cu:
+// 353-360, :381-388).  Eliminating v is row(u) |= row(v) for every u in
+// row(v), minus u and v; the degree is a population count.  An elimination
+// that rebuilds weighted lists took 10-32 us (merge walks of dependent loads
+// and a grid barrier); on bit rows in shared memory it is a block argmin and
+// a few word operations per neighbour.  The weights are computed afterwards,
+// for all vertices, over the blocks of the finished tree (fill_blocks.cu).
+// On one GB300, order and weights together against the list kernels: 42 ->
+// 14 ms on a 264k-vertex road graph (global order 18.8 -> 3.4 ms, 2.1 us a
+// pick), 127 -> 31 ms on a 1M-vertex one (45.9 -> 7.9 ms), 27 -> 3.2 ms for a
+// rebuild of 16 graphs after new weights, which repeats no elimination.
+// Bound: the chain of picks; a pick is an argmin, two to four barriers and one
+// pass over the neighbours' rows.
+//
+// One thread-block cluster per cell; member l's row, counters and key belong
+// to CTA l mod CS.  Per elimination: every CTA's best key (degree + height,
+// degree, id -- packed, members being numbered in id order) goes to all CTAs
+// through distributed shared memory, one cluster barrier, then each CTA copies
+// v's row from its owner and updates the rows it owns, a warp per row.
+//
+// Rules kept from the reference: a cell's first pick uses the stale keys
+// (input degree, height 0), later picks live ones (kernel_functions.cu:462-476);
+// a neighbour's height becomes max(height, HeightNow + 1); the global order
+// starts with live keys that still count repeated entries, then drops them
+// (unordered_map::emplace).
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+
+#include "graph.h"
+
+namespace cg = cooperative_groups;
+
+namespace gh {
+
+namespace {
+
+constexpr int kErrOverflow = 1;  // a list outgrew its capacity
+constexpr int kErrEmpty = 2;     // eliminated a vertex without neighbours
+constexpr int kErrPick = 5;      // no candidate left to pick, or a vertex outside its cell
+
+constexpr int kIdxBits = 14, kDegBits = 22, kSumBits = 28;  // a key: degree + height, degree, member
+constexpr int kMaxMembers = 1 << kIdxBits;
+constexpr unsigned long long kNoKey = ~0ull;
+
+struct SymCell {
+  int start, count, size, src;  // candidates in elim; members; slot buffer its lists are read from
+  int64_t mem, out;             // members; where the ones that stay go (the parent's members)
+};
+
+struct SymArgs {
+  const SymCell *cells;
+  int *slot[2];
+  int64_t *slot_off;
+  int *lsize, *ljunk, *extra, *height, *elim, *members, *err;
+  const int *cap, *deg0, *adj_off, *adj_v;
+  unsigned *grows;  // rows in global memory (kGlobal)
+  unsigned long long *pool_next;
+  int64_t pool_size;
+  unsigned char *fin;  // the slot buffer a vertex's list ended in
+  int smax, npow, heap;
+};
+
+__device__ __forceinline__ unsigned long long pack_key(int deg, int height, int l) {
+  return ((unsigned long long)(deg + height) << (kIdxBits + kDegBits)) | ((unsigned long long)deg << kIdxBits) |
+         (unsigned)l;
+}
+
+__device__ __forceinline__ int find_id(const int *ids, int n, int x) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ids[mid] < x) lo = mid + 1; else hi = mid;
+  }
+  return lo < n && ids[lo] == x ? lo : -1;
+}
+
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long k) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, k, o);
+    k = y < k ? y : k;
+  }
+  return k;
+}
+
+template <bool kGlobal>
+__global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned long long s_wmin[2][16];
+  __shared__ unsigned long long s_best[2][16];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int CS = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int ci = (int)(blockIdx.x / CS);
+  const SymCell c = A.cells[ci];
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
+  const int S = c.size, k = c.count, W = (S + 31) >> 5;
+  if (S == 0) return;  // uniform across the cluster
+  const int ownmax = (A.smax + CS - 1) / CS, Wm = ((A.smax + 31) >> 5) | 1;  // odd row stride: no bank conflicts
+  const int nown = (S - rank + CS - 1) / CS;
+  unsigned long long *key = (unsigned long long *)smem;
+  int *ids = (int *)(key + ownmax);
+  int *vc = ids + A.npow;   // neighbours inside the cell
+  int *outc = vc + ownmax;  // entries outside it
+  int *ext = outc + ownmax; // repeated entries
+  int *junk = ext + ownmax;
+  int *hgt = junk + ownmax;
+  int *cap = hgt + ownmax;  // list capacity (partition cells)
+  unsigned *rowv = (unsigned *)(cap + ownmax);
+  unsigned *cand = rowv + Wm;
+  unsigned *srows = cand + Wm;
+  unsigned *const grows = kGlobal ? A.grows + (int64_t)ci * A.smax * Wm : nullptr;
+  auto own_row = [&](int r) -> unsigned * {
+    return kGlobal ? grows + (int64_t)(r * CS + rank) * Wm : srows + (int64_t)r * Wm;
+  };
+  // ---- members in id order
+  int np2 = 1;
+  while (np2 < S) np2 <<= 1;
+  for (int i = tid; i < np2; i += nthr) ids[i] = i < S ? A.members[c.mem + i] : INT_MAX;
+  for (int i = tid; i < W; i += nthr) cand[i] = 0;
+  __syncthreads();
+  for (int kk = 2; kk <= np2; kk <<= 1)
+    for (int j = kk >> 1; j > 0; j >>= 1) {
+      for (int t = tid; t < np2 >> 1; t += nthr) {
+        const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), p = i | j;
+        const int x = ids[i], y = ids[p];
+        if ((x > y) == ((i & kk) == 0)) {
+          ids[i] = y;
+          ids[p] = x;
+        }
+      }
+      __syncthreads();
+    }
+  for (int i = tid; i < k; i += nthr) {
+    const int l = find_id(ids, S, A.elim[c.start + i]);
+    if (l >= 0) atomicOr(cand + (l >> 5), 1u << (l & 31));
+    else atomicCAS(A.err, 0, kErrPick);
+  }
+  __syncthreads();
+  // ---- rows and counters of the owned members, a warp per member
+  for (int r = wid; r < nown; r += nw) {
+    const int l = r * CS + rank, u = ids[l];
+    unsigned *row = own_row(r);
+    for (int w = lane; w < W; w += 32) row[w] = 0;
+    __syncwarp();
+    const int64_t off = A.slot_off[u];
+    const int n = A.lsize[u];
+    const int *list = A.slot[c.src] + off;
+    int out = 0;
+    for (int e = lane; e < n; e += 32) {
+      const int x = find_id(ids, S, __ldcg(list + e));
+      if (x >= 0) atomicOr(row + (x >> 5), 1u << (x & 31));
+      else out++;
+    }
+    out = __reduce_add_sync(0xffffffffu, out);
+    if (lane == 0) {
+      const int ex = A.extra[u], J = A.ljunk[u], h = A.height[u], in = n - out;
+      vc[r] = in;
+      outc[r] = out;
+      hgt[r] = h;
+      cap[r] = A.heap ? INT_MAX : A.cap[u];
+      ext[r] = A.heap ? 0 : ex;
+      junk[r] = A.heap ? 0 : J;
+      unsigned long long kk = kNoKey;
+      if ((cand[l >> 5] >> (l & 31)) & 1u) kk = A.heap ? pack_key(n + ex, h, l) : pack_key(A.deg0[u], 0, l);
+      key[r] = kk;
+    }
+  }
+  __syncthreads();
+  if (CS > 1) cluster.sync();
+  // Two ways through v's neighbours.  Few of them: a warp takes its rows one
+  // at a time, a lane per word (the rows of a warp are G apart: neighbours
+  // have close ids).  Many: T lanes take a row, 32 / T rows at once, so the
+  // cost is the rows' words and not their number.  The second way pays from
+  // about dense_deg neighbours (60 cycles a row against 10 a word).
+  const int G = max(nw, (nown + 31) >> 5);
+  int T = 1;
+  while (T < 8 && 2 * T * nown <= nthr) T <<= 1;
+  const int per = 32 / T, rounds = (nown + per * nw - 1) / (per * nw);
+  const int dense_deg = kGlobal ? INT_MAX : max(4, rounds * (W / T + 4) * nw * CS / 6);
+  // the counters of owned member r after its row became pc neighbours
+  auto settle = [&](int r, int pc, int lv, int hnow) {
+    const int l = r * CS + rank;
+    int ex = ext[r], mult = 1;  // entries of v in the list
+    const int valid = vc[r] + outc[r] + ex;
+    if (ex > 0) {
+      const int u = ids[l], v = ids[lv];
+      mult = 0;
+      for (int e = A.adj_off[u]; e < A.adj_off[u + 1]; e++) mult += A.adj_v[e] == v;
+      mult = max(1, mult);
+      ex -= mult - 1;
+      ext[r] = ex;
+    }
+    int J = junk[r];
+    J = valid - mult > 0 || A.heap ? 0 : J + valid;  // nothing valid left: the stale size stays as junk
+    const int size = J + pc + outc[r] + ex;
+    const int h = max(hgt[r], hnow + 1);
+    vc[r] = pc;
+    junk[r] = J;
+    hgt[r] = h;
+    if (key[r] != kNoKey) key[r] = pack_key(size, h, l);
+    if (size > cap[r]) atomicCAS(A.err, 0, kErrOverflow);
+  };
+  for (int j = 0; j < k; j++) {
+    const int par = j & 1;
+    // ---- the pick
+    unsigned long long b = kNoKey;
+    for (int r = tid; r < nown; r += nthr) {
+      const unsigned long long x = key[r];
+      b = x < b ? x : b;
+    }
+    b = warp_min(b);
+    if (lane == 0) s_wmin[par][wid] = b;
+    __syncthreads();
+    if (CS == 1) {
+      b = warp_min(lane < nw ? s_wmin[par][lane] : kNoKey);
+    } else {
+      if (wid == 0) {
+        b = warp_min(lane < nw ? s_wmin[par][lane] : kNoKey);
+        if (lane < CS) *cluster.map_shared_rank(&s_best[par][rank], lane) = b;
+      }
+      cluster.sync();
+      b = warp_min(lane < CS ? s_best[par][lane] : kNoKey);
+    }
+    if (b == kNoKey) {  // the same in every CTA of the cluster
+      if (rank == 0 && tid == 0) atomicCAS(A.err, 0, kErrPick);
+      break;
+    }
+    const int lv = (int)(b & (kMaxMembers - 1));
+    const int hnow = (int)(b >> (kIdxBits + kDegBits)) - (int)((b >> kIdxBits) & ((1u << kDegBits) - 1));
+    const int owner = lv % CS;
+    const unsigned *rv;
+    if (CS == 1 && !kGlobal) {
+      rv = own_row(lv);
+    } else {
+      const unsigned *src = kGlobal ? grows + (int64_t)lv * Wm
+                                    : cluster.map_shared_rank(srows, owner) + (int64_t)(lv / CS) * Wm;
+      for (int w = tid; w < W; w += nthr) rowv[w] = kGlobal ? __ldcg(src + w) : src[w];
+      __syncthreads();
+      rv = rowv;
+    }
+    // ---- its neighbours among the owned members
+    if ((int)((b >> kIdxBits) & ((1u << kDegBits) - 1)) < dense_deg) {
+      for (int g = wid; g < G; g += nw) {
+        const int r0 = lane * G + g, l0 = r0 * CS + rank;
+        const bool hit = r0 < nown && ((rv[l0 >> 5] >> (l0 & 31)) & 1u);
+        unsigned todo = __ballot_sync(0xffffffffu, hit);
+        int mine = 0;
+        while (todo) {
+          const int at = __ffs(todo) - 1, r = at * G + g, l = r * CS + rank;
+          todo &= todo - 1;
+          unsigned *row = own_row(r);
+          int pc = 0;
+          for (int w = lane; w < W; w += 32) {
+            unsigned x = (kGlobal ? __ldcg(row + w) : row[w]) | rv[w];
+            if (w == (l >> 5)) x &= ~(1u << (l & 31));
+            if (w == (lv >> 5)) x &= ~(1u << (lv & 31));
+            row[w] = x;
+            pc += __popc(x);
+          }
+          pc = __reduce_add_sync(0xffffffffu, pc);
+          if (lane == at) mine = pc;
+        }
+        if (hit) settle(r0, mine, lv, hnow);
+      }
+    } else {
+      const int sub = lane & (T - 1);
+      for (int g = wid; g * per < nown; g += nw) {
+        const int r = g * per + lane / T, l = r * CS + rank;
+        const bool hit = r < nown && ((rv[l >> 5] >> (l & 31)) & 1u);
+        int pc = 0;
+        if (hit) {
+          unsigned *row = own_row(r);
+          for (int w = sub; w < W; w += T) {
+            unsigned x = row[w] | rv[w];
+            if (w == (l >> 5)) x &= ~(1u << (l & 31));
+            if (w == (lv >> 5)) x &= ~(1u << (lv & 31));
+            row[w] = x;
+            pc += __popc(x);
+          }
+        }
+        for (int o = 1; o < T; o <<= 1) pc += __shfl_xor_sync(0xffffffffu, pc, o);
+        if (hit && sub == 0) settle(r, pc, lv, hnow);
+      }
+    }
+    if (rank == owner && tid == 0) {
+      key[lv / CS] = kNoKey;
+      A.elim[c.start + j] = ids[lv];
+      if (vc[lv / CS] == 0 && !A.heap) atomicCAS(A.err, 0, kErrEmpty);  // a partition cell never isolates a candidate
+    }
+    __syncthreads();
+    if (j == 0 && !A.heap) {  // live keys from the second pick on
+      for (int r = tid; r < nown; r += nthr)
+        if (key[r] != kNoKey) key[r] = pack_key(junk[r] + vc[r] + outc[r] + ext[r], hgt[r], r * CS + rank);
+      __syncthreads();
+    }
+  }
+  // ---- lists: an eliminated member's row is its X in id order, a boundary
+  // member's new list is its row, then its entries outside the cell
+  for (int r = wid; r < nown; r += nw) {
+    const int l = r * CS + rank, u = ids[l];
+    const bool gone = (cand[l >> 5] >> (l & 31)) & 1u;
+    const int in = vc[r], len = in + outc[r];
+    int64_t off = A.slot_off[u];
+    const int64_t old = off;
+    const int cap = A.cap[u], n0 = A.lsize[u];
+    if (A.heap && len > cap) {  // a global-order list may outgrow its range
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(A.pool_next, (unsigned long long)len);
+      off = (int64_t)__shfl_sync(0xffffffffu, at, 0);
+    }
+    const bool fits = A.heap ? off + len <= A.pool_size : len <= cap;
+    if (fits) {
+      int *dst = A.slot[c.src ^ 1] + off;
+      const unsigned *row = own_row(r);
+      int base = 0;
+      for (int w0 = 0; w0 < W; w0 += 32) {
+        const int w = w0 + lane;
+        unsigned x = w < W ? (kGlobal ? __ldcg(row + w) : row[w]) : 0u;
+        const int pc = __popc(x);
+        int incl = pc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        int at = base + incl - pc;
+        while (x) {
+          const int bit = __ffs(x) - 1;
+          x &= x - 1;
+          dst[at++] = ids[w * 32 + bit];
+        }
+        base += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (len > in) {
+        const int *list = A.slot[c.src] + old;
+        int q = in;
+        for (int e0 = 0; e0 < n0; e0 += 32) {
+          const int x = e0 + lane < n0 ? __ldcg(list + e0 + lane) : -1;
+          const bool out = x >= 0 && find_id(ids, S, x) < 0;
+          const unsigned bal = __ballot_sync(0xffffffffu, out);
+          if (out) dst[q + __popc(bal & ((1u << lane) - 1u))] = x;
+          q += __popc(bal);
+        }
+      }
+    }
+    if (lane == 0) {
+      if (!fits) atomicCAS(A.err, 0, kErrOverflow);
+      A.slot_off[u] = off;
+      A.lsize[u] = fits ? len : 0;
+      A.ljunk[u] = gone ? 0 : junk[r];
+      A.extra[u] = ext[r];
+      A.height[u] = hgt[r];
+      A.fin[u] = (unsigned char)(c.src ^ 1);
+    }
+  }
+  if (rank == 0 && wid == 0 && c.out >= 0) {
+    int q = 0;
+    for (int l0 = 0; l0 < S; l0 += 32) {
+      const int l = l0 + lane;
+      const bool stay = l < S && !((cand[l >> 5] >> (l & 31)) & 1u);
+      const unsigned bal = __ballot_sync(0xffffffffu, stay);
+      if (stay) A.members[c.out + q + __popc(bal & ((1u << lane) - 1u))] = ids[l];
+      q += __popc(bal);
+    }
+  }
+  if (CS > 1) cluster.sync();  // no CTA leaves while a peer may still read its rows
+}
+
+// Distinct neighbours of every vertex's input list (in id order) and the
+// number of repeated entries.
+__global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, const int64_t *slot_off, int *slot,
+                                      int *lsize, int *extra, int n) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    int *list = slot + slot_off[v];
+    const int b = adj_off[v], e = adj_off[v + 1];
+    int c = 0;
+    for (int i = b; i < e; i++) {
+      const int x = adj_v[i];
+      int k = c;
+      while (k > 0 && list[k - 1] > x) k--;
+      if (k > 0 && list[k - 1] == x) continue;
+      for (int q = c; q > k; q--) list[q] = list[q - 1];
+      list[k] = x;
+      c++;
+    }
+    lsize[v] = c;
+    extra[v] = e - b - c;
+  }
+}
+
+// The final lists from whichever slot buffer each ended in.  One warp per vertex.
+__global__ void gather_ids_kernel(const int64_t *slot_off, const int *lsize, const unsigned char *fin, const int *slot0,
+                                  const int *slot1, const int64_t *out_off, int *out_nbr, int n) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
+       v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
+    const int *src = (fin[v] ? slot1 : slot0) + slot_off[v];
+    const int64_t oo = out_off[v];
+    const int s = lsize[v];
+    for (int i = lane; i < s; i += 32) out_nbr[oo + i] = src[i];
+  }
+}
+
+template <typename T>
+T *palloc(size_t n, int64_t &bytes) {
+  T *p = nullptr;
+  if (n == 0) n = 1;
+  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  bytes += (int64_t)(n * sizeof(T));
+  return p;
+}
+
+// Alive members of every cell at its level, or false when the cut rows do not
+// nest (each level tiling the positions, a cell split by its two children).
+bool cell_sizes(const Graph &g, std::vector<int> &size) {
+  const int64_t cells = (int64_t(1) << g.H) - 1;
+  size.assign(cells, 0);
+  if (g.cut_l[0] != 0 || g.cut_r[0] != g.n) return false;
+  const int64_t inner = (int64_t(1) << (g.H - 1)) - 1;
+  for (int64_t c = 0; c < inner; c++)
+    if (g.cut_l[2 * c + 1] != g.cut_l[c] || g.cut_r[2 * c + 1] != g.cut_l[2 * c + 2] ||
+        g.cut_r[2 * c + 2] != g.cut_r[c])
+      return false;
+  for (int64_t c = cells - 1; c >= 0; c--) {
+    size[c] = c >= inner ? g.cut_r[c] - g.cut_l[c]
+                         : size[2 * c + 1] - g.cell_count[2 * c + 1] + size[2 * c + 2] - g.cell_count[2 * c + 2];
+    if (size[c] < g.cell_count[c]) return false;
+  }
+  return true;
+}
+
+}  // namespace
+
+// Lays out the elimination on bit rows, if every cell's members fit a row
+// (up to 16,384) and the partition nests.  False: the list kernels run, as
+// they also do when one of their switches is set.  A 16,384-member cell takes
+// 32 MB of rows and about 10 us a pick; past that, sparse lists are the
+// smaller working set (a global order over a whole 264k-vertex graph would
+// scan 33 KB per row).
+bool ElimPlan::plan_bits() {
+  for (const char *e : {"GPUH2H_CLUSTER_HEAP", "GPUH2H_GRID_CELLS", "GPUH2H_GLOBAL_STAGING", "GPUH2H_GRID_ARENA",
+                        "GPUH2H_ELIM_BALANCE", "GPUH2H_LIST_ELIM"})
+    if (std::getenv(e)) return false;
+  const int K = (int)gs.size();
+  if (N >= (1 << (kSumBits - 2))) return false;
+  struct Host {
+    SymCell c;
+    int level;
+  };
+  std::vector<std::vector<Host>> steps;
+  std::vector<std::vector<int>> sizes(K);
+  int nsteps = 0;
+  for (int i = 0; i < K; i++) {
+    if (!cell_sizes(*gs[i], sizes[i])) return false;
+    for (int x : gs[i]->cap)
+      if (x >= (1 << (kDegBits - 1))) return false;
+    nsteps = std::max(nsteps, gs[i]->H - gs[i]->C);
+  }
+  steps.resize(nsteps + 1);
+  std::vector<int> f_members(N);  // the bottom cells' members come first, in partition order
+  int64_t mem = N;
+  for (int i = 0; i < K; i++) {
+    const Graph &g = *gs[i];
+    const int vb = vbase[i], levels = g.H - g.C;
+    for (int q = 0; q < g.n; q++) f_members[vb + q] = (levels > 0 ? g.part_ids[q] : q) + vb;
+    std::vector<int64_t> region(sizes[i].size(), -1);
+    int64_t heap_region = levels > 0 ? -1 : vb;
+    int heap_n = 0;
+    for (int64_t c = 0; c < (int64_t)sizes[i].size() && c < (int64_t(1) << g.C) - 1; c++) heap_n += g.cell_count[c];
+    if (heap_n > kMaxMembers) return false;
+    if (levels > 0) {
+      heap_region = mem;
+      mem += heap_n;
+    }
+    int64_t heap_at = heap_region;
+    for (int h = g.H; h > g.C; h--) {
+      const int64_t lo = (int64_t(1) << (h - 1)) - 1, hi = (int64_t(1) << h) - 2;
+      for (int64_t c = lo; c <= hi; c++) {
+        if (sizes[i][c] > kMaxMembers) return false;
+        if (h == g.H) region[c] = vb + g.cut_l[c];
+        const int stay = sizes[i][c] - g.cell_count[c];
+        int64_t out;
+        if (h - 1 > g.C) {
+          const int64_t p = (c - 1) / 2;
+          if (region[p] < 0) {
+            region[p] = mem;
+            mem += sizes[i][p];
+          }
+          out = region[p] + (c & 1 ? 0 : sizes[i][c - 1] - g.cell_count[c - 1]);
+        } else {
+          out = heap_at;
+          heap_at += stay;
+        }
+        const int st = g.H - h;
+        steps[st].push_back({{vb + g.cell_start[c], g.cell_count[c], sizes[i][c], st & 1, region[c], out},
+                             K > 1 ? -(st + 1) : h});
+      }
+    }
+    if (levels > 0 && heap_at != heap_region + heap_n) return false;
+    int heap_start = g.n - heap_n;
+    steps[nsteps].push_back({{vb + heap_start, heap_n, heap_n, levels & 1, heap_region, -1}, 0});
+  }
+  // ---- launches: a step's cells by size class, each class with its own
+  // cluster size.  A pick costs a fixed part (argmin and barriers: about 0.5
+  // us in one CTA, 1.2 us across a cluster) and its neighbours' rows, which a
+  // cluster shares.
+  cudaFuncAttributes fa;
+  GH_CUDA(cudaFuncGetAttributes(&fa, symbolic_kernel<false>));
+  const int smem_dyn = enable_max_dynamic_smem(symbolic_kernel<false>);
+  enable_max_dynamic_smem(symbolic_kernel<true>);
+  GH_CUDA(cudaFuncSetAttribute(symbolic_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  GH_CUDA(cudaFuncSetAttribute(symbolic_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  int dev = 0;
+  GH_CUDA(cudaGetDevice(&dev));
+  GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  auto pow2 = [](int x) {
+    int p = 1;
+    while (p < x) p <<= 1;
+    return p;
+  };
+  auto smem_for = [&](int smax, int cs, bool global) -> int64_t {
+    const int64_t own = (smax + cs - 1) / cs, w = (smax + 31) / 32 | 1;
+    return own * (8 + 24) + 4LL * pow2(smax) + 8 * w + (global ? 0 : 4 * own * w);
+  };
+  std::vector<SymCell> table;
+  int64_t grow_words = 0;
+  for (int st = 0; st <= nsteps; st++) {
+    std::vector<Host> &cells = steps[st];
+    std::stable_sort(cells.begin(), cells.end(), [](const Host &a, const Host &b) { return a.c.size > b.c.size; });
+    int64_t step_words = 0;
+    for (size_t g0 = 0; g0 < cells.size();) {
+      if (cells[g0].c.size == 0) break;  // only empty cells are left
+      const int smax = cells[g0].c.size;
+      size_t g1 = g0;
+      while (g1 < cells.size() && cells[g1].c.size * 3 > smax * 2) g1++;  // within a third of the largest
+      SymLaunch L{};
+      L.step = st;
+      L.level = cells[g0].level;
+      L.heap = st == nsteps;
+      L.lo = (int64_t)table.size();
+      L.ncell = (int)(g1 - g0);
+      L.smax = smax;
+      L.npow = pow2(smax);
+      L.kmax = 0;
+      for (size_t c = g0; c < g1; c++) {
+        table.push_back(cells[c].c);
+        L.kmax = std::max(L.kmax, cells[c].c.count);
+      }
+      double best = 1e300;
+      for (int global = 0; global < 2 && best > 1e299; global++)  // rows in global memory only where nothing else fits
+        for (int cs = 1; cs <= 16; cs <<= 1) {
+          const int64_t sm = smem_for(smax, cs, global);
+          if (sm > smem_dyn || (global && cs < 16)) continue;
+          const int own = (smax + cs - 1) / cs, w = (smax + 31) / 32;
+          const int nw = own >= 400 || (cs > 1 && own >= 64) ? 16 : own >= 96 ? 8 : 4;
+          int fit = 0;
+          cudaLaunchConfig_t cfg = {};
+          cudaLaunchAttribute attr[1];
+          attr[0].id = cudaLaunchAttributeClusterDimension;
+          attr[0].val.clusterDim.x = cs;
+          attr[0].val.clusterDim.y = 1;
+          attr[0].val.clusterDim.z = 1;
+          cfg.attrs = attr;
+          cfg.numAttrs = 1;
+          cfg.blockDim = dim3(nw * 32);
+          cfg.dynamicSmemBytes = (size_t)sm;
+          cfg.gridDim = dim3(L.ncell * cs);
+          const cudaError_t e = global ? cudaOccupancyMaxActiveClusters(&fit, symbolic_kernel<true>, &cfg)
+                                       : cudaOccupancyMaxActiveClusters(&fit, symbolic_kernel<false>, &cfg);
+          if (e != cudaSuccess || fit < 1) {
+            cudaGetLastError();
+            continue;
+          }
+          const double waves = std::ceil((double)L.ncell / fit);
+          const double words = 0.4 * own * w / (32.0 * nw);  // a lane's words per pick
+          const double cost = waves * ((cs == 1 ? 0.6 : 1.8) + 0.01 * words);
+          if (cost < best * 0.99) {
+            best = cost;
+            L.cs = cs;
+            L.nw = nw;
+            L.smem = sm;
+            L.global = global != 0;
+          }
+        }
+      if (best > 1e299) return false;
+      if (L.global) {
+        L.rows_off = step_words;
+        step_words += (int64_t)L.ncell * smax * ((smax + 31) / 32 | 1);
+      }
+      sym.push_back(L);
+      g0 = g1;
+    }
+    grow_words = std::max(grow_words, step_words);
+  }
+  max_group = 1;
+  for (size_t i = 0; i < sym.size();) {
+    size_t j = i;
+    while (j < sym.size() && sym[j].step == sym[i].step) j++;
+    max_group = std::max(max_group, (int)(j - i));
+    i = j;
+  }
+  try {
+    members = palloc<int>(mem, bytes);
+    extra = palloc<int>(N, bytes);
+    fin = palloc<unsigned char>(N, bytes);
+    sym_cells = palloc<unsigned char>(sizeof(SymCell) * table.size(), bytes);
+    if (grow_words) grows = palloc<unsigned>(grow_words, bytes);
+    GH_CUDA(cudaMemcpy(members, f_members.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(sym_cells, table.data(), sizeof(SymCell) * table.size(), cudaMemcpyHostToDevice));
+  } catch (...) {
+    release();
+    throw;
+  }
+  return true;
+}
+
+void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
+  GH_CUDA(cudaMemcpyAsync(slot_off, slot_off_init, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice, s));
+  GH_CUDA(cudaMemcpyAsync(elim, elim_init, sizeof(int) * N, cudaMemcpyDeviceToDevice, s));
+  GH_CUDA(cudaMemcpyAsync(pool_next, pool_first, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
+  GH_CUDA(cudaMemsetAsync(height, 0, sizeof(int) * N, s));
+  GH_CUDA(cudaMemsetAsync(ljunk, 0, sizeof(int) * N, s));
+  GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  distinct_lists_kernel<<<std::max(1, std::min(4096, (N + 255) / 256)), 256, 0, s>>>(adj_off, adj_v, slot_off, slot_nbr,
+                                                                                     lsize, extra, N);
+  GH_CUDA(cudaGetLastError());
+  auto launch = [&](const SymLaunch &L, cudaStream_t ls) {
+    SymArgs A{};
+    A.cells = reinterpret_cast<const SymCell *>(sym_cells) + L.lo;
+    A.slot[0] = slot_nbr;
+    A.slot[1] = slot_w;
+    A.slot_off = slot_off;
+    A.lsize = lsize;
+    A.ljunk = ljunk;
+    A.extra = extra;
+    A.height = height;
+    A.elim = elim;
+    A.members = members;
+    A.err = err;
+    A.cap = cap_init;
+    A.deg0 = deg_init;
+    A.adj_off = adj_off;
+    A.adj_v = adj_v;
+    A.grows = L.global ? grows + L.rows_off : nullptr;
+    A.pool_next = pool_next;
+    A.pool_size = pool_size;
+    A.fin = fin;
+    A.smax = L.smax;
+    A.npow = L.npow;
+    A.heap = L.heap;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = L.cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(L.nw * 32);
+    cfg.dynamicSmemBytes = (size_t)L.smem;
+    cfg.gridDim = dim3(L.ncell * L.cs);
+    cfg.stream = ls;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    if (trace) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, ls); }
+    if (L.global) GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<true>, A));
+    else GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<false>, A));
+    if (trace) {
+      cudaEventRecord(e1, ls);
+      cudaEventSynchronize(e1);
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      std::fprintf(stderr, "[gpuh2h] elim bits %s %d: %d cells x %d CTAs x %d warps, kmax %d, members %d, smem %lld%s: %.3f ms\n",
+                   L.heap ? "heap" : "level", L.level, L.ncell, L.cs, L.nw, L.kmax, L.smax, (long long)L.smem,
+                   L.global ? " (rows in global memory)" : "", ms);
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+    }
+  };
+  for (size_t li = 0; li < sym.size();) {
+    size_t lj = li;
+    while (lj < sym.size() && sym[lj].step == sym[li].step) lj++;
+    if (sym[li].heap && heap_ev) GH_CUDA(cudaEventRecord(heap_ev[0], s));
+    if (lj - li > 1) GH_CUDA(cudaEventRecord(ev_fork, s));
+    for (size_t k = li; k < lj; k++) {
+      cudaStream_t ls = s;
+      if (k > li) {
+        ls = side[k - li - 1];
+        GH_CUDA(cudaStreamWaitEvent(ls, ev_fork, 0));
+      }
+      launch(sym[k], ls);
+      if (k > li) GH_CUDA(cudaEventRecord(ev_join[k - li - 1], ls));
+    }
+    for (size_t k = li + 1; k < lj; k++) GH_CUDA(cudaStreamWaitEvent(s, ev_join[k - li - 1], 0));
+    li = lj;
+  }
+  if (heap_ev) {
+    if (sym.empty() || !sym.back().heap) GH_CUDA(cudaEventRecord(heap_ev[0], s));
+    GH_CUDA(cudaEventRecord(heap_ev[1], s));
+  }
+}
+
+void ElimPlan::gather_bits(cudaStream_t s) {
+  gather_ids_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256, 0, s>>>(
+      slot_off, lsize, fin, slot_nbr, slot_w, lists.off, lists.id, N);
+  GH_CUDA(cudaGetLastError());
+}
+
+}  // namespace gh
