@@ -26,8 +26,11 @@
 // A fill that takes a warp per (node, column block, separator chunk) tile is
 // bound by one L2 load per update and 13 us per tree level of the narrow top.
 // On one GB300 the blocks took the fill of a 264k-vertex road graph (4.5e9
-// updates) from 28.4 to 4.7 ms and of a 1M-vertex one (3.8e10) from 104 to
-// 18.9 ms.
+// updates) from 28.4 to 3.7 ms and of a 1M-vertex one (3.8e10) from 104 to
+// 14.9 ms.  Narrow levels are a chain of blocks (about 30 us each); below
+// them the kernel issues a min-plus term per lane in over half of the ALU
+// slots (9e9 terms on the 264k-vertex graph, a warp instruction per two
+// cycles and scheduler).
 #include <algorithm>
 #include <climits>
 #include <cstdio>
@@ -44,7 +47,8 @@ constexpr int kRows = 32;     // nodes of a block (rows of its product)
 constexpr int kSmall = 16;    // largest light subtree that joins its father's block whole
 constexpr int kCols = 64;     // columns of one step of the product
 constexpr int kMembers = 32;  // separator members of one step
-constexpr int kEStride = 72;  // row stride of the staged second factor: 16-byte stores of four rows hit all banks
+constexpr int kMaxTiles = 64; // most tiles (of kCols columns) in a task
+constexpr int kEStride = 80;  // row stride of the staged second factor: 16-byte stores of two rows hit all banks
 constexpr unsigned kInf = 0x7fffffffu;
 
 constexpr int kErrWait = 4;    // a dependency wait ran out
@@ -214,7 +218,7 @@ __global__ void block_sizes_kernel(const int *blk_top, const int *count, const i
 // Tasks of every block: the columns above it in one task, or cut into
 // policy.col_block columns each.
 __global__ void block_tasks_kernel(const int *blk_top, const int *depth, const int *mem, const int64_t *boff,
-                                   const int *lvl_cls, TilePolicy pol, int *ntask, int *pieces, int *tcols, int nblk) {
+                                   const int *lvl_cls, TilePolicy pol, int *ntask, int *pieces, int *tcols, int *several, int nblk) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nblk; b += gridDim.x * blockDim.x) {
     int nt = 0, tc = kCols;
     if (b < nblk) {
@@ -223,12 +227,18 @@ __global__ void block_tasks_kernel(const int *blk_top, const int *depth, const i
       const int cols = d - 1;
       tc = (pol.col_block[wb][sb] + kCols - 1) / kCols * kCols;
       if ((int64_t)m * d <= pol.small_work[wb][sb]) tc = max(kCols, (cols + kCols - 1) / kCols * kCols);
+      tc = min(tc, kCols * kMaxTiles);
       nt = max(1, (cols + tc - 1) / tc);
     }
     ntask[b] = nt;
     pieces[b] = b < nblk ? nt * (int)(boff[b + 1] - boff[b]) : 0;
     tcols[b] = tc;
+    several[b] = nt > 1;
   }
+}
+
+__global__ void narrow_kernel(const int64_t *in, int *out, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = (int)in[i];
 }
 
 __global__ void scatter_nodes_kernel(const int *top_of, const int *blk_of_top, const int64_t *boff, int *fill, int *bnode,
@@ -762,6 +772,8 @@ struct FillKernelArgs {
   const int *tcols;
   int ntasks;
   int *done, *count, *next;
+  const int *mslot;  // blocks of several tasks: their in-block matrix in mbuf, combined by atomicMin
+  unsigned *mbuf;
   long long spin_limit;
   int max_segs;
   unsigned long long *trace_t;  // non-null (GPUH2H_TRACE): each node's publish time, ns
@@ -776,14 +788,21 @@ struct FillKernelArgs {
 // columns inside the block and publishes it.  Rows produced in the launch are
 // read through L2 (ld.global.cg).  A quad of four columns that lies above a
 // member (p_u >= J + 4) is one 128-bit load of u's row; below it, four
-// ancestors' entries at p_u, 16 members of consecutive positions per warp
-// request.
-__global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
+// ancestors' entries at p_u, eight members of consecutive positions per warp
+// request (a third of a 32-byte sector per entry on a 264k-vertex graph).
+// Five CTAs per SM: with six the compiler holds 80 registers and shared memory
+// takes the L1 (4.3 ms against 3.8 on the 264k-vertex graph), with four there
+// are too few warps (4.0).
+__global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
   extern __shared__ __align__(16) int s_seg[];
   __shared__ __align__(16) unsigned s_E[kMembers * kEStride];
   __shared__ __align__(16) unsigned s_S[kMembers * kRows];
   __shared__ __align__(16) int64_t s_arow[2][kCols];
+  __shared__ __align__(16) unsigned s_O[kCols * 36];   // a finished tile, [column][row]
+  __shared__ int64_t s_mrow[2][kMembers];  // a step's members: rows and positions (-1: none)
+  __shared__ int s_mp[2][kMembers];
   __shared__ int64_t s_rowoff[kRows];
+  __shared__ int s_kb[kMaxTiles + 1];  // first member at or after each tile's first column
   __shared__ unsigned s_M[kRows * 33];
   __shared__ int s_tw[kRows * 32];
   __shared__ unsigned char s_tl[kRows * 32];
@@ -793,8 +812,7 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
   const BlockArgs &B = A.B;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   int *const s_top = s_seg, *const s_pos = s_seg + A.max_segs;
-  const int hk = (wid >> 1) * 16 + (lane >> 1);         // the member of a step this thread loads
-  const int q0 = (wid & 1) * 8 + (lane & 1);            // its quads of columns: q0, q0 + 2, q0 + 4, q0 + 6
+  const int em = lane >> 2, ec = 16 * wid + 4 * (lane & 3);  // loads members em, em + 8, .. at columns ec .. ec + 3
   const int ry = tid >> 4, cx = tid & 15;               // its patch of the result
   for (;;) {
     __syncthreads();  // the last task's shared memory is free
@@ -819,6 +837,25 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
       s_pos[i] = __ldg(A.seg_pos + sb + i);
     }
     if (tid < R) s_rowoff[tid] = __ldg(B.drow + __ldg(B.bnode + bo + tid));
+    const int my = tid >> 3, mx = tid & 7;  // this thread's 2 x 4 patch of the in-block matrix
+    for (int i = wid; i < R; i += 4) {
+      const int v = __ldg(B.bnode + bo + i);
+      const int c = stage_inner(B, v, dt, s_tl + 32 * i, s_tw + 32 * i, lane);
+      if (lane == 0) {
+        s_tc[i] = c;
+        s_dcol[i] = __ldg(B.depth + v) - 1;
+        s_par[i] = i > 0 ? B.loc_of[__ldg(B.father + v)] : 0;
+      }
+    }
+    if (tid <= (c1 - c0 + kCols - 1) / kCols) {
+      const int j = min(c0 + kCols * tid, c1);
+      int lo = 0, hi = m;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(B.bm_p + m0 + mid) < j) lo = mid + 1; else hi = mid;
+      }
+      s_kb[tid] = lo;
+    }
     __syncthreads();
     auto ancestor_row = [&](int j) -> int64_t {  // row offset of the ancestor at depth j + 1
       if (j >= c1) return 0;
@@ -843,36 +880,46 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
       reinterpret_cast<uint4 *>(s_S)[tid] = sbuf[0];
       reinterpret_cast<uint4 *>(s_S)[tid + 128] = sbuf[1];
     };
-    auto issue_e = [&](int T, int k0) {
-      const int k = k0 + hk;
-      const bool kv = k < m;
-      const int p = kv ? __ldg(B.bm_p + m0 + k) : -1;
-      const int64_t row = kv ? __ldg(B.bm_row + m0 + k) : 0;
-      const int64_t *ar = s_arow[T & 1];
+    int p2 = -1;  // warp 0: a member of the step after the next
+    int64_t row2 = 0;
+    auto load_member = [&](int k0) {
+      const int k = k0 + lane;
+      p2 = k < m ? __ldg(B.bm_p + m0 + k) : -1;
+      row2 = k < m ? __ldg(B.bm_row + m0 + k) : 0;
+    };
+    // members of a step in buffer `mb` at the columns of tile T; a warp takes
+    // 16 columns of eight members at a time, so that it mostly goes one way
+    auto issue_e = [&](int T, int mb, int kn) {
+      const int J = c0 + T * kCols + ec;
+      const int64_t *ar = s_arow[T & 1] + ec;
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int q = q0 + 2 * i, J = c0 + T * kCols + 4 * q;
+      for (int g = 0; g < 4; g++) {
         uint4 e = make_uint4(kInf, kInf, kInf, kInf);
-        if (kv && J < c1) {
+        if (8 * g < kn && J < c1) {
+          const int k = 8 * g + em, p = s_mp[mb][k];
+          const int *row = A.dis + s_mrow[mb][k];
           if (p >= J + 4) {
-            e = __ldcg(reinterpret_cast<const uint4 *>(A.dis + row + J));
-          } else {
+            e = __ldcg(reinterpret_cast<const uint4 *>(row + J));
+          } else if (p >= 0) {
+            const int *col = A.dis + p;  // past column c1 the ancestor's row is 0: a read that counts for nothing
             unsigned x[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-              const int j = J + c;
-              x[c] = j < p    ? (unsigned)__ldcg(A.dis + row + j)
-                     : j == p ? 0u
-                     : j < c1 ? (unsigned)__ldcg(A.dis + ar[4 * q + c] + p)
-                              : kInf;
-            }
+            for (int c = 0; c < 4; c++)
+              x[c] = (unsigned)(J + c > p ? __ldcg(col + ar[c]) : J + c == p ? 0 : __ldcg(row + J + c));
             e = make_uint4(x[0], x[1], x[2], x[3]);
           }
         }
-        eb[i] = e;
+        eb[g] = e;
       }
     };
-    if (nsteps > 0) issue_s(B.closed, 0);
+    if (nsteps > 0) {
+      issue_s(B.closed, 0);
+      if (wid < 2 && wid < nchunk) {  // the first two steps' members
+        load_member(wid * kMembers);
+        s_mp[wid][lane] = p2;
+        s_mrow[wid][lane] = row2;
+      }
+    }
     if (tid == 0) {
       int ok = 1;
       const int f = __ldg(B.father + top);
@@ -892,18 +939,28 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
     }
     __syncthreads();
     if (!s_flag) return;
-    if (nsteps > 0) issue_e(0, 0);
+    if (nsteps > 0) {
+      issue_e(0, 0, min(kMembers, m));
+    }
+    unsigned mm[2][4];  // in-block matrix: the part over members above the block
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) mm[r][c] = kInf;
     unsigned acc[4][4];
 #pragma unroll
     for (int r = 0; r < 4; r++)
 #pragma unroll
       for (int c = 0; c < 4; c++) acc[r][c] = kInf;
     int64_t arow_next = 0;  // threads below 64: the column's ancestor row two tiles ahead
-    for (int s = 0, T = 0, ch = 0; s < nsteps; s++) {
+    for (int s = 0, T = 0, ch = 0, ch2 = 2 % max(nchunk, 1); s < nsteps; s++) {
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        *reinterpret_cast<uint4 *>(s_E + hk * kEStride + 4 * (q0 + 2 * i)) = eb[i];
+      for (int g = 0; g < 4; g++) *reinterpret_cast<uint4 *>(s_E + (8 * g + em) * kEStride + ec) = eb[g];
       if (nchunk > 1 || s == 0) store_s();
+      if (nchunk > 1 && s > 0 && wid == 0) {
+        s_mp[(s + 1) & 1][lane] = p2;
+        s_mrow[(s + 1) & 1][lane] = row2;
+      }
       if (ch == 0 && T > 0 && tid < kCols) s_arow[(T + 1) & 1][tid] = arow_next;
       __syncthreads();
       const int kn = min(kMembers, m - ch * kMembers);
@@ -913,8 +970,12 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
         nT++;
       }
       if (s + 1 < nsteps) {
-        if (nchunk > 1) issue_s(B.closed, nch * kMembers);
-        issue_e(nT, nch * kMembers);
+        issue_e(nT, nchunk > 1 ? (s + 1) & 1 : 0, min(kMembers, m - nch * kMembers));
+        if (nchunk > 1) {
+          issue_s(B.closed, nch * kMembers);
+          if (wid == 0) load_member(ch2 * kMembers);
+          if (++ch2 == nchunk) ch2 = 0;
+        }
       }
       if (ch == 0 && tid < kCols) arow_next = ancestor_row(c0 + (T + 2) * kCols + tid);
       if (4 * ry < Rp) {
@@ -933,8 +994,15 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
           }
         }
       }
+      const int kb = s_kb[T], ke = nch == 0 ? s_kb[T + 1] : kb;  // members inside a completed tile
       if (nch == 0) {  // the tile is complete
         const int j = c0 + T * kCols + 4 * cx;
+        if (kb < ke && R > 1) {
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            *reinterpret_cast<uint4 *>(s_O + (4 * cx + c) * 36 + 4 * ry) =
+                make_uint4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
+        }
 #pragma unroll
         for (int r = 0; r < 4; r++) {
           const int i = 4 * ry + r;
@@ -952,11 +1020,39 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
           for (int c = 0; c < 4; c++) acc[r][c] = kInf;
         }
       }
+      __syncthreads();
+      // columns inside the block, for nodes i below a (both in the block):
+      //   M(i, a) = min over u in X(i) of sc(i, u) + E(u, a); the part over u
+      // above the block takes column p_u of row a, which this tile has just
+      // completed (the next tile is not written before the next barrier)
+      if (R > 1 && 2 * my < Rp) {
+        const int J = c0 + T * kCols;
+#pragma unroll 4
+        for (int k = kb; k < ke; k++) {
+          const uint2 w = __ldg(reinterpret_cast<const uint2 *>(B.direct + so + (int64_t)k * Rp + 2 * my));
+          const uint4 e = *reinterpret_cast<const uint4 *>(s_O + (__ldg(B.bm_p + m0 + k) - J) * 36 + 4 * mx);
+          const unsigned wr[2] = {w.x, w.y};
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            mm[r][0] = add_min(wr[r], e.x, mm[r][0]);
+            mm[r][1] = add_min(wr[r], e.y, mm[r][1]);
+            mm[r][2] = add_min(wr[r], e.z, mm[r][2]);
+            mm[r][3] = add_min(wr[r], e.w, mm[r][3]);
+          }
+        }
+      }
       T = nT;
       ch = nch;
-      __syncthreads();
     }
     // ---- the last task of the block finishes it
+    unsigned *const mb = ntask > 1 ? A.mbuf + (int64_t)__ldg(A.mslot + b) * (kRows * kRows) : nullptr;
+    if (mb && R > 1) {
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+          if (mm[r][c] < kInf) atomicMin(mb + (2 * my + r) * kRows + 4 * mx + c, mm[r][c]);
+    }
     __syncthreads();
     if (tid == 0) {
       __threadfence();
@@ -965,73 +1061,13 @@ __global__ void __launch_bounds__(128, 6) block_fill_kernel(FillKernelArgs A) {
     }
     __syncthreads();
     if (!s_flag) continue;
-    // columns inside the block.  For nodes i below a (both in the block):
-    //   M(i, a) = min over u in X(i) of sc(i, u) + E(u, a); the part over u
-    // above the block is a product of the direct weights with column p_u of
-    // row a, just completed
-    unsigned mm[2][4];
 #pragma unroll
     for (int r = 0; r < 2; r++)
 #pragma unroll
-      for (int c = 0; c < 4; c++) mm[r][c] = kInf;
-    if (R > 1 && m > 0) {
-      unsigned gb[8];
-      auto issue_g = [&](int k0) {
-        const bool kv = k0 + lane < m;
-        const int p = kv ? __ldg(B.bm_p + m0 + k0 + lane) : 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int a = wid + 4 * i;
-          gb[i] = kv && a < R ? (unsigned)__ldcg(A.dis + s_rowoff[a] + p) : kInf;
-        }
-      };
-      issue_s(B.direct, 0);
-      issue_g(0);
-      const int my = tid >> 3, mx = tid & 7;
-      for (int ch = 0; ch < nchunk; ch++) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) s_E[lane * 36 + wid + 4 * i] = gb[i];
-        store_s();
-        __syncthreads();
-        const int kn = min(kMembers, m - ch * kMembers);
-        if (ch + 1 < nchunk) {
-          issue_s(B.direct, (ch + 1) * kMembers);
-          issue_g((ch + 1) * kMembers);
-        }
-        if (2 * my < Rp) {
-#pragma unroll 4
-          for (int k = 0; k < kn; k++) {
-            const uint4 e = *reinterpret_cast<const uint4 *>(s_E + k * 36 + 4 * mx);
-            const uint2 w = *reinterpret_cast<const uint2 *>(s_S + k * Rp + 2 * my);
-            const unsigned wr[2] = {w.x, w.y};
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-              mm[r][0] = add_min(wr[r], e.x, mm[r][0]);
-              mm[r][1] = add_min(wr[r], e.y, mm[r][1]);
-              mm[r][2] = add_min(wr[r], e.z, mm[r][2]);
-              mm[r][3] = add_min(wr[r], e.w, mm[r][3]);
-            }
-          }
-        }
-        __syncthreads();
+      for (int c = 0; c < 4; c++) {
+        const int at = (2 * my + r) * kRows + 4 * mx + c;
+        s_M[(2 * my + r) * 33 + 4 * mx + c] = mb ? __ldcg(mb + at) : mm[r][c];
       }
-    }
-    {
-      const int my = tid >> 3, mx = tid & 7;
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) s_M[(2 * my + r) * 33 + 4 * mx + c] = mm[r][c];
-    }
-    for (int i = wid; i < R; i += 4) {
-      const int v = __ldg(B.bnode + bo + i);
-      const int c = stage_inner(B, v, dt, s_tl + 32 * i, s_tw + 32 * i, lane);
-      if (lane == 0) {
-        s_tc[i] = c;
-        s_dcol[i] = __ldg(B.depth + v) - 1;
-        s_par[i] = i > 0 ? B.loc_of[__ldg(B.father + v)] : 0;
-      }
-    }
     __syncthreads();
     if (wid == 0) {
       // nodes in depth-first order; lane a holds the entry for the node at
@@ -1307,18 +1343,30 @@ std::vector<int> FillPlan::level_classes() const {
 void FillPlan::build_tiles(const TilePolicy &pol) {
   policy = pol;
   Workspace ws;
-  int *ntask = ws.get<int>(nblk + 1), *pieces = ws.get<int>(nblk + 1);
-  int64_t *piece0 = ws.get<int64_t>(nblk + 1);
+  int *ntask = ws.get<int>(nblk + 1), *pieces = ws.get<int>(nblk + 1), *several = ws.get<int>(nblk + 1);
+  int64_t *piece0 = ws.get<int64_t>(nblk + 1), *slot0 = ws.get<int64_t>(nblk + 1);
   if (!task0) {
     task0 = dalloc<int64_t>(nblk + 1, work_bytes);
     tcols = dalloc<int>(nblk + 1, work_bytes);
+    mslot = dalloc<int>(nblk + 1, work_bytes);
   }
   block_tasks_kernel<<<grid_for(nblk + 1, nsm), 256>>>(blk_top, depth, blk_mem, blk_boff, lvl_cls, pol, ntask, pieces,
-                                                            tcols, nblk);
+                                                            tcols, several, nblk);
   GH_CUDA(cudaGetLastError());
   exclusive_scan<int>(ntask, task0, nblk + 1, ws, 0);
   exclusive_scan<int>(pieces, piece0, nblk + 1, ws, 0);
+  exclusive_scan<int>(several, slot0, nblk + 1, ws, 0);
+  narrow_kernel<<<grid_for(nblk + 1, nsm), 256>>>(slot0, mslot, nblk + 1);
+  GH_CUDA(cudaGetLastError());
   ntasks = read_one(task0 + nblk);
+  mslots = read_one(slot0 + nblk);
+  if (mslots > mslots_cap) {
+    cudaFree(mbuf);
+    mbuf = nullptr;
+    mslots_cap = 0;
+    mbuf = dalloc<unsigned>(mslots * kRows * kRows, work_bytes);
+    mslots_cap = mslots;
+  }
   ntiles = read_one(piece0 + nblk);
   GH_CHECK(ntasks >= nblk && ntasks < INT32_MAX, H2H_ERR_ARG, "too many fill tasks");
   if (ntasks > tasks_cap) {
@@ -1356,6 +1404,8 @@ void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
   A.done = done;
   A.count = done + nblk;
   A.next = next;
+  A.mslot = mslot;
+  A.mbuf = mbuf;
   A.spin_limit = spin_limit_cycles();
   A.max_segs = std::max(max_segs, 1);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1371,6 +1421,7 @@ void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
     GH_CUDA(capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s));
   };
   if (fill_ev) record(fill_ev[0]);
+  if (mslots) fill_inf_kernel<<<grid_for(mslots * 256, nsm), 256, 0, s>>>(mbuf, mslots * kRows * kRows);
   block_fill_kernel<<<blocks, 128, smem, s>>>(A);
   GH_CUDA(cudaGetLastError());
   if (fill_ev) record(fill_ev[1]);

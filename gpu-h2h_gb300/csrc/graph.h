@@ -281,6 +281,9 @@ struct FillPlan {
   unsigned *upd = nullptr;
   int64_t wtasks = 0, upd_total = 0;
   unsigned long long *trace_t = nullptr;  // publish time per node (GPUH2H_TRACE)
+  int *mslot = nullptr;  // blocks of several tasks: their in-block matrix
+  unsigned *mbuf = nullptr;
+  int64_t mslots = 0, mslots_cap = 0;
   int64_t ntasks = 0, tasks_cap = 0;
   int64_t ntiles = 0;  // row pieces: every node of a block once per task of the block
   int max_segs = 1, blocks = 1;

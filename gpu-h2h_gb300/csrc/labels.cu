@@ -309,11 +309,12 @@ __global__ void build_positions_kernel(const int64_t *list_off, const int *list_
 
 }  // namespace
 
-// A narrow level's blocks are cut as finely as the kernel's step (64 columns):
-// they are the chain the fill waits for.  Elsewhere a task is about 16k
-// (member, column) pairs, so a block of the bottom (m <= 16) is one task.
+// A narrow level's blocks are the chain the fill waits for and are cut finely;
+// elsewhere a task is a whole row range, because a task's own start (tables,
+// members, ancestors) costs as much as several steps: 64 / 256-column tasks
+// there took the 1M-vertex fill from 14.8 to 17.4 ms.
 TilePolicy::TilePolicy() {
-  static const int cb[kWidth][kSep] = {{64, 64, 64, 64}, {1024, 256, 64, 64}, {1024, 256, 64, 64}};
+  static const int cb[kWidth][kSep] = {{256, 256, 128, 64}, {4096, 4096, 512, 64}, {4096, 4096, 512, 64}};
   for (int w = 0; w < kWidth; w++)
     for (int b = 0; b < kSep; b++) {
       small_work[w][b] = 1024;
@@ -519,14 +520,15 @@ void FillPlan::release_work() {
   void *ps[] = {pos_w,    pos_src,  hld,      htop,  hpos,   seg_off, seg_top, seg_pos, done,   next,   err,    tasks,   trace_t,
                 hld_row,  blk_top,  blk_mem,  blk_boff, blk_moff, blk_soff, bnode, blk_of, loc_of, lvl_cls, bm_p, bm_row,
                 direct,   closed,   task0,    tcols,  blk_up, bm_up,   wtask_blk, pending, pend_init, blk_uoff, wtask0,
-                arc_cell, upd};
+                arc_cell, upd,      mslot,    mbuf};
   for (void *p : ps) cudaFree(p);
   trace_t = nullptr;
   pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = tasks = nullptr;
   blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;
   hld_row = seg_off = blk_boff = blk_moff = blk_soff = bm_row = task0 = nullptr;
   loc_of = nullptr;
-  direct = closed = upd = nullptr;
+  direct = closed = upd = mbuf = nullptr;
+  mslot = nullptr;
   blk_up = bm_up = wtask_blk = pending = pend_init = nullptr;
   blk_uoff = wtask0 = arc_cell = nullptr;
 }
