@@ -56,7 +56,7 @@ struct h2h_batch {
     info.vertices = elim->N;
     info.elim_launches = elim->launch_count();
     info.fill_tiles = fill->ntiles;
-    int64_t db = elim->bytes + fill->work_bytes;
+    int64_t db = elim->bytes() + fill->work_bytes();
     int64_t upd = 0;
     for (gh::Graph *g : gs) {
       db += g->dev.bytes;

@@ -112,7 +112,7 @@ int load_common(const std::string &edge, const std::string &idf, const std::stri
     GH_CHECK(g.C <= g.H, H2H_ERR_ARG, "ChangeToGlobalHeight exceeds the partition height");
     gh::Clock clk;
     {
-      gh::Pool pool(g.threads);
+      gh::Pool pool(gh::useful_threads(g.threads, g.m));
       check_symmetric(g, pool);
       check_connected(g, pool);
     }

@@ -1236,11 +1236,7 @@ __global__ void father_kernel(const int64_t *off, const int *id, const int *rank
 struct ListArrays {
   int64_t *off = nullptr;
   int *id = nullptr, *w = nullptr;
-  ~ListArrays() {
-    cudaFree(off);
-    cudaFree(id);
-    cudaFree(w);
-  }
+  DeviceArena mem;
 };
 
 template <typename T>
@@ -1267,13 +1263,6 @@ GraphLevels graph_levels(const Graph &g) {
   L.heap_start = (int)heap_start;
   L.heap_n = g.n - (int)heap_start;
   return L;
-}
-
-template <typename T>
-T *palloc(size_t n, int64_t &bytes) {
-  T *p = dalloc<T>(n);
-  bytes += (int64_t)(std::max<size_t>(n, 1) * sizeof(T));
-  return p;
 }
 
 }  // namespace
@@ -1341,6 +1330,7 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
       const Graph &g = *gs[i];
       for (int j = L[i].heap_start; j < g.n; j++) f_heap[hbase[i] + j - L[i].heap_start] = g.elim[j] + vbase[i];
     };
+    threads = useful_threads(threads, N);
     Pool pool(threads);
     if (K >= threads) {  // a batch: a graph per task
       pool.parallel_for(K, 1, [&](int64_t lo, int64_t hi, int) {
@@ -1366,36 +1356,39 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
   const int64_t pstage_ints = LL.pstage_ints, partial_max = LL.partial_max;
   // ---- device state
   try {
-    slot_nbr = palloc<int>(pool_size + 4, bytes);  // + 4: a list's last 128-bit load stays inside
-    slot_w = palloc<int>(pool_size + 4, bytes);
-    pool_next = palloc<unsigned long long>(1, bytes);
-    pool_first = palloc<unsigned long long>(1, bytes);
-    slot_off = palloc<int64_t>(N, bytes);
-    slot_off_init = palloc<int64_t>(N, bytes);
-    lsize = palloc<int>(N, bytes);
-    cap = palloc<int>(N, bytes);
-    cap_init = palloc<int>(N, bytes);
-    height = palloc<int>(N, bytes);
-    elim = palloc<int>(N, bytes);
-    elim_init = palloc<int>(N, bytes);
-    deg0 = palloc<int>(N, bytes);
-    deg_init = palloc<int>(N, bytes);
-    h0 = palloc<int>(N, bytes);
-    cpos = palloc<int>(N, bytes);
-    err = palloc<int>(1, bytes);
-    ljunk = palloc<int>(N, bytes);
-    cell_start = palloc<int>(fcs.size(), bytes);
-    cell_count = palloc<int>(fcc.size(), bytes);
-    adj_off = palloc<int>(N + 1, bytes);
-    adj_v = palloc<int>(std::max<int64_t>(M, 1), bytes);
-    adj_w = palloc<int>(std::max<int64_t>(M, 1), bytes);
-    heap_verts = palloc<int>(std::max(heap_total, 1), bytes);
-    if (pstage_ints) pstage = palloc<int>(pstage_ints, bytes);
+    // large slot arrays are freed as soon as the lists are compacted
+    own_slots = bits && pool_size >= (int64_t(16) << 20);
+    slot_nbr = own_slots ? dalloc<int>(pool_size + 4) : mem.get<int>(pool_size + 4);  // + 4: a list's last 128-bit load stays inside
+    slot_w = own_slots ? dalloc<int>(pool_size + 4) : mem.get<int>(pool_size + 4);
+    slot_bytes = own_slots ? 8 * (pool_size + 4) : 0;
+    pool_next = mem.get<unsigned long long>(1);
+    pool_first = mem.get<unsigned long long>(1);
+    slot_off = mem.get<int64_t>(N);
+    slot_off_init = mem.get<int64_t>(N);
+    lsize = mem.get<int>(N);
+    cap = mem.get<int>(N);
+    cap_init = mem.get<int>(N);
+    height = mem.get<int>(N);
+    elim = mem.get<int>(N);
+    elim_init = mem.get<int>(N);
+    deg0 = mem.get<int>(N);
+    deg_init = mem.get<int>(N);
+    h0 = mem.get<int>(N);
+    cpos = mem.get<int>(N);
+    err = mem.get<int>(1);
+    ljunk = mem.get<int>(N);
+    cell_start = mem.get<int>(fcs.size());
+    cell_count = mem.get<int>(fcc.size());
+    adj_off = mem.get<int>(N + 1);
+    adj_v = mem.get<int>(std::max<int64_t>(M, 1));
+    adj_w = mem.get<int>(std::max<int64_t>(M, 1));
+    heap_verts = mem.get<int>(std::max(heap_total, 1));
+    if (pstage_ints) pstage = mem.get<int>(pstage_ints);
     if (!gmap.empty()) {
-      hg_partial = palloc<int4>(2 * partial_max, bytes);  // per block: argmin, then (first word) merge count
+      hg_partial = mem.get<int4>(2 * partial_max);  // per block: argmin, then (first word) merge count
       partial_cap = partial_max;
-      grid_map = palloc<int>(gmap.size(), bytes);
-      grid_bar = palloc<unsigned>(grid_bar_words, bytes);
+      grid_map = mem.get<int>(gmap.size());
+      grid_bar = mem.get<unsigned>(grid_bar_words);
       GH_CUDA(cudaMemcpy(grid_map, gmap.data(), sizeof(int) * gmap.size(), cudaMemcpyHostToDevice));
     }
     for (int k = 1; k < max_group; k++) {
@@ -1694,22 +1687,19 @@ void ElimPlan::plan_lists(const int *f_elim, const std::vector<GraphLevels> &L, 
 ElimPlan::~ElimPlan() { release(); }
 
 void ElimPlan::release() {
-  void *ps[] = {slot_nbr, slot_w, pool_next, pool_first, slot_off, slot_off_init, lsize, cap, cap_init, height, elim,
-                elim_init, deg0, deg_init, h0, cpos, err, ljunk, cell_start, cell_count, adj_off, adj_v, adj_w,
-                heap_verts, pstage};
-  for (void *p : ps) cudaFree(p);
-  for (void *p : {(void *)members, (void *)extra, (void *)fin, (void *)sym_cells, (void *)grows}) cudaFree(p);
+  if (own_slots) {
+    cudaFree(slot_nbr);
+    cudaFree(slot_w);
+    own_slots = false;
+    slot_bytes = 0;
+  }
+  mem.release();
   members = extra = nullptr;
   fin = sym_cells = nullptr;
   grows = nullptr;
-  cudaFree(hg_partial);
-  cudaFree(grid_map);
-  cudaFree(grid_bar);
   grid_map = nullptr;
   hg_partial = nullptr;
   grid_bar = nullptr;
-  cudaFree(rank);
-  cudaFree(father_dev);
   rank = father_dev = nullptr;
   for (cudaStream_t st : side) cudaStreamDestroy(st);
   for (cudaEvent_t e : ev_join) cudaEventDestroy(e);
@@ -1862,33 +1852,35 @@ void ElimPlan::check_error() {
 void ElimPlan::build_lists() {
   int threads = 1;
   for (const Graph *g : gs) threads = std::max(threads, g->threads);
-  Pool pool(threads);
+  Pool pool(useful_threads(threads, N));
   std::vector<int, NoInit<int>> f_lsize(N), f_elim(N), f_father(N);
   GH_CUDA(cudaMemcpy(f_lsize.data(), lsize, sizeof(int) * N, cudaMemcpyDeviceToHost));
   std::vector<int64_t, NoInit<int64_t>> off(N + 1);
   parallel_prefix(pool, N, off.data(), [&](int64_t v) { return (int64_t)f_lsize[v]; });
   const int64_t tot = off[N];
   auto la = std::make_shared<ListArrays>();
-  la->off = dalloc<int64_t>(N + 1);
-  la->id = dalloc<int>(std::max<int64_t>(tot, 1));
-  la->w = dalloc<int>(std::max<int64_t>(tot, 1));
+  la->off = la->mem.get<int64_t>(N + 1);
+  la->id = la->mem.get<int>(tot);
+  la->w = la->mem.get<int>(tot);
   lists.off = la->off;
   lists.id = la->id;
   lists.w = la->w;
   lists.total = tot;
   lists.keep = la;
-  if (!rank) rank = palloc<int>(N, bytes);
-  if (!father_dev) father_dev = palloc<int>(N, bytes);
+  if (!rank) rank = mem.get<int>(N);
+  if (!father_dev) father_dev = mem.get<int>(N);
   GH_CUDA(cudaMemcpy(lists.off, off.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
   enqueue_gather(0);
   rank_kernel<<<std::max(1, std::min(4096, (N + 255) / 256)), 256>>>(elim, rank, N);
   GH_CUDA(cudaGetLastError());
   father_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256>>>(lists.off, lists.id, rank, father_dev, N);
   GH_CUDA(cudaGetLastError());
-  if (bits) {  // the lists never run again: only their weights are replayed
-    GH_CUDA(cudaFree(slot_nbr));
-    GH_CUDA(cudaFree(slot_w));
+  if (own_slots) {  // the lists never run again: only their weights are replayed
+    cudaFree(slot_nbr);
+    cudaFree(slot_w);
     slot_nbr = slot_w = nullptr;
+    own_slots = false;
+    slot_bytes = 0;
   }
   GH_CUDA(cudaMemcpy(f_elim.data(), elim, sizeof(int) * N, cudaMemcpyDeviceToHost));
   GH_CUDA(cudaMemcpy(f_father.data(), father_dev, sizeof(int) * N, cudaMemcpyDeviceToHost));
@@ -1928,9 +1920,9 @@ ListStore upload_lists(const std::vector<int64_t> &off, const std::vector<int> &
   ListStore L;
   auto la = std::make_shared<ListArrays>();
   const int64_t t = off.empty() ? 0 : off.back();
-  la->off = dalloc<int64_t>(std::max<size_t>(off.size(), 1));
-  la->id = dalloc<int>(std::max<int64_t>(t, 1));
-  la->w = dalloc<int>(std::max<int64_t>(t, 1));
+  la->off = la->mem.get<int64_t>((int64_t)off.size());
+  la->id = la->mem.get<int>(t);
+  la->w = la->mem.get<int>(t);
   L.off = la->off;
   L.id = la->id;
   L.w = la->w;

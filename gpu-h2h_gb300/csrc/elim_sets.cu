@@ -27,6 +27,7 @@
 // writes its interior vertices in position order and retires them.
 #include <algorithm>
 
+#include "arena.h"
 #include "graph.h"
 
 namespace gh {
@@ -244,14 +245,6 @@ __global__ void __launch_bounds__(kThreads) write_kernel(SetsArgs A) {
   }
 }
 
-template <typename T>
-T *sets_alloc(size_t n, std::vector<void *> &owned) {
-  T *p = nullptr;
-  GH_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
-  owned.push_back(p);
-  return p;
-}
-
 }  // namespace
 
 void build_elimination_sets(const std::vector<Graph *> &gs) {
@@ -311,26 +304,22 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
     nchunk_total += (int64_t)lv[h].size();
   }
   // ---- device state
-  std::vector<void *> owned;
-  auto cleanup = [&]() {
-    for (void *p : owned) cudaFree(p);
-    owned.clear();
-  };
+  DeviceArena ws;
   std::vector<int> f_cell_start(CELLS), f_cell_count(CELLS), f_cell_bound(CELLS), f_cap(N), f_dup(N), f_elim(N),
       f_fill(K);
-  try {
+  {
     SetsArgs S{};
-    int *d_vbase = sets_alloc<int>(K, owned), *d_abase = sets_alloc<int>(K, owned), *d_mbase = sets_alloc<int>(K, owned);
-    int *d_adj_off = sets_alloc<int>(A, owned), *d_adj_v = sets_alloc<int>(M, owned);
-    int *d_part = sets_alloc<int>(N, owned), *d_pos = sets_alloc<int>(N, owned), *d_dup = sets_alloc<int>(N, owned);
-    int *d_vgraph = sets_alloc<int>(N, owned);
-    int *d_cut_l = sets_alloc<int>(CELLS, owned), *d_cut_r = sets_alloc<int>(CELLS, owned);
-    unsigned char *d_alive = sets_alloc<unsigned char>(N, owned), *d_flag = sets_alloc<unsigned char>(N, owned);
-    int *d_cap = sets_alloc<int>(N, owned), *d_elim = sets_alloc<int>(N, owned);
-    int *d_cell = sets_alloc<int>(4 * CELLS, owned);  // size, bound, start, count
-    int *d_chunk_cnt = sets_alloc<int>(nchunk_max, owned), *d_chunk_out = sets_alloc<int>(nchunk_max, owned);
-    Chunk *d_chunks = sets_alloc<Chunk>(std::max<int64_t>(nchunk_total, 1), owned);
-    int *d_fill = sets_alloc<int>(K, owned);
+    int *d_vbase = ws.get<int>(K), *d_abase = ws.get<int>(K), *d_mbase = ws.get<int>(K);
+    int *d_adj_off = ws.get<int>(A), *d_adj_v = ws.get<int>(M);
+    int *d_part = ws.get<int>(N), *d_pos = ws.get<int>(N), *d_dup = ws.get<int>(N);
+    int *d_vgraph = ws.get<int>(N);
+    int *d_cut_l = ws.get<int>(CELLS), *d_cut_r = ws.get<int>(CELLS);
+    unsigned char *d_alive = ws.get<unsigned char>(N), *d_flag = ws.get<unsigned char>(N);
+    int *d_cap = ws.get<int>(N), *d_elim = ws.get<int>(N);
+    int *d_cell = ws.get<int>(4 * CELLS);  // size, bound, start, count
+    int *d_chunk_cnt = ws.get<int>(nchunk_max), *d_chunk_out = ws.get<int>(nchunk_max);
+    Chunk *d_chunks = ws.get<Chunk>(std::max<int64_t>(nchunk_total, 1));
+    int *d_fill = ws.get<int>(K);
     GH_CUDA(cudaMemcpy(d_vbase, vbase.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(d_abase, abase.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(d_mbase, mbase.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
@@ -413,11 +402,8 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
     GH_CUDA(cudaMemcpy(f_cell_bound.data(), S.cell_bound, sizeof(int) * CELLS, cudaMemcpyDeviceToHost));
     GH_CUDA(cudaMemcpy(f_cell_start.data(), S.cell_start, sizeof(int) * CELLS, cudaMemcpyDeviceToHost));
     GH_CUDA(cudaMemcpy(f_cell_count.data(), S.cell_count, sizeof(int) * CELLS, cudaMemcpyDeviceToHost));
-  } catch (...) {
-    cleanup();
-    throw;
   }
-  cleanup();
+  ws.release();
   const long long t_sets = clk.us();
   // ---- per graph: tables, LUB layout (GraphPartition.cu:270-292), level rates
   for (int i = 0; i < K; i++) {

@@ -1172,16 +1172,16 @@ void FillPlan::build_blocks() {
   exclusive_scan<int>(lvl_tops, lvl_first, nlev + 1, ws, 0);
   nblk = (int)read_one(lvl_first + nlev);
   GH_CHECK(nblk >= 1 && nblk <= N, H2H_ERR_STATE, "fill blocks do not cover the tree");
-  blk_top = dalloc<int>(nblk, work_bytes);
-  blk_mem = dalloc<int>(nblk + 1, work_bytes);
-  blk_boff = dalloc<int64_t>(nblk + 1, work_bytes);
-  blk_moff = dalloc<int64_t>(nblk + 1, work_bytes);
-  blk_soff = dalloc<int64_t>(nblk + 1, work_bytes);
-  bnode = dalloc<int>(N, work_bytes);
-  blk_of = dalloc<int>(N, work_bytes);
-  loc_of = dalloc<unsigned char>(N, work_bytes);
-  lvl_cls = dalloc<int>(nlev, work_bytes);
-  done = dalloc<int>(2 * (int64_t)nblk, work_bytes);  // done flags, then finished tasks per block
+  blk_top = work.get<int>(nblk);
+  blk_mem = work.get<int>(nblk + 1);
+  blk_boff = work.get<int64_t>(nblk + 1);
+  blk_moff = work.get<int64_t>(nblk + 1);
+  blk_soff = work.get<int64_t>(nblk + 1);
+  bnode = work.get<int>(N);
+  blk_of = work.get<int>(N);
+  loc_of = work.get<unsigned char>(N);
+  lvl_cls = work.get<int>(nlev);
+  done = work.get<int>(2 * (int64_t)nblk);  // done flags, then finished tasks per block
   unsigned long long per_node = 1ull << 18;
   if (const char *e = std::getenv("GPUH2H_HEAVY_LEVEL_WORK")) per_node = (unsigned long long)std::max(1LL, std::atoll(e));
   level_class_kernel<<<grid_for(nlev, nsm), 256>>>(lvl_width, lvl_work, nlev, nsm, per_node, lvl_cls);
@@ -1196,10 +1196,10 @@ void FillPlan::build_blocks() {
   GH_CHECK(read_one(blk_boff + nblk) == N, H2H_ERR_STATE, "fill blocks do not cover the tree");
   const int64_t members = read_one(blk_moff + nblk);
   cell_total = read_one(blk_soff + nblk);
-  bm_p = dalloc<int>(members, work_bytes);
-  bm_row = dalloc<int64_t>(members, work_bytes);
-  direct = dalloc<unsigned>(cell_total, work_bytes);
-  closed = dalloc<unsigned>(cell_total, work_bytes);
+  bm_p = work.get<int>(members);
+  bm_row = work.get<int64_t>(members);
+  direct = work.get<unsigned>(cell_total);
+  closed = work.get<unsigned>(cell_total);
   scatter_nodes_kernel<<<grid, 256>>>(top_of, blk_of_top, blk_boff, filled, bnode, N);
   block_nodes_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(blk_top, blk_boff, blk_moff, hpos, pos_hash, pos_pos,
                                                                  pos_id, drow, bnode, blk_of, loc_of, bm_p, bm_row,
@@ -1247,14 +1247,14 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   int *ntask = ws.get<int>(nblk + 1);
   int64_t *ucells = ws.get<int64_t>(nblk + 1);
   unsigned char *global = ws.get<unsigned char>(N);
-  wtask0 = dalloc<int64_t>(nblk + 1, work_bytes);
-  blk_up = dalloc<int>(nblk, work_bytes);
-  blk_uoff = dalloc<int64_t>(nblk + 1, work_bytes);
-  pending = dalloc<int>(nblk, work_bytes);
-  pend_init = dalloc<int>(nblk, work_bytes);
+  wtask0 = work.get<int64_t>(nblk + 1);
+  blk_up = work.get<int>(nblk);
+  blk_uoff = work.get<int64_t>(nblk + 1);
+  pending = work.get<int>(nblk);
+  pend_init = work.get<int>(nblk);
   const int64_t members = read_one(blk_moff + nblk);
-  bm_up = dalloc<int>(members, work_bytes);
-  arc_cell = dalloc<int64_t>(from.M, work_bytes);
+  bm_up = work.get<int>(members);
+  arc_cell = work.get<int64_t>(from.M);
   const BlockArgs B = block_args(*this);
   const int gb = grid_for(nblk + 1, nsm), gw = grid_for((int64_t)nblk * 32, nsm);
   weight_tasks_kernel<<<gb, 256>>>(blk_mem, ntask, nblk);
@@ -1262,7 +1262,7 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   exclusive_scan<int>(ntask, wtask0, nblk + 1, ws, 0);
   wtasks = read_one(wtask0 + nblk);
   GH_CHECK(wtasks < INT32_MAX, H2H_ERR_ARG, "too many weight tasks");
-  wtask_blk = dalloc<int>(wtasks, work_bytes);
+  wtask_blk = work.get<int>(wtasks);
   expand_tasks_kernel<<<gw, 256>>>(wtask0, wtask_blk, nblk);
   GH_CUDA(cudaMemset(err, 0, sizeof(int)));
   GH_CUDA(cudaMemset(pend_init, 0, sizeof(int) * nblk));
@@ -1275,7 +1275,7 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   GH_CUDA(cudaMemGetInfo(&fr, &tot));
   weights_fit = (uint64_t)upd_total * 4 <= fr / 2;
   if (!weights_fit) return;
-  upd = dalloc<unsigned>(upd_total, work_bytes);
+  upd = work.get<unsigned>(upd_total);
   GH_CUDA(cudaMemset(global, 0, N));
   if (from.heap_total) {
     mark_kernel<<<grid_for(from.heap_total, nsm), 256>>>(from.heap_verts, from.heap_total, global);
@@ -1346,9 +1346,9 @@ void FillPlan::build_tiles(const TilePolicy &pol) {
   int *ntask = ws.get<int>(nblk + 1), *pieces = ws.get<int>(nblk + 1), *several = ws.get<int>(nblk + 1);
   int64_t *piece0 = ws.get<int64_t>(nblk + 1), *slot0 = ws.get<int64_t>(nblk + 1);
   if (!task0) {
-    task0 = dalloc<int64_t>(nblk + 1, work_bytes);
-    tcols = dalloc<int>(nblk + 1, work_bytes);
-    mslot = dalloc<int>(nblk + 1, work_bytes);
+    task0 = work.get<int64_t>(nblk + 1);
+    tcols = work.get<int>(nblk + 1);
+    mslot = work.get<int>(nblk + 1);
   }
   block_tasks_kernel<<<grid_for(nblk + 1, nsm), 256>>>(blk_top, depth, blk_mem, blk_boff, lvl_cls, pol, ntask, pieces,
                                                             tcols, several, nblk);
@@ -1363,8 +1363,9 @@ void FillPlan::build_tiles(const TilePolicy &pol) {
   if (mslots > mslots_cap) {
     cudaFree(mbuf);
     mbuf = nullptr;
+    grown_bytes -= mslots_cap * kRows * kRows * 4;
     mslots_cap = 0;
-    mbuf = dalloc<unsigned>(mslots * kRows * kRows, work_bytes);
+    mbuf = dalloc<unsigned>(mslots * kRows * kRows, grown_bytes);
     mslots_cap = mslots;
   }
   ntiles = read_one(piece0 + nblk);
@@ -1372,8 +1373,9 @@ void FillPlan::build_tiles(const TilePolicy &pol) {
   if (ntasks > tasks_cap) {
     cudaFree(tasks);
     tasks = nullptr;
+    grown_bytes -= tasks_cap * 4;
     tasks_cap = 0;
-    tasks = dalloc<int>(ntasks, work_bytes);
+    tasks = dalloc<int>(ntasks, grown_bytes);
     tasks_cap = ntasks;
   }
   expand_tasks_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(task0, tasks, nblk);

@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "arena.h"
 #include "common.h"
 
 namespace gh {
@@ -53,7 +54,7 @@ struct DeviceIndex {
   int id_base = 0;
   int64_t bytes = 0, rmq_bytes = 0;
   std::vector<void *> owned;      // label-side allocations of this handle
-  std::vector<void *> owned_rmq;  // first, rmq_hash, rmq_id (built with the tree)
+  std::unique_ptr<DeviceArena> owned_rmq;  // first, rmq_hash, rmq_id (built with the tree)
   std::shared_ptr<void> keep;
   void release();
   void release_labels();  // everything but the sparse table
@@ -198,7 +199,10 @@ struct ElimPlan {
   void *hg_partial = nullptr;
   unsigned *grid_bar = nullptr;
   int64_t grid_bar_words = 0;
-  int64_t bytes = 0;
+  DeviceArena mem;          // every array but large slot arrays
+  bool own_slots = false;   // slot_nbr and slot_w are allocations of their own
+  int64_t slot_bytes = 0;
+  int64_t bytes() const { return mem.bytes + slot_bytes; }
   explicit ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits = true);
   ~ElimPlan();
   bool plan_bits();
@@ -289,7 +293,9 @@ struct FillPlan {
   int max_segs = 1, blocks = 1;
   size_t smem = 0;
   int nsm = 0;
-  int64_t work_bytes = 0;
+  DeviceArena work;       // the plan's arrays but tasks and mbuf, which grow with the policy
+  int64_t grown_bytes = 0;
+  int64_t work_bytes() const { return work.bytes + grown_bytes; }
   // The blocks and, when `arcs` made the order on bit rows, where each of its
   // arcs enters the blocks' weights.  lists: the graphs' X lists in the same
   // forest numbering.

@@ -324,7 +324,7 @@ void load_graph(Graph &g, const std::string &edge, const std::string &idf, const
     // by tail in increasing order, as Edge files are written, the lists are
     // the arc arrays themselves and the offsets the group starts (found in
     // parallel); otherwise a counting pass and a placement pass
-    Pool pool(std::max(1, g.threads));
+    Pool pool(useful_threads(std::max(1, g.threads), g.n));
     std::atomic<bool> sorted{true};
     pool.parallel_for(g.m, 1 << 16, [&](int64_t lo, int64_t hi, int) {
       for (int64_t i = std::max<int64_t>(lo, 1); i < hi; i++)

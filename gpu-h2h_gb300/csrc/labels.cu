@@ -48,8 +48,7 @@ void DeviceIndex::release() {
   lists = ListStore();
   x_base = pos_base = 0;
   id_base = 0;
-  for (void *p : owned_rmq) cudaFree(p);
-  owned_rmq.clear();
+  owned_rmq.reset();
   first = rmq_id = nullptr;
   rmq_hash = nullptr;
   bytes = rmq_bytes = 0;
@@ -74,21 +73,6 @@ T *dalloc_owned(size_t n, DeviceIndex &D) {
   D.owned.push_back(p);
   return p;
 }
-
-// Device arrays shared by the graphs of one forest fill.
-struct DevArrays {
-  std::vector<void *> p;
-  int64_t bytes = 0;
-  template <typename T>
-  T *alloc(size_t n) {
-    T *q = dalloc<T>(n, bytes);
-    p.push_back(q);
-    return q;
-  }
-  ~DevArrays() {
-    for (void *q : p) cudaFree(q);
-  }
-};
 
 // Initial rows (mallocH2HLabel_noHub, H2HConsturction.cu:636-654): INT_MAX,
 // shortcut weights at the positions of X(v), 0 at the own position.
@@ -375,7 +359,9 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
   const int64_t nvr = (int64_t)vr.size();
   std::vector<int64_t> rdis(nvr, 0), rbase(nvr, 0);
   std::vector<int> rmax_m(nvr, 0);
-  Pool pool(host_threads);
+  int64_t total_n = 0;
+  for (const Graph *g : gs) total_n += g->n;
+  Pool pool(useful_threads(host_threads, total_n));
   pool.parallel_for(nvr, 1, [&](int64_t lo, int64_t hi, int) {
     for (int64_t r = lo; r < hi; r++) {
       const Graph &g = *gs[vr[r].g];
@@ -449,31 +435,31 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
   int dev = 0;
   GH_CUDA(cudaGetDevice(&dev));
   GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  auto st = std::make_shared<DevArrays>();
+  auto st = std::make_shared<DeviceArena>();
   storage = st;
-  drow = st->alloc<int64_t>(N + 1);
-  pos_hash = st->alloc<int64_t>(N + 1);
-  pos_pos = st->alloc<int>(pos_total);
-  pos_id = st->alloc<int>(pos_total);
-  father = st->alloc<int>(N);
-  depth = st->alloc<int>(N);
+  drow = st->get<int64_t>(N + 1);
+  pos_hash = st->get<int64_t>(N + 1);
+  pos_pos = st->get<int>(pos_total);
+  pos_id = st->get<int>(pos_total);
+  father = st->get<int>(N);
+  depth = st->get<int>(N);
   try {
-    pos_w = dalloc<int>(pos_total, work_bytes);
-    pos_src = dalloc<int>(pos_total, work_bytes);
-    hld = dalloc<int>(N, work_bytes);
-    htop = dalloc<int>(N, work_bytes);
-    hpos = dalloc<int>(N, work_bytes);
-    seg_off = dalloc<int64_t>(N + 1, work_bytes);
-    seg_top = dalloc<int>(std::max<int64_t>(seg_total, 1), work_bytes);
-    seg_pos = dalloc<int>(std::max<int64_t>(seg_total, 1), work_bytes);
-    next = dalloc<int>(1, work_bytes);
-    err = dalloc<int>(1, work_bytes);
+    pos_w = work.get<int>(pos_total);
+    pos_src = work.get<int>(pos_total);
+    hld = work.get<int>(N);
+    htop = work.get<int>(N);
+    hpos = work.get<int>(N);
+    seg_off = work.get<int64_t>(N + 1);
+    seg_top = work.get<int>(std::max<int64_t>(seg_total, 1));
+    seg_pos = work.get<int>(std::max<int64_t>(seg_total, 1));
+    next = work.get<int>(1);
+    err = work.get<int>(1);
     GH_CUDA(cudaMemcpy(drow, f_drow.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(pos_hash, f_pos_hash.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(father, f_father.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(depth, f_depth.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(hld, f_hld.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    hld_row = dalloc<int64_t>(N, work_bytes);
+    hld_row = work.get<int64_t>(N);
     hld_row_kernel<<<std::max(1, std::min(8192, (N + 255) / 256)), 256>>>(hld, drow, hld_row, N);
     GH_CUDA(cudaGetLastError());
     mark("allocations and uploads");
@@ -512,16 +498,14 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
 FillPlan::~FillPlan() { release_work(); }
 
 void FillPlan::prepare(const TilePolicy &pol) {
-  dis = static_cast<DevArrays *>(storage.get())->alloc<int>(dis_total);
+  dis = static_cast<DeviceArena *>(storage.get())->get<int>(dis_total);
   build_tiles(pol);
 }
 
 void FillPlan::release_work() {
-  void *ps[] = {pos_w,    pos_src,  hld,      htop,  hpos,   seg_off, seg_top, seg_pos, done,   next,   err,    tasks,   trace_t,
-                hld_row,  blk_top,  blk_mem,  blk_boff, blk_moff, blk_soff, bnode, blk_of, loc_of, lvl_cls, bm_p, bm_row,
-                direct,   closed,   task0,    tcols,  blk_up, bm_up,   wtask_blk, pending, pend_init, blk_uoff, wtask0,
-                arc_cell, upd,      mslot,    mbuf};
-  for (void *p : ps) cudaFree(p);
+  work.release();
+  for (void *p : {(void *)tasks, (void *)mbuf, (void *)trace_t}) cudaFree(p);
+  grown_bytes = tasks_cap = mslots_cap = 0;
   trace_t = nullptr;
   pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = tasks = nullptr;
   blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;

@@ -37,6 +37,12 @@ struct NoInit : std::allocator<T> {
   }
 };
 
+// Threads worth starting for `items` vertices or arcs of light work: one per
+// 16k (starting sixteen costs about as much as one thread's pass over 64k).
+inline int useful_threads(int threads, int64_t items) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(threads, items >> 14));
+}
+
 class Pool {
  public:
   explicit Pool(int threads) : nthreads_(std::max(1, threads)) {

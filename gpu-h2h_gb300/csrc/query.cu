@@ -18,16 +18,6 @@ namespace gh {
 
 namespace {
 
-template <typename T>
-T *dalloc(size_t n, int64_t &bytes) {
-  T *p = nullptr;
-  if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  bytes += (int64_t)(n * sizeof(T));
-  return p;
-}
-
 struct QArgs {
   const int *x, *y;
   int *out;
@@ -220,6 +210,24 @@ __global__ void rmq_level_kernel(const RmqJob *jobs, const int64_t *off, int njo
   }
 }
 
+// firstAppeare, RMQHash and RMQ_ID on the device.
+void allocate_rmq(Graph &g) {
+  DeviceIndex &D = g.dev;
+  D.bytes -= D.rmq_bytes;
+  D.rmq_bytes = 0;
+  D.first = nullptr;
+  D.rmq_hash = nullptr;
+  D.rmq_id = nullptr;
+  D.owned_rmq = std::make_unique<DeviceArena>();
+  D.euler = g.euler_n;
+  D.rmq = g.rmq_total;
+  D.first = D.owned_rmq->get<int>(g.n);
+  D.rmq_hash = D.owned_rmq->get<int64_t>(D.euler);
+  D.rmq_id = D.owned_rmq->get<int>(D.rmq);
+  D.rmq_bytes = D.owned_rmq->bytes;
+  D.bytes += D.rmq_bytes;
+}
+
 }  // namespace
 
 void build_rmq_gpu(const std::vector<Graph *> &gs) {
@@ -236,34 +244,17 @@ void build_rmq_gpu(const std::vector<Graph *> &gs) {
     levels = std::max(levels, ilog2_floor(g.euler_n));
   }
   const int64_t total = off[K];
-  int64_t tmp = 0;
-  int *d_eid = nullptr, *d_depth = nullptr;
-  int64_t *d_off = nullptr;
-  RmqJob *d_jobs = nullptr;
-  auto cleanup = [&]() { cudaFree(d_eid); cudaFree(d_depth); cudaFree(d_off); cudaFree(d_jobs); };
-  try {
-    d_eid = dalloc<int>(total, tmp);
-    d_depth = dalloc<int>(voff[K], tmp);
-    d_off = dalloc<int64_t>(K + 1, tmp);
-    d_jobs = dalloc<RmqJob>(K, tmp);
+  DeviceArena ws;
+  {
+    int *d_eid = ws.get<int>(total), *d_depth = ws.get<int>(voff[K]);
+    int64_t *d_off = ws.get<int64_t>(K + 1);
+    RmqJob *d_jobs = ws.get<RmqJob>(K);
     std::vector<RmqJob> jobs(K);
     for (int i = 0; i < K; i++) {
       Graph &g = *gs[i];
       DeviceIndex &D = g.dev;
-      for (void *p : D.owned_rmq) cudaFree(p);
-      D.owned_rmq.clear();
-      D.bytes -= D.rmq_bytes;
-      D.rmq_bytes = 0;
-      D.euler = g.euler_n;
       g.rmq_total = rmq_prefix(g.euler_n);
-      D.rmq = g.rmq_total;
-      D.first = dalloc<int>(g.n, D.rmq_bytes);
-      D.owned_rmq.push_back(D.first);
-      D.rmq_hash = dalloc<int64_t>(D.euler, D.rmq_bytes);
-      D.owned_rmq.push_back(D.rmq_hash);
-      D.rmq_id = dalloc<int>(D.rmq, D.rmq_bytes);
-      D.owned_rmq.push_back(D.rmq_id);
-      D.bytes += D.rmq_bytes;
+      allocate_rmq(g);
       GH_CUDA(cudaMemcpy(D.first, g.first.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
       GH_CUDA(cudaMemcpy(d_eid + off[i], g.euler_id.data(), sizeof(int) * g.euler_n, cudaMemcpyHostToDevice));
       GH_CUDA(cudaMemcpy(d_depth + voff[i], g.depth.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
@@ -282,11 +273,8 @@ void build_rmq_gpu(const std::vector<Graph *> &gs) {
       GH_CUDA(cudaGetLastError());
     }
     GH_CUDA(cudaDeviceSynchronize());
-  } catch (...) {
-    cleanup();
-    throw;
   }
-  cleanup();
+  ws.release();
   const long long us = clk.us();
   for (Graph *g : gs) {
     std::vector<int>().swap(g->euler_id);
@@ -295,20 +283,8 @@ void build_rmq_gpu(const std::vector<Graph *> &gs) {
 }
 
 void upload_rmq(Graph &g, const std::vector<int64_t> &rmq_hash, const std::vector<int> &rmq_id) {
+  allocate_rmq(g);
   DeviceIndex &D = g.dev;
-  for (void *p : D.owned_rmq) cudaFree(p);
-  D.owned_rmq.clear();
-  D.bytes -= D.rmq_bytes;
-  D.rmq_bytes = 0;
-  D.euler = g.euler_n;
-  D.rmq = g.rmq_total;
-  D.first = dalloc<int>(g.n, D.rmq_bytes);
-  D.owned_rmq.push_back(D.first);
-  D.rmq_hash = dalloc<int64_t>(D.euler, D.rmq_bytes);
-  D.owned_rmq.push_back(D.rmq_hash);
-  D.rmq_id = dalloc<int>(D.rmq, D.rmq_bytes);
-  D.owned_rmq.push_back(D.rmq_id);
-  D.bytes += D.rmq_bytes;
   GH_CUDA(cudaMemcpy(D.first, g.first.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
   GH_CUDA(cudaMemcpy(D.rmq_hash, rmq_hash.data(), sizeof(int64_t) * D.euler, cudaMemcpyHostToDevice));
   GH_CUDA(cudaMemcpy(D.rmq_id, rmq_id.data(), sizeof(int) * D.rmq, cudaMemcpyHostToDevice));

@@ -5,9 +5,8 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <vector>
 
-#include "common.h"
+#include "arena.h"
 
 namespace gh {
 
@@ -63,19 +62,7 @@ __global__ void scan_add_kernel(int64_t *out, int64_t n, const int64_t *tile_off
 }
 
 // Device scratch of one build, freed together.
-struct Workspace {
-  std::vector<void *> p;
-  template <typename T>
-  T *get(int64_t n) {
-    T *q = nullptr;
-    GH_CUDA(cudaMalloc(&q, sizeof(T) * (size_t)std::max<int64_t>(n, 1)));
-    p.push_back(q);
-    return q;
-  }
-  ~Workspace() {
-    for (void *q : p) cudaFree(q);
-  }
-};
+using Workspace = DeviceArena;
 
 // out[i] = sum of in[0 .. i) for i < n (tile sums scanned recursively).
 template <typename T>

@@ -418,16 +418,6 @@ __global__ void gather_ids_kernel(const int64_t *slot_off, const int *lsize, con
   }
 }
 
-template <typename T>
-T *palloc(size_t n, int64_t &bytes) {
-  T *p = nullptr;
-  if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  bytes += (int64_t)(n * sizeof(T));
-  return p;
-}
-
 // Alive members of every cell at its level, or false when the cut rows do not
 // nest (each level tiling the positions, a cell split by its two children).
 bool cell_sizes(const Graph &g, std::vector<int> &size) {
@@ -476,7 +466,7 @@ bool ElimPlan::plan_bits() {
   }
   steps.resize(nsteps + 1);
   std::vector<int> f_members(N);  // the bottom cells' members come first, in partition order
-  int64_t mem = N;
+  int64_t mem_total = N;
   for (int i = 0; i < K; i++) {
     const Graph &g = *gs[i];
     const int vb = vbase[i], levels = g.H - g.C;
@@ -487,8 +477,8 @@ bool ElimPlan::plan_bits() {
     for (int64_t c = 0; c < (int64_t)sizes[i].size() && c < (int64_t(1) << g.C) - 1; c++) heap_n += g.cell_count[c];
     if (heap_n > kMaxMembers) return false;
     if (levels > 0) {
-      heap_region = mem;
-      mem += heap_n;
+      heap_region = mem_total;
+      mem_total += heap_n;
     }
     int64_t heap_at = heap_region;
     for (int h = g.H; h > g.C; h--) {
@@ -501,8 +491,8 @@ bool ElimPlan::plan_bits() {
         if (h - 1 > g.C) {
           const int64_t p = (c - 1) / 2;
           if (region[p] < 0) {
-            region[p] = mem;
-            mem += sizes[i][p];
+            region[p] = mem_total;
+            mem_total += sizes[i][p];
           }
           out = region[p] + (c & 1 ? 0 : sizes[i][c - 1] - g.cell_count[c - 1]);
         } else {
@@ -618,11 +608,11 @@ bool ElimPlan::plan_bits() {
     i = j;
   }
   try {
-    members = palloc<int>(mem, bytes);
-    extra = palloc<int>(N, bytes);
-    fin = palloc<unsigned char>(N, bytes);
-    sym_cells = palloc<unsigned char>(sizeof(SymCell) * table.size(), bytes);
-    if (grow_words) grows = palloc<unsigned>(grow_words, bytes);
+    members = mem.get<int>(mem_total);
+    extra = mem.get<int>(N);
+    fin = mem.get<unsigned char>(N);
+    sym_cells = mem.get<unsigned char>(sizeof(SymCell) * table.size());
+    if (grow_words) grows = mem.get<unsigned>(grow_words);
     GH_CUDA(cudaMemcpy(members, f_members.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(sym_cells, table.data(), sizeof(SymCell) * table.size(), cudaMemcpyHostToDevice));
   } catch (...) {

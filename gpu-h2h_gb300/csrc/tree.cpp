@@ -107,14 +107,14 @@ void prefix_sums(Pool &pool, int64_t n, std::vector<int64_t> &out, F val) {
 }  // namespace
 
 void position_offsets(Graph &g) {
-  Pool pool(g.threads);
+  Pool pool(useful_threads(g.threads, g.n));
   prefix_sums(pool, g.n, g.pos_hash, [&](int64_t v) { return (int64_t)(g.x_off[v + 1] - g.x_off[v]) + 1; });
 }
 
 void allocate_labels_and_bfs(Graph &g) {
   Clock clk;
   const int n = g.n;
-  Pool pool(g.threads);
+  Pool pool(useful_threads(g.threads, g.n));
   if (!g.tree_layout) prefix_sums(pool, n, g.dis_hash, [&](int64_t v) { return (int64_t)g.depth[v]; });
   if (!g.plan) prefix_sums(pool, n, g.pos_hash, [&](int64_t v) { return (int64_t)(g.x_off[v + 1] - g.x_off[v]) + 1; });
   // host position lists only for the level-synchronous fill; the block
