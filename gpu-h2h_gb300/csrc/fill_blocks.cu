@@ -555,6 +555,8 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
   __shared__ __align__(16) unsigned s_L[kRows * 36];
   __shared__ __align__(16) unsigned s_P[2][kRows * 68];
   __shared__ int s_up[2][64];
+  __shared__ int64_t s_pso, s_puo;  // the parent's cells, triangle, members and row padding
+  __shared__ int s_pm, s_pRp;
   __shared__ int s_t, s_flag;
   const BlockArgs &B = A.B;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -579,6 +581,12 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
     if (p >= 0) {
       const int k = 64 * (tid < 64 ? X : Y) + (tid & 63);
       s_up[tid >> 6][tid & 63] = k < m ? __ldg(A.bm_up + m0 + k) : 0;
+      if (tid == 32) {
+        s_pso = __ldg(B.soff + p);
+        s_puo = __ldg(A.uoff + p);
+        s_pm = (int)(__ldg(B.moff + p + 1) - __ldg(B.moff + p));
+        s_pRp = ((int)(__ldg(B.boff + p + 1) - __ldg(B.boff + p)) + 3) & ~3;
+      }
     }
     if (tid == 0) {
       int ok = 1;
@@ -597,36 +605,27 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
     __syncthreads();
     if (!s_flag) return;
     unsigned *const cells = B.direct + so;
-    // the block's own triangle
-    for (int i = tid; i < kRows * 36; i += 128) s_L[i] = kInf;
-    __syncthreads();
-    for (int i = tid; i < R * Rp; i += 128) {
-      const int c = i / Rp, r = i - c * Rp;
-      if (r > c && r < R) s_L[r * 36 + c] = __ldcg(cells + (int64_t)(m + c) * Rp + r);
-    }
-    __syncthreads();
-    for (int i = R - 1; i > 1; i--) {
-      const unsigned li = s_L[i * 36 + lane];
-      unsigned ups = __ballot_sync(0xffffffffu, li != kInf && lane < i);
-      int turn = 0;
-      while (ups) {
-        const int u = __ffs(ups) - 1;
-        ups &= ups - 1;
-        if ((turn++ & 3) == wid && lane < u)
-          s_L[u * 36 + lane] = add_min(s_L[i * 36 + u], li, s_L[u * 36 + lane]);
-      }
-      __syncthreads();
-    }
-    if (sub == 0)
-      for (int i = tid; i < R * Rp; i += 128) {
-        const int c = i / Rp, r = i - c * Rp;
-        if (r > c && r < R) cells[(int64_t)(m + c) * Rp + r] = s_L[r * 36 + c];
-      }
-    // the tile's columns, one per lane
+    // loads first: the update triangle's tile (what the blocks below added),
+    // the columns, one per lane, and the block's own triangle
+    const int xg = tid & 15, yg = tid >> 4;  // this thread's patch: 4 x by 8 y, lanes along x
+    const int x0 = 64 * X + 4 * xg, y0 = 64 * Y + 8 * yg;
     const int half = wid >> 1;  // warps 0, 1: X's columns; 2, 3: Y's
     const int k = 64 * (half ? Y : X) + 32 * (wid & 1) + lane;
-    if (!(diag && half) && 64 * (half ? Y : X) + 32 * (wid & 1) < m) {
-      unsigned col[kRows];
+    const bool solve = !(diag && half) && 64 * (half ? Y : X) + 32 * (wid & 1) < m;
+    unsigned acc[8][4];
+    {
+      const int64_t uo = __ldg(A.uoff + b);
+      const bool below = __ldg(A.uoff + b + 1) > uo;
+#pragma unroll
+      for (int y = 0; y < 8; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          const int xx = x0 + x, yy = y0 + y;
+          acc[y][x] = below && yy < m && xx < yy ? __ldcg(A.upd + uo + (int64_t)yy * (yy - 1) / 2 + xx) : kInf;
+        }
+    }
+    unsigned col[kRows];
+    if (solve) {
       const uint4 *src = reinterpret_cast<const uint4 *>(cells + (int64_t)min(k, m - 1) * Rp);
 #pragma unroll
       for (int q = 0; q < kRows / 4; q++) {
@@ -636,6 +635,31 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
         col[4 * q + 2] = x.z;
         col[4 * q + 3] = x.w;
       }
+    }
+    // the block's own triangle, eliminated by the last warp (which on the
+    // diagonal has no columns): lane c holds column c of every row
+    if (wid == 3) {
+      unsigned row[kRows];
+      const unsigned *src = cells + (int64_t)(m + lane) * Rp;
+#pragma unroll
+      for (int i = 0; i < kRows; i++) row[i] = lane < i && i < R ? __ldcg(src + i) : kInf;
+#pragma unroll
+      for (int i = kRows - 1; i > 1; i--)
+        if (i < R) {
+#pragma unroll
+          for (int u = 1; u < i; u++) row[u] = add_min(__shfl_sync(0xffffffffu, row[i], u), lane < u ? row[i] : kInf, row[u]);
+        }
+#pragma unroll
+      for (int i = 0; i < kRows; i++) s_L[i * 36 + lane] = row[i];
+    }
+    __syncthreads();
+    if (sub == 0)
+      for (int i = tid; i < R * Rp; i += 128) {
+        const int c = i / Rp, r = i - c * Rp;
+        if (r > c && r < R) cells[(int64_t)(m + c) * Rp + r] = s_L[r * 36 + c];
+      }
+    // the tile's columns
+    if (solve) {
 #pragma unroll
       for (int i = kRows - 1; i > 0; i--)
         if (i < R) {
@@ -663,15 +687,7 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
     }
     if (p < 0) continue;
     __syncthreads();
-    // the tile of the update: lanes along x, so an address run of the parent
-    const int xg = tid & 15, yg = tid >> 4;
-    const int x0 = 64 * X + 4 * xg, y0 = 64 * Y + 8 * yg;
     if (x0 < m && y0 < m) {
-      unsigned acc[8][4];
-#pragma unroll
-      for (int y = 0; y < 8; y++)
-#pragma unroll
-        for (int x = 0; x < 4; x++) acc[y][x] = kInf;
       const unsigned *px = s_P[0] + 4 * xg, *py = s_P[diag ? 0 : 1] + 8 * yg;
 #pragma unroll 2
       for (int i = 0; i < R; i++) {
@@ -687,11 +703,8 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
           acc[y][3] = add_min(yv[y], a.w, acc[y][3]);
         }
       }
-      const int64_t uo = __ldg(A.uoff + b);
-      const bool below = __ldg(A.uoff + b + 1) > uo;
-      const int64_t pso = __ldg(B.soff + p), puo = __ldg(A.uoff + p);
-      const int pm = (int)(__ldg(B.moff + p + 1) - __ldg(B.moff + p));
-      const int pRp = ((int)(__ldg(B.boff + p + 1) - __ldg(B.boff + p)) + 3) & ~3;
+      const int64_t pso = s_pso, puo = s_puo;
+      const int pm = s_pm, pRp = s_pRp;
 #pragma unroll
       for (int y = 0; y < 8; y++) {
         const int yy = y0 + y;
@@ -701,8 +714,7 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
         for (int x = 0; x < 4; x++) {
           const int xx = x0 + x;
           if (xx >= yy) break;
-          unsigned v = acc[y][x];
-          if (below) v = min(v, __ldcg(A.upd + uo + (int64_t)yy * (yy - 1) / 2 + xx));
+          const unsigned v = acc[y][x];
           if (v >= kInf) continue;
           const int cx = s_up[0][4 * xg + x];
           unsigned *dst;
