@@ -17,12 +17,13 @@
 // and a grid barrier); on bit rows in shared memory it is a block argmin and
 // a few word operations per neighbour.  The weights are computed afterwards,
 // for all vertices, over the blocks of the finished tree (fill_blocks.cu).
-// On one GB300, order and weights together against the list kernels: 42 ->
-// 14 ms on a 264k-vertex road graph (global order 18.8 -> 3.4 ms, 2.1 us a
-// pick), 127 -> 31 ms on a 1M-vertex one (45.9 -> 7.9 ms), 27 -> 3.2 ms for a
-// rebuild of 16 graphs after new weights, which repeats no elimination.
-// Bound: the chain of picks; a pick is an argmin, two to four barriers and one
-// pass over the neighbours' rows.
+// On one GB300, against the list kernels: partition levels 23 -> 2.9 ms and
+// global order 18.8 -> 2.8 ms (1.8 us a pick) on a 264k-vertex road graph, 81
+// -> 8.0 and 45.9 -> 6.7 ms on a 1M-vertex one, where they also made the
+// weights (1.5 and 4.6 ms here); a rebuild after new weights repeats no
+// elimination (16 graphs: 27 -> 2.5 ms).  Bound: the chain of picks; a pick is
+// an argmin over the row groups, two or three barriers and one pass over the
+// neighbours' rows.
 //
 // One thread-block cluster per cell; member l's row, counters and key belong
 // to CTA l mod CS.  Per elimination: every CTA's best key (degree + height,
@@ -57,11 +58,13 @@ constexpr int kErrPick = 5;      // no candidate left to pick, or a vertex outsi
 
 constexpr int kIdxBits = 14, kDegBits = 22, kSumBits = 28;  // a key: degree + height, degree, member
 constexpr int kMaxMembers = 1 << kIdxBits;
+constexpr int kMaxGroups = 64;
 constexpr unsigned long long kNoKey = ~0ull;
 
 struct SymCell {
   int start, count, size, src;  // candidates in elim; members; slot buffer its lists are read from
-  int64_t mem, out;             // members; where the ones that stay go (the parent's members)
+  int64_t mem, out;             // members; where the ones that stay go (a run of the parent's members)
+  int obase;                    // that run's start within the parent's members
 };
 
 struct SymArgs {
@@ -92,19 +95,16 @@ __device__ __forceinline__ int find_id(const int *ids, int n, int x) {
 }
 
 __device__ __forceinline__ unsigned long long warp_min(unsigned long long k) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long y = __shfl_xor_sync(0xffffffffu, k, o);
-    k = y < k ? y : k;
-  }
-  return k;
+  const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
+  const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : ~0u);
+  return ((unsigned long long)hi << 32) | lo;
 }
 
 template <bool kGlobal>
 __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ unsigned long long s_wmin[2][16];
-  __shared__ unsigned long long s_best[2][16];
+  __shared__ unsigned long long s_gmin[2][kMaxGroups];  // best key of every group of rows
+  __shared__ unsigned long long s_best[2][16];          // best key of every CTA
   cg::cluster_group cluster = cg::this_cluster();
   const int CS = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int ci = (int)(blockIdx.x / CS);
@@ -112,8 +112,9 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
   const int S = c.size, k = c.count, W = (S + 31) >> 5;
   if (S == 0) return;  // uniform across the cluster
-  const int ownmax = (A.smax + CS - 1) / CS, Wm = ((A.smax + 31) >> 5) | 1;  // odd row stride: no bank conflicts
-  const int nown = (S - rank + CS - 1) / CS;
+  const int csh = 31 - __clz(CS);  // clusters are powers of two
+  const int ownmax = (A.smax + CS - 1) >> csh, Wm = ((A.smax + 31) >> 5) | 1;  // odd row stride: no bank conflicts
+  const int nown = (S - rank + CS - 1) >> csh;
   unsigned long long *key = (unsigned long long *)smem;
   int *ids = (int *)(key + ownmax);
   int *vc = ids + A.npow;   // neighbours inside the cell
@@ -122,7 +123,8 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
   int *junk = ext + ownmax;
   int *hgt = junk + ownmax;
   int *cap = hgt + ownmax;  // list capacity (partition cells)
-  unsigned *rowv = (unsigned *)(cap + ownmax);
+  int *map = cap + ownmax;  // place in id order of every entry of the members' array; then the rank of the ones that stay
+  unsigned *rowv = (unsigned *)(map + A.smax);
   unsigned *cand = rowv + Wm;
   unsigned *srows = cand + Wm;
   unsigned *const grows = kGlobal ? A.grows + (int64_t)ci * A.smax * Wm : nullptr;
@@ -147,6 +149,7 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
       }
       __syncthreads();
     }
+  for (int i = tid; i < S; i += nthr) map[i] = find_id(ids, S, A.members[c.mem + i]);
   for (int i = tid; i < k; i += nthr) {
     const int l = find_id(ids, S, A.elim[c.start + i]);
     if (l >= 0) atomicOr(cand + (l >> 5), 1u << (l & 31));
@@ -162,9 +165,13 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
     const int64_t off = A.slot_off[u];
     const int n = A.lsize[u];
     const int *list = A.slot[c.src] + off;
+    // an entry is a place in the members' array, or ~id of a vertex that was
+    // outside the cell below
     int out = 0;
+#pragma unroll 4
     for (int e = lane; e < n; e += 32) {
-      const int x = find_id(ids, S, __ldcg(list + e));
+      const int y = __ldcg(list + e);
+      const int x = y < 0 ? find_id(ids, S, ~y) : y < S ? map[y] : -1;
       if (x >= 0) atomicOr(row + (x >> 5), 1u << (x & 31));
       else out++;
     }
@@ -184,12 +191,26 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
   }
   __syncthreads();
   if (CS > 1) cluster.sync();
-  // Two ways through v's neighbours.  Few of them: a warp takes its rows one
-  // at a time, a lane per word (the rows of a warp are G apart: neighbours
-  // have close ids).  Many: T lanes take a row, 32 / T rows at once, so the
-  // cost is the rows' words and not their number.  The second way pays from
-  // about dense_deg neighbours (60 cycles a row against 10 a word).
+  // Row r belongs to group r mod G, a lane of the group's warp (neighbours
+  // have close ids, so they spread over the groups).  Each group's best key is
+  // kept, so a pick looks at the groups and an update at the groups it hits.
+  // Two ways through v's neighbours.  Few of them: a group's warp takes its
+  // rows one at a time, a lane per word.  Many: T lanes take a row, 32 / T rows
+  // at once, so the cost is the rows' words and not their number, and every
+  // group's best key is taken anew.  The second way pays from about dense_deg
+  // neighbours (60 cycles a row against 10 a word).
   const int G = max(nw, (nown + 31) >> 5);
+  for (int g = tid; g < 2 * kMaxGroups; g += nthr) s_gmin[g / kMaxGroups][g % kMaxGroups] = kNoKey;
+  __syncthreads();
+  auto regroup = [&](int buf) {  // every group's best key
+    for (int g = wid; g < G; g += nw) {
+      const int r = lane * G + g;
+      const unsigned long long best = warp_min(r < nown ? key[r] : kNoKey);
+      if (lane == 0) s_gmin[buf][g] = best;
+    }
+    __syncthreads();
+  };
+  regroup(0);
   int T = 1;
   while (T < 8 && 2 * T * nown <= nthr) T <<= 1;
   const int per = 32 / T, rounds = (nown + per * nw - 1) / (per * nw);
@@ -220,19 +241,16 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
   for (int j = 0; j < k; j++) {
     const int par = j & 1;
     // ---- the pick
-    unsigned long long b = kNoKey;
-    for (int r = tid; r < nown; r += nthr) {
-      const unsigned long long x = key[r];
-      b = x < b ? x : b;
+    unsigned long long b;
+    {
+      const unsigned long long x = s_gmin[par][lane], y = s_gmin[par][lane + 32];
+      b = x < y ? x : y;
     }
-    b = warp_min(b);
-    if (lane == 0) s_wmin[par][wid] = b;
-    __syncthreads();
     if (CS == 1) {
-      b = warp_min(lane < nw ? s_wmin[par][lane] : kNoKey);
+      b = warp_min(b);
     } else {
       if (wid == 0) {
-        b = warp_min(lane < nw ? s_wmin[par][lane] : kNoKey);
+        b = warp_min(b);
         if (lane < CS) *cluster.map_shared_rank(&s_best[par][rank], lane) = b;
       }
       cluster.sync();
@@ -244,41 +262,55 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
     }
     const int lv = (int)(b & (kMaxMembers - 1));
     const int hnow = (int)(b >> (kIdxBits + kDegBits)) - (int)((b >> kIdxBits) & ((1u << kDegBits) - 1));
-    const int owner = lv % CS;
+    const int owner = lv & (CS - 1);
     const unsigned *rv;
     if (CS == 1 && !kGlobal) {
       rv = own_row(lv);
     } else {
       const unsigned *src = kGlobal ? grows + (int64_t)lv * Wm
-                                    : cluster.map_shared_rank(srows, owner) + (int64_t)(lv / CS) * Wm;
+                                    : cluster.map_shared_rank(srows, owner) + (int64_t)(lv >> csh) * Wm;
       for (int w = tid; w < W; w += nthr) rowv[w] = kGlobal ? __ldcg(src + w) : src[w];
       __syncthreads();
       rv = rowv;
     }
     // ---- its neighbours among the owned members
+    const int rlv = owner == rank ? lv >> csh : -1;  // v's own row, if it is one of this CTA's
+    auto retire = [&]() {
+      key[rlv] = kNoKey;
+      A.elim[c.start + j] = ids[lv];
+      if (vc[rlv] == 0 && !A.heap) atomicCAS(A.err, 0, kErrEmpty);  // a partition cell never isolates a candidate
+    };
     if ((int)((b >> kIdxBits) & ((1u << kDegBits) - 1)) < dense_deg) {
       for (int g = wid; g < G; g += nw) {
         const int r0 = lane * G + g, l0 = r0 * CS + rank;
         const bool hit = r0 < nown && ((rv[l0 >> 5] >> (l0 & 31)) & 1u);
         unsigned todo = __ballot_sync(0xffffffffu, hit);
-        int mine = 0;
-        while (todo) {
-          const int at = __ffs(todo) - 1, r = at * G + g, l = r * CS + rank;
-          todo &= todo - 1;
-          unsigned *row = own_row(r);
-          int pc = 0;
-          for (int w = lane; w < W; w += 32) {
-            unsigned x = (kGlobal ? __ldcg(row + w) : row[w]) | rv[w];
-            if (w == (l >> 5)) x &= ~(1u << (l & 31));
-            if (w == (lv >> 5)) x &= ~(1u << (lv & 31));
-            row[w] = x;
-            pc += __popc(x);
+        const bool mine = __any_sync(0xffffffffu, r0 == rlv);
+        unsigned long long best = s_gmin[par][g];
+        if (todo || mine) {
+          int deg = 0;
+          while (todo) {
+            const int at = __ffs(todo) - 1, r = at * G + g, l = r * CS + rank;
+            todo &= todo - 1;
+            unsigned *row = own_row(r);
+            int pc = 0;
+            for (int w = lane; w < W; w += 32) {
+              unsigned x = (kGlobal ? __ldcg(row + w) : row[w]) | rv[w];
+              if (w == (l >> 5)) x &= ~(1u << (l & 31));
+              if (w == (lv >> 5)) x &= ~(1u << (lv & 31));
+              row[w] = x;
+              pc += __popc(x);
+            }
+            pc = __reduce_add_sync(0xffffffffu, pc);
+            if (lane == at) deg = pc;
           }
-          pc = __reduce_add_sync(0xffffffffu, pc);
-          if (lane == at) mine = pc;
+          if (hit) settle(r0, deg, lv, hnow);
+          if (r0 == rlv) retire();
+          best = warp_min(r0 < nown ? key[r0] : kNoKey);  // each lane reads the key it alone writes
         }
-        if (hit) settle(r0, mine, lv, hnow);
+        if (lane == 0) s_gmin[par ^ 1][g] = best;
       }
+      __syncthreads();
     } else {
       const int sub = lane & (T - 1);
       for (int g = wid; g * per < nown; g += nw) {
@@ -298,66 +330,65 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
         for (int o = 1; o < T; o <<= 1) pc += __shfl_xor_sync(0xffffffffu, pc, o);
         if (hit && sub == 0) settle(r, pc, lv, hnow);
       }
+      if (rlv >= 0 && tid == 0) retire();
+      __syncthreads();
+      regroup(par ^ 1);
     }
-    if (rank == owner && tid == 0) {
-      key[lv / CS] = kNoKey;
-      A.elim[c.start + j] = ids[lv];
-      if (vc[lv / CS] == 0 && !A.heap) atomicCAS(A.err, 0, kErrEmpty);  // a partition cell never isolates a candidate
-    }
-    __syncthreads();
     if (j == 0 && !A.heap) {  // live keys from the second pick on
       for (int r = tid; r < nown; r += nthr)
         if (key[r] != kNoKey) key[r] = pack_key(junk[r] + vc[r] + outc[r] + ext[r], hgt[r], r * CS + rank);
       __syncthreads();
+      regroup(par ^ 1);
     }
   }
-  // ---- lists: an eliminated member's row is its X in id order, a boundary
-  // member's new list is its row, then its entries outside the cell
+  // ---- lists: an eliminated member's row is its X in id order; a member that
+  // stays lists its entries outside the cell, then its row as places in the
+  // parent's members (the ones that stay go there in id order)
+  if (wid == 0) {
+    int q = 0;
+    for (int l0 = 0; l0 < S; l0 += 32) {
+      const int l = l0 + lane;
+      const bool stay = l < S && !((cand[l >> 5] >> (l & 31)) & 1u);
+      const unsigned bal = __ballot_sync(0xffffffffu, stay);
+      const int at = q + __popc(bal & ((1u << lane) - 1u));
+      if (l < S) map[l] = c.obase + at;
+      if (stay && rank == 0 && c.out >= 0) A.members[c.out + at] = ids[l];
+      q += __popc(bal);
+    }
+  }
+  __syncthreads();
   for (int r = wid; r < nown; r += nw) {
     const int l = r * CS + rank, u = ids[l];
     const bool gone = (cand[l >> 5] >> (l & 31)) & 1u;
-    const int in = vc[r], len = in + outc[r];
+    const int out = gone ? 0 : outc[r], len = vc[r] + out;
     int64_t off = A.slot_off[u];
     const int64_t old = off;
-    const int cap = A.cap[u], n0 = A.lsize[u];
-    if (A.heap && len > cap) {  // a global-order list may outgrow its range
+    if (A.heap && len > A.cap[u]) {  // a global-order list may outgrow its range
       unsigned long long at = 0;
       if (lane == 0) at = atomicAdd(A.pool_next, (unsigned long long)len);
       off = (int64_t)__shfl_sync(0xffffffffu, at, 0);
     }
-    const bool fits = A.heap ? off + len <= A.pool_size : len <= cap;
+    const bool fits = A.heap ? off + len <= A.pool_size : len <= cap[r];
     if (fits) {
       int *dst = A.slot[c.src ^ 1] + off;
-      const unsigned *row = own_row(r);
-      int base = 0;
-      for (int w0 = 0; w0 < W; w0 += 32) {
-        const int w = w0 + lane;
-        unsigned x = w < W ? (kGlobal ? __ldcg(row + w) : row[w]) : 0u;
-        const int pc = __popc(x);
-        int incl = pc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += y;
-        }
-        int at = base + incl - pc;
-        while (x) {
-          const int bit = __ffs(x) - 1;
-          x &= x - 1;
-          dst[at++] = ids[w * 32 + bit];
-        }
-        base += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (len > in) {
+      int q = 0;
+      if (out > 0) {
         const int *list = A.slot[c.src] + old;
-        int q = in;
-        for (int e0 = 0; e0 < n0; e0 += 32) {
-          const int x = e0 + lane < n0 ? __ldcg(list + e0 + lane) : -1;
-          const bool out = x >= 0 && find_id(ids, S, x) < 0;
-          const unsigned bal = __ballot_sync(0xffffffffu, out);
-          if (out) dst[q + __popc(bal & ((1u << lane) - 1u))] = x;
+        const int n0 = A.lsize[u];
+        for (int e0 = 0; e0 < n0 && q < out; e0 += 32) {
+          const int y = e0 + lane < n0 ? __ldcg(list + e0 + lane) : 0;
+          const bool o = y < 0 && find_id(ids, S, ~y) < 0;
+          const unsigned bal = __ballot_sync(0xffffffffu, o);
+          if (o) dst[q + __popc(bal & ((1u << lane) - 1u))] = y;
           q += __popc(bal);
         }
+      }
+      const unsigned *row = own_row(r);
+      const int *name = gone ? ids : map;
+      for (int w = 0; w < W; w++) {
+        const unsigned x = kGlobal ? __ldcg(row + w) : row[w];
+        if ((x >> lane) & 1u) dst[q + __popc(x & ((1u << lane) - 1u))] = name[w * 32 + lane];
+        q += __popc(x);
       }
     }
     if (lane == 0) {
@@ -370,21 +401,11 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
       A.fin[u] = (unsigned char)(c.src ^ 1);
     }
   }
-  if (rank == 0 && wid == 0 && c.out >= 0) {
-    int q = 0;
-    for (int l0 = 0; l0 < S; l0 += 32) {
-      const int l = l0 + lane;
-      const bool stay = l < S && !((cand[l >> 5] >> (l & 31)) & 1u);
-      const unsigned bal = __ballot_sync(0xffffffffu, stay);
-      if (stay) A.members[c.out + q + __popc(bal & ((1u << lane) - 1u))] = ids[l];
-      q += __popc(bal);
-    }
-  }
   if (CS > 1) cluster.sync();  // no CTA leaves while a peer may still read its rows
 }
 
-// Distinct neighbours of every vertex's input list (in id order) and the
-// number of repeated entries.
+// Distinct neighbours of every vertex's input list as ~id and the number of
+// repeated entries.
 __global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, const int64_t *slot_off, int *slot,
                                       int *lsize, int *extra, int n) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
@@ -392,13 +413,10 @@ __global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, cons
     const int b = adj_off[v], e = adj_off[v + 1];
     int c = 0;
     for (int i = b; i < e; i++) {
-      const int x = adj_v[i];
-      int k = c;
-      while (k > 0 && list[k - 1] > x) k--;
-      if (k > 0 && list[k - 1] == x) continue;
-      for (int q = c; q > k; q--) list[q] = list[q - 1];
-      list[k] = x;
-      c++;
+      const int x = ~adj_v[i];
+      bool seen = false;
+      for (int q = 0; q < c && !seen; q++) seen = list[q] == x;
+      if (!seen) list[c++] = x;
     }
     lsize[v] = c;
     extra[v] = e - b - c;
@@ -487,31 +505,38 @@ bool ElimPlan::plan_bits() {
         if (sizes[i][c] > kMaxMembers) return false;
         if (h == g.H) region[c] = vb + g.cut_l[c];
         const int stay = sizes[i][c] - g.cell_count[c];
-        int64_t out;
+        int64_t out, parent;
         if (h - 1 > g.C) {
           const int64_t p = (c - 1) / 2;
           if (region[p] < 0) {
             region[p] = mem_total;
             mem_total += sizes[i][p];
           }
-          out = region[p] + (c & 1 ? 0 : sizes[i][c - 1] - g.cell_count[c - 1]);
+          parent = region[p];
+          out = parent + (c & 1 ? 0 : sizes[i][c - 1] - g.cell_count[c - 1]);
         } else {
+          parent = heap_region;
           out = heap_at;
           heap_at += stay;
         }
         const int st = g.H - h;
-        steps[st].push_back({{vb + g.cell_start[c], g.cell_count[c], sizes[i][c], st & 1, region[c], out},
+        steps[st].push_back({{vb + g.cell_start[c], g.cell_count[c], sizes[i][c], st & 1, region[c], out,
+                              (int)(out - parent)},
                              K > 1 ? -(st + 1) : h});
       }
     }
     if (levels > 0 && heap_at != heap_region + heap_n) return false;
     int heap_start = g.n - heap_n;
-    steps[nsteps].push_back({{vb + heap_start, heap_n, heap_n, levels & 1, heap_region, -1}, 0});
+    steps[nsteps].push_back({{vb + heap_start, heap_n, heap_n, levels & 1, heap_region, -1, 0}, 0});
   }
   // ---- launches: a step's cells by size class, each class with its own
-  // cluster size.  A pick costs a fixed part (argmin and barriers: about 0.5
-  // us in one CTA, 1.2 us across a cluster) and its neighbours' rows, which a
-  // cluster shares.
+  // cluster size.  A pick costs a fixed part (argmin and barriers: 1.1 us in
+  // one CTA, 1.5 us across a cluster) and its neighbours' rows, 1 us + 45 ps
+  // per word of the cell, which a cluster shares.  Measured us per pick with 1
+  // / 2 / 4 / 8 / 16 CTAs: 716 members 3.4 / 2.9 / 2.3 / 1.9 / 1.9, 1,604 members
+  // - / - / 2.5 / 2.0 / 1.8, 2,968 members - / - / - / 2.7 / 2.3.  Cells that
+  // outnumber the SMs keep few warps (1,024 cells of 259 members: 0.54 ms with
+  // 4 warps, 0.67 with 8; 2,048 cells of 489: 3.7 with 4, 2.8 with 8, 3.9 with 16).
   cudaFuncAttributes fa;
   GH_CUDA(cudaFuncGetAttributes(&fa, symbolic_kernel<false>));
   const int smem_dyn = enable_max_dynamic_smem(symbolic_kernel<false>);
@@ -528,7 +553,7 @@ bool ElimPlan::plan_bits() {
   };
   auto smem_for = [&](int smax, int cs, bool global) -> int64_t {
     const int64_t own = (smax + cs - 1) / cs, w = (smax + 31) / 32 | 1;
-    return own * (8 + 24) + 4LL * pow2(smax) + 8 * w + (global ? 0 : 4 * own * w);
+    return own * (8 + 24) + 4LL * smax + 4LL * pow2(smax) + 8 * w + (global ? 0 : 4 * own * w);
   };
   std::vector<SymCell> table;
   int64_t grow_words = 0;
@@ -560,7 +585,8 @@ bool ElimPlan::plan_bits() {
           const int64_t sm = smem_for(smax, cs, global);
           if (sm > smem_dyn || (global && cs < 16)) continue;
           const int own = (smax + cs - 1) / cs, w = (smax + 31) / 32;
-          const int nw = own >= 400 || (cs > 1 && own >= 64) ? 16 : own >= 96 ? 8 : 4;
+          int nw = cs > 1 ? (own >= 64 ? 16 : 8) : L.ncell > 4 * nsm ? (own >= 384 ? 8 : 4) : own >= 300 ? 16 : 8;
+          if ((own + 31) / 32 > kMaxGroups) continue;
           int fit = 0;
           cudaLaunchConfig_t cfg = {};
           cudaLaunchAttribute attr[1];
@@ -580,8 +606,7 @@ bool ElimPlan::plan_bits() {
             continue;
           }
           const double waves = std::ceil((double)L.ncell / fit);
-          const double words = 0.4 * own * w / (32.0 * nw);  // a lane's words per pick
-          const double cost = waves * ((cs == 1 ? 0.6 : 1.8) + 0.01 * words);
+          const double cost = waves * ((cs == 1 ? 1.1 : 1.5) + (1.0 + 4.5e-5 * smax * w) / cs);
           if (cost < best * 0.99) {
             best = cost;
             L.cs = cs;
