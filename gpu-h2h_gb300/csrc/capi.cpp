@@ -248,6 +248,27 @@ int h2h_query_batch_host(const h2h_graph *hc, const int *x, const int *y, int *o
     gh::HostQueryStage &s = h->stage;
     std::lock_guard<std::mutex> lock(s.mu);
     if (!s.stream) GH_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+    // Up to 4,096 pairs go through page-locked memory that the kernel reads and
+    // writes in place: one launch instead of a launch and four copies (a single
+    // pair took 29 us with the copies).
+    constexpr int64_t kSmall = gh::HostQueryStage::kSmall;
+    if (n <= kSmall) {
+      if (!s.pin) {
+        GH_CUDA(cudaHostAlloc(&s.pin, sizeof(int) * (3 * kSmall + 1), cudaHostAllocMapped));
+        GH_CUDA(cudaHostGetDevicePointer(&s.dpin, s.pin, 0));
+        s.pin[3 * kSmall] = 0;
+      }
+      std::memcpy(s.pin, x, sizeof(int) * n);
+      std::memcpy(s.pin + kSmall, y, sizeof(int) * n);
+      gh::run_query_batch(g, s.dpin, s.dpin + kSmall, s.dpin + 2 * kSmall, n, mode, s.stream, s.dpin + 3 * kSmall);
+      GH_CUDA(cudaStreamSynchronize(s.stream));
+      std::memcpy(out, s.pin + 2 * kSmall, sizeof(int) * n);
+      if (s.pin[3 * kSmall]) {
+        s.pin[3 * kSmall] = 0;
+        throw gh::Error(H2H_ERR_ARG, "vertex id out of range in batch (those pairs answered -1)");
+      }
+      return;
+    }
     if (!s.stream2) GH_CUDA(cudaStreamCreateWithFlags(&s.stream2, cudaStreamNonBlocking));
     if (!s.joined) GH_CUDA(cudaEventCreateWithFlags(&s.joined, cudaEventDisableTiming));
     if (!s.dbad) {

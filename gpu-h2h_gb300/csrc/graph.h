@@ -35,6 +35,7 @@ struct ListStore {
 struct DeviceIndex {
   int n = 0;
   int64_t euler = 0, rmq = 0, pos = 0, dis_padded = 0;
+  bool rmq_closed = true;     // RMQHash is the closed form of build_rmq_gpu
   int *first = nullptr;       // firstAppeare           [n]
   int *depth = nullptr;       // H2H_TreeHeight_Hash    [n]
   int64_t *rmq_hash = nullptr;// RMQHash                [euler]

@@ -20,7 +20,12 @@ struct HostQueryStage {
   cudaStream_t stream = nullptr, stream2 = nullptr;  // large batches alternate chunks between them
   cudaEvent_t joined = nullptr;
   int *dbad = nullptr;  // this path's own out-of-range flag (device batches on the graph never touch it)
+  // small batches: pairs, answers and the flag in page-locked memory that the
+  // kernel reads and writes in place (x, y, out, flag)
+  static constexpr int64_t kSmall = 4096;
+  int *pin = nullptr, *dpin = nullptr;
   ~HostQueryStage() {
+    cudaFreeHost(pin);
     cudaFree(dx); cudaFree(dy); cudaFree(dout); cudaFree(dbad);
     if (stream) cudaStreamDestroy(stream);
     if (stream2) cudaStreamDestroy(stream2);

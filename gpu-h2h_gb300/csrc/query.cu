@@ -31,6 +31,8 @@ struct QArgs {
   const int64_t *drow;
   const int *dis;
   int *bad;  // set to 1 when a pair holds an id outside [0, nv)
+  int64_t tiles;             // ceil(n / TILE)
+  int64_t euler, rmq_total;  // tour and table lengths; euler 0: row starts are read from rmq_hash
 };
 
 // G lanes cooperate on one query.  Every lane of the group resolves the LCA
@@ -73,21 +75,48 @@ __global__ void query_kernel(QArgs A) {
   }
 }
 
-// Warp-tiled batch: a warp owns TILE consecutive queries.  Phase 1: lane i
-// < TILE resolves query i (ids, LCA through the sparse table, row bases, the
-// position range) -- TILE independent dependent-load chains in flight.
-// Phase 2: the whole warp walks each query's positions in turn with 4-way
-// unrolled loads (position, then the two label entries) and a warp min
-// (__reduce_min_sync); the owning lane keeps the answer and the answers
-// leave in one coalesced store.  TILE = 32 for large batches; a batch too
-// small to fill the GPU's resident warps takes a narrower tile, so more
-// warps share its walks and the batch finishes sooner.
+// Start of row i of the sparse table (see build_rmq_gpu): S(L) - S(L - i).
+__host__ __device__ inline int64_t rmq_prefix(int64_t x) {
+  if (x <= 0) return 0;
+#ifdef __CUDA_ARCH__
+  const int k = 63 - __clzll(x);
+#else
+  int k = 0;
+  while ((int64_t(2) << k) <= x) k++;
+#endif
+  return ((int64_t)(k - 1) << k) + 1 + (x - (int64_t(1) << k) + 1) * (k + 1);
+}
+
+__device__ __forceinline__ int64_t rmq_row(const QArgs &A, int i) {
+  return A.euler > 0 ? A.rmq_total - rmq_prefix(A.euler - i) : __ldg(A.rmq_hash + i);
+}
+
+// A warp owns TILE queries.  Phase 1: lane i < TILE resolves query i (ids, row
+// bases, LCA through the sparse table) -- TILE chains of dependent loads in
+// flight.  The table's row starts are computed and the position ranges of both
+// LCA candidates fetched with their depths, so a chain is five loads long, not
+// seven.  Phase 2: the warp walks the queries one after another in pieces of
+// 128 entries; while the label entries of a piece are on their way it loads
+// the positions (noLCA mode: the entries) of the next one, this query's or
+// the next query's, so only one load's latency is left per piece.  The answers
+// leave in one store.
+//
+// Bound: HBM on large batches, the chain of dependent loads on small ones.  On
+// one GB300, against loading positions and entries of one query in turn: 2e6
+// pairs on a 264k-vertex road graph 800 -> 690 us (0.91 of HBM), 1e5 pairs 73
+// -> 61 us, 1e5 pairs in noLCA mode on a 70k-vertex graph 66 -> 45 us, 1e3
+// pairs 9.6 -> 7.8 us.  Spreading a warp over several queries (8 lanes each)
+// took 2,200 us: a row is then read in 128-byte pieces at different times,
+// which DRAM serves at a third of its rate.
 template <bool LCA_MODE, int TILE>
-__global__ void __launch_bounds__(256, 8) query_tile_kernel(QArgs A) {
+__global__ void __launch_bounds__(256, 6) query_tile_kernel(QArgs A) {
+  constexpr int U = 4;
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t tile = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; tile * TILE < A.n; tile += nwarps) {
-    const int64_t q = tile * TILE + lane;
+  for (int64_t tile = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; tile < A.tiles; tile += nwarps) {
+    // narrow tiles (one wave) deal the batch out like cards: a run of far or
+    // near pairs then spreads over all warps, and no warp gets only long walks
+    const int64_t q = TILE < 32 ? lane * A.tiles + tile : tile * TILE + lane;
     int res = INT_MAX, len = 0;
     int64_t pb = 0, bx = 0, by = 0;
     if (lane < TILE && q < A.n) {
@@ -95,7 +124,7 @@ __global__ void __launch_bounds__(256, 8) query_tile_kernel(QArgs A) {
       const bool valid = (unsigned)a < (unsigned)A.nv && (unsigned)b < (unsigned)A.nv;
       if (!valid) {
         res = -1;
-        atomicExch(A.bad, 1);
+        *(volatile int *)A.bad = 1;
       } else if (a == b) {
         res = 0;
       } else {
@@ -104,47 +133,110 @@ __global__ void __launch_bounds__(256, 8) query_tile_kernel(QArgs A) {
         by = __ldg(A.drow + b);
         const int l = min(fa, fb), r = max(fa, fb);
         const int k = 31 - __clz(r - l + 1);
-        const int i1 = __ldg(A.rmq_id + __ldg(A.rmq_hash + l) + k);
-        const int i2 = __ldg(A.rmq_id + __ldg(A.rmq_hash + r - (1 << k) + 1) + k);
+        const int i1 = __ldg(A.rmq_id + rmq_row(A, l) + k);
+        const int i2 = __ldg(A.rmq_id + rmq_row(A, r - (1 << k) + 1) + k);
         const int d1 = __ldg(A.depth + i1), d2 = __ldg(A.depth + i2);
         if (LCA_MODE) {
-          const int lca = d1 <= d2 ? i1 : i2;
-          pb = __ldg(A.pos_hash + lca);
-          len = (int)(__ldg(A.pos_hash + lca + 1) - pb);
+          const int64_t b1 = __ldg(A.pos_hash + i1), e1 = __ldg(A.pos_hash + i1 + 1);
+          const int64_t b2 = __ldg(A.pos_hash + i2), e2 = __ldg(A.pos_hash + i2 + 1);
+          pb = d1 <= d2 ? b1 : b2;
+          len = (int)(d1 <= d2 ? e1 - b1 : e2 - b2);
         } else {
           len = min(d1, d2);
         }
       }
     }
-#pragma unroll 1
-    for (int s = 0; s < TILE; s++) {
-      const int L = __shfl_sync(0xffffffffu, len, s);
-      if (L == 0) continue;
-      const int64_t PB = __shfl_sync(0xffffffffu, pb, s);
-      const int *rx = A.dis + __shfl_sync(0xffffffffu, bx, s);
-      const int *ry = A.dis + __shfl_sync(0xffffffffu, by, s);
-      int m = INT_MAX;
-      for (int t0 = 0; t0 < L; t0 += 128) {
-        int p[4];
-        bool ok[4];
+    unsigned todo = __ballot_sync(0xffffffffu, len > 0);
+    if (LCA_MODE) {
+      if (todo) {
+        int s = __ffs(todo) - 1, t0 = 0;
+        int L = __shfl_sync(0xffffffffu, len, s);
+        int64_t PB = __shfl_sync(0xffffffffu, pb, s);
+        int p[U];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int t = t0 + (u << 5) + lane;
-          ok[u] = t < L;
-          p[u] = ok[u] ? (LCA_MODE ? __ldg(A.pos_pos + PB + t) : t) : 0;
+        for (int u = 0; u < U; u++) p[u] = 32 * u + lane < L ? __ldg(A.pos_pos + PB + 32 * u + lane) : -1;
+        const int *rx = A.dis + __shfl_sync(0xffffffffu, bx, s), *ry = A.dis + __shfl_sync(0xffffffffu, by, s);
+        int m = INT_MAX;
+        for (;;) {
+          int xv[U], yv[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            xv[u] = p[u] >= 0 ? __ldg(rx + p[u]) : 0;
+            yv[u] = p[u] >= 0 ? __ldg(ry + p[u]) : 0;
+          }
+          // the positions of the next piece: this query's next 128, or the next query's first
+          const int cur = s;
+          const bool last = t0 + 32 * U >= L;
+          int next[U];
+          if (last) {
+            todo &= todo - 1;
+            s = todo ? __ffs(todo) - 1 : s;
+            t0 = 0;
+            L = todo ? __shfl_sync(0xffffffffu, len, s) : 0;
+            PB = __shfl_sync(0xffffffffu, pb, s);
+          } else {
+            t0 += 32 * U;
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const int t = t0 + 32 * u + lane;
+            next[u] = t < L ? __ldg(A.pos_pos + PB + t) : -1;
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            if (p[u] >= 0) m = min(m, xv[u] + yv[u]);
+            p[u] = next[u];
+          }
+          if (last) {
+            m = __reduce_min_sync(0xffffffffu, m);
+            if (lane == cur) res = m;
+            if (!todo) break;
+            m = INT_MAX;
+            rx = A.dis + __shfl_sync(0xffffffffu, bx, s);
+            ry = A.dis + __shfl_sync(0xffffffffu, by, s);
+          }
         }
-        int xv[4], yv[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          xv[u] = ok[u] ? __ldg(rx + p[u]) : 0;
-          yv[u] = ok[u] ? __ldg(ry + p[u]) : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          if (ok[u]) m = min(m, xv[u] + yv[u]);
       }
-      m = __reduce_min_sync(0xffffffffu, m);
-      if (lane == s) res = m;
+    } else if (todo) {
+      // pieces of 128 entries, four per lane (rows start on 16 bytes and are
+      // padded to them); the next piece, this query's or the next one's, is
+      // loaded before this one is used
+      int s = __ffs(todo) - 1, t0 = 0;
+      int L = __shfl_sync(0xffffffffu, len, s);
+      const int *rx = A.dis + __shfl_sync(0xffffffffu, bx, s), *ry = A.dis + __shfl_sync(0xffffffffu, by, s);
+      const int4 none = make_int4(0, 0, 0, 0);
+      int4 xv = 4 * lane < L ? __ldg(reinterpret_cast<const int4 *>(rx) + lane) : none;
+      int4 yv = 4 * lane < L ? __ldg(reinterpret_cast<const int4 *>(ry) + lane) : none;
+      int m = INT_MAX;
+      for (;;) {
+        const int cur = s, left = L - t0 - 4 * lane;  // entries of this lane's four that count
+        const bool last = t0 + 128 >= L;
+        if (last) {
+          todo &= todo - 1;
+          s = todo ? __ffs(todo) - 1 : s;
+          t0 = 0;
+          L = todo ? __shfl_sync(0xffffffffu, len, s) : 0;
+          rx = A.dis + __shfl_sync(0xffffffffu, bx, s);
+          ry = A.dis + __shfl_sync(0xffffffffu, by, s);
+        } else {
+          t0 += 128;
+        }
+        const int j = t0 + 4 * lane;
+        const int4 xn = j < L ? __ldg(reinterpret_cast<const int4 *>(rx + j)) : none;
+        const int4 yn = j < L ? __ldg(reinterpret_cast<const int4 *>(ry + j)) : none;
+        if (left > 0) m = min(m, xv.x + yv.x);
+        if (left > 1) m = min(m, xv.y + yv.y);
+        if (left > 2) m = min(m, xv.z + yv.z);
+        if (left > 3) m = min(m, xv.w + yv.w);
+        xv = xn;
+        yv = yn;
+        if (last) {
+          m = __reduce_min_sync(0xffffffffu, m);
+          if (lane == cur) res = m;
+          if (!todo) break;
+          m = INT_MAX;
+        }
+      }
     }
     if (lane < TILE && q < A.n) A.out[q] = res;
   }
@@ -170,13 +262,6 @@ struct RmqJob {
   int *id;           // RMQ_ID  [S(L)]
   int64_t L;
 };
-
-__host__ __device__ inline int64_t rmq_prefix(int64_t x) {
-  if (x <= 0) return 0;
-  int k = 0;
-  while ((int64_t(2) << k) <= x) k++;
-  return ((int64_t)(k - 1) << k) + 1 + (x - (int64_t(1) << k) + 1) * (k + 1);
-}
 
 __device__ __forceinline__ int job_of(const int64_t *off, int njobs, int64_t p) {
   int lo = 0, hi = njobs - 1;  // last job with off[job] <= p
@@ -283,8 +368,16 @@ void build_rmq_gpu(const std::vector<Graph *> &gs) {
 }
 
 void upload_rmq(Graph &g, const std::vector<int64_t> &rmq_hash, const std::vector<int> &rmq_id) {
+  // a file's row starts are usually the closed form's; otherwise the queries read them
+  const int64_t total = rmq_prefix(g.euler_n);
+  bool closed = total == g.rmq_total;
+  for (int64_t i = 0, start = 0; i < g.euler_n && closed; i++) {
+    closed = rmq_hash[i] == start;
+    start += 64 - __builtin_clzll((unsigned long long)(g.euler_n - i));
+  }
   allocate_rmq(g);
   DeviceIndex &D = g.dev;
+  D.rmq_closed = closed;
   GH_CUDA(cudaMemcpy(D.first, g.first.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
   GH_CUDA(cudaMemcpy(D.rmq_hash, rmq_hash.data(), sizeof(int64_t) * D.euler, cudaMemcpyHostToDevice));
   GH_CUDA(cudaMemcpy(D.rmq_id, rmq_id.data(), sizeof(int) * D.rmq, cudaMemcpyHostToDevice));
@@ -307,19 +400,19 @@ void run_query_batch(const Graph &g, const int *x, const int *y, int *out, int64
   if (n <= 0) return;
   const DeviceIndex &D = g.dev;
   QArgs A{x, y, out, n, g.n, D.first, D.depth, D.rmq_hash, D.rmq_id, D.pos_hash, D.pos_pos, D.drow, D.dis,
-          bad ? bad : D.err};
+          bad ? bad : D.err, 0, D.rmq_closed ? D.euler : 0, D.rmq};
   const int threads = 256;
   const int mi = mode == H2H_QUERY_LCA ? 0 : 1;
   using Kernel = void (*)(QArgs);
-  static const Kernel kernels[2][4] = {
+  static const Kernel kernels[2][6] = {
       {query_tile_kernel<true, 32>, query_tile_kernel<true, 16>, query_tile_kernel<true, 8>,
-       query_tile_kernel<true, 4>},
+       query_tile_kernel<true, 4>, query_tile_kernel<true, 2>, query_tile_kernel<true, 1>},
       {query_tile_kernel<false, 32>, query_tile_kernel<false, 16>, query_tile_kernel<false, 8>,
-       query_tile_kernel<false, 4>}};
+       query_tile_kernel<false, 4>, query_tile_kernel<false, 2>, query_tile_kernel<false, 1>}};
   // device shape, looked up once (thread-safe static initialisation: the
   // server's worker and callers' threads may arrive together)
   struct Shape {
-    int nsm = 1, per_sm[2] = {1, 1};  // resident 256-thread blocks per SM (all tile widths use 32 registers)
+    int nsm = 1, per_sm[2] = {1, 1};  // resident 256-thread blocks per SM (all tile widths use 40 registers)
   };
   static const Shape shape = [] {
     Shape sh;
@@ -337,11 +430,12 @@ void run_query_batch(const Graph &g, const int *x, const int *y, int *out, int64
   // narrowest tile whose warps still fit one wave of resident warps
   const int64_t resident_warps = (int64_t)nsm * per_sm[mi] * (threads / 32);
   int ti = 0, tile = 32;
-  while (ti < 3 && ((n + tile / 2 - 1) / (tile / 2)) <= resident_warps) {
+  while (ti < 5 && ((n + tile / 2 - 1) / (tile / 2)) <= resident_warps) {
     tile /= 2;
     ti++;
   }
   const int64_t tiles = (n + tile - 1) / tile;
+  A.tiles = tiles;
   // one wave of resident blocks, grid-striding over the tiles
   const int blocks = (int)std::min<int64_t>((tiles + 7) / 8, (int64_t)nsm * per_sm[mi]);
   kernels[mi][ti]<<<std::max(1, blocks), threads, 0, s>>>(A);
@@ -352,7 +446,8 @@ void run_query_batch_plain(const Graph &g, const int *x, const int *y, int *out,
                            cudaStream_t s) {
   if (n <= 0) return;
   const DeviceIndex &D = g.dev;
-  QArgs A{x, y, out, n, g.n, D.first, D.depth, D.rmq_hash, D.rmq_id, D.pos_hash, D.pos_pos, D.drow, D.dis, D.err};
+  QArgs A{x, y, out, n, g.n, D.first, D.depth, D.rmq_hash, D.rmq_id, D.pos_hash, D.pos_pos, D.drow, D.dis, D.err,
+          0,      0,      0};
   const int threads = 256;
   int blocks = (int)std::min<int64_t>((n + threads - 1) / threads, INT32_MAX);
   if (mode == H2H_QUERY_LCA) query_kernel<1, true><<<blocks, threads, 0, s>>>(A);
