@@ -184,6 +184,23 @@ int h2h_build_labels(h2h_graph *h, int parallel_fine, int use_gpu_construct, int
   });
 }
 
+// Device address of page-locked host memory, nullptr for any other memory.
+static int *mapped_address(const int *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return a.type == cudaMemoryTypeHost ? static_cast<int *>(a.devicePointer) : nullptr;
+}
+
+// Whether the answers may be written while pairs are still read: a query reads
+// its own pair before it writes its own answer, so only a shifted overlap is
+// a conflict.
+static bool in_place_safe(const int *in, const int *out, int64_t n) {
+  return in == out || in + n <= out || out + n <= in;
+}
+
 static int single_query(const h2h_graph *h, int x, int y, int mode) {
   if (!h) { gh::set_last_error("null handle"); return -1; }
   int res = -1;
@@ -251,18 +268,33 @@ int h2h_query_batch_host(const h2h_graph *hc, const int *x, const int *y, int *o
     // Up to 4,096 pairs go through page-locked memory that the kernel reads and
     // writes in place: one launch instead of a launch and four copies (a single
     // pair took 29 us with the copies).
+    // Larger batches in page-locked buffers are read and written in place too:
+    // the kernel streams 12 bytes a pair over the host link while it runs (2e6
+    // pairs on a 264k-vertex graph 975 us, 1,050 with overlapped copies).
     constexpr int64_t kSmall = gh::HostQueryStage::kSmall;
-    if (n <= kSmall) {
+    const bool small = n <= kSmall;
+    int *mx = nullptr, *my = nullptr, *mo = nullptr;
+    if (!small && in_place_safe(x, out, n) && in_place_safe(y, out, n)) {
+      mx = mapped_address(x);
+      my = mx ? mapped_address(y) : nullptr;
+      mo = my ? mapped_address(out) : nullptr;
+    }
+    if (small || mo) {
       if (!s.pin) {
         GH_CUDA(cudaHostAlloc(&s.pin, sizeof(int) * (3 * kSmall + 1), cudaHostAllocMapped));
         GH_CUDA(cudaHostGetDevicePointer(&s.dpin, s.pin, 0));
         s.pin[3 * kSmall] = 0;
       }
-      std::memcpy(s.pin, x, sizeof(int) * n);
-      std::memcpy(s.pin + kSmall, y, sizeof(int) * n);
-      gh::run_query_batch(g, s.dpin, s.dpin + kSmall, s.dpin + 2 * kSmall, n, mode, s.stream, s.dpin + 3 * kSmall);
+      if (small) {
+        std::memcpy(s.pin, x, sizeof(int) * n);
+        std::memcpy(s.pin + kSmall, y, sizeof(int) * n);
+        mx = s.dpin;
+        my = s.dpin + kSmall;
+        mo = s.dpin + 2 * kSmall;
+      }
+      gh::run_query_batch(g, mx, my, mo, n, mode, s.stream, s.dpin + 3 * kSmall);
       GH_CUDA(cudaStreamSynchronize(s.stream));
-      std::memcpy(out, s.pin + 2 * kSmall, sizeof(int) * n);
+      if (small) std::memcpy(out, s.pin + 2 * kSmall, sizeof(int) * n);
       if (s.pin[3 * kSmall]) {
         s.pin[3 * kSmall] = 0;
         throw gh::Error(H2H_ERR_ARG, "vertex id out of range in batch (those pairs answered -1)");

@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(256, 6) query_tile_kernel(QArgs A) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t tile = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; tile < A.tiles; tile += nwarps) {
-    // narrow tiles (one wave) deal the batch out like cards: a run of far or
-    // near pairs then spreads over all warps, and no warp gets only long walks
-    const int64_t q = TILE < 32 ? lane * A.tiles + tile : tile * TILE + lane;
+    // narrow tiles (one wave) take half their queries from each half of the
+    // batch: a run of near or far pairs spreads over more warps, and fewer get
+    // only long walks
+    constexpr int RUN = TILE < 32 && TILE > 1 ? TILE / 2 : TILE;
+    const int64_t q = (lane / RUN * A.tiles + tile) * RUN + lane % RUN;
     int res = INT_MAX, len = 0;
     int64_t pb = 0, bx = 0, by = 0;
     if (lane < TILE && q < A.n) {

@@ -4,8 +4,8 @@
 //
 // Requests (pairs of one graph in one mode) are queued by any thread and
 // answered asynchronously.  One worker thread owns all CUDA work.  It keeps
-// up to `slots` device batches in flight, each on its own stream: copy the
-// pairs in, run the query kernel, copy the answers out, record an event.
+// up to `slots` device batches in flight, each on its own stream: the query
+// kernel on page-locked host buffers, then an event.
 // Whenever a batch retires, its answers are scattered to the requests and
 // the slot is refilled at once from the pending queue: the oldest request
 // picks the (graph, mode) and later requests with the same key join the
@@ -36,15 +36,22 @@ double now_us() {
 }
 
 // cudaMemoryTypeHost for page-locked memory, Unregistered for pageable
-// memory, Device / Managed for memory the server does not take.
-cudaMemoryType memory_type(const void *p) {
+// memory, Device / Managed for memory the server does not take; *dev receives
+// the device address of page-locked memory.
+cudaMemoryType memory_type(const void *p, int **dev) {
+  *dev = nullptr;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return cudaMemoryTypeUnregistered;
   }
+  if (a.type == cudaMemoryTypeHost) *dev = static_cast<int *>(a.devicePointer);
   return a.type;
 }
+
+// A piece of at least this many pairs in page-locked buffers is a launch of
+// its own on them; smaller ones are gathered in the slot's staging.
+constexpr int64_t kDirectPairs = 4096;
 
 struct Request {
   uint64_t id = 0;
@@ -54,7 +61,7 @@ struct Request {
   int64_t n = 0;
   int64_t next = 0;      // first pair not yet placed in a batch
   int64_t remaining = 0; // pairs not yet answered
-  bool pinned = false;
+  int *dx = nullptr, *dy = nullptr, *dout = nullptr;  // device addresses when all three buffers are page-locked
   double t_submit = 0, t_done = 0;
   bool done = false;
 };
@@ -62,13 +69,13 @@ struct Request {
 struct Piece {
   Request *r;
   int64_t req_off, slot_off, count;
+  bool direct() const { return r->dout && count >= kDirectPairs; }
 };
 
 struct Slot {
   int64_t cap = 0;
-  int *dx = nullptr, *dy = nullptr, *dout = nullptr;
   int *dbad = nullptr;  // this slot's out-of-range flag (answers carry -1 instead)
-  int *hx = nullptr, *hy = nullptr, *hout = nullptr;  // pinned staging
+  int *hx = nullptr, *hy = nullptr, *hout = nullptr;  // page-locked staging, read and written by the kernel
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr, k0 = nullptr, k1 = nullptr;
   std::vector<Piece> pieces;
@@ -106,7 +113,7 @@ struct h2h_server {
     if (worker.joinable()) worker.join();
     for (Slot &s : slots) {
       if (s.stream) cudaStreamSynchronize(s.stream);
-      cudaFree(s.dx); cudaFree(s.dy); cudaFree(s.dout); cudaFree(s.dbad);
+      cudaFree(s.dbad);
       cudaFreeHost(s.hx); cudaFreeHost(s.hy); cudaFreeHost(s.hout);
       if (s.done) cudaEventDestroy(s.done);
       if (s.k0) cudaEventDestroy(s.k0);
@@ -138,46 +145,24 @@ struct h2h_server {
     return true;
   }
 
+  // The kernels read pairs from and write answers to page-locked host memory:
+  // no copies, one launch for all gathered pieces and one per large piece.
   void launch(Slot &s, const gh::Graph &g, int mode) {
-    for (const Piece &p : s.pieces) {
-      if (p.r->pinned) {
-        GH_CUDA(cudaMemcpyAsync(s.dx + p.slot_off, p.r->x + p.req_off, sizeof(int) * p.count,
-                                cudaMemcpyHostToDevice, s.stream));
-        GH_CUDA(cudaMemcpyAsync(s.dy + p.slot_off, p.r->y + p.req_off, sizeof(int) * p.count,
-                                cudaMemcpyHostToDevice, s.stream));
-      } else {
-        std::memcpy(s.hx + p.slot_off, p.r->x + p.req_off, sizeof(int) * p.count);
-        std::memcpy(s.hy + p.slot_off, p.r->y + p.req_off, sizeof(int) * p.count);
-      }
-    }
-    bool staged = false;
-    for (const Piece &p : s.pieces) staged |= !p.r->pinned;
-    if (staged) {  // one copy of the staged range (pinned pieces land on top in stream order first)
-      // copy only the staged pieces, merged where contiguous
-      int64_t a = -1, b = -1;
-      auto flush = [&]() {
-        if (a < 0) return;
-        GH_CUDA(cudaMemcpyAsync(s.dx + a, s.hx + a, sizeof(int) * (b - a), cudaMemcpyHostToDevice, s.stream));
-        GH_CUDA(cudaMemcpyAsync(s.dy + a, s.hy + a, sizeof(int) * (b - a), cudaMemcpyHostToDevice, s.stream));
-        a = b = -1;
-      };
-      for (const Piece &p : s.pieces) {
-        if (p.r->pinned) { flush(); continue; }
-        if (a >= 0 && b == p.slot_off) b += p.count;
-        else { flush(); a = p.slot_off; b = p.slot_off + p.count; }
-      }
-      flush();
+    int64_t staged = 0;
+    for (Piece &p : s.pieces) {
+      if (p.direct()) continue;
+      p.slot_off = staged;
+      std::memcpy(s.hx + staged, p.r->x + p.req_off, sizeof(int) * p.count);
+      std::memcpy(s.hy + staged, p.r->y + p.req_off, sizeof(int) * p.count);
+      staged += p.count;
     }
     GH_CUDA(cudaEventRecord(s.k0, s.stream));
-    gh::run_query_batch(g, s.dx, s.dy, s.dout, s.pairs, mode, s.stream, s.dbad);
+    for (const Piece &p : s.pieces)
+      if (p.direct())
+        gh::run_query_batch(g, p.r->dx + p.req_off, p.r->dy + p.req_off, p.r->dout + p.req_off, p.count, mode, s.stream,
+                            s.dbad);
+    if (staged) gh::run_query_batch(g, s.hx, s.hy, s.hout, staged, mode, s.stream, s.dbad);
     GH_CUDA(cudaEventRecord(s.k1, s.stream));
-    for (const Piece &p : s.pieces) {
-      if (p.r->pinned)
-        GH_CUDA(cudaMemcpyAsync(p.r->out + p.req_off, s.dout + p.slot_off, sizeof(int) * p.count,
-                                cudaMemcpyDeviceToHost, s.stream));
-    }
-    if (staged)
-      GH_CUDA(cudaMemcpyAsync(s.hout, s.dout, sizeof(int) * s.pairs, cudaMemcpyDeviceToHost, s.stream));
     GH_CUDA(cudaEventRecord(s.done, s.stream));
     s.busy = true;
   }
@@ -186,7 +171,7 @@ struct h2h_server {
     float kms = 0;
     cudaEventElapsedTime(&kms, s.k0, s.k1);
     for (const Piece &p : s.pieces)
-      if (!p.r->pinned) std::memcpy(p.r->out + p.req_off, s.hout + p.slot_off, sizeof(int) * p.count);
+      if (!p.direct()) std::memcpy(p.r->out + p.req_off, s.hout + p.slot_off, sizeof(int) * p.count);
     const double t = now_us();
     {
       std::lock_guard<std::mutex> l(mu);
@@ -298,9 +283,6 @@ int h2h_server_create(const h2h_server_config *cfg, h2h_server **out) {
     s->slots.resize(c.slots);
     for (Slot &sl : s->slots) {
       sl.cap = c.slot_pairs;
-      GH_CUDA(cudaMalloc(&sl.dx, sizeof(int) * sl.cap));
-      GH_CUDA(cudaMalloc(&sl.dy, sizeof(int) * sl.cap));
-      GH_CUDA(cudaMalloc(&sl.dout, sizeof(int) * sl.cap));
       GH_CUDA(cudaMalloc(&sl.dbad, sizeof(int)));
       GH_CUDA(cudaMallocHost(&sl.hx, sizeof(int) * sl.cap));
       GH_CUDA(cudaMallocHost(&sl.hy, sizeof(int) * sl.cap));
@@ -355,11 +337,14 @@ int h2h_server_submit(h2h_server *s, int graph_id, const int *x, const int *y, i
     GH_CHECK(mode == H2H_QUERY_LCA || mode == H2H_QUERY_NOLCA, H2H_ERR_ARG, "mode must be 0 (LCA) or 1 (noLCA)");
     GH_CHECK(n >= 1, H2H_ERR_ARG, "a request holds at least one pair");
     GH_CHECK(x && y && out, H2H_ERR_ARG, "null buffer");
-    const cudaMemoryType tx = memory_type(x), ty = memory_type(y), to = memory_type(out);
+    int *dx, *dy, *dout;
+    const cudaMemoryType tx = memory_type(x, &dx), ty = memory_type(y, &dy), to = memory_type(out, &dout);
     for (cudaMemoryType t : {tx, ty, to})
       GH_CHECK(t == cudaMemoryTypeHost || t == cudaMemoryTypeUnregistered, H2H_ERR_ARG,
                "the server takes host buffers (pageable or page-locked)");
-    const bool pinned = tx == cudaMemoryTypeHost && ty == cudaMemoryTypeHost && to == cudaMemoryTypeHost;
+    // answers may be written while pairs are read only where the buffers coincide or lie apart
+    auto apart = [n](const int *a, const int *b) { return a == b || a + n <= b || b + n <= a; };
+    const bool in_place = dx && dy && dout && apart(x, out) && apart(y, out);
     auto r = std::make_unique<Request>();
     r->graph = graph_id;
     r->mode = mode;
@@ -368,7 +353,11 @@ int h2h_server_submit(h2h_server *s, int graph_id, const int *x, const int *y, i
     r->out = out;
     r->n = n;
     r->remaining = n;
-    r->pinned = pinned;
+    if (in_place) {
+      r->dx = dx;
+      r->dy = dy;
+      r->dout = dout;
+    }
     {
       std::lock_guard<std::mutex> l(s->mu);
       GH_CHECK(s->worker_error.empty(), H2H_ERR_CUDA, "server worker stopped: " + s->worker_error);

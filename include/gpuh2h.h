@@ -99,9 +99,10 @@ int h2h_query_nolca_nohub(const h2h_graph *g, int x, int y);
 int h2h_query_batch(const h2h_graph *g, const int *x_dev, const int *y_dev, int *out_dev, int64_t n,
                     int mode, void *stream);
 
-/* The same from host buffers: copies x, y to the device, runs the batch and
- * copies the answers back before returning (the Query_noHub flow,
- * main.cu:218-240: translateQuery, kernel, translateQueryResultBack).
+/* The same from host buffers, the answers in `out` on return (the Query_noHub
+ * flow, main.cu:218-240: translateQuery, kernel, translateQueryResultBack).
+ * Page-locked buffers and batches of up to 4,096 pairs are read and written
+ * by the kernel over the host link; larger pageable ones are copied.
  * Returns H2H_ERR_ARG when a pair holds an id outside [0, n) (those pairs
  * answer -1); the flag it reads belongs to this call path alone. */
 int h2h_query_batch_host(const h2h_graph *g, const int *x, const int *y, int *out, int64_t n, int mode);
@@ -226,8 +227,8 @@ void h2h_batch_free(h2h_batch *b);
  * and answered asynchronously by a worker that keeps `slots` device batches
  * in flight on separate streams and refills a slot from the queue as soon as
  * it retires, joining requests of the same graph and mode (a request larger
- * than a slot spans several).  Page-locked request buffers are transferred
- * directly; pageable ones go through the slot's page-locked staging.  Pairs
+ * than a slot spans several).  Large requests in page-locked buffers are read
+ * and answered in place; others go through the slot's page-locked staging.  Pairs
  * with a vertex id out of range answer -1.  Graphs must outlive the server
  * (or be removed first). */
 typedef struct h2h_server h2h_server;
