@@ -298,7 +298,7 @@ __global__ void build_positions_kernel(const int64_t *list_off, const int *list_
 // members, ancestors) costs as much as several steps: 64 / 256-column tasks
 // there took the 1M-vertex fill from 14.8 to 17.4 ms.
 TilePolicy::TilePolicy() {
-  static const int cb[kWidth][kSep] = {{256, 256, 128, 64}, {4096, 4096, 512, 64}, {4096, 4096, 512, 64}};
+  static const int cb[kWidth][kSep] = {{64, 64, 64, 64}, {4096, 4096, 512, 128}, {4096, 4096, 512, 128}};
   for (int w = 0; w < kWidth; w++)
     for (int b = 0; b < kSep; b++) {
       small_work[w][b] = 1024;
