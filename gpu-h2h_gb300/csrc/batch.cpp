@@ -201,6 +201,7 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch 
       b->fill->attach(true);
       for (gh::Graph *g : b->gs) {
         gh::upload_query_index(*g);
+        g->sets.reset();
         g->labelled = true;
       }
       b->info.t_attach_us = clk.us();

@@ -111,7 +111,7 @@ int load_common(const std::string &edge, const std::string &idf, const std::stri
     gh::load_graph(g, edge, idf, cut);
     GH_CHECK(g.C <= g.H, H2H_ERR_ARG, "ChangeToGlobalHeight exceeds the partition height");
     gh::Clock clk;
-    {
+    if (!g.input) {  // parsed on the device: checked there
       gh::Pool pool(gh::useful_threads(g.threads, g.m));
       check_symmetric(g, pool);
       check_connected(g, pool);
@@ -464,7 +464,7 @@ int h2h_copy_labels(const h2h_graph *h, int64_t *dis_hash, int *dis, int64_t *po
 int h2h_copy_input_arcs(const h2h_graph *h, int *adj_off, int *adj_v, int *adj_w) {
   if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
   return guarded([&] {
-    const gh::Graph &g = h->g;
+    const gh::HostInput &g = gh::input_host(h->g);
     if (adj_off) std::copy(g.adj_off.begin(), g.adj_off.end(), adj_off);
     if (adj_v) std::copy(g.adj_v.begin(), g.adj_v.end(), adj_v);
     if (adj_w) std::copy(g.adj_w.begin(), g.adj_w.end(), adj_w);
@@ -474,8 +474,8 @@ int h2h_copy_input_arcs(const h2h_graph *h, int *adj_off, int *adj_v, int *adj_w
 int h2h_copy_partition(const h2h_graph *h, int *part_ids, int *id_hash) {
   if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
   return guarded([&] {
-    const gh::Graph &g = h->g;
-    GH_CHECK((int)g.part_ids.size() == g.n, H2H_ERR_STATE, "no partition array (a loaded index has none)");
+    const gh::HostInput &g = gh::input_host(h->g);
+    GH_CHECK((int)g.part_ids.size() == h->g.n, H2H_ERR_STATE, "no partition array (a loaded index has none)");
     if (part_ids) std::copy(g.part_ids.begin(), g.part_ids.end(), part_ids);
     if (id_hash) std::copy(g.id_hash.begin(), g.id_hash.end(), id_hash);
   });
@@ -527,12 +527,12 @@ int h2h_gen_uniform_pairs(int n_vertices, int64_t n, uint64_t seed, int *x, int 
 
 int h2h_gen_local_pairs(const h2h_graph *h, int64_t n, int max_hops, uint64_t seed, int *x, int *y) {
   if (!h || n < 0 || (n > 0 && (!x || !y))) { gh::set_last_error("bad argument"); return H2H_ERR_ARG; }
-  if ((int)h->g.adj_off.size() != h->g.n + 1 || h->g.n == 0) {
-    gh::set_last_error("the input arcs are not loaded (an index read by h2h_load_index has none)");
-    return H2H_ERR_STATE;
-  }
-  gh::gen_local_pairs_csr(h->g.n, h->g.adj_off.data(), h->g.adj_v.data(), n, max_hops, seed, x, y);
-  return H2H_OK;
+  return guarded([&] {
+    const gh::HostInput &g = gh::input_host(h->g);
+    GH_CHECK((int)g.adj_off.size() == h->g.n + 1 && h->g.n != 0, H2H_ERR_STATE,
+             "the input arcs are not loaded (an index read by h2h_load_index has none)");
+    gh::gen_local_pairs_csr(h->g.n, g.adj_off.data(), g.adj_v.data(), n, max_hops, seed, x, y);
+  });
 }
 
 }  // extern "C"

@@ -1252,6 +1252,17 @@ T *dalloc(size_t n) {
 
 namespace {
 
+// A graph's arcs at its place in the forest's arrays.
+__global__ void forest_arcs_kernel(const int *off, const int *v, const int *w, int n, int64_t m, int vb, int mb,
+                                   int *f_off, int *f_v, int *f_w) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += step) f_off[vb + i] = off[i] + mb;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += step) {
+    f_v[mb + i] = v[i] + vb;
+    f_w[mb + i] = w[i];
+  }
+}
+
 GraphLevels graph_levels(const Graph &g) {
   GraphLevels L;
   int64_t heap_start = INT32_MAX;
@@ -1272,13 +1283,9 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
   GH_CHECK(K >= 1, H2H_ERR_ARG, "no graph to contract");
   // cell list bounds come with the elimination sets (build_elimination_sets)
   std::vector<GraphLevels> L(K);
-  int threads = 1;
-  for (const Graph *g : gs) {
-    threads = std::max(threads, g->threads);
-    GH_CHECK(g->cell_bound.size() == g->cell_start.size(), H2H_ERR_STATE, "elimination sets not built");
-  }
+  const std::shared_ptr<SetsStore> sets = gs[0]->sets;
+  GH_CHECK(sets && sets->gs == gs, H2H_ERR_STATE, "elimination sets not built");
   for (int i = 0; i < K; i++) L[i] = graph_levels(*gs[i]);
-  std::vector<int64_t> lbase(K);
   vbase.assign(K, 0);
   mbase.assign(K, 0);
   int64_t pool_extra = 1024;
@@ -1286,7 +1293,6 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
     Graph &g = *gs[i];
     vbase[i] = N;
     mbase[i] = M;
-    lbase[i] = lub;
     GH_CHECK((int64_t)N + g.n < INT32_MAX, H2H_ERR_ARG, "too many vertices in one batch");
     N += g.n;
     M += g.m;
@@ -1299,59 +1305,13 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
   // slot arrays: the LUB ranges, then a pool for global-order lists that
   // outgrow theirs
   pool_size = lub + pool_extra;
-  // ---- forest arrays (written in full below, so not zero-filled first)
-  std::vector<int64_t, NoInit<int64_t>> f_slot_off(N);
-  std::vector<int, NoInit<int>> f_deg(N), f_cap(N), f_elim(N), f_adj_off(N + 1), f_adj_v(std::max<int64_t>(M, 1)),
-      f_adj_w(std::max<int64_t>(M, 1)), f_heap(std::max(heap_total, 1));
-  f_adj_v[0] = f_adj_w[0] = f_heap[0] = 0;  // defined when there is nothing to copy
-  {
-    std::vector<int> hbase(K, 0);
-    for (int i = 1; i < K; i++) hbase[i] = hbase[i - 1] + L[i - 1].heap_n;
-    auto verts = [&](int i, int64_t lo, int64_t hi) {
-      const Graph &g = *gs[i];
-      const int vb = vbase[i];
-      for (int64_t v = lo; v < hi; v++) {
-        f_slot_off[vb + v] = g.slot_off[v] + lbase[i];
-        f_deg[vb + v] = g.adj_off[v + 1] - g.adj_off[v];
-        f_cap[vb + v] = g.cap[v];
-        f_elim[vb + v] = g.elim[v] + vb;
-        f_adj_off[vb + v] = g.adj_off[v] + (int)mbase[i];
-      }
-    };
-    auto arcs = [&](int i, int64_t lo, int64_t hi) {
-      const Graph &g = *gs[i];
-      const int vb = vbase[i];
-      for (int64_t e = lo; e < hi; e++) {
-        f_adj_v[mbase[i] + e] = g.adj_v[e] + vb;
-        f_adj_w[mbase[i] + e] = g.adj_w[e];
-      }
-    };
-    auto heap = [&](int i) {
-      const Graph &g = *gs[i];
-      for (int j = L[i].heap_start; j < g.n; j++) f_heap[hbase[i] + j - L[i].heap_start] = g.elim[j] + vbase[i];
-    };
-    threads = useful_threads(threads, N);
-    Pool pool(threads);
-    if (K >= threads) {  // a batch: a graph per task
-      pool.parallel_for(K, 1, [&](int64_t lo, int64_t hi, int) {
-        for (int64_t i = lo; i < hi; i++) {
-          verts((int)i, 0, gs[i]->n);
-          arcs((int)i, 0, gs[i]->m);
-          heap((int)i);
-        }
-      });
-    } else {  // few graphs: ranges of each graph's vertices and arcs per task
-      for (int i = 0; i < K; i++) {
-        pool.parallel_for(gs[i]->n, 1 << 16, [&](int64_t lo, int64_t hi, int) { verts(i, lo, hi); });
-        pool.parallel_for(gs[i]->m, 1 << 17, [&](int64_t lo, int64_t hi, int) { arcs(i, lo, hi); });
-        heap(i);
-      }
-    }
-  }
-  f_adj_off[N] = (int)M;
   ListLaunches LL;
   bits = allow_bits && plan_bits();
-  if (!bits) plan_lists(f_elim.data(), L, LL);
+  if (!bits) {
+    std::vector<int> f_elim(N);
+    GH_CUDA(cudaMemcpy(f_elim.data(), sets->elim, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost));
+    plan_lists(f_elim.data(), L, LL);
+  }
   const std::vector<int> &fcs = LL.fcs, &fcc = LL.fcc, &gmap = LL.gmap;
   const int64_t pstage_ints = LL.pstage_ints, partial_max = LL.partial_max;
   // ---- device state
@@ -1400,17 +1360,23 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
       ev_join.push_back(e);
     }
     GH_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    GH_CUDA(cudaMemcpy(slot_off_init, f_slot_off.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(deg_init, f_deg.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(cap_init, f_cap.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(elim_init, f_elim.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(cell_start, fcs.data(), sizeof(int) * fcs.size(), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(cell_count, fcc.data(), sizeof(int) * fcc.size(), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(adj_off, f_adj_off.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(adj_v, f_adj_v.data(), sizeof(int) * f_adj_v.size(), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(adj_w, f_adj_w.data(), sizeof(int) * f_adj_w.size(), cudaMemcpyHostToDevice));
-    if (heap_total)
-      GH_CUDA(cudaMemcpy(heap_verts, f_heap.data(), sizeof(int) * heap_total, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpyAsync(slot_off_init, sets->slot, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice));
+    GH_CUDA(cudaMemcpyAsync(deg_init, sets->deg, sizeof(int) * N, cudaMemcpyDeviceToDevice));
+    GH_CUDA(cudaMemcpyAsync(cap_init, sets->cap, sizeof(int) * N, cudaMemcpyDeviceToDevice));
+    GH_CUDA(cudaMemcpyAsync(elim_init, sets->elim, sizeof(int) * N, cudaMemcpyDeviceToDevice));
+    if (!fcs.empty()) GH_CUDA(cudaMemcpy(cell_start, fcs.data(), sizeof(int) * fcs.size(), cudaMemcpyHostToDevice));
+    if (!fcc.empty()) GH_CUDA(cudaMemcpy(cell_count, fcc.data(), sizeof(int) * fcc.size(), cudaMemcpyHostToDevice));
+    for (int i = 0, hb = 0; i < K; hb += L[i].heap_n, i++) {
+      const DeviceInput &in = input_device(*gs[i]);
+      const int n = gs[i]->n;
+      const int64_t m = gs[i]->m;
+      forest_arcs_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, (n + m + 256) / 256)), 256>>>(
+          in.off, in.v, in.w, n, m, vbase[i], (int)mbase[i], adj_off, adj_v, adj_w);
+      GH_CUDA(cudaGetLastError());
+      if (L[i].heap_n)
+        GH_CUDA(cudaMemcpyAsync(heap_verts + hb, elim_init + vbase[i] + L[i].heap_start, sizeof(int) * L[i].heap_n,
+                                cudaMemcpyDeviceToDevice));
+    }
     const unsigned long long first_free = (unsigned long long)lub;
     GH_CUDA(cudaMemcpy(pool_first, &first_free, sizeof(first_free), cudaMemcpyHostToDevice));
   } catch (...) {
@@ -1887,6 +1853,7 @@ void ElimPlan::build_lists() {
   for (size_t i = 0; i < gs.size(); i++) {
     Graph &g = *gs[i];
     const int vb = vbase[i];
+    g.elim.resize(g.n);
     g.father.resize(g.n);
     g.x_off.resize(g.n + 1);
     pool.parallel_for(g.n, 1 << 16, [&](int64_t lo, int64_t hi, int) {
@@ -2004,6 +1971,7 @@ void contract_gpu(Graph &g) {
       clk.reset();
     }
     owned.reset();  // the elimination's device state is freed here, inside the timed phase
+    g.sets.reset();
     g.t.translate_back += clk.us();
     return;
   }

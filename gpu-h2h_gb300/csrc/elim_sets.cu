@@ -24,11 +24,15 @@
 // arcs, interior flag, capacity and cell bound, interior count per chunk; a
 // one-block segmented scan over the level's chunks (per graph, continuing
 // from the levels below) gives every chunk and cell its offset; each chunk
-// writes its interior vertices in position order and retires them.
+// writes its interior vertices in position order and retires them.  The list
+// ranges follow from a scan of the capacities in partition-array order
+// (GraphPartition.cu:270-292).  The sets stay on the device: the host reads the
+// per-cell tables and a few sums (with the arrays going through the host the
+// sets and the elimination's tables of a 1M-vertex graph took 8.7 ms, now 2.5).
 #include <algorithm>
 
-#include "arena.h"
 #include "graph.h"
+#include "scan.h"
 
 namespace gh {
 
@@ -44,23 +48,27 @@ struct Chunk {
   int end;
 };
 
+struct SetsGraph {
+  const int *off, *nbr;    // n + 1 offsets, local neighbour ids
+  const int *part, *pos;   // local vertex per local position and its inverse
+  int vbase;               // the graph's first forest vertex and position
+};
+
 struct SetsArgs {
   const Chunk *chunks;     // this level's chunks, graph-major, cells from the highest index down
   int nchunks;
-  const int *vbase, *abase, *mbase;  // per graph: vertex / position base, adj_off base, arc base
-  const int *adj_off;      // per graph n + 1 offsets (local), at abase
-  const int *adj_v;        // local neighbour ids, at mbase
-  const int *part;         // local vertex per local position, at vbase
-  const int *pos;          // local position per local vertex, at vbase
+  const SetsGraph *graphs;
+  int ngraphs;
   int *dup;                // parallel arcs per vertex (forest)
   const int *cut_l, *cut_r;  // per global cell, local positions
   unsigned char *alive;    // per forest vertex
   unsigned char *flag;     // per forest position: interior at this level
-  int *cap;                // per forest vertex
+  int *cap, *deg;          // per forest vertex
+  int *cap_max;
   int *cell_sz, *cell_bound, *cell_start, *cell_count;  // per global cell
   int *chunk_cnt, *chunk_out;  // per chunk of the level
   int *gfill;              // per graph: elim entries written so far
-  int *elim;               // per graph's vertices, local ids, at vbase
+  int *elim;               // forest vertices, graph i's from its vbase
 };
 
 __device__ __forceinline__ int block_sum(int v, int *red) {
@@ -75,17 +83,28 @@ __device__ __forceinline__ int block_sum(int v, int *red) {
   return t;  // valid in thread 0
 }
 
-// Parallel arcs of every vertex: entries whose neighbour id appeared earlier
-// in the same input list.  One warp per vertex.
-__global__ void dup_kernel(SetsArgs A, const int *vertex_graph, int N) {
+// The graph of a forest vertex.
+__device__ __forceinline__ const SetsGraph &graph_of(const SetsArgs &A, int V) {
+  int lo = 0, hi = A.ngraphs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (A.graphs[mid].vbase <= V) lo = mid;
+    else hi = mid - 1;
+  }
+  return A.graphs[lo];
+}
+
+// Degree of every vertex, which its capacity starts from, and its parallel
+// arcs: entries whose neighbour id appeared earlier in the same input list.
+// One warp per vertex.
+__global__ void dup_kernel(SetsArgs A, int N) {
   const int lane = threadIdx.x & 31;
   for (int64_t V = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; V < N;
        V += (gridDim.x * (int64_t)blockDim.x) >> 5) {
-    const int gi = vertex_graph[V];
-    const int v = (int)V - A.vbase[gi];
-    const int *off = A.adj_off + A.abase[gi];
-    const int *nb = A.adj_v + A.mbase[gi];
-    const int b = off[v], e = off[v + 1];
+    const SetsGraph &G = graph_of(A, (int)V);
+    const int v = (int)V - G.vbase;
+    const int *nb = G.nbr;
+    const int b = G.off[v], e = G.off[v + 1];
     int d = 0;
     for (int i = b + lane; i < e; i += 32) {
       const int x = nb[i];
@@ -94,7 +113,11 @@ __global__ void dup_kernel(SetsArgs A, const int *vertex_graph, int N) {
       d += seen;
     }
     for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-    if (lane == 0) A.dup[V] = d;
+    if (lane == 0) {
+      A.dup[V] = d;
+      A.deg[V] = A.cap[V] = e - b;
+      A.alive[V] = 1;
+    }
   }
 }
 
@@ -103,9 +126,9 @@ __global__ void __launch_bounds__(kThreads) count_alive_kernel(SetsArgs A) {
   __shared__ int red[32];
   for (int k = blockIdx.x; k < A.nchunks; k += gridDim.x) {
     const Chunk c = A.chunks[k];
-    const int vb = A.vbase[c.graph];
+    const SetsGraph G = A.graphs[c.graph];
     int n = 0;
-    for (int j = c.start + threadIdx.x; j < c.end; j += blockDim.x) n += A.alive[vb + A.part[j]];
+    for (int j = c.start + threadIdx.x; j < c.end; j += blockDim.x) n += A.alive[G.vbase + G.part[j - G.vbase]];
     const int t = block_sum(n, red);
     if (threadIdx.x == 0 && t) atomicAdd(A.cell_sz + c.cell, t);
   }
@@ -116,20 +139,20 @@ __global__ void __launch_bounds__(kThreads) classify_kernel(SetsArgs A) {
   __shared__ int red[32];
   for (int k = blockIdx.x; k < A.nchunks; k += gridDim.x) {
     const Chunk c = A.chunks[k];
-    const int gi = c.graph, vb = A.vbase[gi];
-    const int *off = A.adj_off + A.abase[gi];
-    const int *nb = A.adj_v + A.mbase[gi];
+    const SetsGraph G = A.graphs[c.graph];
+    const int vb = G.vbase;
+    const int *off = G.off, *nb = G.nbr;
     const int cl = A.cut_l[c.cell], cr = A.cut_r[c.cell];  // local positions
     const int sz = A.cell_sz[c.cell];
     int interior = 0, bound = 0;
     for (int j = c.start + threadIdx.x; j < c.end; j += blockDim.x) {
-      const int v = A.part[j];  // local
+      const int v = G.part[j - vb];  // local
       unsigned char f = 0;
       if (A.alive[vb + v]) {
         int out = 0;
         for (int e = off[v]; e < off[v + 1]; e++) {
           const int u = nb[e];
-          const int pu = A.pos[vb + u];
+          const int pu = G.pos[u];
           out += A.alive[vb + u] && (pu < cl || pu >= cr);
         }
         f = out == 0;
@@ -219,7 +242,8 @@ __global__ void __launch_bounds__(kThreads) write_kernel(SetsArgs A) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int k = blockIdx.x; k < A.nchunks; k += gridDim.x) {
     const Chunk c = A.chunks[k];
-    const int vb = A.vbase[c.graph];
+    const SetsGraph G = A.graphs[c.graph];
+    const int vb = G.vbase;
     if (threadIdx.x == 0) s_base = A.chunk_out[k];
     __syncthreads();
     for (int j0 = c.start; j0 < c.end; j0 += blockDim.x) {
@@ -234,9 +258,9 @@ __global__ void __launch_bounds__(kThreads) write_kernel(SetsArgs A) {
         total += s_warp[w];
       }
       if (f) {
-        const int v = A.part[j];
-        A.elim[vb + s_base + before + __popc(bal & ((1u << lane) - 1u))] = v;
-        A.alive[vb + v] = 0;
+        const int V = vb + G.part[j - vb];
+        A.elim[vb + s_base + before + __popc(bal & ((1u << lane) - 1u))] = V;
+        A.alive[V] = 0;
       }
       __syncthreads();
       if (threadIdx.x == 0) s_base += total;
@@ -245,23 +269,46 @@ __global__ void __launch_bounds__(kThreads) write_kernel(SetsArgs A) {
   }
 }
 
+// Capacities in partition-array order (len[N] = 0) and the largest.
+__global__ void capacity_order_kernel(SetsArgs A, int *len, int N) {
+  int most = 0;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= N; j += gridDim.x * blockDim.x) {
+    int c = 0;
+    if (j < N) {
+      const SetsGraph &G = graph_of(A, j);
+      c = A.cap[G.vbase + G.part[j - G.vbase]];
+    }
+    len[j] = c;
+    most = max(most, c);
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(A.cap_max, most);
+}
+
+// List starts per vertex, and where every graph's lists end.
+__global__ void slot_kernel(SetsArgs A, const int64_t *start, int64_t *slot, int64_t *graph_end, int N) {
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
+    const SetsGraph &G = graph_of(A, j);
+    slot[G.vbase + G.part[j - G.vbase]] = start[j];
+  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.ngraphs; i += gridDim.x * blockDim.x)
+    graph_end[i] = start[i + 1 < A.ngraphs ? A.graphs[i + 1].vbase : N];
+}
+
 }  // namespace
 
 void build_elimination_sets(const std::vector<Graph *> &gs) {
   Clock clk;
   const int K = (int)gs.size();
   GH_CHECK(K >= 1, H2H_ERR_ARG, "no graph");
-  std::vector<int> vbase(K), abase(K), mbase(K), cbase(K);
-  int64_t N = 0, A = 0, M = 0, CELLS = 0;
+  std::vector<int> vbase(K), cbase(K);
+  int64_t N = 0, M = 0, CELLS = 0;
   int Hmax = 0;
   for (int i = 0; i < K; i++) {
     const Graph &g = *gs[i];
     vbase[i] = (int)N;
-    abase[i] = (int)A;
-    mbase[i] = (int)M;
     cbase[i] = (int)CELLS;
     N += g.n;
-    A += g.n + 1;
     M += g.m;
     CELLS += (int64_t(1) << g.H) - 1;
     Hmax = std::max(Hmax, g.H);
@@ -304,43 +351,34 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
     nchunk_total += (int64_t)lv[h].size();
   }
   // ---- device state
-  DeviceArena ws;
-  std::vector<int> f_cell_start(CELLS), f_cell_count(CELLS), f_cell_bound(CELLS), f_cap(N), f_dup(N), f_elim(N),
-      f_fill(K);
+  Workspace ws;
+  auto sets = std::make_shared<SetsStore>();
+  sets->gs = gs;
+  std::vector<int> f_cell(4 * CELLS), f_fill(K + 1);  // size, bound, start, count; placed per graph, largest capacity
+  std::vector<int64_t> graph_end(K);
   {
     SetsArgs S{};
-    int *d_vbase = ws.get<int>(K), *d_abase = ws.get<int>(K), *d_mbase = ws.get<int>(K);
-    int *d_adj_off = ws.get<int>(A), *d_adj_v = ws.get<int>(M);
-    int *d_part = ws.get<int>(N), *d_pos = ws.get<int>(N), *d_dup = ws.get<int>(N);
-    int *d_vgraph = ws.get<int>(N);
+    sets->elim = sets->mem.get<int>(N);
+    sets->cap = sets->mem.get<int>(N);
+    sets->deg = sets->mem.get<int>(N);
+    sets->slot = sets->mem.get<int64_t>(N);
+    SetsGraph *d_graphs = ws.get<SetsGraph>(K);
+    int *d_dup = ws.get<int>(N), *d_len = ws.get<int>(N + 1);
+    int64_t *d_start = ws.get<int64_t>(N + 1), *d_end = ws.get<int64_t>(K);
     int *d_cut_l = ws.get<int>(CELLS), *d_cut_r = ws.get<int>(CELLS);
     unsigned char *d_alive = ws.get<unsigned char>(N), *d_flag = ws.get<unsigned char>(N);
-    int *d_cap = ws.get<int>(N), *d_elim = ws.get<int>(N);
-    int *d_cell = ws.get<int>(4 * CELLS);  // size, bound, start, count
+    int *d_cell = ws.get<int>(4 * CELLS);
     int *d_chunk_cnt = ws.get<int>(nchunk_max), *d_chunk_out = ws.get<int>(nchunk_max);
     Chunk *d_chunks = ws.get<Chunk>(std::max<int64_t>(nchunk_total, 1));
-    int *d_fill = ws.get<int>(K);
-    GH_CUDA(cudaMemcpy(d_vbase, vbase.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(d_abase, abase.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(d_mbase, mbase.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
+    int *d_fill = ws.get<int>(K + 1);
+    std::vector<SetsGraph> table(K);
+    for (int i = 0; i < K; i++) {
+      const DeviceInput &in = input_device(*gs[i]);
+      table[i] = {in.off, in.v, in.part, in.pos, vbase[i]};
+    }
+    GH_CUDA(cudaMemcpy(d_graphs, table.data(), sizeof(SetsGraph) * K, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(d_cut_l, f_cut_l.data(), sizeof(int) * CELLS, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(d_cut_r, f_cut_r.data(), sizeof(int) * CELLS, cudaMemcpyHostToDevice));
-    {
-      std::vector<int> vgraph(N);
-      for (int i = 0; i < K; i++) {
-        const Graph &g = *gs[i];
-        std::fill(vgraph.begin() + vbase[i], vgraph.begin() + vbase[i] + g.n, i);
-        GH_CUDA(cudaMemcpy(d_adj_off + abase[i], g.adj_off.data(), sizeof(int) * (g.n + 1), cudaMemcpyHostToDevice));
-        if (g.m) GH_CUDA(cudaMemcpy(d_adj_v + mbase[i], g.adj_v.data(), sizeof(int) * g.m, cudaMemcpyHostToDevice));
-        if (g.n) {
-          GH_CUDA(cudaMemcpy(d_part + vbase[i], g.part_ids.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
-          GH_CUDA(cudaMemcpy(d_pos + vbase[i], g.id_hash.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
-        }
-        for (int v = 0; v < g.n; v++) f_cap[vbase[i] + v] = g.adj_off[v + 1] - g.adj_off[v];
-      }
-      GH_CUDA(cudaMemcpy(d_vgraph, vgraph.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    }
-    GH_CUDA(cudaMemcpy(d_cap, f_cap.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     {
       int64_t at = 0;
       for (int h = Hmax; h >= 1; h--) {
@@ -349,22 +387,18 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
         at += (int64_t)lv[h].size();
       }
     }
-    GH_CUDA(cudaMemset(d_alive, 1, N));
     GH_CUDA(cudaMemset(d_cell, 0, sizeof(int) * 4 * CELLS));
-    GH_CUDA(cudaMemset(d_fill, 0, sizeof(int) * K));
-    S.vbase = d_vbase;
-    S.abase = d_abase;
-    S.mbase = d_mbase;
-    S.adj_off = d_adj_off;
-    S.adj_v = d_adj_v;
-    S.part = d_part;
-    S.pos = d_pos;
+    GH_CUDA(cudaMemset(d_fill, 0, sizeof(int) * (K + 1)));
+    S.graphs = d_graphs;
+    S.ngraphs = K;
     S.dup = d_dup;
     S.cut_l = d_cut_l;
     S.cut_r = d_cut_r;
     S.alive = d_alive;
     S.flag = d_flag;
-    S.cap = d_cap;
+    S.cap = sets->cap;
+    S.deg = sets->deg;
+    S.cap_max = d_fill + K;
     S.cell_sz = d_cell;
     S.cell_bound = d_cell + CELLS;
     S.cell_start = d_cell + 2 * CELLS;
@@ -372,12 +406,12 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
     S.chunk_cnt = d_chunk_cnt;
     S.chunk_out = d_chunk_out;
     S.gfill = d_fill;
-    S.elim = d_elim;
+    S.elim = sets->elim;
     int dev = 0, nsm = 0;
     GH_CUDA(cudaGetDevice(&dev));
     GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     if (N) {
-      dup_kernel<<<std::max(1, std::min<int>(nsm * 16, (int)((N * 32 + 255) / 256))), 256>>>(S, d_vgraph, (int)N);
+      dup_kernel<<<std::max(1, std::min<int>(nsm * 16, (int)((N * 32 + 255) / 256))), 256>>>(S, (int)N);
       GH_CUDA(cudaGetLastError());
     }
     int64_t at = 0;
@@ -395,15 +429,18 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
       write_kernel<<<grid, kThreads>>>(S);
       GH_CUDA(cudaGetLastError());
     }
-    GH_CUDA(cudaMemcpy(f_fill.data(), d_fill, sizeof(int) * K, cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_elim.data(), d_elim, sizeof(int) * N, cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_cap.data(), d_cap, sizeof(int) * N, cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_dup.data(), d_dup, sizeof(int) * N, cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_cell_bound.data(), S.cell_bound, sizeof(int) * CELLS, cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_cell_start.data(), S.cell_start, sizeof(int) * CELLS, cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_cell_count.data(), S.cell_count, sizeof(int) * CELLS, cudaMemcpyDeviceToHost));
+    const int grid = std::max(1, std::min<int>(nsm * 8, (int)((N + 256) / 256)));
+    capacity_order_kernel<<<grid, 256>>>(S, d_len, (int)N);
+    GH_CUDA(cudaGetLastError());
+    exclusive_scan<int>(d_len, d_start, N + 1, ws, 0);
+    slot_kernel<<<grid, 256>>>(S, d_start, sets->slot, d_end, (int)N);
+    GH_CUDA(cudaGetLastError());
+    GH_CUDA(cudaMemcpy(f_fill.data(), d_fill, sizeof(int) * (K + 1), cudaMemcpyDeviceToHost));
+    GH_CUDA(cudaMemcpy(graph_end.data(), d_end, sizeof(int64_t) * K, cudaMemcpyDeviceToHost));
+    GH_CUDA(cudaMemcpy(f_cell.data(), d_cell, sizeof(int) * 4 * CELLS, cudaMemcpyDeviceToHost));
   }
   ws.release();
+  sets->cap_max = f_fill[K];
   const long long t_sets = clk.us();
   // ---- per graph: tables, LUB layout (GraphPartition.cu:270-292), level rates
   for (int i = 0; i < K; i++) {
@@ -412,13 +449,11 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
     GH_CHECK(f_fill[i] == g.n, H2H_ERR_FORMAT,
              "partition does not cover every vertex (root cut row must span all vertices)");
     const int64_t cells = (int64_t(1) << g.H) - 1;
-    g.cell_start.assign(f_cell_start.begin() + cbase[i], f_cell_start.begin() + cbase[i] + cells);
-    g.cell_count.assign(f_cell_count.begin() + cbase[i], f_cell_count.begin() + cbase[i] + cells);
+    const int *bound = f_cell.data() + CELLS + cbase[i], *start = bound + CELLS, *count = start + CELLS;
+    g.cell_start.assign(start, start + cells);
+    g.cell_count.assign(count, count + cells);
     g.cell_bound.resize(cells);
-    for (int64_t c = 0; c < cells; c++) g.cell_bound[c] = std::max(1, f_cell_bound[cbase[i] + c]);
-    g.elim.assign(f_elim.begin() + vbase[i], f_elim.begin() + vbase[i] + g.n);
-    g.cap.assign(f_cap.begin() + vbase[i], f_cap.begin() + vbase[i] + g.n);
-    g.dup.assign(f_dup.begin() + vbase[i], f_dup.begin() + vbase[i] + g.n);
+    for (int64_t c = 0; c < cells; c++) g.cell_bound[c] = std::max(1, bound[c]);
     g.layer_rate.assign(g.H + 1, 0.0);
     int64_t done = 0;
     for (int h = g.H; h > 0; h--) {
@@ -426,14 +461,8 @@ void build_elimination_sets(const std::vector<Graph *> &gs) {
       for (int64_t c = lo; c <= hi; c++) done += g.cell_count[c];
       g.layer_rate[h] = g.n ? (double)done / g.n : 0.0;
     }
-    g.slot_off.assign(g.n, 0);
-    int64_t off = 0;
-    for (int j = 0; j < g.n; j++) {
-      const int v = g.part_ids[j];
-      g.slot_off[v] = off;
-      off += g.cap[v];
-    }
-    g.lub = off;
+    g.lub = graph_end[i] - (i ? graph_end[i - 1] : 0);
+    g.sets = sets;
     g.t.rank_tree = t_sets;
     g.t.lub = clk.us();
   }

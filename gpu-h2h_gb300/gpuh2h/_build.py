@@ -23,7 +23,7 @@ LIB = os.path.join(OUT, "libgpuh2h.so")
 CLI = os.path.join(OUT, "G2H")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-LIB_SOURCES = ["io.cpp", "gen.cpp", "elim_sets.cu", "tree.cpp", "tree_gpu.cu", "capi.cpp", "contract.cu", "symbolic.cu", "labels.cu", "fill_blocks.cu", "query.cu", "noalloc.cu", "batch.cpp", "server.cpp", "loadgen.cpp", "index_io.cpp"]
+LIB_SOURCES = ["io.cpp", "gen.cpp", "input_gpu.cu", "elim_sets.cu", "tree.cpp", "tree_gpu.cu", "capi.cpp", "contract.cu", "symbolic.cu", "labels.cu", "fill_blocks.cu", "query.cu", "noalloc.cu", "batch.cpp", "server.cpp", "loadgen.cpp", "index_io.cpp"]
 
 
 def cuda_home() -> str:
@@ -90,7 +90,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     libdir = os.path.join(cuda, "lib64")
     if force or _stale(LIB, objs):
         tmp = LIB + ".tmp%d" % os.getpid()
-        subprocess.check_call([nvcc, *ARCH, "-shared", "-o", tmp, *objs, "-L" + libdir, "-lcudart", "-lpthread"])
+        subprocess.check_call([nvcc, *ARCH, "-shared", "-o", tmp, *objs, "-L" + libdir, "-lcudart", "-ldl", "-lpthread"])
         os.replace(tmp, LIB)
     main_obj = os.path.join(OBJ, "g2h_main.cpp.o")
     if force or _stale(CLI, [LIB, main_obj]):
