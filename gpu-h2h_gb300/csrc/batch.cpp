@@ -7,8 +7,8 @@
 // few SMs.  Here the graphs' vertices share one numbering: ElimPlan runs
 // level H_i - s of every graph in launch s and every graph's global order in
 // one last launch; FillPlan fills the forest of all trees in one
-// launch.  Host phases between them (elimination sets, tree, Euler tour,
-// sparse table, label layout) run per graph on a thread pool.
+// launch.  The phases between them (elimination sets, trees, sparse tables,
+// label layout) are launches over all graphs too.
 //
 // The list structure, the elimination order, the tree and the label layout
 // depend only on the arcs, never on their weights, so a rebuild after new
@@ -23,7 +23,6 @@
 
 #include "gpuh2h.h"
 #include "handle.h"
-#include "pool.h"
 
 namespace gh {
 std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds);
@@ -60,8 +59,7 @@ struct h2h_batch {
     int64_t upd = 0;
     for (gh::Graph *g : gs) {
       db += g->dev.bytes;
-      for (int v = 0; v < g->n; v++)
-        upd += (g->pos_hash[v + 1] - g->pos_hash[v] - 1) * (int64_t)std::max(g->depth[v] - 2, 0);
+      upd += g->updates;
     }
     info.device_bytes = db;
     info.label_updates = upd;
@@ -87,7 +85,7 @@ void copy_policy(const std::string &p, char *out, int cap) {
 
 extern "C" {
 
-int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch **out) {
+int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_batch **out) {
   if (out) *out = nullptr;
   if (!graphs || count <= 0 || !out) {
     gh::set_last_error("need graphs, count >= 1 and an output pointer");
@@ -104,32 +102,6 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch 
       b->gs.push_back(&g);
     }
     gh::Clock total, clk;
-    gh::Pool pool(std::max(1, threads));
-    // per-graph host phases run one graph per thread, largest graph first
-    std::vector<int> by_size(count);
-    for (int i = 0; i < count; i++) by_size[i] = i;
-    std::stable_sort(by_size.begin(), by_size.end(), [&](int x, int y) { return b->gs[x]->m > b->gs[y]->m; });
-    auto per_graph = [&](const std::function<void(gh::Graph &)> &fn) {
-      std::vector<int> saved(count);
-      for (int i = 0; i < count; i++) {
-        saved[i] = b->gs[i]->threads;
-        b->gs[i]->threads = 1;
-      }
-      std::vector<std::exception_ptr> errs(count);
-      pool.parallel_for(count, 1, [&](int64_t lo, int64_t hi, int) {
-        for (int64_t k = lo; k < hi; k++) {
-          const int i = by_size[k];
-          try {
-            fn(*b->gs[i]);
-          } catch (...) {
-            errs[i] = std::current_exception();
-          }
-        }
-      });
-      for (int i = 0; i < count; i++) b->gs[i]->threads = saved[i];
-      for (auto &e : errs)
-        if (e) std::rethrow_exception(e);
-    };
     gh::build_elimination_sets(b->gs);
     b->info.t_sets_us = clk.us();
     clk.reset();
@@ -155,26 +127,16 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch 
       }
       b->info.t_download_us = clk.us();
       clk.reset();
-      per_graph([](gh::Graph &g) {
-        gh::build_tree(g);
-        g.contracted = true;
-        g.parallel_fine = 2;
-        g.construct_device = 1;
-        g.label_mode = H2H_LABEL_L4;
-        gh::allocate_labels_and_bfs(g);
-      });
+      gh::build_tree_gpu(b->gs);
       gh::build_rmq_gpu(b->gs);
-      b->info.t_tree_us = clk.us();
-      if (std::getenv("GPUH2H_TRACE")) {
-        long long sum = 0, mx = 0;
-        for (gh::Graph *g : b->gs) {
-          const long long t = g->t.tree + g->t.malloc_labels + g->t.bfs;
-          sum += t;
-          mx = std::max(mx, t);
-        }
-        std::fprintf(stderr, "[gpuh2h] batch tree phase: %lld us wall, per-graph sum %lld us, max %lld us\n",
-                     (long long)b->info.t_tree_us, sum, mx);
+      for (gh::Graph *g : b->gs) {
+        g->contracted = true;
+        g->parallel_fine = 2;
+        g->construct_device = 1;
+        g->label_mode = H2H_LABEL_L4;
+        gh::allocate_labels_and_bfs(*g);
       }
+      b->info.t_tree_us = clk.us();
       clk.reset();
       gh::TilePolicy pol;
       if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))

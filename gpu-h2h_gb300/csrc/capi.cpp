@@ -361,16 +361,16 @@ int h2h_get_info(const h2h_graph *h, h2h_info *info) {
   info->change_height = g.C;
   info->head = g.head;
   info->tree_height = g.tree_height;
-  info->n_levels = g.tree_hash.empty() ? 0 : (int)g.tree_hash.size() - 1;
+  info->n_levels = g.n_levels;
   info->gpu_vertices = g.gpu_vertices;
   info->label_mode = g.label_mode;
   info->m = g.m;
   info->label_size = g.h2h_size;
-  info->pos_size = g.pos_hash.empty() ? 0 : g.pos_hash.back();
+  info->pos_size = g.pos_n;
   info->rmq_size = g.rmq_total;
   info->euler_size = g.euler_n;
   info->lub_size = g.lub;
-  info->adj_size = g.x_off.empty() ? 0 : g.x_off.back();
+  info->adj_size = g.x_total;
   info->device_bytes = g.dev.bytes;
   info->lub_mb = (double)g.lub * 12.0 / MB;
   info->decomposition_tree_mb = (double)g.decomposition_size * 12.0 / MB;
@@ -395,10 +395,7 @@ int h2h_get_info(const h2h_graph *h, h2h_info *info) {
     gh::set_last_error(e.what());
     return e.code;
   }
-  info->label_updates = 0;
-  if (!g.pos_hash.empty() && (int)g.depth.size() == g.n)
-    for (int v = 0; v < g.n; v++)
-      info->label_updates += (g.pos_hash[v + 1] - g.pos_hash[v] - 1) * (int64_t)std::max(g.depth[v] - 2, 0);
+  info->label_updates = g.pos_n ? g.updates : 0;
   return H2H_OK;
 }
 
@@ -406,7 +403,7 @@ int h2h_copy_order(const h2h_graph *h, int *order) {
   if (!h || !order) { gh::set_last_error("null argument"); return H2H_ERR_ARG; }
   return guarded([&] {
     GH_CHECK(h->g.contracted, H2H_ERR_STATE, "not contracted");
-    std::copy(h->g.elim.begin(), h->g.elim.end(), order);
+    gh::download_tree(h->g, order, nullptr, nullptr, nullptr, nullptr);
   });
 }
 
@@ -415,9 +412,7 @@ int h2h_copy_tree(const h2h_graph *h, int *father, int *depth, int *first) {
   return guarded([&] {
     const gh::Graph &g = h->g;
     GH_CHECK(g.contracted, H2H_ERR_STATE, "not contracted");
-    if (father) std::copy(g.father.begin(), g.father.end(), father);
-    if (depth) std::copy(g.depth.begin(), g.depth.end(), depth);
-    if (first) std::copy(g.first.begin(), g.first.end(), first);
+    gh::download_tree(g, nullptr, father, depth, first, nullptr);
   });
 }
 
@@ -435,7 +430,7 @@ int h2h_copy_adj(const h2h_graph *h, int64_t *adj_hash, int *adj_id, int *adj_w)
   return guarded([&] {
     const gh::Graph &g = h->g;
     GH_CHECK(g.contracted, H2H_ERR_STATE, "not contracted");
-    if (adj_hash) std::copy(g.x_off.begin(), g.x_off.end(), adj_hash);
+    gh::download_tree(g, nullptr, nullptr, nullptr, nullptr, adj_hash);
     if (adj_id || adj_w) {
       gh::Graph &gm = const_cast<gh::Graph &>(g);
       gh::download_lists(gm);  // the lists live on the device
@@ -454,6 +449,7 @@ int h2h_copy_labels(const h2h_graph *h, int64_t *dis_hash, int *dis, int64_t *po
   return guarded([&] {
     const gh::Graph &g = h->g;
     GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
+    if (dis_hash || dis || pos_hash) gh::host_tree(g);
     if (dis_hash) std::copy(g.dis_hash.begin(), g.dis_hash.end(), dis_hash);
     if (dis) gh::download_labels(g, dis);
     if (pos_hash) std::copy(g.pos_hash.begin(), g.pos_hash.end(), pos_hash);
@@ -486,6 +482,7 @@ int h2h_copy_bfs(const h2h_graph *h, int *tree_bfs, int *tree_hash) {
   return guarded([&] {
     const gh::Graph &g = h->g;
     GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
+    gh::host_tree(g);
     if (tree_bfs) std::copy(g.tree_bfs.begin(), g.tree_bfs.end(), tree_bfs);
     if (tree_hash) std::copy(g.tree_hash.begin(), g.tree_hash.end(), tree_hash);
   });

@@ -58,7 +58,7 @@
 #include <queue>
 
 #include "graph.h"
-#include "pool.h"
+#include "scan.h"
 
 namespace cg = cooperative_groups;
 
@@ -1325,7 +1325,7 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
     pool_first = mem.get<unsigned long long>(1);
     slot_off = mem.get<int64_t>(N);
     slot_off_init = mem.get<int64_t>(N);
-    lsize = mem.get<int>(N);
+    lsize = mem.get<int>((int64_t)N + 1);  // + 1: the end of a scan
     cap = mem.get<int>(N);
     cap_init = mem.get<int>(N);
     height = mem.get<int>(N);
@@ -1666,7 +1666,7 @@ void ElimPlan::release() {
   grid_map = nullptr;
   hg_partial = nullptr;
   grid_bar = nullptr;
-  rank = father_dev = nullptr;
+  rank = nullptr;
   for (cudaStream_t st : side) cudaStreamDestroy(st);
   for (cudaEvent_t e : ev_join) cudaEventDestroy(e);
   if (ev_fork) cudaEventDestroy(ev_fork);
@@ -1816,30 +1816,33 @@ void ElimPlan::check_error() {
 }
 
 void ElimPlan::build_lists() {
-  int threads = 1;
-  for (const Graph *g : gs) threads = std::max(threads, g->threads);
-  Pool pool(useful_threads(threads, N));
-  std::vector<int, NoInit<int>> f_lsize(N), f_elim(N), f_father(N);
-  GH_CUDA(cudaMemcpy(f_lsize.data(), lsize, sizeof(int) * N, cudaMemcpyDeviceToHost));
-  std::vector<int64_t, NoInit<int64_t>> off(N + 1);
-  parallel_prefix(pool, N, off.data(), [&](int64_t v) { return (int64_t)f_lsize[v]; });
-  const int64_t tot = off[N];
   auto la = std::make_shared<ListArrays>();
-  la->off = la->mem.get<int64_t>(N + 1);
-  la->id = la->mem.get<int>(tot);
-  la->w = la->mem.get<int>(tot);
+  la->off = la->mem.get<int64_t>((int64_t)N + 1);
+  {
+    Workspace ws;
+    GH_CUDA(cudaMemsetAsync(lsize + N, 0, sizeof(int)));
+    exclusive_scan<int>(lsize, la->off, (int64_t)N + 1, ws, 0);
+    GH_CUDA(cudaMemcpy(&lists.total, la->off + N, sizeof(int64_t), cudaMemcpyDeviceToHost));
+  }
+  la->id = la->mem.get<int>(lists.total);
+  la->w = la->mem.get<int>(lists.total);
   lists.off = la->off;
   lists.id = la->id;
   lists.w = la->w;
-  lists.total = tot;
   lists.keep = la;
+  auto tree = std::make_shared<TreeStore>();
+  tree->gs = gs;
+  tree->vbase = vbase;
+  tree->vbase.push_back(N);
+  tree->n = N;
+  tree->elim = tree->mem.get<int>(N);
+  tree->father = tree->mem.get<int>(N);
   if (!rank) rank = mem.get<int>(N);
-  if (!father_dev) father_dev = mem.get<int>(N);
-  GH_CUDA(cudaMemcpy(lists.off, off.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
   enqueue_gather(0);
+  GH_CUDA(cudaMemcpyAsync(tree->elim, elim, sizeof(int) * N, cudaMemcpyDeviceToDevice));
   rank_kernel<<<std::max(1, std::min(4096, (N + 255) / 256)), 256>>>(elim, rank, N);
   GH_CUDA(cudaGetLastError());
-  father_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256>>>(lists.off, lists.id, rank, father_dev, N);
+  father_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256>>>(lists.off, lists.id, rank, tree->father, N);
   GH_CUDA(cudaGetLastError());
   if (own_slots) {  // the lists never run again: only their weights are replayed
     cudaFree(slot_nbr);
@@ -1848,28 +1851,13 @@ void ElimPlan::build_lists() {
     own_slots = false;
     slot_bytes = 0;
   }
-  GH_CUDA(cudaMemcpy(f_elim.data(), elim, sizeof(int) * N, cudaMemcpyDeviceToHost));
-  GH_CUDA(cudaMemcpy(f_father.data(), father_dev, sizeof(int) * N, cudaMemcpyDeviceToHost));
   for (size_t i = 0; i < gs.size(); i++) {
     Graph &g = *gs[i];
-    const int vb = vbase[i];
-    g.elim.resize(g.n);
-    g.father.resize(g.n);
-    g.x_off.resize(g.n + 1);
-    pool.parallel_for(g.n, 1 << 16, [&](int64_t lo, int64_t hi, int) {
-      for (int64_t v = lo; v < hi; v++) {
-        g.elim[v] = f_elim[vb + v] - vb;
-        g.father[v] = f_father[vb + v] < 0 ? -1 : f_father[vb + v] - vb;
-        g.x_off[v + 1] = off[vb + v + 1] - off[vb];
-      }
-    });
-    g.x_off[0] = 0;
-    g.decomposition_size = g.x_off[g.n] + g.n;
+    std::vector<int>().swap(g.elim);
     std::vector<int>().swap(g.x_id);
     std::vector<int>().swap(g.x_w);
+    g.tree = tree;
     g.dev.lists = lists;
-    g.dev.x_base = off[vb];
-    g.dev.id_base = vb;
   }
 }
 
@@ -1905,8 +1893,8 @@ ListStore upload_lists(const std::vector<int64_t> &off, const std::vector<int> &
 
 void download_lists(Graph &g) {
   const ListStore &L = g.dev.lists;
-  GH_CHECK(L.id && (int64_t)g.x_off.size() == g.n + 1, H2H_ERR_STATE, "not contracted");
-  const int64_t t = g.x_off[g.n];
+  GH_CHECK(L.id, H2H_ERR_STATE, "not contracted");
+  const int64_t t = g.x_total;
   g.x_id.resize(t);
   g.x_w.resize(t);
   if (t) {
@@ -1919,9 +1907,8 @@ void download_lists(Graph &g) {
 
 // Whole contraction of one graph on the GPU: partition levels H..C+1, then
 // the global order over the vertices of levels <= C, the tree and the sparse
-// table.  Fills g.elim (elimination order), g.father, g.x_off and
-// g.gpu_vertices; the lists X(v)\{v} (sorted by id, the lists at elimination
-// time) stay on the device.  On bit rows the lists' weights follow from the
+// table.  The order, the fathers and the lists X(v)\{v} (sorted by id, the
+// lists at elimination time) stay on the device.  On bit rows the lists' weights follow from the
 // tree's blocks, which g.plan keeps for the label fill.
 void contract_gpu(Graph &g) {
   Clock clk;
@@ -1954,10 +1941,10 @@ void contract_gpu(Graph &g) {
     clk.reset();
     plan.build_lists();
     g.t.translate_back = clk.us();
-    build_tree_and_rmq(g);
+    build_tree_gpu({&g});
+    build_rmq_gpu({&g});
     clk.reset();
     if (plan.bits) {
-      position_offsets(g);
       g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, plan.lists, &plan);
       if (!g.plan->weights_fit) {  // very wide separators: the list kernels, which need no update triangles
         g.plan.reset();

@@ -1160,9 +1160,6 @@ T read_one(const T *p) {
 // Cuts the forest into blocks and lays out their tables (weights come later,
 // with enqueue).
 void FillPlan::build_blocks() {
-  int height = 0;
-  for (const Graph *g : gs) height = std::max(height, (int)g->tree_hash.size() - 1);
-  nlev = height;
   const int grid = grid_for(N, nsm);
   Workspace ws;
   int *size = ws.get<int>(N), *weight = ws.get<int>(N), *block_top = ws.get<int>(N), *top_of = ws.get<int>(N);

@@ -56,6 +56,31 @@ struct SetsStore {
   int cap_max = 0;
 };
 
+// The trees of the graphs contracted together, on the device in the
+// contraction's numbering (tree_gpu.cu): graph i's vertices are vbase[i] ..
+// vbase[i + 1] - 1.
+struct TreeStore {
+  DeviceArena mem;                // of the arrays that live as long as the labels
+  std::vector<Graph *> gs;
+  std::vector<int> vbase;         // [graphs + 1]
+  int n = 0;
+  int *elim = nullptr, *father = nullptr, *depth = nullptr;  // order; father (-1: a root); depth, roots 1
+  int64_t *drow = nullptr, *pos_hash = nullptr;              // padded row and position-list offsets [n + 1]
+  int64_t pos_total = 0, dis_total = 0, seg_total = 0;
+  int height = 0, max_segs = 0, max_list = 0;
+  // until the sparse tables are built: first appearance (per graph) and the
+  // Euler tours (graph-local vertices), graph i's from 2 * vbase[i] - i
+  std::unique_ptr<DeviceArena> tour;
+  int *first = nullptr, *euler = nullptr;
+  // until the labels are built: hld lists the heavy paths one after another,
+  // top to bottom (hpos[v] = v's index, htop[v] = the top of v's path); node
+  // v's root path is the segments seg_off[v] .. seg_off[v+1]-1, shallowest
+  // first, one per heavy path it crosses (written by FillPlan)
+  std::shared_ptr<DeviceArena> layout;
+  int *hld = nullptr, *htop = nullptr, *hpos = nullptr;
+  int64_t *seg_off = nullptr;
+};
+
 // Device-resident index used by the label fill and the query kernels.
 // Label rows are padded so every row starts on a 16-byte boundary
 // (drow[v] is a multiple of 4 ints); the reference layout is restored on
@@ -112,39 +137,34 @@ struct Graph : HostInput {
   std::vector<int> cut_l, cut_r;   // partition_Tree rows [2^H-1]
   // elimination sets (GraphPartition.cu:178-308)
   std::vector<int> cell_start, cell_count;  // NANHash first / NodeID per cell
-  std::vector<int> elim;                    // elimination order
+  std::vector<int> elim;                    // elimination order (host_tree)
   std::vector<int> cell_bound;              // per partition cell: bound on a list while its level runs
   std::shared_ptr<SetsStore> sets;          // until the graph is contracted
   int64_t lub = 0;
   std::vector<double> layer_rate;           // afs[h] / n for the PartitionRate CSV
-  // contraction results
-  std::vector<int> height;                  // CHInfo.second after the partition levels
+  // contraction results: on the device (tree, dev.lists); the host arrays
+  // below are filled by host_tree, the lists by download_lists
+  std::shared_ptr<TreeStore> tree;
   std::vector<int64_t> x_off;               // X(v)\{v}: upper neighbours, CSR by vertex [n+1]
-  std::vector<int> x_id, x_w;               //   sorted by id, shortcut weights (host copies on demand)
+  std::vector<int> x_id, x_w;               //   sorted by id, shortcut weights
   int gpu_vertices = 0;                     // vertexesConstructedInGPU
+  int64_t x_total = 0;                      // entries of the lists
   int64_t decomposition_size = 0;           // size1 = sum(|X(v)|+1)
   bool contracted = false;
   // tree (TreeStructure.cu)
-  int head = -1, tree_height = 0;
-  std::vector<int> father, depth, first, child_off, childs;
-  std::vector<int> euler_id;                // Euler tour (vertex per position), until the table is built
+  int head = -1, tree_height = 0, n_levels = 0;
+  std::vector<int> father, depth, first;
   int64_t euler_n = 0, h2h_size = 0, rmq_total = 0;  // rmq_total: RMQ_ID entries (the table is on the GPU)
   // labels (H2HConsturction.cu), reference layout on the host
   std::vector<int64_t> dis_hash, pos_hash;
+  int64_t pos_n = 0;                        // entries of the position lists, once the labels are laid out
+  int64_t updates = 0;                      // min-plus updates of the fill
   // host position lists: built for L3 labels only (L4 builds them on the GPU;
   // accessors download them)
   std::vector<int> pos_id, pos_pos, pos_w;  // pos_w: shortcut weight per pos entry (0 for v itself)
   std::vector<int64_t> drow_host;           // padded device row offsets (absolute in a batch's forest)
+  int64_t row0 = 0, row1 = 0;               // the first and the end
   std::vector<int> tree_bfs, tree_hash;     // TreeBFS / TreeHash
-  // heavy-path decomposition of the tree for ancestor lookups in the fill:
-  // hld lists the heavy paths one after another, top to bottom (hpos[v] =
-  // v's index, htop[v] = the top of v's path); node v's root path is the
-  // segments seg_off[v] .. seg_off[v+1]-1, shallowest first, one per heavy
-  // path it crosses (written on the GPU by FillPlan)
-  std::vector<int> hld, htop, hpos;
-  std::vector<int64_t> seg_off;
-  int max_segs = 0;
-  bool tree_layout = false;  // depth, first, level order, heavy paths, segments and dis_hash built on the GPU
   bool labelled = false;
   int64_t max_label = 0;  // -1: not computed yet (label_max computes it)
   // device
@@ -153,6 +173,12 @@ struct Graph : HostInput {
   Timings t;
 
   ~Graph() { dev.release(); }
+};
+
+// The label arrays of graphs filled together.
+struct LabelStore {
+  DeviceArena mem;
+  std::shared_ptr<TreeStore> tree;
 };
 
 // Where a graph's global order starts: the vertices of the cells at levels
@@ -223,7 +249,7 @@ struct ElimPlan {
   int64_t *slot_off = nullptr, *slot_off_init = nullptr;
   unsigned long long *pool_next = nullptr, *pool_first = nullptr;
   ListStore lists;       // compact final lists (forest numbering), after build_lists()
-  int *rank = nullptr, *father_dev = nullptr;
+  int *rank = nullptr;
   // cell_grid_kernel state: per-block argmins, block maps, barrier counters
   int *grid_map = nullptr;
   void *hg_partial = nullptr;
@@ -249,10 +275,9 @@ struct ElimPlan {
   void enqueue(cudaStream_t s, cudaEvent_t *heap_ev = nullptr, bool trace = false);
   void launch_one(const Launch &Lc, cudaStream_t s, bool trace);
   void check_error();  // synchronises; throws on a kernel error code
-  // After the first enqueue: compact the final lists on the device, pick each
-  // vertex's father (min elimination rank over its list) there, and hand each
-  // graph its elimination order, list offsets and fathers; the lists stay on
-  // the device (each graph's DeviceIndex gets a view).
+  // After the first enqueue: compact the final lists and pick each vertex's
+  // father (min elimination rank over its list), all on the device; every
+  // graph gets the lists and the tree they start.
   void build_lists();
   // Refreshes the compact lists' entries from the slot arrays (replays).
   void enqueue_gather(cudaStream_t s);
@@ -285,7 +310,7 @@ struct FillPlan {
   int N = 0;
   int64_t pos_total = 0, dis_total = 0;
   TilePolicy policy;
-  std::shared_ptr<void> storage;  // forest arrays shared with the graphs' views
+  std::shared_ptr<struct LabelStore> storage;  // forest arrays shared with the graphs' views
   int64_t *drow = nullptr, *pos_hash = nullptr;
   int *pos_pos = nullptr, *pos_id = nullptr, *pos_w = nullptr, *pos_src = nullptr, *father = nullptr;
   ListStore lists;
@@ -324,8 +349,9 @@ struct FillPlan {
   size_t smem = 0;
   int nsm = 0;
   DeviceArena work;       // the plan's arrays but tasks and mbuf, which grow with the policy
+  std::shared_ptr<DeviceArena> layout;  // the tree's heavy paths and segment offsets
   int64_t grown_bytes = 0;
-  int64_t work_bytes() const { return work.bytes + grown_bytes; }
+  int64_t work_bytes() const { return work.bytes + (layout ? layout->bytes : 0) + grown_bytes; }
   // The blocks and, when `arcs` made the order on bit rows, where each of its
   // arcs enters the blocks' weights.  lists: the graphs' X lists in the same
   // forest numbering.
@@ -346,7 +372,7 @@ struct FillPlan {
   void enqueue(cudaStream_t s, cudaEvent_t *fill_ev = nullptr);
   void check_error();            // synchronises; throws if a dependency wait ran out
   void trace_report();           // GPUH2H_TRACE: the last fill's time per level class
-  void attach(bool first);       // per-graph views, max_label; first: also drow_host
+  void attach(bool first);       // per-graph views; first: of new arrays
 };
 
 // Phases (one translation unit each).
@@ -359,22 +385,17 @@ void load_graph(Graph &g, const std::string &edge, const std::string &idf, const
 // bounds and parallel-arc counts of one or more graphs, on the GPU
 void build_elimination_sets(const std::vector<Graph *> &gs);
 // contract.cu: partition levels H..C+1 and the global heap over levels <= C;
-// fills g.elim (elimination order) and g.x_off / x_id / x_w
-// contraction (then the tree, sparse table and weights of one graph)
+// (then the tree, sparse table and weights of one graph)
 void contract_gpu(Graph &g);
-void position_offsets(Graph &g);                       // tree.cpp: pos_hash
-void build_tree(Graph &g);                             // tree.cpp: father, children, Euler tour
-// tree_gpu.cu: the same on the GPU, plus the level order, heavy paths and
-// root-path segment offsets (sets g.tree_layout)
-void build_tree_gpu(Graph &g);
+// tree_gpu.cu: the tree of every graph contracted together (children, tour,
+// depths, heavy paths, offsets) from the fathers, on the GPU
+void build_tree_gpu(const std::vector<Graph *> &gs);
+const Graph &host_tree(const Graph &g);                // tree_gpu.cu: fills the host arrays of the tree
+void download_tree(const Graph &g, int *order, int *father, int *depth, int *first, int64_t *x_off);  // tree_gpu.cu
 // query.cu: the compacted sparse tables of the graphs' Euler tours on the
 // GPU (first, rmq_hash, rmq_id in each graph's DeviceIndex)
 void build_rmq_gpu(const std::vector<Graph *> &gs);
 void download_rmq(const Graph &g, int64_t *rmq_hash, int *rmq_id);  // query.cu
-inline void build_tree_and_rmq(Graph &g) {
-  build_tree_gpu(g);
-  build_rmq_gpu({&g});
-}
 void allocate_labels_and_bfs(Graph &g);                // tree.cpp
 void fill_labels_gpu(Graph &g);                        // labels.cu
 // The level-synchronous fill (L3 labels, or L4 with GPUH2H_LEVEL_FILL set)

@@ -104,6 +104,7 @@ int h2h_save_index(const h2h_graph *h, const char *path) {
     gh::Graph &g = const_cast<gh::Graph &>(h->g);
     GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
     const int n = g.n;
+    gh::host_tree(g);
     std::vector<int64_t> rmq_hash(g.euler_n);
     std::vector<int> rmq_id(g.rmq_total);
     gh::download_rmq(g, rmq_hash.data(), rmq_id.data());
@@ -259,6 +260,10 @@ int h2h_load_index(const char *path, h2h_graph **out) {
     int64_t h2h = 0;
     for (int v = 0; v < n; v++) h2h += g.depth[v];
     g.h2h_size = h2h;
+    g.n_levels = hd.n_levels;
+    g.x_total = hd.x_total;
+    g.pos_n = hd.pos_total;
+    for (int v = 0; v < n; v++) g.updates += (g.x_off[v + 1] - g.x_off[v]) * (int64_t)std::max(g.depth[v] - 2, 0);
     // device index
     gh::upload_rmq(g, rmq_hash, rmq_id);
     g.dev.lists = gh::upload_lists(g.x_off, g.x_id, g.x_w);

@@ -30,7 +30,6 @@
 #include <sstream>
 
 #include "graph.h"
-#include "pool.h"
 
 namespace gh {
 
@@ -344,125 +343,45 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
     std::fprintf(stderr, "[gpuh2h] fill plan: %s %.3f ms\n", what, tclk.us() / 1e3);
     tclk.reset();
   };
-  const int K = (int)gs.size();
-  GH_CHECK(K >= 1, H2H_ERR_ARG, "no graph to label");
-  int host_threads = 1;
-  for (const Graph *g : gs) host_threads = std::max(host_threads, g->threads);
-  // vertex ranges of every graph, in parallel: padded row totals and the
-  // widest separator
-  struct VRange {
-    int g, v0, v1;
-  };
-  std::vector<VRange> vr;
-  for (int i = 0; i < K; i++)
-    for (int v = 0; v < gs[i]->n; v += 65536) vr.push_back({i, v, std::min(gs[i]->n, v + 65536)});
-  const int64_t nvr = (int64_t)vr.size();
-  std::vector<int64_t> rdis(nvr, 0), rbase(nvr, 0);
-  std::vector<int> rmax_m(nvr, 0);
-  int64_t total_n = 0;
-  for (const Graph *g : gs) total_n += g->n;
-  Pool pool(useful_threads(host_threads, total_n));
-  pool.parallel_for(nvr, 1, [&](int64_t lo, int64_t hi, int) {
-    for (int64_t r = lo; r < hi; r++) {
-      const Graph &g = *gs[vr[r].g];
-      int64_t d = 0, mm = 0;
-      for (int v = vr[r].v0; v < vr[r].v1; v++) {
-        d += (g.depth[v] + 3) & ~3;
-        mm = std::max<int64_t>(mm, g.x_off[v + 1] - g.x_off[v]);
-      }
-      rdis[r] = d;
-      rmax_m[r] = (int)mm;
-    }
-  });
-  std::vector<int64_t> gdis(K, 0);
-  std::vector<int> gmax_m(K, 0);
-  for (int64_t r = 0; r < nvr; r++) {
-    rbase[r] = gdis[vr[r].g];  // offset inside the graph's rows
-    gdis[vr[r].g] += rdis[r];
-    gmax_m[vr[r].g] = std::max(gmax_m[vr[r].g], rmax_m[r]);
-  }
-  vbase.assign(K, 0);
-  std::vector<int64_t> pbase(K, 0), dbase(K, 0);
-  int max_m = 0;
-  for (int i = 0; i < K; i++) {
-    const Graph &g = *gs[i];
-    GH_CHECK((int64_t)N + g.n < INT32_MAX, H2H_ERR_ARG, "too many vertices in one batch");
-    vbase[i] = N;
-    pbase[i] = pos_total;
-    dbase[i] = dis_total;
-    N += g.n;
-    pos_total += g.pos_hash[g.n];
-    dis_total += gdis[i];
-    max_m = std::max(max_m, gmax_m[i]);
-  }
-  // forest arrays, every entry written below (so not zero-filled first)
-  std::vector<int64_t, NoInit<int64_t>> f_drow(N + 1), f_pos_hash(N + 1);
-  std::vector<int, NoInit<int>> f_father(N), f_depth(N), f_hld(N);
-  std::vector<int64_t> sbase(K, 0);
-  int64_t seg_total = 0;
-  for (int i = 0; i < K; i++) {
-    sbase[i] = seg_total;
-    seg_total += gs[i]->seg_off[gs[i]->n];
-    max_segs = std::max(max_segs, gs[i]->max_segs);
-  }
-  std::vector<int64_t, NoInit<int64_t>> f_seg_off(N + 1);
-  std::vector<int, NoInit<int>> f_htop(N), f_hpos(N);
-  pool.parallel_for(nvr, 1, [&](int64_t lo, int64_t hi, int) {
-    for (int64_t r = lo; r < hi; r++) {
-      const int i = vr[r].g;
-      const Graph &g = *gs[i];
-      const int vb = vbase[i];
-      const int64_t pb = pbase[i];
-      int64_t d = dbase[i] + rbase[r];
-      for (int v = vr[r].v0; v < vr[r].v1; v++) {
-        const int V = vb + v;
-        f_drow[V] = d;
-        d += (g.depth[v] + 3) & ~3;
-        f_pos_hash[V] = pb + g.pos_hash[v];
-        f_father[V] = g.father[v] < 0 ? -1 : g.father[v] + vb;
-        f_depth[V] = g.depth[v];
-        f_hld[V] = g.hld[v] + vb;
-        f_htop[V] = g.htop[v] + vb;
-        f_hpos[V] = g.hpos[v] + vb;
-        f_seg_off[V] = sbase[i] + g.seg_off[v];
-      }
-    }
-  });
-  f_drow[N] = dis_total;
-  f_pos_hash[N] = pos_total;
-  f_seg_off[N] = seg_total;
-  mark("host assembly");
+  GH_CHECK(!gs.empty(), H2H_ERR_ARG, "no graph to label");
+  const std::shared_ptr<TreeStore> tree = gs[0]->tree;
+  GH_CHECK(tree && tree->gs == gs && tree->layout, H2H_ERR_STATE, "tree not built");
+  vbase = tree->vbase;
+  vbase.pop_back();
+  N = tree->n;
+  pos_total = tree->pos_total;
+  dis_total = tree->dis_total;
+  max_segs = std::max(max_segs, tree->max_segs);
+  nlev = tree->height;
+  layout = tree->layout;
   int dev = 0;
   GH_CUDA(cudaGetDevice(&dev));
   GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  auto st = std::make_shared<DeviceArena>();
-  storage = st;
-  drow = st->get<int64_t>(N + 1);
-  pos_hash = st->get<int64_t>(N + 1);
-  pos_pos = st->get<int>(pos_total);
-  pos_id = st->get<int>(pos_total);
-  father = st->get<int>(N);
-  depth = st->get<int>(N);
+  storage = std::make_shared<LabelStore>();
+  storage->tree = tree;
+  drow = tree->drow;
+  pos_hash = tree->pos_hash;
+  father = tree->father;
+  depth = tree->depth;
+  hld = tree->hld;
+  htop = tree->htop;
+  hpos = tree->hpos;
+  seg_off = tree->seg_off;
+  const int64_t seg_total = tree->seg_total;
+  const int max_m = tree->max_list;
+  pos_pos = storage->mem.get<int>(pos_total);
+  pos_id = storage->mem.get<int>(pos_total);
   try {
     pos_w = work.get<int>(pos_total);
     pos_src = work.get<int>(pos_total);
-    hld = work.get<int>(N);
-    htop = work.get<int>(N);
-    hpos = work.get<int>(N);
-    seg_off = work.get<int64_t>(N + 1);
     seg_top = work.get<int>(std::max<int64_t>(seg_total, 1));
     seg_pos = work.get<int>(std::max<int64_t>(seg_total, 1));
     next = work.get<int>(1);
     err = work.get<int>(1);
-    GH_CUDA(cudaMemcpy(drow, f_drow.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(pos_hash, f_pos_hash.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(father, f_father.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(depth, f_depth.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(hld, f_hld.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     hld_row = work.get<int64_t>(N);
     hld_row_kernel<<<std::max(1, std::min(8192, (N + 255) / 256)), 256>>>(hld, drow, hld_row, N);
     GH_CUDA(cudaGetLastError());
-    mark("allocations and uploads");
+    mark("allocations");
     {
       const size_t ksmem = (size_t)(max_m + 1) * sizeof(int);
       const int kdyn = enable_max_dynamic_smem(build_positions_kernel);
@@ -476,9 +395,6 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
       GH_CHECK(e == 0, H2H_ERR_STATE, "an upper neighbour is not an ancestor in the tree");
     }
     mark("position lists");
-    GH_CUDA(cudaMemcpy(seg_off, f_seg_off.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(htop, f_htop.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    GH_CUDA(cudaMemcpy(hpos, f_hpos.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     root_path_segments_kernel<<<std::max(1, std::min(8192, (N + 255) / 256)), 256>>>(father, depth, htop, hpos,
                                                                                      seg_off, seg_top, seg_pos, N);
     GH_CUDA(cudaGetLastError());
@@ -498,12 +414,13 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
 FillPlan::~FillPlan() { release_work(); }
 
 void FillPlan::prepare(const TilePolicy &pol) {
-  dis = static_cast<DeviceArena *>(storage.get())->get<int>(dis_total);
+  dis = storage->mem.get<int>(dis_total);
   build_tiles(pol);
 }
 
 void FillPlan::release_work() {
   work.release();
+  layout.reset();
   for (void *p : {(void *)tasks, (void *)mbuf, (void *)trace_t}) cudaFree(p);
   grown_bytes = tasks_cap = mslots_cap = 0;
   trace_t = nullptr;
@@ -566,13 +483,6 @@ void FillPlan::check_error() {
 }
 
 void FillPlan::attach(bool first) {
-  std::vector<int64_t> f_drow, f_pos_hash;
-  if (first) {
-    f_drow.resize(N + 1);
-    f_pos_hash.resize(N + 1);
-    GH_CUDA(cudaMemcpy(f_drow.data(), drow, sizeof(int64_t) * (N + 1), cudaMemcpyDeviceToHost));
-    GH_CUDA(cudaMemcpy(f_pos_hash.data(), pos_hash, sizeof(int64_t) * (N + 1), cudaMemcpyDeviceToHost));
-  }
   for (size_t i = 0; i < gs.size(); i++) {
     Graph &g = *gs[i];
     DeviceIndex &D = g.dev;
@@ -588,15 +498,15 @@ void FillPlan::attach(bool first) {
       D.pos_pos = pos_pos;
       D.pos_id = pos_id;
       D.dis = dis;
-      D.pos = f_pos_hash[vb + g.n] - f_pos_hash[vb];
-      D.pos_base = f_pos_hash[vb];
-      D.dis_padded = f_drow[vb + g.n] - f_drow[vb];
+      D.pos = g.pos_n;
+      D.pos_base = D.x_base + vb;
+      D.dis_padded = g.row1 - g.row0;
       D.err = dalloc_owned<int>(1, D);
       D.bytes += (int64_t)(g.n + 1) * 16 + (int64_t)g.n * 8 + D.pos * 8 + D.dis_padded * 4;
-      g.drow_host.assign(f_drow.begin() + vb, f_drow.begin() + vb + g.n + 1);
     }
     g.max_label = -1;  // the largest label is computed when it is first asked for (label_max)
   }
+  if (first) storage->tree->layout.reset();  // the plan's own reference is the last
 }
 
 // The largest finite label of g's rows, computed on first request (a pass
@@ -607,8 +517,7 @@ int64_t label_max(const Graph &gc) {
   std::lock_guard<std::mutex> lock(mu);
   Graph &g = const_cast<Graph &>(gc);
   if (g.max_label >= 0 || !g.dev.dis || !g.dev.err) return std::max<int64_t>(g.max_label, 0);
-  const int64_t r0 = g.drow_host.empty() ? 0 : g.drow_host[0];
-  const int64_t r1 = g.drow_host.empty() ? g.dev.dis_padded : g.drow_host[g.n];
+  const int64_t r0 = g.row0, r1 = g.row1;
   int dev = 0, nsm = 1;
   GH_CUDA(cudaGetDevice(&dev));
   GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -633,12 +542,14 @@ std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
   bool used[TilePolicy::kWidth][TilePolicy::kSep] = {};
   {
     const std::vector<int> lcls = plan.level_classes();
-    for (const Graph *g : plan.gs)
+    for (const Graph *g : plan.gs) {
+      host_tree(*g);
       for (int l = 0; l + 1 < (int)g->tree_hash.size(); l++)
         for (int q = g->tree_hash[l]; q < g->tree_hash[l + 1]; q++) {
           const int v = g->tree_bfs[q];
           used[lcls[l]][TilePolicy::sep_bucket((int)(g->pos_hash[v + 1] - g->pos_hash[v]) - 1)] = true;
         }
+    }
   }
   cudaEvent_t ev[2];
   GH_CUDA(cudaEventCreate(&ev[0]));
@@ -739,6 +650,7 @@ void fill_labels_gpu(Graph &g) {
     return;
   }
   g.plan.reset();
+  g.tree.reset();  // its host copies are made (allocate_labels_and_bfs)
   D.release_labels();
   D.n = n;
   D.pos_base = 0;
@@ -836,6 +748,8 @@ void fill_labels_gpu(Graph &g) {
   }
   cleanup();
   g.drow_host.swap(drow);
+  g.row0 = 0;
+  g.row1 = D.dis_padded;
 }
 
 // Copies the filled labels back into the reference's unpadded layout.
@@ -893,6 +807,8 @@ void upload_labels(Graph &g, const std::vector<int> &dis, const std::vector<int>
   }
   cudaFreeHost(stage);
   g.drow_host.swap(drow);
+  g.row0 = 0;
+  g.row1 = D.dis_padded;
 }
 
 // Runs one of the reference's GPU fill mappings (mapping 0: a thread per
@@ -906,7 +822,8 @@ void fill_labels_plain(const Graph &g, int mapping, double *ms, int64_t *mismatc
   GH_CHECK(g.labelled && g.label_mode == H2H_LABEL_L4, H2H_ERR_STATE, "needs built L4 labels");
   const DeviceIndex &D = g.dev;
   const int n = g.n;
-  const int64_t np = g.pos_hash[n];
+  host_tree(g);
+  const int64_t np = g.pos_n;
   std::vector<int> pid(np), ppos(np);
   download_positions(g, pid.data(), ppos.data());
   // (v, k) pairs per tree level, k over v's entries other than v itself
@@ -1027,7 +944,7 @@ void fill_labels_plain(const Graph &g, int mapping, double *ms, int64_t *mismatc
 // Position lists in the reference layout with graph-local ids: the host
 // copies (L3) or the graph's range of the device arrays (L4).
 void download_positions(const Graph &g, int *pos_id, int *pos_pos) {
-  const int64_t np = g.pos_hash.empty() ? 0 : g.pos_hash[g.n];
+  const int64_t np = g.pos_n;
   if ((int64_t)g.pos_id.size() == np && np) {
     if (pos_id) std::copy(g.pos_id.begin(), g.pos_id.end(), pos_id);
     if (pos_pos) std::copy(g.pos_pos.begin(), g.pos_pos.end(), pos_pos);
@@ -1043,11 +960,12 @@ void download_positions(const Graph &g, int *pos_id, int *pos_pos) {
   }
 }
 
-// The graph's rows are [drow_host[0], drow_host[n]) of the device array
+// The graph's rows are [row0, row1) of the device array
 // (a batch's forest array holds other graphs' rows around them).
 void download_labels(const Graph &g, int *dis_out) {
   const int n = g.n;
-  const int64_t r0 = g.drow_host[0], r1 = g.drow_host[n];
+  host_tree(g);
+  const int64_t r0 = g.row0, r1 = g.row1;
   GH_CHECK(r1 - r0 == g.dev.dis_padded, H2H_ERR_STATE, "label rows and device index disagree");
   std::vector<int> tmp(r1 - r0);
   GH_CUDA(cudaMemcpy(tmp.data(), g.dev.dis + r0, sizeof(int) * (r1 - r0), cudaMemcpyDeviceToHost));

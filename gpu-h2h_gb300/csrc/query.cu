@@ -320,32 +320,28 @@ void allocate_rmq(Graph &g) {
 void build_rmq_gpu(const std::vector<Graph *> &gs) {
   Clock clk;
   const int K = (int)gs.size();
-  std::vector<int64_t> off(K + 1, 0), voff(K + 1, 0);
+  const std::shared_ptr<TreeStore> tree = gs[0]->tree;
+  GH_CHECK(tree && tree->gs == gs && tree->euler, H2H_ERR_STATE, "Euler tour missing");
+  std::vector<int64_t> off(K + 1, 0);
   int levels = 0;
   for (int i = 0; i < K; i++) {
-    const Graph &g = *gs[i];
-    GH_CHECK((int64_t)g.euler_id.size() == g.euler_n && g.euler_n == 2 * (int64_t)g.n - 1, H2H_ERR_STATE,
-             "Euler tour missing");
-    off[i + 1] = off[i] + g.euler_n;
-    voff[i + 1] = voff[i] + g.n;
-    levels = std::max(levels, ilog2_floor(g.euler_n));
+    off[i + 1] = off[i] + gs[i]->euler_n;
+    levels = std::max(levels, ilog2_floor(gs[i]->euler_n));
   }
   const int64_t total = off[K];
   DeviceArena ws;
   {
-    int *d_eid = ws.get<int>(total), *d_depth = ws.get<int>(voff[K]);
     int64_t *d_off = ws.get<int64_t>(K + 1);
     RmqJob *d_jobs = ws.get<RmqJob>(K);
     std::vector<RmqJob> jobs(K);
     for (int i = 0; i < K; i++) {
       Graph &g = *gs[i];
       DeviceIndex &D = g.dev;
+      const int vb = tree->vbase[i];
       g.rmq_total = rmq_prefix(g.euler_n);
       allocate_rmq(g);
-      GH_CUDA(cudaMemcpy(D.first, g.first.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
-      GH_CUDA(cudaMemcpy(d_eid + off[i], g.euler_id.data(), sizeof(int) * g.euler_n, cudaMemcpyHostToDevice));
-      GH_CUDA(cudaMemcpy(d_depth + voff[i], g.depth.data(), sizeof(int) * g.n, cudaMemcpyHostToDevice));
-      jobs[i] = RmqJob{d_eid + off[i], d_depth + voff[i], D.rmq_hash, D.rmq_id, g.euler_n};
+      GH_CUDA(cudaMemcpyAsync(D.first, tree->first + vb, sizeof(int) * g.n, cudaMemcpyDeviceToDevice));
+      jobs[i] = RmqJob{tree->euler + off[i], tree->depth + vb, D.rmq_hash, D.rmq_id, g.euler_n};
     }
     GH_CUDA(cudaMemcpy(d_jobs, jobs.data(), sizeof(RmqJob) * K, cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemcpy(d_off, off.data(), sizeof(int64_t) * (K + 1), cudaMemcpyHostToDevice));
@@ -362,11 +358,10 @@ void build_rmq_gpu(const std::vector<Graph *> &gs) {
     GH_CUDA(cudaDeviceSynchronize());
   }
   ws.release();
+  tree->tour.reset();
+  tree->first = tree->euler = nullptr;
   const long long us = clk.us();
-  for (Graph *g : gs) {
-    std::vector<int>().swap(g->euler_id);
-    g->t.tree += us / K;
-  }
+  for (Graph *g : gs) g->t.tree += us / K;
 }
 
 void upload_rmq(Graph &g, const std::vector<int64_t> &rmq_hash, const std::vector<int> &rmq_id) {

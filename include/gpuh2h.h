@@ -191,8 +191,8 @@ typedef struct {
 } h2h_batch_info;
 
 /* Builds `count` graphs loaded by h2h_load / h2h_load_files and not yet
- * contracted.  threads: host threads for the per-graph host phases (each
- * graph's own phase runs on one thread). */
+ * contracted.  threads: kept for callers; every phase runs on the GPU over all
+ * graphs. */
 int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch **out);
 /* Replaces the arc weights of graph `index` for the next h2h_batch_rebuild:
  * w holds one weight per stored arc in h2h_copy_input_arcs order. */
