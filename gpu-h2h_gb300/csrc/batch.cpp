@@ -114,8 +114,7 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       clk.reset();
       GH_CUDA(cudaEventRecord(b->ev[0], b->stream));
       cudaEvent_t hev[2] = {b->ev[1], b->ev[2]};
-      b->elim->enqueue(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr);
-      b->elim->check_error();
+      if (!b->elim->run(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr)) continue;  // the list kernels
       b->info.t_contract_us = event_us(b->ev[0], b->ev[1]);
       b->info.t_global_us = event_us(b->ev[1], b->ev[2]);
       clk.reset();

@@ -71,6 +71,7 @@ constexpr int kErrEmpty = 2;     // eliminated a vertex without neighbours (the 
 constexpr int kErrStaging = 3;   // a list outgrew the per-level staging bound
 constexpr int kErrTimeout = 4;   // a cell barrier wait ran out (cell_grid_kernel)
 constexpr int kErrPick = 5;      // no candidate left to pick (inconsistent cell table)
+constexpr int kErrPool = 6;      // bit rows: the list pool is full
 
 struct ElimArgs {
   int *slot_nbr;
@@ -1304,7 +1305,7 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
   GH_CHECK(M < INT32_MAX, H2H_ERR_ARG, "too many arcs in one batch");
   // slot arrays: the LUB ranges, then a pool for global-order lists that
   // outgrow theirs
-  pool_size = lub + pool_extra;
+  slots_size = lub + pool_extra;
   ListLaunches LL;
   bits = allow_bits && plan_bits();
   if (!bits) {
@@ -1316,15 +1317,25 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
   const int64_t pstage_ints = LL.pstage_ints, partial_max = LL.partial_max;
   // ---- device state
   try {
-    // large slot arrays are freed as soon as the lists are compacted
-    own_slots = bits && pool_size >= (int64_t(16) << 20);
-    slot_nbr = own_slots ? dalloc<int>(pool_size + 4) : mem.get<int>(pool_size + 4);  // + 4: a list's last 128-bit load stays inside
-    slot_w = own_slots ? dalloc<int>(pool_size + 4) : mem.get<int>(pool_size + 4);
-    slot_bytes = own_slots ? 8 * (pool_size + 4) : 0;
+    if (bits) {
+      // every list of every level is written once: on road graphs some 40
+      // entries a vertex (19 of them final); the slot ranges, sized for the
+      // longest list each vertex can ever have, took 4 GB on 1M vertices, and
+      // their cudaMalloc and cudaFree 3.5 ms
+      pool_size = std::min<int64_t>(2 * (slots_size + 4), M + 64 * (int64_t)N + (1 << 16));
+      own_pool = pool_size >= (int64_t(2) << 20);
+      if (own_pool) GH_CUDA(cudaMalloc(&pool, sizeof(int) * (size_t)pool_size));
+      else pool = mem.get<int>(pool_size);
+      slot_bytes = own_pool ? 4 * pool_size : 0;
+    } else {
+      pool_size = slots_size;
+      slot_nbr = mem.get<int>(pool_size + 4);  // + 4: a list's last 128-bit load stays inside
+      slot_w = mem.get<int>(pool_size + 4);
+      slot_off_init = mem.get<int64_t>(N);
+    }
     pool_next = mem.get<unsigned long long>(1);
     pool_first = mem.get<unsigned long long>(1);
     slot_off = mem.get<int64_t>(N);
-    slot_off_init = mem.get<int64_t>(N);
     lsize = mem.get<int>((int64_t)N + 1);  // + 1: the end of a scan
     cap = mem.get<int>(N);
     cap_init = mem.get<int>(N);
@@ -1360,7 +1371,8 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
       ev_join.push_back(e);
     }
     GH_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    GH_CUDA(cudaMemcpyAsync(slot_off_init, sets->slot, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice));
+    if (!bits)
+      GH_CUDA(cudaMemcpyAsync(slot_off_init, sets->slot, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice));
     GH_CUDA(cudaMemcpyAsync(deg_init, sets->deg, sizeof(int) * N, cudaMemcpyDeviceToDevice));
     GH_CUDA(cudaMemcpyAsync(cap_init, sets->cap, sizeof(int) * N, cudaMemcpyDeviceToDevice));
     GH_CUDA(cudaMemcpyAsync(elim_init, sets->elim, sizeof(int) * N, cudaMemcpyDeviceToDevice));
@@ -1377,7 +1389,7 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
         GH_CUDA(cudaMemcpyAsync(heap_verts + hb, elim_init + vbase[i] + L[i].heap_start, sizeof(int) * L[i].heap_n,
                                 cudaMemcpyDeviceToDevice));
     }
-    const unsigned long long first_free = (unsigned long long)lub;
+    const unsigned long long first_free = (unsigned long long)(bits ? M : lub);
     GH_CUDA(cudaMemcpy(pool_first, &first_free, sizeof(first_free), cudaMemcpyHostToDevice));
   } catch (...) {
     release();
@@ -1653,15 +1665,10 @@ void ElimPlan::plan_lists(const int *f_elim, const std::vector<GraphLevels> &L, 
 ElimPlan::~ElimPlan() { release(); }
 
 void ElimPlan::release() {
-  if (own_slots) {
-    cudaFree(slot_nbr);
-    cudaFree(slot_w);
-    own_slots = false;
-    slot_bytes = 0;
-  }
+  free_pool();
   mem.release();
   members = extra = nullptr;
-  fin = sym_cells = nullptr;
+  sym_cells = nullptr;
   grows = nullptr;
   grid_map = nullptr;
   hg_partial = nullptr;
@@ -1803,15 +1810,32 @@ void ElimPlan::enqueue(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
   if (heap_ev) GH_CUDA(cudaEventRecord(heap_ev[1], s));
 }
 
-void ElimPlan::check_error() {
+bool ElimPlan::run(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
+  for (;;) {
+    enqueue(s, heap_ev, trace);
+    if (!bits || read_error() != kErrPool) {
+      check_error();
+      return true;
+    }
+    if (!grow_pool()) return false;
+  }
+}
+
+int ElimPlan::read_error() {
   GH_CUDA(cudaDeviceSynchronize());
   int e = 0;
   GH_CUDA(cudaMemcpy(&e, err, sizeof(int), cudaMemcpyDeviceToHost));
+  return e;
+}
+
+void ElimPlan::check_error() {
+  const int e = read_error();
   GH_CHECK(e == 0, H2H_ERR_DEVICE,
            e == kErrOverflow ? "contraction: a list outgrew its LUB capacity"
            : e == kErrEmpty  ? "contraction: eliminated a vertex with an empty list (disconnected input)"
            : e == kErrTimeout ? "contraction: a cell barrier wait ran out"
            : e == kErrPick    ? "contraction: no candidate left to pick"
+           : e == kErrPool    ? "contraction: the list pool is full"
                               : "contraction: a list outgrew the staging bound");
 }
 
@@ -1844,13 +1868,7 @@ void ElimPlan::build_lists() {
   GH_CUDA(cudaGetLastError());
   father_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256>>>(lists.off, lists.id, rank, tree->father, N);
   GH_CUDA(cudaGetLastError());
-  if (own_slots) {  // the lists never run again: only their weights are replayed
-    cudaFree(slot_nbr);
-    cudaFree(slot_w);
-    slot_nbr = slot_w = nullptr;
-    own_slots = false;
-    slot_bytes = 0;
-  }
+  if (bits) free_pool();  // the lists never run again: only their weights are replayed
   for (size_t i = 0; i < gs.size(); i++) {
     Graph &g = *gs[i];
     std::vector<int>().swap(g.elim);
@@ -1924,8 +1942,11 @@ void contract_gpu(Graph &g) {
     GH_CUDA(cudaEventCreate(&ev[1]));
     long long heap_us = 0;
     try {
-      plan.enqueue(0, ev, trace);
-      plan.check_error();
+      if (!plan.run(0, ev, trace)) {  // lists longer than the list kernels' slots in all
+        cudaEventDestroy(ev[0]);
+        cudaEventDestroy(ev[1]);
+        continue;
+      }
       float hms = 0;
       GH_CUDA(cudaEventElapsedTime(&hms, ev[0], ev[1]));
       heap_us = (long long)(hms * 1000.0f);

@@ -229,10 +229,14 @@ struct ElimPlan {
   bool bits = false;
   std::vector<SymLaunch> sym;
   int *members = nullptr, *extra = nullptr;
-  unsigned char *fin = nullptr, *sym_cells = nullptr;
+  unsigned char *sym_cells = nullptr;
+  // the lists on bit rows, level after level; from 8 MiB an allocation of its
+  // own, freed once they are compacted
+  int *pool = nullptr;
+  bool own_pool = false;
   unsigned *grows = nullptr;
   int N = 0, heap_total = 0;
-  int64_t M = 0, lub = 0, pool_size = 0;
+  int64_t M = 0, lub = 0, slots_size = 0, pool_size = 0;
   std::vector<Launch> launches;  // in step order; launches of one step are independent
   int nsm = 0, max_group = 1;
   bool elim_balance = true;  // cooperative steps: merges split over a cell's blocks by work
@@ -255,8 +259,7 @@ struct ElimPlan {
   void *hg_partial = nullptr;
   unsigned *grid_bar = nullptr;
   int64_t grid_bar_words = 0;
-  DeviceArena mem;          // every array but large slot arrays
-  bool own_slots = false;   // slot_nbr and slot_w are allocations of their own
+  DeviceArena mem;          // every array but the pool
   int64_t slot_bytes = 0;
   int64_t bytes() const { return mem.bytes + slot_bytes; }
   explicit ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits = true);
@@ -265,6 +268,8 @@ struct ElimPlan {
   void plan_lists(const int *f_elim, const std::vector<GraphLevels> &L, ListLaunches &LL);
   void enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace);
   void gather_bits(cudaStream_t s);
+  bool grow_pool();
+  void free_pool();
   int launch_count() const { return (int)(bits ? sym.size() : launches.size()); }
   void release();
   ElimPlan(const ElimPlan &) = delete;
@@ -274,6 +279,10 @@ struct ElimPlan {
   // heap_ev[1] after it.
   void enqueue(cudaStream_t s, cudaEvent_t *heap_ev = nullptr, bool trace = false);
   void launch_one(const Launch &Lc, cudaStream_t s, bool trace);
+  // The first enqueue, waited for; again with a larger pool where the lists
+  // outgrew it.  False: they take more than the list kernels would.
+  bool run(cudaStream_t s, cudaEvent_t *heap_ev, bool trace);
+  int read_error();    // synchronises
   void check_error();  // synchronises; throws on a kernel error code
   // After the first enqueue: compact the final lists and pick each vertex's
   // father (min elimination rank over its list), all on the device; every

@@ -55,6 +55,7 @@ namespace {
 constexpr int kErrOverflow = 1;  // a list outgrew its capacity
 constexpr int kErrEmpty = 2;     // eliminated a vertex without neighbours
 constexpr int kErrPick = 5;      // no candidate left to pick, or a vertex outside its cell
+constexpr int kErrPool = 6;      // the list pool is full
 
 constexpr int kIdxBits = 14, kDegBits = 22, kSumBits = 28;  // a key: degree + height, degree, member
 constexpr int kMaxMembers = 1 << kIdxBits;
@@ -62,21 +63,20 @@ constexpr int kMaxGroups = 64;
 constexpr unsigned long long kNoKey = ~0ull;
 
 struct SymCell {
-  int start, count, size, src;  // candidates in elim; members; slot buffer its lists are read from
+  int start, count, size;       // candidates in elim; members
   int64_t mem, out;             // members; where the ones that stay go (a run of the parent's members)
   int obase;                    // that run's start within the parent's members
 };
 
 struct SymArgs {
   const SymCell *cells;
-  int *slot[2];
-  int64_t *slot_off;
+  int *pool;          // lists, each written once and taken from the pool's end
+  int64_t *slot_off;  // where a vertex's list is
   int *lsize, *ljunk, *extra, *height, *elim, *members, *err;
   const int *cap, *deg0, *adj_off, *adj_v;
   unsigned *grows;  // rows in global memory (kGlobal)
   unsigned long long *pool_next;
   int64_t pool_size;
-  unsigned char *fin;  // the slot buffer a vertex's list ended in
   int smax, npow, heap;
 };
 
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
     __syncwarp();
     const int64_t off = A.slot_off[u];
     const int n = A.lsize[u];
-    const int *list = A.slot[c.src] + off;
+    const int *list = A.pool + off;
     // an entry is a place in the members' array, or ~id of a vertex that was
     // outside the cell below
     int out = 0;
@@ -356,24 +356,39 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
       q += __popc(bal);
     }
   }
+  // the lists' places: one run of the pool for the CTA
+  __syncthreads();
+  if (wid == 0) {
+    unsigned long long total = 0;
+    for (int r0 = 0; r0 < nown; r0 += 32) {
+      const int r = r0 + lane, l = r * CS + rank;
+      const int len = r < nown ? vc[r] + ((cand[l >> 5] >> (l & 31)) & 1u ? 0 : outc[r]) : 0;
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (r < nown) key[r] = total + (unsigned)(incl - len);
+      total += (unsigned)__shfl_sync(0xffffffffu, incl, 31);
+    }
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(A.pool_next, total);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int r = lane; r < nown; r += 32) key[r] += at;
+  }
   __syncthreads();
   for (int r = wid; r < nown; r += nw) {
     const int l = r * CS + rank, u = ids[l];
     const bool gone = (cand[l >> 5] >> (l & 31)) & 1u;
     const int out = gone ? 0 : outc[r], len = vc[r] + out;
-    int64_t off = A.slot_off[u];
-    const int64_t old = off;
-    if (A.heap && len > A.cap[u]) {  // a global-order list may outgrow its range
-      unsigned long long at = 0;
-      if (lane == 0) at = atomicAdd(A.pool_next, (unsigned long long)len);
-      off = (int64_t)__shfl_sync(0xffffffffu, at, 0);
-    }
-    const bool fits = A.heap ? off + len <= A.pool_size : len <= cap[r];
+    const int64_t old = A.slot_off[u], off = (int64_t)key[r];
+    const bool room = off + len <= A.pool_size, fits = room && len <= cap[r];
     if (fits) {
-      int *dst = A.slot[c.src ^ 1] + off;
+      int *dst = A.pool + off;
       int q = 0;
       if (out > 0) {
-        const int *list = A.slot[c.src] + old;
+        const int *list = A.pool + old;
         const int n0 = A.lsize[u];
         for (int e0 = 0; e0 < n0 && q < out; e0 += 32) {
           const int y = e0 + lane < n0 ? __ldcg(list + e0 + lane) : 0;
@@ -392,13 +407,12 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
       }
     }
     if (lane == 0) {
-      if (!fits) atomicCAS(A.err, 0, kErrOverflow);
+      if (!fits) atomicCAS(A.err, 0, room ? kErrOverflow : kErrPool);
       A.slot_off[u] = off;
       A.lsize[u] = fits ? len : 0;
       A.ljunk[u] = gone ? 0 : junk[r];
       A.extra[u] = ext[r];
       A.height[u] = hgt[r];
-      A.fin[u] = (unsigned char)(c.src ^ 1);
     }
   }
   if (CS > 1) cluster.sync();  // no CTA leaves while a peer may still read its rows
@@ -406,11 +420,12 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
 
 // Distinct neighbours of every vertex's input list as ~id and the number of
 // repeated entries.
-__global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, const int64_t *slot_off, int *slot,
-                                      int *lsize, int *extra, int n) {
+__global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, int64_t *slot_off, int *pool, int *lsize,
+                                      int *extra, int n) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    int *list = slot + slot_off[v];
     const int b = adj_off[v], e = adj_off[v + 1];
+    int *list = pool + b;  // the pool starts with the input lists' places
+    slot_off[v] = b;
     int c = 0;
     for (int i = b; i < e; i++) {
       const int x = ~adj_v[i];
@@ -423,13 +438,13 @@ __global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, cons
   }
 }
 
-// The final lists from whichever slot buffer each ended in.  One warp per vertex.
-__global__ void gather_ids_kernel(const int64_t *slot_off, const int *lsize, const unsigned char *fin, const int *slot0,
-                                  const int *slot1, const int64_t *out_off, int *out_nbr, int n) {
+// The final lists one after another.  One warp per vertex.
+__global__ void gather_ids_kernel(const int64_t *slot_off, const int *lsize, const int *pool, const int64_t *out_off,
+                                  int *out_nbr, int n) {
   const int lane = threadIdx.x & 31;
   for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
        v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
-    const int *src = (fin[v] ? slot1 : slot0) + slot_off[v];
+    const int *src = pool + slot_off[v];
     const int64_t oo = out_off[v];
     const int s = lsize[v];
     for (int i = lane; i < s; i += 32) out_nbr[oo + i] = src[i];
@@ -523,14 +538,14 @@ bool ElimPlan::plan_bits() {
           heap_at += stay;
         }
         const int st = g.H - h;
-        steps[st].push_back({{vb + g.cell_start[c], g.cell_count[c], sizes[i][c], st & 1, region[c], out,
+        steps[st].push_back({{vb + g.cell_start[c], g.cell_count[c], sizes[i][c], region[c], out,
                               (int)(out - parent)},
                              K > 1 ? -(st + 1) : h});
       }
     }
     if (levels > 0 && heap_at != heap_region + heap_n) return false;
     int heap_start = g.n - heap_n;
-    steps[nsteps].push_back({{vb + heap_start, heap_n, heap_n, levels & 1, heap_region, -1, 0}, 0});
+    steps[nsteps].push_back({{vb + heap_start, heap_n, heap_n, heap_region, -1, 0}, 0});
   }
   // ---- launches: a step's cells by size class, each class with its own
   // cluster size.  A pick costs a fixed part (argmin and barriers: 1.1 us in
@@ -638,7 +653,6 @@ bool ElimPlan::plan_bits() {
   try {
     members = mem.get<int>(mem_total);
     extra = mem.get<int>(N);
-    fin = mem.get<unsigned char>(N);
     sym_cells = mem.get<unsigned char>(sizeof(SymCell) * table.size());
     if (grow_words) grows = mem.get<unsigned>(grow_words);
     for (int i = 0; i < K; i++) {
@@ -656,20 +670,18 @@ bool ElimPlan::plan_bits() {
 }
 
 void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
-  GH_CUDA(cudaMemcpyAsync(slot_off, slot_off_init, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice, s));
   GH_CUDA(cudaMemcpyAsync(elim, elim_init, sizeof(int) * N, cudaMemcpyDeviceToDevice, s));
   GH_CUDA(cudaMemcpyAsync(pool_next, pool_first, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
   GH_CUDA(cudaMemsetAsync(height, 0, sizeof(int) * N, s));
   GH_CUDA(cudaMemsetAsync(ljunk, 0, sizeof(int) * N, s));
   GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-  distinct_lists_kernel<<<std::max(1, std::min(4096, (N + 255) / 256)), 256, 0, s>>>(adj_off, adj_v, slot_off, slot_nbr,
+  distinct_lists_kernel<<<std::max(1, std::min(4096, (N + 255) / 256)), 256, 0, s>>>(adj_off, adj_v, slot_off, pool,
                                                                                      lsize, extra, N);
   GH_CUDA(cudaGetLastError());
   auto launch = [&](const SymLaunch &L, cudaStream_t ls) {
     SymArgs A{};
     A.cells = reinterpret_cast<const SymCell *>(sym_cells) + L.lo;
-    A.slot[0] = slot_nbr;
-    A.slot[1] = slot_w;
+    A.pool = pool;
     A.slot_off = slot_off;
     A.lsize = lsize;
     A.ljunk = ljunk;
@@ -685,7 +697,6 @@ void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
     A.grows = L.global ? grows + L.rows_off : nullptr;
     A.pool_next = pool_next;
     A.pool_size = pool_size;
-    A.fin = fin;
     A.smax = L.smax;
     A.npow = L.npow;
     A.heap = L.heap;
@@ -740,9 +751,31 @@ void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
   }
 }
 
+// A larger pool for another run, unless the list kernels' slot arrays would
+// take no more.
+bool ElimPlan::grow_pool() {
+  const int64_t most = 2 * (slots_size + 4);
+  if (pool_size >= most) return false;
+  free_pool();
+  pool_size = std::min(most, 4 * pool_size);
+  if (std::getenv("GPUH2H_TRACE"))
+    std::fprintf(stderr, "[gpuh2h] elim bits: list pool grown to %lld entries\n", (long long)pool_size);
+  GH_CUDA(cudaMalloc(&pool, sizeof(int) * (size_t)pool_size));
+  own_pool = true;
+  slot_bytes = 4 * pool_size;
+  return true;
+}
+
+void ElimPlan::free_pool() {
+  if (own_pool) cudaFree(pool);
+  pool = nullptr;
+  own_pool = false;
+  slot_bytes = 0;
+}
+
 void ElimPlan::gather_bits(cudaStream_t s) {
   gather_ids_kernel<<<std::max(1, std::min(8192, (N * 32 + 255) / 256)), 256, 0, s>>>(
-      slot_off, lsize, fin, slot_nbr, slot_w, lists.off, lists.id, N);
+      slot_off, lsize, pool, lists.off, lists.id, N);
   GH_CUDA(cudaGetLastError());
 }
 
