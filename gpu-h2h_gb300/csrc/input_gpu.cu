@@ -20,6 +20,8 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstdio>
+#include <cstdlib>
 
 #include "graph.h"
 #include "sort.h"
@@ -289,11 +291,20 @@ bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, 
   RelaxedCapture relaxed;
   Workspace ws;
   QuietStream q;
+  const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
+  Clock tclk;
+  auto mark = [&](const char *what) {
+    if (!trace) return;
+    cudaStreamSynchronize(q.s);
+    std::fprintf(stderr, "[gpuh2h] load: %s %.3f ms\n", what, tclk.us() / 1e3);
+    tclk.reset();
+  };
   char *id_text, *text;
   int64_t *id_first, *first;
   if (number_lines(ids, ids_size, ws, q, &id_text, &id_first) != n ||
       number_lines(arcs, arcs_size, ws, q, &text, &first) != m)
     return false;
+  mark("text copied, lines numbered");
   auto in = std::make_shared<DeviceInput>();
   in->off = in->mem.get<int>((int64_t)n + 1);
   in->v = in->mem.get<int>(m);
@@ -314,6 +325,7 @@ bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, 
   GH_CUDA(cudaGetLastError());
   LoadFlags f{};
   q.read(&f, flags, sizeof(f));
+  mark("lines parsed");
   if (f.odd) return false;
   if (f.unsorted) {  // the arcs of a vertex in file order: a stable sort by tail
     int *from = ws.get<int>(m), *v2 = in->mem.get<int>(m), *w2 = in->mem.get<int>(m);
@@ -337,6 +349,7 @@ bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, 
   check_connected_kernel<<<blocks_for(n), 256, 0, q.s>>>(parent, n, flags);
   GH_CUDA(cudaGetLastError());
   q.read(&f, flags, sizeof(f));
+  mark("checks");
   if (f.missing || f.split) return false;
   g.m = m;
   g.input = in;

@@ -24,8 +24,9 @@ namespace gh {
 
 namespace {
 
-// A whole file in memory, read by several threads at once (pread of 16 MB
-// pieces into an uninitialised buffer).
+// A whole file in memory, read by several threads at once (pread of 2 MB
+// pieces into an uninitialised buffer: its pages are made as it is written, so
+// two files of 30 MB take 3.2 ms in 16 MB pieces, 2.6 in 2 MB ones).
 struct FileBytes {
   std::unique_ptr<char[]> data;
   size_t size = 0;
@@ -42,7 +43,7 @@ FileBytes read_file(const std::string &path, int threads) {
   FileBytes f;
   f.size = st.st_size > 0 ? (size_t)st.st_size : 0;
   f.data.reset(new char[f.size + 1]);
-  const size_t piece = size_t(16) << 20;
+  const size_t piece = size_t(2) << 20;
   const int64_t np = (int64_t)((f.size + piece - 1) / piece);
   std::atomic<bool> ok{true};
   auto read_pieces = [&](int64_t lo, int64_t hi, int) {
@@ -370,6 +371,7 @@ void load_graph(Graph &g, const std::string &edge, const std::string &idf, const
       arcs = read_file(edge, g.threads);
       Cursor ce(arcs, edge);
       const long long n2 = ce.integer(), m = ce.integer();
+      if (std::getenv("GPUH2H_TRACE")) std::fprintf(stderr, "[gpuh2h] load: files read %.3f ms\n", clk.us() / 1e3);
       on_gpu = n2 == n && load_input_gpu(g, ci.p, ci.e - ci.p, ce.p, ce.e - ce.p, m);
       if (on_gpu && std::getenv("GPUH2H_TRACE"))
         std::fprintf(stderr, "[gpuh2h] load: files parsed on the device: %.3f ms\n", clk.us() / 1e3);

@@ -255,36 +255,110 @@ __global__ void max_label_kernel(const int *dis, int64_t n, int *out) {
 // Position lists (mallocH2HLabel_noHub, H2HConsturction.cu:656-700): X(v)
 // and v itself ordered by position (depth - 1 of the member).  Positions of
 // one list are distinct, so an entry's slot is the number of smaller
-// positions in the list.  One block per vertex, the list's positions staged
-// in shared memory.  A member that is not a proper ancestor (position >=
-// d - 1) sets *err = 5.
-__global__ void build_positions_kernel(const int64_t *list_off, const int *list_id, const int *list_w,
-                                       const int *depth, const int64_t *pos_hash, int *pos_pos, int *pos_id,
-                                       int *pos_w, int *pos_src, int *err, int n) {
-  extern __shared__ int keys[];
-  const int tid = threadIdx.x, T = blockDim.x;
-  for (int v = blockIdx.x; v < n; v += gridDim.x) {
-    const int64_t b = list_off[v];
-    const int m = (int)(list_off[v + 1] - b);
-    const int d = depth[v];
-    const int64_t pb = pos_hash[v];
-    for (int i = tid; i <= m; i += T) {
-      int key = d - 1;
-      if (i < m) {
-        key = depth[list_id[b + i]] - 1;
-        if (key < 0 || key >= d - 1) atomicCAS(err, 0, 5);
-      }
-      keys[i] = key;
+// positions in the list.  A member that is not a proper ancestor (position >=
+// d - 1) sets *err = 5.  list_w: nullptr where the weights come later.
+//
+// Lists that fit a warp's lanes (nine in ten of a road graph's) take a warp
+// each, positions compared through shuffles; the others go to a second kernel,
+// a block per list that ranks positions in a bit map of the depth (comparing
+// every pair costs m * m, and the global order's lists are thousands long).  Bound: the
+// loads of the members' depths; 20M entries of 1M lists take 0.5 ms (1.2 with a
+// block per list and every pair compared).
+struct PosArgs {
+  const int64_t *list_off;
+  const int *list_id, *list_w, *depth;
+  const int64_t *pos_hash;
+  int *pos_pos, *pos_id, *pos_w, *pos_src;
+  int *large, *count;  // vertices with longer lists
+  int *err;
+};
+
+__device__ __forceinline__ int member_position(const PosArgs &A, int u, int d) {
+  const int key = A.depth[u] - 1;
+  if (key < 0 || key >= d - 1) atomicCAS(A.err, 0, 5);
+  return key;
+}
+
+__device__ __forceinline__ void put_position(const PosArgs &A, int64_t at, int key, int id, int w, int src) {
+  A.pos_pos[at] = key;
+  A.pos_id[at] = id;
+  if (A.list_w) A.pos_w[at] = w;
+  A.pos_src[at] = src;
+}
+
+__global__ void short_positions_kernel(PosArgs A, int n) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n;
+       v += (gridDim.x * (int64_t)blockDim.x) >> 5) {
+    const int64_t b = A.list_off[v];
+    const int m = (int)(A.list_off[v + 1] - b), d = A.depth[v];
+    if (m > 31) {
+      if (lane == 0) A.large[atomicAdd(A.count, 1)] = (int)v;
+      continue;
     }
-    __syncthreads();
-    for (int i = tid; i <= m; i += T) {
-      const int key = keys[i];
-      int r = 0;
-      for (int j = 0; j <= m; j++) r += keys[j] < key;
-      pos_pos[pb + r] = key;
-      pos_id[pb + r] = i < m ? list_id[b + i] : v;
-      pos_w[pb + r] = i < m ? list_w[b + i] : 0;
-      pos_src[pb + r] = i < m ? i : -1;
+    const int id = lane < m ? A.list_id[b + lane] : (int)v;
+    const int key = lane < m ? member_position(A, id, d) : d - 1;
+    int r = 0;
+    for (int j = 0; j <= m; j++) r += __shfl_sync(0xffffffffu, key, j) < key;
+    if (lane <= m)
+      put_position(A, A.pos_hash[v] + r, key, id, A.list_w && lane < m ? A.list_w[b + lane] : 0, lane < m ? lane : -1);
+  }
+}
+
+__global__ void long_positions_kernel(PosArgs A, int room) {
+  extern __shared__ int words[];
+  __shared__ int s_total;
+  const int tid = threadIdx.x, T = blockDim.x;
+  for (int q = blockIdx.x; q < *A.count; q += gridDim.x) {
+    const int v = A.large[q];
+    const int64_t b = A.list_off[v], pb = A.pos_hash[v];
+    const int m = (int)(A.list_off[v + 1] - b), d = A.depth[v];
+    const int W = (d + 31) >> 5;
+    if (2 * W <= room) {  // a bit per position, then the bits before each word
+      unsigned *bits = reinterpret_cast<unsigned *>(words);
+      int *before = words + W;
+      for (int w = tid; w < W; w += T) bits[w] = 0;
+      __syncthreads();
+      for (int i = tid; i <= m; i += T) {
+        const int key = i < m ? member_position(A, A.list_id[b + i], d) : d - 1;
+        if (key >= 0 && key < d) atomicOr(bits + (key >> 5), 1u << (key & 31));
+      }
+      __syncthreads();
+      if (tid < 32) {
+        int run = 0;
+        for (int w0 = 0; w0 < W; w0 += 32) {
+          const int c = w0 + tid < W ? __popc(bits[w0 + tid]) : 0;
+          int incl = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (tid >= o) incl += y;
+          }
+          if (w0 + tid < W) before[w0 + tid] = run + incl - c;
+          run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (tid == 0) s_total = run;
+      }
+      __syncthreads();
+      for (int i = tid; i <= m; i += T) {
+        const int id = i < m ? A.list_id[b + i] : v, key = A.depth[id] - 1;
+        if (s_total != m + 1 || key < 0 || key >= d) {  // a position out of range, or twice
+          atomicCAS(A.err, 0, 5);
+          continue;
+        }
+        put_position(A, pb + before[key >> 5] + __popc(bits[key >> 5] & ((1u << (key & 31)) - 1u)), key, id,
+                     A.list_w && i < m ? A.list_w[b + i] : 0, i < m ? i : -1);
+      }
+    } else {  // deep for its length: the number of smaller positions in the list
+      for (int i = tid; i <= m; i += T) words[i] = i < m ? member_position(A, A.list_id[b + i], d) : d - 1;
+      __syncthreads();
+      for (int i = tid; i <= m; i += T) {
+        const int key = words[i];
+        int r = 0;
+        for (int j = 0; j <= m; j++) r += words[j] < key;
+        put_position(A, pb + r, key, i < m ? A.list_id[b + i] : v, A.list_w && i < m ? A.list_w[b + i] : 0,
+                     i < m ? i : -1);
+      }
     }
     __syncthreads();
   }
@@ -383,12 +457,17 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
     GH_CUDA(cudaGetLastError());
     mark("allocations");
     {
-      const size_t ksmem = (size_t)(max_m + 1) * sizeof(int);
-      const int kdyn = enable_max_dynamic_smem(build_positions_kernel);
+      const int room = std::max(max_m + 1, 1024);  // ints of staging: a list, or the bits of 16,384 positions
+      const size_t ksmem = (size_t)room * sizeof(int);
+      const int kdyn = enable_max_dynamic_smem(long_positions_kernel);
       GH_CHECK(ksmem <= (size_t)kdyn, H2H_ERR_DEVICE, "separator too large for the position-list staging");
+      DeviceArena ws;
+      PosArgs A{lists.off, lists.id, from && from->bits ? nullptr : lists.w, depth, pos_hash, pos_pos, pos_id, pos_w,
+                pos_src, ws.get<int>(N), ws.get<int>(1), err};
       GH_CUDA(cudaMemset(err, 0, sizeof(int)));
-      build_positions_kernel<<<std::max(1, std::min(N, nsm * 16)), 128, ksmem>>>(
-          lists.off, lists.id, lists.w, depth, pos_hash, pos_pos, pos_id, pos_w, pos_src, err, N);
+      GH_CUDA(cudaMemset(A.count, 0, sizeof(int)));
+      short_positions_kernel<<<std::max(1, std::min(nsm * 8, (N + 7) / 8)), 256>>>(A, N);
+      if (max_m > 31) long_positions_kernel<<<std::max(1, std::min(N, nsm * 16)), 128, ksmem>>>(A, room);
       GH_CUDA(cudaGetLastError());
       int e = 0;
       GH_CUDA(cudaMemcpy(&e, err, sizeof(int), cudaMemcpyDeviceToHost));
