@@ -1318,11 +1318,12 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
   // ---- device state
   try {
     if (bits) {
-      // every list of every level is written once: on road graphs some 40
-      // entries a vertex (19 of them final); the slot ranges, sized for the
-      // longest list each vertex can ever have, took 4 GB on 1M vertices, and
-      // their cudaMalloc and cudaFree 3.5 ms
-      pool_size = std::min<int64_t>(2 * (slots_size + 4), M + 64 * (int64_t)N + (1 << 16));
+      // Every list of every level is written once: some 20 entries a vertex of
+      // final lists and 5 per level of those handed up, 70 in all on a 1M-vertex
+      // road graph.  The room is 2.5 times that, since a run that outgrows it is
+      // repeated.  (Slot ranges sized for the longest list each vertex can ever
+      // have took 4 GB there, and their cudaMalloc and cudaFree 3.5 ms.)
+      pool_size = std::min<int64_t>(2 * (slots_size + 4), M + 192 * (int64_t)N + (1 << 16));
       own_pool = pool_size >= (int64_t(2) << 20);
       if (own_pool) GH_CUDA(cudaMalloc(&pool, sizeof(int) * (size_t)pool_size));
       else pool = mem.get<int>(pool_size);
@@ -1813,7 +1814,13 @@ void ElimPlan::enqueue(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
 bool ElimPlan::run(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
   for (;;) {
     enqueue(s, heap_ev, trace);
-    if (!bits || read_error() != kErrPool) {
+    const int e = read_error();
+    if (bits && trace) {
+      unsigned long long used = 0;
+      GH_CUDA(cudaMemcpy(&used, pool_next, sizeof(used), cudaMemcpyDeviceToHost));
+      std::fprintf(stderr, "[gpuh2h] elim bits: %llu of %lld entries of the list pool\n", used, (long long)pool_size);
+    }
+    if (!bits || e != kErrPool) {
       check_error();
       return true;
     }

@@ -1,5 +1,5 @@
 """Lists that outgrow the pool of the elimination on bit rows: a random graph
-of degree 6 fills in to about half of a clique, several times the 64 entries a
+of degree 6 fills in to about half of a clique, more than the 192 entries a
 vertex the pool starts with.  The run is repeated with a larger pool; order
 and lists equal the list kernels' (zero tolerance)."""
 import random
@@ -26,7 +26,7 @@ def _random(n, degree, seed):
 @pytest.mark.parametrize("batch", (False, True))
 def test_pool_grows(tmp_path, monkeypatch, capfd, H, batch):
     import gpuh2h
-    n, edges = _random(2000, 6, 7)
+    n, edges = _random(3200, 6, 7)
     (tmp_path / "a").mkdir()
     (tmp_path / "b").mkdir()
     files = [write(tmp_path / "a", n, edges, H)]
