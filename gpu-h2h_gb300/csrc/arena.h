@@ -21,15 +21,23 @@ class DeviceArena {
   DeviceArena &operator=(const DeviceArena &) = delete;
   ~DeviceArena() { release(); }
 
-  // n elements, aligned to 256 bytes, uninitialised.  Arrays of 8 MiB and more
-  // are allocations of their own; smaller ones share chunks that double up to
-  // 64 MiB.
+  // Room for arrays of `total` bytes in all (each rounded up to 256) in one
+  // allocation, for a phase that knows what it will take.
+  void reserve(size_t total) {
+    cur_ = chunk(total);
+    cap_ = total;
+    used_ = 0;
+  }
+
+  // n elements, aligned to 256 bytes, uninitialised.  What the current chunk
+  // has no room for and takes 8 MiB or more is an allocation of its own; smaller
+  // arrays share chunks that double up to 64 MiB.
   template <typename T>
   T *get(int64_t n) {
     const size_t want = ((size_t)std::max<int64_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
     bytes += (int64_t)((size_t)std::max<int64_t>(n, 1) * sizeof(T));
-    if (want >= (size_t(8) << 20)) return reinterpret_cast<T *>(chunk(want));
     if (want > cap_ - used_) {
+      if (want >= (size_t(8) << 20)) return reinterpret_cast<T *>(chunk(want));
       next_ = std::min<size_t>(std::max<size_t>(2 * next_, size_t(1) << 20), size_t(64) << 20);
       const size_t size = std::max(want, next_);
       cur_ = chunk(size);

@@ -112,7 +112,7 @@ struct DeviceIndex {
   int id_base = 0;
   int64_t bytes = 0, rmq_bytes = 0;
   std::vector<void *> owned;      // label-side allocations of this handle
-  std::unique_ptr<DeviceArena> owned_rmq;  // first, rmq_hash, rmq_id (built with the tree)
+  std::shared_ptr<DeviceArena> owned_rmq;  // first, rmq_hash, rmq_id (built with the trees)
   std::shared_ptr<void> keep;
   void release();
   void release_labels();  // everything but the sparse table
