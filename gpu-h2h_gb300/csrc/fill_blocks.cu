@@ -17,20 +17,24 @@
 //   S(i, u) = min(sc(i, u), min over w in X(i) inside the block of sc(i, w) + S(w, u)).
 // S needs no label (closure_kernel computes it for all blocks at once), and
 // the columns above the block become one min-plus product [32 x |X(t)|] by
-// [|X(t)| x depth(t)] whose second factor is loaded once for 32 rows.  The
-// columns inside the block follow from a second, 32 x 32 product with the
-// direct weights and a short sequential pass.  Sums are those of the
-// recursion, regrouped; they are taken in unsigned 32-bit arithmetic, where
-// two values below 2^31 cannot wrap, with INT_MAX for "no entry".
+// [|X(t)| x depth(t)] whose second factor is loaded once for 32 rows.  For two
+// nodes i below a of one block the way either stays inside the block or passes
+// a last u in X(t),
+//   D(i, a) = min(W(i, a), min over u in X(t) of S(i, u) + D(a, u)),
+// where W, the recursion over the block's nodes alone, needs no label either
+// (inner_closure_kernel) and column u of row a has just been computed.  D is
+// the distance in the graph whose arc {v, u} weighs what the endpoint eliminated
+// first says, so both forms of a sum agree.  Sums are taken in unsigned 32-bit
+// arithmetic, where two values below 2^31 cannot wrap, with INT_MAX for "no
+// entry".
 //
 // A fill that takes a warp per (node, column block, separator chunk) tile is
 // bound by one L2 load per update and 13 us per tree level of the narrow top.
 // On one GB300 the blocks took the fill of a 264k-vertex road graph (4.5e9
-// updates) from 28.4 to 3.7 ms and of a 1M-vertex one (3.8e10) from 104 to
-// 14.9 ms.  Narrow levels are a chain of blocks (about 30 us each); below
-// them the kernel issues a min-plus term per lane in over half of the ALU
-// slots (9e9 terms on the 264k-vertex graph, a warp instruction per two
-// cycles and scheduler).
+// updates) from 28.4 to 2.65 ms and of a 1M-vertex one (3.8e10) from 104 to 12.9
+// ms.  Narrow levels are a chain of blocks (about 30 us each, a step of 32
+// members 4,000 clocks); below them a term costs an ALU slot of half rate and the
+// kernel fills half of those slots.
 #include <algorithm>
 #include <climits>
 #include <cstdio>
@@ -64,6 +68,15 @@ T *dalloc(size_t n, int64_t &bytes) {
   return p;
 }
 
+__device__ __forceinline__ void cp_async16(void *smem, const void *global) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *global) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ int ld_acquire(const int *p) {
   int v;
   asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -302,8 +315,9 @@ struct BlockArgs {
   const int64_t *drow, *pos_hash;
   const int *pos_pos, *pos_id, *pos_w;
   // per block [column][row], rows padded to a multiple of four: the columns
-  // are the top's members, then (direct only) the block's own nodes
+  // are the top's members, then the block's own nodes (closed: W)
   unsigned *direct, *closed;
+  unsigned *anc;  // per node in the blocks' order: its ancestors inside the block, a bit per place
   int nblk;
   int *err;
 };
@@ -323,10 +337,9 @@ __device__ __forceinline__ int stage_inner(const BlockArgs &A, int v, int dt, un
 
 constexpr int kClosureWarps = 4;
 
-// S and the direct weights of every block, 32 members at a time: a warp
-// scatters its block's list entries into a 32 x 32 tile (row i, member), writes
-// it out as the direct weights, then lane k carries member k's column through
-// the block's nodes in depth-first order.  Columns are independent, so the
+// S of every block from the lists, 32 members at a time: a warp scatters its
+// block's list entries into a 32 x 32 tile (row i, member), then lane k carries
+// member k's column through the block's nodes in depth-first order.  Columns are independent, so the
 // chunks of a wide separator run in different warps (blockIdx.y).  Bound:
 // latency of the scattered list reads; 0.1 ms beside the product's 2 ms on
 // the 264k-vertex graph.
@@ -389,9 +402,6 @@ __global__ void __launch_bounds__(32 * kClosureWarps) closure_kernel(BlockArgs A
     }
     __syncwarp();
     const int64_t out = A.soff[b] + (int64_t)k0 * Rp;
-    for (int k = 0; k < kn; k++)
-      if (lane < Rp) A.direct[out + k * Rp + lane] = lane < R ? row[lane * 33 + k] : kInf;
-    __syncwarp();
     for (int i = 1; i < R; i++) {
       unsigned r = row[i * 33 + lane];
       const int c = __shfl_sync(0xffffffffu, tc, i);
@@ -403,6 +413,73 @@ __global__ void __launch_bounds__(32 * kClosureWarps) closure_kernel(BlockArgs A
       if (lane < Rp) A.closed[out + k * Rp + lane] = lane < R ? row[lane * 33 + k] : kInf;
     __syncwarp();
   }
+}
+
+// W of every block and the nodes' ancestors inside it: a warp takes the block's
+// nodes in depth-first order, lane a holding the entry for the node at place a.
+// The matrix stays symmetric over finished pairs, so W between an inner
+// neighbour w and a is one read whichever lies deeper.  Bound: a chain of up to
+// 31 rows, 0.4 us each; it used to end every block of the fill (14 us of the 45 a
+// narrow level took), here all blocks run side by side (0.39 ms on the
+// 1M-vertex graph).
+__global__ void __launch_bounds__(32 * kClosureWarps) inner_closure_kernel(BlockArgs A) {
+  __shared__ unsigned s_M[kClosureWarps][kRows * 33];
+  __shared__ int s_tw[kClosureWarps][kRows * 32];
+  __shared__ unsigned char s_tl[kClosureWarps][kRows * 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int b = blockIdx.x * kClosureWarps + wid;
+  if (b >= A.nblk) return;
+  unsigned *M = s_M[wid];
+  int *tw = s_tw[wid];
+  unsigned char *tl = s_tl[wid];
+  const int64_t o = A.boff[b];
+  const int R = (int)(A.boff[b + 1] - o), Rp = (R + 3) & ~3;
+  const int m = (int)(A.moff[b + 1] - A.moff[b]);
+  const int dt = A.depth[A.blk_top[b]] - 1;
+  int tc = 0, par = 0;  // lane i: inner members of node i, its father's place
+  int64_t pb = 0, pe = 0;
+  if (lane < R) {
+    const int v = A.bnode[o + lane];
+    pb = A.pos_hash[v];
+    pe = A.pos_hash[v + 1] - 2;
+    if (lane > 0) par = A.loc_of[A.father[v]];
+  }
+#pragma unroll 4
+  for (int i = 0; i < R; i++) {  // stage_inner for every node, several in flight
+    const int64_t e = __shfl_sync(0xffffffffu, pe, i) - lane;
+    const bool in = e >= __shfl_sync(0xffffffffu, pb, i) && __ldg(A.pos_pos + e) >= dt;
+    if (in) {
+      tl[32 * i + lane] = A.loc_of[__ldg(A.pos_id + e)];
+      tw[32 * i + lane] = __ldg(A.pos_w + e);
+    }
+    const int c = __popc(__ballot_sync(0xffffffffu, in));
+    if (lane == i) tc = c;
+  }
+  for (int i = 0; i < kRows; i++) M[i * 33 + lane] = kInf;
+  __syncwarp();
+  unsigned anc = 0;
+  for (int i = 1; i < R; i++) {
+    const int pi = __shfl_sync(0xffffffffu, par, i);
+    const unsigned ai = __shfl_sync(0xffffffffu, anc, pi) | (1u << pi);
+    if (lane == i) anc = ai;
+    unsigned r = kInf;
+    const int c = __shfl_sync(0xffffffffu, tc, i);
+#pragma unroll 4
+    for (int x = 0; x < c; x++) {
+      const int w = tl[32 * i + x];
+      r = add_min((unsigned)tw[32 * i + x], w == lane ? 0u : M[w * 33 + lane], r);
+    }
+    __syncwarp();
+    if ((ai >> lane) & 1u) {
+      M[i * 33 + lane] = r;
+      M[lane * 33 + i] = r;
+    }
+    __syncwarp();
+  }
+  if (lane < R) A.anc[o + lane] = anc;
+  unsigned *out = A.closed + A.soff[b] + (int64_t)m * Rp;
+  for (int c = 0; c < R; c++)
+    if (lane < Rp) out[c * Rp + lane] = M[lane * 33 + c];  // rows past R: no entry
 }
 
 // ------------------------------------------------------------ the weights
@@ -796,8 +873,9 @@ struct FillKernelArgs {
 // columns 64 at a time and the top's members 32 at a time: the second factor
 // E goes through registers into shared memory one step ahead (so a step's
 // loads overlap the product before it), every thread owns a 4 x 4 patch of
-// the 32 x 64 result.  The last task of a block to finish fills in the
-// columns inside the block and publishes it.  Rows produced in the launch are
+// the 32 x 64 result.  A completed tile adds its columns' part of the matrix
+// inside the block, whose weights came to shared memory with the tile; the last
+// task of a block to finish writes that matrix and publishes the block.  Rows produced in the launch are
 // read through L2 (ld.global.cg).  A quad of four columns that lies above a
 // member (p_u >= J + 4) is one 128-bit load of u's row; below it, four
 // ancestors' entries at p_u, eight members of consecutive positions per warp
@@ -815,10 +893,9 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
   __shared__ int s_mp[2][kMembers];
   __shared__ int64_t s_rowoff[kRows];
   __shared__ int s_kb[kMaxTiles + 1];  // first member at or after each tile's first column
-  __shared__ unsigned s_M[kRows * 33];
-  __shared__ int s_tw[kRows * 32];
-  __shared__ unsigned char s_tl[kRows * 32];
-  __shared__ int s_tc[kRows], s_dcol[kRows], s_par[kRows];
+  __shared__ __align__(16) unsigned s_D[kCols * kRows];  // a tile's members: S and positions
+  __shared__ int s_pd[kCols];
+  __shared__ int s_dcol[kRows];
   __shared__ unsigned s_anc[kRows];
   __shared__ int s_t, s_flag;
   const BlockArgs &B = A.B;
@@ -848,17 +925,13 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
       s_top[i] = __ldg(A.seg_top + sb + i);
       s_pos[i] = __ldg(A.seg_pos + sb + i);
     }
-    if (tid < R) s_rowoff[tid] = __ldg(B.drow + __ldg(B.bnode + bo + tid));
-    const int my = tid >> 3, mx = tid & 7;  // this thread's 2 x 4 patch of the in-block matrix
-    for (int i = wid; i < R; i += 4) {
-      const int v = __ldg(B.bnode + bo + i);
-      const int c = stage_inner(B, v, dt, s_tl + 32 * i, s_tw + 32 * i, lane);
-      if (lane == 0) {
-        s_tc[i] = c;
-        s_dcol[i] = __ldg(B.depth + v) - 1;
-        s_par[i] = i > 0 ? B.loc_of[__ldg(B.father + v)] : 0;
-      }
+    if (tid < R) {
+      const int v = __ldg(B.bnode + bo + tid);
+      s_rowoff[tid] = __ldg(B.drow + v);
+      s_dcol[tid] = __ldg(B.depth + v) - 1;
+      s_anc[tid] = B.anc[bo + tid];
     }
+    const int my = tid >> 3, mx = tid & 7;  // this thread's 2 x 4 patch of the in-block matrix
     if (tid <= (c1 - c0 + kCols - 1) / kCols) {
       const int j = min(c0 + kCols * tid, c1);
       int lo = 0, hi = m;
@@ -924,8 +997,27 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
         eb[g] = e;
       }
     };
+    // the members whose positions lie inside a tile: their rows of S go to
+    // shared memory beside the tile's product (one chunk: they are in s_S)
+    auto issue_d = [&](int T) {
+      const int kb = s_kb[T], nd = s_kb[T + 1] - kb;
+      const unsigned *src = B.closed + so + (int64_t)kb * Rp;
+      for (int i = tid; i < nd * (Rp >> 2); i += 128) cp_async16(s_D + 4 * i, src + 4 * i);
+      if (tid < nd) cp_async4(s_pd + tid, B.bm_p + m0 + kb + tid);
+    };
+    unsigned mm[2][4];  // in-block matrix: W, then the part over members above the block
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int a = 4 * mx + c;
+      const uint2 w = t == task0 && a < R && 2 * my < Rp
+                          ? *reinterpret_cast<const uint2 *>(B.closed + so + (int64_t)(m + a) * Rp + 2 * my)
+                          : make_uint2(kInf, kInf);
+      mm[0][c] = w.x;
+      mm[1][c] = w.y;
+    }
     if (nsteps > 0) {
       issue_s(B.closed, 0);
+      if (nchunk > 1 && R > 1) issue_d(0);
       if (wid < 2 && wid < nchunk) {  // the first two steps' members
         load_member(wid * kMembers);
         s_mp[wid][lane] = p2;
@@ -954,11 +1046,6 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
     if (nsteps > 0) {
       issue_e(0, 0, min(kMembers, m));
     }
-    unsigned mm[2][4];  // in-block matrix: the part over members above the block
-#pragma unroll
-    for (int r = 0; r < 2; r++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) mm[r][c] = kInf;
     unsigned acc[4][4];
 #pragma unroll
     for (int r = 0; r < 4; r++)
@@ -989,6 +1076,7 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
           if (++ch2 == nchunk) ch2 = 0;
         }
       }
+      if (ch == 0 && T > 0 && nchunk > 1 && R > 1) issue_d(T);
       if (ch == 0 && tid < kCols) arow_next = ancestor_row(c0 + (T + 2) * kCols + tid);
       if (4 * ry < Rp) {
         const unsigned *pe = s_E + 4 * cx, *ps = s_S + 4 * ry;
@@ -1031,18 +1119,20 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
 #pragma unroll
           for (int c = 0; c < 4; c++) acc[r][c] = kInf;
         }
+        cp_async_wait();
       }
       __syncthreads();
-      // columns inside the block, for nodes i below a (both in the block):
-      //   M(i, a) = min over u in X(i) of sc(i, u) + E(u, a); the part over u
-      // above the block takes column p_u of row a, which this tile has just
+      // columns inside the block, for nodes i below a (both in the block): the
+      // way over a member u takes column p_u of row a, which this tile has just
       // completed (the next tile is not written before the next barrier)
       if (R > 1 && 2 * my < Rp) {
         const int J = c0 + T * kCols;
+        const unsigned *pd = (nchunk > 1 ? s_D : s_S + kb * Rp) + 2 * my;
+        const int *pp = nchunk > 1 ? s_pd : s_mp[0] + kb;
 #pragma unroll 4
-        for (int k = kb; k < ke; k++) {
-          const uint2 w = __ldg(reinterpret_cast<const uint2 *>(B.direct + so + (int64_t)k * Rp + 2 * my));
-          const uint4 e = *reinterpret_cast<const uint4 *>(s_O + (__ldg(B.bm_p + m0 + k) - J) * 36 + 4 * mx);
+        for (int k = 0; k < ke - kb; k++) {
+          const uint2 w = *reinterpret_cast<const uint2 *>(pd + k * Rp);
+          const uint4 e = *reinterpret_cast<const uint4 *>(s_O + (pp[k] - J) * 36 + 4 * mx);
           const unsigned wr[2] = {w.x, w.y};
 #pragma unroll
           for (int r = 0; r < 2; r++) {
@@ -1058,63 +1148,45 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
     }
     // ---- the last task of the block finishes it
     unsigned *const mb = ntask > 1 ? A.mbuf + (int64_t)__ldg(A.mslot + b) * (kRows * kRows) : nullptr;
-    if (mb && R > 1) {
+    if (mb) {
 #pragma unroll
       for (int r = 0; r < 2; r++)
 #pragma unroll
+        for (int c = 0; c < 4; c++) {
+          const int i = 2 * my + r, a = 4 * mx + c;
+          if (i < R && ((s_anc[i] >> a) & 1u) && mm[r][c] < kInf) atomicMin(mb + i * kRows + a, mm[r][c]);
+        }
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        s_flag = atomicAdd(A.count + b, 1) == ntask - 1;
+        __threadfence();
+      }
+      __syncthreads();
+      if (!s_flag) continue;
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(mb + (2 * my + r) * kRows + 4 * mx));
+        mm[r][0] = x.x;
+        mm[r][1] = x.y;
+        mm[r][2] = x.z;
+        mm[r][3] = x.w;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int i = 2 * my + r;
+      if (i < R) {
+        int *row = A.dis + s_rowoff[i];
+        const unsigned anc = s_anc[i] >> (4 * mx);
+#pragma unroll
         for (int c = 0; c < 4; c++)
-          if (mm[r][c] < kInf) atomicMin(mb + (2 * my + r) * kRows + 4 * mx + c, mm[r][c]);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      s_flag = ntask == 1 || atomicAdd(A.count + b, 1) == ntask - 1;
-      __threadfence();
-    }
-    __syncthreads();
-    if (!s_flag) continue;
-#pragma unroll
-    for (int r = 0; r < 2; r++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const int at = (2 * my + r) * kRows + 4 * mx + c;
-        s_M[(2 * my + r) * 33 + 4 * mx + c] = mb ? __ldcg(mb + at) : mm[r][c];
-      }
-    __syncthreads();
-    if (wid == 0) {
-      // nodes in depth-first order; lane a holds the entry for the node at
-      // place a.  M stays symmetric over finished pairs, so E(w, a) is one
-      // read whichever of w and a lies deeper.
-      unsigned anc = 0;
-      for (int i = 1; i < R; i++) {
-        const int par = s_par[i];
-        const unsigned ai = __shfl_sync(0xffffffffu, anc, par) | (1u << par);
-        if (lane == i) anc = ai;
-        unsigned r = s_M[i * 33 + lane];
-        const int c = s_tc[i];
-#pragma unroll 4
-        for (int x = 0; x < c; x++) {
-          const int w = s_tl[32 * i + x];
-          r = add_min((unsigned)s_tw[32 * i + x], w == lane ? 0u : s_M[w * 33 + lane], r);
+          if ((anc >> c) & 1u) row[s_dcol[4 * mx + c]] = (int)mm[r][c];
+        if (mx < 4) {  // 0 for the node itself, INT_MAX in the row's padding
+          const int own = s_dcol[i], j = own + mx;
+          if (mx == 0) row[j] = 0;
+          else if (j < ((own + 4) & ~3)) row[j] = INT_MAX;
         }
-        __syncwarp();
-        if ((ai >> lane) & 1u) {
-          s_M[i * 33 + lane] = r;
-          s_M[lane * 33 + i] = r;
-        }
-        __syncwarp();
-      }
-      s_anc[lane] = anc;
-    }
-    __syncthreads();
-    for (int i = wid; i < R; i += 4) {
-      int *row = A.dis + s_rowoff[i];
-      const int own = s_dcol[i];
-      if ((s_anc[i] >> lane) & 1u) row[s_dcol[lane]] = (int)s_M[i * 33 + lane];
-      if (lane < 4) {  // 0 for the node itself, INT_MAX in the row's padding
-        const int j = own + lane;
-        if (lane == 0) row[j] = 0;
-        else if (j < ((own + 4) & ~3)) row[j] = INT_MAX;
       }
     }
     __syncthreads();
@@ -1188,6 +1260,7 @@ void FillPlan::build_blocks() {
   blk_soff = work.get<int64_t>(nblk + 1);
   bnode = work.get<int>(N);
   blk_of = work.get<int>(N);
+  blk_anc = work.get<unsigned>(N);
   loc_of = work.get<unsigned char>(N);
   lvl_cls = work.get<int>(nlev);
   done = work.get<int>(2 * (int64_t)nblk);  // done flags, then finished tasks per block
@@ -1238,6 +1311,7 @@ BlockArgs block_args(const FillPlan &P) {
   B.pos_w = P.pos_w;
   B.direct = P.direct;
   B.closed = P.closed;
+  B.anc = P.blk_anc;
   B.nblk = P.nblk;
   B.err = P.err;
   return B;
@@ -1299,10 +1373,12 @@ void FillPlan::enqueue_weights(cudaStream_t s) {
   const BlockArgs B = block_args(*this);
   const int gn = std::max(1, std::min(8192, (N + 7) / 8));  // a warp per vertex
   GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  const int gi = (nblk + kClosureWarps - 1) / kClosureWarps;
   if (!arcs) {  // the lists carry the weights
     gather_pos_weights_kernel<<<gn, 256, 0, s>>>(pos_hash, pos_src, lists.off, lists.w, pos_w, N);
     GH_CUDA(cudaGetLastError());
-    closure_kernel<<<dim3((nblk + kClosureWarps - 1) / kClosureWarps, 4), 32 * kClosureWarps, 0, s>>>(B);
+    closure_kernel<<<dim3(gi, 4), 32 * kClosureWarps, 0, s>>>(B);
+    inner_closure_kernel<<<gi, 32 * kClosureWarps, 0, s>>>(B);
     GH_CUDA(cudaGetLastError());
     return;
   }
@@ -1339,6 +1415,7 @@ void FillPlan::enqueue_weights(cudaStream_t s) {
                  (long long)wtasks, upd_total * 4e-6, clk.us() / 1e3);
   }
   list_weights_kernel<<<gn, 256, 0, s>>>(B, pos_src, lists.off, lists.w, pos_w, N);
+  inner_closure_kernel<<<gi, 32 * kClosureWarps, 0, s>>>(B);
   GH_CUDA(cudaGetLastError());
 }
 

@@ -338,7 +338,7 @@ struct FillPlan {
       *tcols = nullptr;
   int64_t *blk_boff = nullptr, *blk_moff = nullptr, *blk_soff = nullptr, *bm_row = nullptr, *task0 = nullptr;
   unsigned char *loc_of = nullptr;
-  unsigned *direct = nullptr, *closed = nullptr;
+  unsigned *direct = nullptr, *closed = nullptr, *blk_anc = nullptr;
   int64_t cell_total = 0;
   // weights from arcs: parent block and the members' places in it, update
   // triangles, task tables, arrivals a block waits for, each arc's cell

@@ -507,7 +507,7 @@ void FillPlan::release_work() {
   blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;
   hld_row = seg_off = blk_boff = blk_moff = blk_soff = bm_row = task0 = nullptr;
   loc_of = nullptr;
-  direct = closed = upd = mbuf = nullptr;
+  direct = closed = blk_anc = upd = mbuf = nullptr;
   mslot = nullptr;
   blk_up = bm_up = wtask_blk = pending = pend_init = nullptr;
   blk_uoff = wtask0 = arc_cell = nullptr;
