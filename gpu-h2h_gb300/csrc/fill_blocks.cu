@@ -31,10 +31,10 @@
 // A fill that takes a warp per (node, column block, separator chunk) tile is
 // bound by one L2 load per update and 13 us per tree level of the narrow top.
 // On one GB300 the blocks took the fill of a 264k-vertex road graph (4.5e9
-// updates) from 28.4 to 2.65 ms and of a 1M-vertex one (3.8e10) from 104 to 12.9
-// ms.  Narrow levels are a chain of blocks (about 30 us each, a step of 32
-// members 4,000 clocks); below them a term costs an ALU slot of half rate and the
-// kernel fills half of those slots.
+// updates) from 28.4 to 2.4 ms and of a 1M-vertex one (3.8e10) from 104 to 12.1
+// ms.  Narrow levels are a chain of blocks (about 22 us each, a step of 32
+// members 3,100 clocks); below them a term costs an ALU slot of half rate and the
+// kernel fills over half of those slots.
 #include <algorithm>
 #include <climits>
 #include <cstdio>
@@ -52,7 +52,7 @@ constexpr int kSmall = 16;    // largest light subtree that joins its father's b
 constexpr int kCols = 64;     // columns of one step of the product
 constexpr int kMembers = 32;  // separator members of one step
 constexpr int kMaxTiles = 64; // most tiles (of kCols columns) in a task
-constexpr int kEStride = 80;  // row stride of the staged second factor: 16-byte stores of two rows hit all banks
+constexpr int kEStride = 84;  // row stride of the staged second factor: 16-byte stores of eight rows hit all banks, of two rows nearly
 constexpr unsigned kInf = 0x7fffffffu;
 
 constexpr int kErrWait = 4;    // a dependency wait ran out
@@ -876,17 +876,21 @@ struct FillKernelArgs {
 // the 32 x 64 result.  A completed tile adds its columns' part of the matrix
 // inside the block, whose weights came to shared memory with the tile; the last
 // task of a block to finish writes that matrix and publishes the block.  Rows produced in the launch are
-// read through L2 (ld.global.cg).  A quad of four columns that lies above a
-// member (p_u >= J + 4) is one 128-bit load of u's row; below it, four
-// ancestors' entries at p_u, eight members of consecutive positions per warp
-// request (a third of a 32-byte sector per entry on a 264k-vertex graph).
-// Five CTAs per SM: with six the compiler holds 80 registers and shared memory
-// takes the L1 (4.3 ms against 3.8 on the 264k-vertex graph), with four there
-// are too few warps (4.0).
+// read through L2 (ld.global.cg).  A member at or below a tile is a row of it,
+// 16 columns of eight members to a warp request; of a member above it, column
+// p_u of each of the tile's ancestors, where lanes along the members read one
+// ancestor's row at neighbouring positions.  The product holds the next
+// member's operands while it sums: with 57 clocks a member for 32 of sums it
+// was the longest part of a narrow step.  1M-vertex graph: 12.9 ms with one
+// mapping of loads and without the operands ahead, 12.1 with both; each alone
+// gains nothing.
+// Five CTAs per SM (four: 12.3 ms; six hold 80 registers and spill).  Loads two
+// or three steps ahead, with 128 registers, gain nothing: a step waits 270
+// clocks of 4,000 for them.
 __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
   extern __shared__ __align__(16) int s_seg[];
-  __shared__ __align__(16) unsigned s_E[kMembers * kEStride];
-  __shared__ __align__(16) unsigned s_S[kMembers * kRows];
+  __shared__ __align__(16) unsigned s_E[(kMembers + 1) * kEStride];  // + 1: the product reads a row ahead
+  __shared__ __align__(16) unsigned s_S[(kMembers + 1) * kRows];
   __shared__ __align__(16) int64_t s_arow[2][kCols];
   __shared__ __align__(16) unsigned s_O[kCols * 36];   // a finished tile, [column][row]
   __shared__ int64_t s_mrow[2][kMembers];  // a step's members: rows and positions (-1: none)
@@ -942,14 +946,18 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
       s_kb[tid] = lo;
     }
     __syncthreads();
+    int seg = 0;  // the root-path segment of this thread's last column: they only move on
+    {
+      int hi = ns - 1;
+      while (seg < hi) {
+        const int mid = (seg + hi + 1) >> 1;
+        if (s_top[mid] <= c0 + tid + 1) seg = mid; else hi = mid - 1;
+      }
+    }
     auto ancestor_row = [&](int j) -> int64_t {  // row offset of the ancestor at depth j + 1
       if (j >= c1) return 0;
-      int lo = 0, hi = ns - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_top[mid] <= j + 1) lo = mid; else hi = mid - 1;
-      }
-      return __ldg(A.hld_row + s_pos[lo] + (j + 1 - s_top[lo]));
+      while (seg + 1 < ns && s_top[seg + 1] <= j + 1) seg++;
+      return __ldg(A.hld_row + s_pos[seg] + (j + 1 - s_top[seg]));
     };
     s_arow[tid >> 6][tid & 63] = ancestor_row(c0 + tid);
     const int nchunk = (m + kMembers - 1) / kMembers, ntile = (c1 - c0 + kCols - 1) / kCols;
@@ -972,10 +980,35 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
       p2 = k < m ? __ldg(B.bm_p + m0 + k) : -1;
       row2 = k < m ? __ldg(B.bm_row + m0 + k) : 0;
     };
-    // members of a step in buffer `mb` at the columns of tile T; a warp takes
-    // 16 columns of eight members at a time, so that it mostly goes one way
-    auto issue_e = [&](int T, int mb, int kn) {
-      const int J = c0 + T * kCols + ec;
+    // members k0 .. k0 + kn of a step, in buffer `mb`, at the columns of tile T.
+    // All above the tile (p_u before its columns): a lane per member, so that a
+    // request reads one ancestor's row at consecutive positions.  Otherwise a
+    // warp takes 16 columns of eight members at a time, rows of 64 bytes.
+    bool along = false;  // eb holds a member per lane
+    auto issue_e = [&](int T, int mb, int k0, int kn) {
+      const int J0 = c0 + T * kCols;
+      along = k0 + kn <= s_kb[T];
+      if (along) {
+        const int *col = A.dis + (lane < kn ? s_mp[mb][lane] : 0);
+        const int64_t *ar = s_arow[T & 1] + 16 * wid;
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+          if (J0 + 16 * wid + 4 * g < c1) {  // past column c1 the ancestor's row is 0: a read that counts for nothing
+            eb[g].x = (unsigned)__ldcg(col + ar[4 * g]);
+            eb[g].y = (unsigned)__ldcg(col + ar[4 * g + 1]);
+            eb[g].z = (unsigned)__ldcg(col + ar[4 * g + 2]);
+            eb[g].w = (unsigned)__ldcg(col + ar[4 * g + 3]);
+          }
+        }
+        return;
+      }
+      const int J = J0 + ec;
+      if (k0 >= s_kb[T + 1]) {  // all below it
+#pragma unroll
+        for (int g = 0; g < 4; g++)
+          if (8 * g + em < kn && J < c1) eb[g] = __ldcg(reinterpret_cast<const uint4 *>(A.dis + s_mrow[mb][8 * g + em] + J));
+        return;
+      }
       const int64_t *ar = s_arow[T & 1] + ec;
 #pragma unroll
       for (int g = 0; g < 4; g++) {
@@ -986,7 +1019,7 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
           if (p >= J + 4) {
             e = __ldcg(reinterpret_cast<const uint4 *>(row + J));
           } else if (p >= 0) {
-            const int *col = A.dis + p;  // past column c1 the ancestor's row is 0: a read that counts for nothing
+            const int *col = A.dis + p;
             unsigned x[4];
 #pragma unroll
             for (int c = 0; c < 4; c++)
@@ -1044,7 +1077,7 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
     __syncthreads();
     if (!s_flag) return;
     if (nsteps > 0) {
-      issue_e(0, 0, min(kMembers, m));
+      issue_e(0, 0, 0, min(kMembers, m));
     }
     unsigned acc[4][4];
 #pragma unroll
@@ -1054,7 +1087,8 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
     int64_t arow_next = 0;  // threads below 64: the column's ancestor row two tiles ahead
     for (int s = 0, T = 0, ch = 0, ch2 = 2 % max(nchunk, 1); s < nsteps; s++) {
 #pragma unroll
-      for (int g = 0; g < 4; g++) *reinterpret_cast<uint4 *>(s_E + (8 * g + em) * kEStride + ec) = eb[g];
+      for (int g = 0; g < 4; g++)
+        *reinterpret_cast<uint4 *>(along ? s_E + lane * kEStride + 16 * wid + 4 * g : s_E + (8 * g + em) * kEStride + ec) = eb[g];
       if (nchunk > 1 || s == 0) store_s();
       if (nchunk > 1 && s > 0 && wid == 0) {
         s_mp[(s + 1) & 1][lane] = p2;
@@ -1069,7 +1103,7 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
         nT++;
       }
       if (s + 1 < nsteps) {
-        issue_e(nT, nchunk > 1 ? (s + 1) & 1 : 0, min(kMembers, m - nch * kMembers));
+        issue_e(nT, nchunk > 1 ? (s + 1) & 1 : 0, nch * kMembers, min(kMembers, m - nch * kMembers));
         if (nchunk > 1) {
           issue_s(B.closed, nch * kMembers);
           if (wid == 0) load_member(ch2 * kMembers);
@@ -1080,10 +1114,12 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
       if (ch == 0 && tid < kCols) arow_next = ancestor_row(c0 + (T + 2) * kCols + tid);
       if (4 * ry < Rp) {
         const unsigned *pe = s_E + 4 * cx, *ps = s_S + 4 * ry;
+        uint4 e = *reinterpret_cast<const uint4 *>(pe), w = *reinterpret_cast<const uint4 *>(ps);
 #pragma unroll 4
-        for (int k = 0; k < kn; k++) {
-          const uint4 e = *reinterpret_cast<const uint4 *>(pe + k * kEStride);
-          const uint4 w = *reinterpret_cast<const uint4 *>(ps + k * Rp);
+        for (int k = 0; k < kn; k++) {  // the next member's row is on its way during this one's sums
+          pe += kEStride;
+          ps += Rp;
+          const uint4 en = *reinterpret_cast<const uint4 *>(pe), wn = *reinterpret_cast<const uint4 *>(ps);
           const unsigned wr[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int r = 0; r < 4; r++) {
@@ -1092,6 +1128,8 @@ __global__ void __launch_bounds__(128, 5) block_fill_kernel(FillKernelArgs A) {
             acc[r][2] = add_min(wr[r], e.z, acc[r][2]);
             acc[r][3] = add_min(wr[r], e.w, acc[r][3]);
           }
+          e = en;
+          w = wn;
         }
       }
       const int kb = s_kb[T], ke = nch == 0 ? s_kb[T + 1] : kb;  // members inside a completed tile
