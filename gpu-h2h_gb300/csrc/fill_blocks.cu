@@ -623,13 +623,25 @@ struct WeightArgs {
 };
 
 // A CTA takes a 64 x 64 tile of a block's update triangle, blocks from the
-// deepest up (a block's tasks wait for the tasks of the blocks below it).  It
-// eliminates the block's triangle, solves the tile's (at most 128) columns,
-// one per lane in registers, and forms the tile.  The diagonal tiles write
-// their columns back, direct and closed (see the closure); a tile may read
-// columns another has already written back, which solves to the same values.
+// deepest up (a block's tasks wait for the tasks of the blocks below it).  One
+// warp eliminates the block's triangle and closes it: C(i, u) is the least sum
+// of weights down a chain i > .. > u of the block's nodes.  With C a column's
+// elimination is a product, col(u) = min over i >= u of C(i, u) + col(i), and so
+// is its closure, S(i) = min over u <= i of C(i, u) + col(u).  Then the CTA forms
+// the tile; the diagonal tiles write their columns back, direct and closed,
+// after the parent has been told.  A tile may read columns another has already
+// written back, which solves to the same values (C is closed).
+//
+// Bound: the chain of blocks, 13 us each: 1 for the loads, 5 for the triangle, 2
+// for the columns, 1.5 for the tile and 3 for its atomics (66 blocks of a
+// 264k-vertex graph 1.48 -> 1.18 ms, 118 of a 1M-vertex one 4.55 -> 3.45).  The
+// loops over nodes stay loops: as straight-line code (6 us for the triangle, 4.5
+// for the columns) they ran at the speed of instruction fetches.  Four warps
+// to the triangle lose more in barriers (1.39 and 3.98 ms).
 __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
-  __shared__ __align__(16) unsigned s_L[kRows * 36];
+  __shared__ __align__(16) unsigned s_L[kRows * 36];   // row i of the triangle, columns moved up by kRows - 1 - i
+  __shared__ __align__(16) unsigned s_C[kRows * 36];   // C(i, u), [i][u] and [u][i]
+  __shared__ __align__(16) unsigned s_Ct[kRows * 36];
   __shared__ __align__(16) unsigned s_P[2][kRows * 68];
   __shared__ int s_up[2][64];
   __shared__ int64_t s_pso, s_puo;  // the parent's cells, triangle, members and row padding
@@ -713,58 +725,68 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
         col[4 * q + 3] = x.w;
       }
     }
-    // the block's own triangle, eliminated by the last warp (which on the
-    // diagonal has no columns): lane c holds column c of every row
+    // the block's own triangle, by the last warp (which on the diagonal has no
+    // columns): lane i holds row i, whose columns move up a register per node
+    // so that the node's own column is always the last.  Node w's row is final
+    // when its turn comes; rows above it (lanes below w) take the elimination's
+    // update, rows below it (lanes above w) extend their chains through w.
     if (wid == 3) {
       unsigned row[kRows];
-      const unsigned *src = cells + (int64_t)(m + lane) * Rp;
 #pragma unroll
-      for (int i = 0; i < kRows; i++) row[i] = lane < i && i < R ? __ldcg(src + i) : kInf;
-#pragma unroll
-      for (int i = kRows - 1; i > 1; i--)
-        if (i < R) {
-#pragma unroll
-          for (int u = 1; u < i; u++) row[u] = add_min(__shfl_sync(0xffffffffu, row[i], u), lane < u ? row[i] : kInf, row[u]);
-        }
-#pragma unroll
-      for (int i = 0; i < kRows; i++) s_L[i * 36 + lane] = row[i];
-    }
-    __syncthreads();
-    if (sub == 0)
-      for (int i = tid; i < R * Rp; i += 128) {
-        const int c = i / Rp, r = i - c * Rp;
-        if (r > c && r < R) cells[(int64_t)(m + c) * Rp + r] = s_L[r * 36 + c];
+      for (int q = 0; q < kRows; q++) {
+        const int c = q - (kRows - R);
+        row[q] = c >= 0 && c < lane && lane < R ? __ldcg(cells + (int64_t)(m + c) * Rp + lane) : kInf;
       }
-    // the tile's columns
+      for (int w = R; w < Rp; w++) s_C[lane * 36 + w] = kInf;  // the rows' padding
+#pragma unroll 1
+      for (int w = R - 1; w >= 0; w--) {
+        unsigned *const piv = s_L + w * 36;
+        if (lane == w) {
+#pragma unroll
+          for (int q = 0; q < kRows / 4; q++)
+            reinterpret_cast<uint4 *>(piv)[q] = make_uint4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]);
+        }
+        const unsigned chain = lane > w ? row[kRows - 1] : lane == w ? 0 : kInf;  // C(lane, w)
+        s_C[lane * 36 + w] = chain;
+        s_Ct[w * 36 + lane] = chain;
+        __syncwarp();
+        const unsigned by = lane < w ? piv[lane + kRows - 1 - w] : lane > w ? chain : kInf;
+#pragma unroll
+        for (int q = kRows / 4 - 1; q >= 0; q--) {
+          const uint4 x = reinterpret_cast<const uint4 *>(piv)[q];
+          if (q < kRows / 4 - 1) row[4 * q + 4] = add_min(by, x.w, row[4 * q + 3]);
+          row[4 * q + 3] = add_min(by, x.z, row[4 * q + 2]);
+          row[4 * q + 2] = add_min(by, x.y, row[4 * q + 1]);
+          row[4 * q + 1] = add_min(by, x.x, row[4 * q]);
+        }
+        row[0] = kInf;
+      }
+    }
     if (solve) {
 #pragma unroll
-      for (int i = kRows - 1; i > 0; i--)
-        if (i < R) {
-#pragma unroll
-          for (int u = 0; u < i; u++) col[u] = add_min(s_L[i * 36 + u], col[i], col[u]);
-        }
-#pragma unroll
       for (int i = 0; i < kRows; i++) s_P[half][i * 68 + 32 * (wid & 1) + lane] = col[i];
-      if (diag) {
-        uint4 *dst = reinterpret_cast<uint4 *>(cells + (int64_t)k * Rp);
-        uint4 *cls = reinterpret_cast<uint4 *>(B.closed + so + (int64_t)k * Rp);
-#pragma unroll
-        for (int q = 0; q < kRows / 4; q++)
-          if (4 * q < Rp && k < m) dst[q] = make_uint4(col[4 * q], col[4 * q + 1], col[4 * q + 2], col[4 * q + 3]);
-#pragma unroll
-        for (int i = 1; i < kRows; i++)
-          if (i < R) {
-#pragma unroll
-            for (int u = 0; u < i; u++) col[i] = add_min(s_L[i * 36 + u], col[u], col[i]);
-          }
-#pragma unroll
-        for (int q = 0; q < kRows / 4; q++)
-          if (4 * q < Rp && k < m) cls[q] = make_uint4(col[4 * q], col[4 * q + 1], col[4 * q + 2], col[4 * q + 3]);
-      }
     }
-    if (p < 0) continue;
     __syncthreads();
-    if (x0 < m && y0 < m) {
+    // the tile's columns
+    unsigned *const mine = s_P[half] + 32 * (wid & 1) + lane;
+    if (solve) {
+#pragma unroll 1
+      for (int i = 1; i < R; i++) {  // col holds row i itself: C(i, i) = 0
+        const unsigned x = mine[i * 68];
+#pragma unroll
+        for (int q = 0; q < kRows / 4; q++) {
+          const uint4 y = *reinterpret_cast<const uint4 *>(s_C + i * 36 + 4 * q);
+          col[4 * q] = add_min(y.x, x, col[4 * q]);
+          col[4 * q + 1] = add_min(y.y, x, col[4 * q + 1]);
+          col[4 * q + 2] = add_min(y.z, x, col[4 * q + 2]);
+          col[4 * q + 3] = add_min(y.w, x, col[4 * q + 3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kRows; i++) mine[i * 68] = col[i];
+    }
+    __syncthreads();
+    if (p >= 0 && x0 < m && y0 < m) {
       const unsigned *px = s_P[0] + 4 * xg, *py = s_P[diag ? 0 : 1] + 8 * yg;
 #pragma unroll 2
       for (int i = 0; i < R; i++) {
@@ -804,9 +826,39 @@ __global__ void __launch_bounds__(128, 4) weights_kernel(WeightArgs A) {
       }
     }
     __syncthreads();
-    if (tid == 0) {
+    if (p >= 0 && tid == 0) {
       __threadfence();
       atomicSub(A.pending + p, 1);
+    }
+    // what only later kernels read
+    if (sub == 0)
+      for (int i = tid; i < R * Rp; i += 128) {
+        const int c = i / Rp, r = i - c * Rp;
+        if (r > c && r < R) cells[(int64_t)(m + c) * Rp + r] = s_L[r * 36 + c + kRows - 1 - r];
+      }
+    if (diag && solve && k < m) {
+      uint4 *dst = reinterpret_cast<uint4 *>(cells + (int64_t)k * Rp);
+      uint4 *cls = reinterpret_cast<uint4 *>(B.closed + so + (int64_t)k * Rp);
+#pragma unroll
+      for (int i = 0; i < kRows; i++) col[i] = mine[i * 68];
+#pragma unroll
+      for (int q = 0; q < kRows / 4; q++)
+        if (4 * q < Rp) dst[q] = make_uint4(col[4 * q], col[4 * q + 1], col[4 * q + 2], col[4 * q + 3]);
+#pragma unroll 1
+      for (int u = 0; u < R - 1; u++) {
+        const unsigned x = mine[u * 68];
+#pragma unroll
+        for (int q = 0; q < kRows / 4; q++) {
+          const uint4 y = *reinterpret_cast<const uint4 *>(s_Ct + u * 36 + 4 * q);
+          col[4 * q] = add_min(y.x, x, col[4 * q]);
+          col[4 * q + 1] = add_min(y.y, x, col[4 * q + 1]);
+          col[4 * q + 2] = add_min(y.z, x, col[4 * q + 2]);
+          col[4 * q + 3] = add_min(y.w, x, col[4 * q + 3]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kRows / 4; q++)
+        if (4 * q < Rp) cls[q] = make_uint4(col[4 * q], col[4 * q + 1], col[4 * q + 2], col[4 * q + 3]);
     }
   }
 }
