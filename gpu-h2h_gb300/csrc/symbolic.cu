@@ -552,7 +552,9 @@ bool ElimPlan::plan_bits() {
   // one CTA, 1.5 us across a cluster) and its neighbours' rows, 1 us + 45 ps
   // per word of the cell, which a cluster shares.  Measured us per pick with 1
   // / 2 / 4 / 8 / 16 CTAs: 716 members 3.4 / 2.9 / 2.3 / 1.9 / 1.9, 1,604 members
-  // - / - / 2.5 / 2.0 / 1.8, 2,968 members - / - / - / 2.7 / 2.3.  Cells that
+  // - / - / 2.5 / 2.0 / 1.8, 2,968 members - / - / - / 2.7 / 2.3.  The bottom
+  // cells' members have the input's few arcs, so their rows cost a tenth: 32 cells
+  // of 469 members 0.44 ms with one CTA each, 0.62 with 2, 0.59 with 4, 0.70 with 16.  Cells that
   // outnumber the SMs keep few warps (1,024 cells of 259 members: 0.54 ms with
   // 4 warps, 0.67 with 8; 2,048 cells of 489: 3.7 with 4, 2.8 with 8, 3.9 with 16).
   cudaFuncAttributes fa;
@@ -624,7 +626,8 @@ bool ElimPlan::plan_bits() {
             continue;
           }
           const double waves = std::ceil((double)L.ncell / fit);
-          const double cost = waves * ((cs == 1 ? 1.1 : 1.5) + (1.0 + 4.5e-5 * smax * w) / cs);
+          const double rows = (st == 0 && nsteps > 0 ? 0.1 : 1.0) * (1.0 + 4.5e-5 * smax * w);
+          const double cost = waves * ((cs == 1 ? 1.1 : 1.5) + rows / cs);
           if (cost < best * 0.99) {
             best = cost;
             L.cs = cs;
