@@ -77,16 +77,39 @@ __device__ __forceinline__ int line_starts(const char *text, int64_t size, int64
   return __popcll(m);
 }
 
-__global__ void __launch_bounds__(kTextThreads) count_lines_kernel(const char *text, int64_t size, int *count) {
+// The two files' records: the ID file's text first, the Edge file's at a
+// 256-byte boundary behind it, each in blocks of its own.
+struct LoadArgs {
+  const char *text[2];
+  int64_t size[2];
+  unsigned blocks[2];
+  int *count;            // lines per block, and one word more
+  const int64_t *first;  // lines before each block
+  int n;
+  int64_t m;
+  int *part, *pos, *tail, *v, *w, *parent;
+  LoadFlags *flags;
+};
+
+// Lines per block; what the parser only sets in part starts unset.
+__global__ void __launch_bounds__(kTextThreads) count_lines_kernel(LoadArgs A) {
   __shared__ int s_sum;
   if (threadIdx.x == 0) s_sum = 0;
   __syncthreads();
+  const int f = blockIdx.x >= A.blocks[0];
+  const int64_t base = (blockIdx.x - (f ? A.blocks[0] : 0)) * kTextBlock + (int64_t)threadIdx.x * kBytes;
   unsigned long long m;
-  int c = line_starts(text, size, blockIdx.x * kTextBlock + (int64_t)threadIdx.x * kBytes, &m);
+  int c = line_starts(A.text[f], A.size[f], base, &m);
   c = __reduce_add_sync(0xffffffffu, c);
   if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, c);
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t == 0) {
+    A.count[A.blocks[0] + A.blocks[1]] = 0;
+    *A.flags = LoadFlags{};
+  }
+  for (int64_t i = t; i < A.n; i += (int64_t)gridDim.x * blockDim.x) A.part[i] = A.pos[i] = -1;
   __syncthreads();
-  if (threadIdx.x == 0) count[blockIdx.x] = s_sum;
+  if (threadIdx.x == 0) A.count[blockIdx.x] = s_sum;
 }
 
 struct Reader {
@@ -118,19 +141,20 @@ struct Reader {
   }
 };
 
-// kArcs: "a u v w" into a = tail, b = head, c = weight; else "idx lon lat id"
-// into a[idx] = id, b[id] = idx.
-template <bool kArcs>
-__global__ void __launch_bounds__(kTextThreads) parse_lines_kernel(const char *text, int64_t size,
-                                                                   const int64_t *first, int64_t records, int n,
-                                                                   int *a, int *b, int *c, LoadFlags *flags) {
-  if (first[gridDim.x] != records) {  // lines in all
-    if (blockIdx.x == 0 && threadIdx.x == 0) flags->odd = 1;
+// "a u v w" into tail, v and w; "idx lon lat id" into part[idx] = id, pos[id] = idx.
+__global__ void __launch_bounds__(kTextThreads) parse_lines_kernel(LoadArgs A) {
+  const unsigned nb = A.blocks[0] + A.blocks[1];
+  const int n = A.n;
+  if (A.first[A.blocks[0]] != n || A.first[nb] - n != A.m) {  // lines in all
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.flags->odd = 1;
     return;
   }
+  const bool arcs = blockIdx.x >= A.blocks[0];
+  const char *text = A.text[arcs];
+  const int64_t size = A.size[arcs], records = arcs ? A.m : n;
   __shared__ int s_warp[kTextThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t base = blockIdx.x * kTextBlock + (int64_t)threadIdx.x * kBytes;
+  const int64_t base = (blockIdx.x - (arcs ? A.blocks[0] : 0)) * kTextBlock + (int64_t)threadIdx.x * kBytes;
   unsigned long long m;
   const int cnt = line_starts(text, size, base, &m);
   int incl = cnt;
@@ -141,7 +165,7 @@ __global__ void __launch_bounds__(kTextThreads) parse_lines_kernel(const char *t
   }
   if (lane == 31) s_warp[wid] = incl;
   __syncthreads();
-  int64_t k = first[blockIdx.x] + incl - cnt;
+  int64_t k = A.first[blockIdx.x] - (arcs ? n : 0) + incl - cnt;
   for (int w = 0; w < wid; w++) k += s_warp[w];
   bool odd = false;
   while (m) {
@@ -149,35 +173,44 @@ __global__ void __launch_bounds__(kTextThreads) parse_lines_kernel(const char *t
     Reader r{text + at, text + min(size, at + kLineBytes)};
     m &= m - 1;
     long long x, y, z;
-    if (kArcs) {
+    if (arcs) {
       bool ok = r.at() == 'a';
       r.p++;
       ok = ok && r.blanks() && r.number(x) && r.blanks() && r.number(y) && r.blanks() && r.number(z) && r.end(text + size);
       ok = ok && x >= 1 && x <= n && y >= 1 && y <= n && x != y && z <= INT_MAX && k < records;
       if (ok) {
-        a[k] = (int)x - 1;
-        b[k] = (int)y - 1;
-        c[k] = (int)z;
+        A.tail[k] = (int)x - 1;
+        A.v[k] = (int)y - 1;
+        A.w[k] = (int)z;
       }
       odd |= !ok;
     } else {
       bool ok = r.number(x) && r.blanks() && r.field() && r.blanks() && r.field() && r.blanks() && r.number(y) && r.end(text + size);
       ok = ok && x < n && y < n && k < records;
       if (ok) {
-        a[x] = (int)y;
-        b[y] = (int)x;
+        A.part[x] = (int)y;
+        A.pos[y] = (int)x;
       }
       odd |= !ok;
     }
     k++;
   }
-  if (odd) flags->odd = 1;
+  if (odd) A.flags->odd = 1;
 }
 
-__global__ void sorted_kernel(const int *tail, int64_t m, LoadFlags *flags) {
-  if (flags->odd) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x + 1; i < m; i += (int64_t)gridDim.x * blockDim.x)
-    if (tail[i] < tail[i - 1]) flags->unsorted = 1;
+// Whether the tails come in order and every position and vertex has its line;
+// every vertex a component of its own.
+__global__ void sorted_kernel(LoadArgs A) {
+  if (A.flags->odd) return;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t + 1; i < A.m; i += step)
+    if (A.tail[i] < A.tail[i - 1]) A.flags->unsorted = 1;
+  bool odd = false;
+  for (int64_t i = t; i < A.n; i += step) {
+    odd |= A.part[i] < 0 || A.pos[i] < 0;
+    A.parent[i] = (int)i;
+  }
+  if (odd) A.flags->odd = 1;
 }
 
 __global__ void iota_kernel(int *a, int64_t m) {
@@ -201,14 +234,6 @@ __global__ void offsets_kernel(const int *tail, int64_t m, int n, int *off, cons
   }
 }
 
-__global__ void check_ids_kernel(const int *part, const int *pos, const int *off, int n, LoadFlags *flags) {
-  if (stopped(flags)) return;
-  bool odd = false;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    odd |= part[i] < 0 || pos[i] < 0 || off[i + 1] - off[i] > kScanDegree;
-  if (odd) flags->odd = 1;
-}
-
 __device__ __forceinline__ int find_root(int *parent, int x) {
   for (;;) {
     const int p = *(volatile int *)(parent + x);
@@ -226,8 +251,13 @@ __global__ void check_arcs_kernel(const int *tail, const int *head, const int *o
   if (stopped(flags)) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
     const int u = tail[i], v = head[i];
+    const int b0 = off[v], b1 = off[v + 1];
+    if (b1 - b0 > kScanDegree) {  // too long to search arc by arc
+      flags->odd = 1;
+      return;
+    }
     bool back = false;
-    for (int e = off[v]; e < off[v + 1] && !back; e++) back = __ldg(head + e) == u;
+    for (int e = b0; e < b1 && !back; e++) back = __ldg(head + e) == u;
     if (!back) flags->missing = 1;
     if (u < v) continue;
     int a = find_root(parent, u), b = find_root(parent, v);
@@ -279,36 +309,17 @@ struct QuietStream {
   }
 };
 
-int64_t text_blocks(int64_t size) { return (size + kTextBlock - 1) / kTextBlock; }
-
-// Copies a file's records to the device and numbers their lines (first: per
-// block, and the number of lines at its end).
-const char *number_lines(const char *text, int64_t size, Workspace &ws, cudaStream_t s, int64_t **first) {
-  char *d_text = ws.get<char>(size);
-  GH_CUDA(cudaMemcpyAsync(d_text, text, size, cudaMemcpyHostToDevice, s));
-  const int64_t nb = text_blocks(size);
-  int *count = ws.get<int>(nb + 1);
-  *first = ws.get<int64_t>(nb + 1);
-  GH_CUDA(cudaMemsetAsync(count + nb, 0, sizeof(int), s));
-  count_lines_kernel<<<(unsigned)nb, kTextThreads, 0, s>>>(d_text, size, count);
-  GH_CUDA(cudaGetLastError());
-  exclusive_scan<int>(count, *first, nb + 1, ws, s);
-  return d_text;
-}
-
 // Offsets and checks of arcs sorted by tail.
-void check_arcs(const DeviceInput &in, int *tail, int64_t m, int n, int *parent, LoadFlags *flags, cudaStream_t s) {
-  offsets_kernel<<<blocks_for(m + 1), 256, 0, s>>>(tail, m, n, in.off, flags);
-  check_ids_kernel<<<blocks_for(n), 256, 0, s>>>(in.part, in.pos, in.off, n, flags);
-  iota_kernel<<<blocks_for(n), 256, 0, s>>>(parent, n);
-  check_arcs_kernel<<<blocks_for(m), 256, 0, s>>>(tail, in.v, in.off, m, parent, flags);
-  check_connected_kernel<<<blocks_for(n), 256, 0, s>>>(parent, n, flags);
+void check_arcs(const DeviceInput &in, const LoadArgs &A, cudaStream_t s) {
+  offsets_kernel<<<blocks_for(A.m + 1), 256, 0, s>>>(A.tail, A.m, A.n, in.off, A.flags);
+  check_arcs_kernel<<<blocks_for(A.m), 256, 0, s>>>(A.tail, in.v, in.off, A.m, A.parent, A.flags);
+  check_connected_kernel<<<blocks_for(A.n), 256, 0, s>>>(A.parent, A.n, A.flags);
   GH_CUDA(cudaGetLastError());
 }
 
-// One allocation for the graph, one for the scratch, one wait: a batch's loads
-// are short (0.25 ms for a 15k-vertex graph; 0.5 with a wait and an allocation
-// per step).
+// One allocation for the graph, one for the scratch, seven kernels and one
+// wait: a batch's loads are short (a 4,096-vertex graph's 0.5 ms with a wait and
+// an allocation per step, 0.31 with one of each and thirteen kernels, 0.27 now).
 bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, int64_t arcs_size, int64_t m) {
   const int n = g.n;
   if (n > ids_size / 7 || m > arcs_size / 7) return false;  // a record takes eight bytes, the last one seven
@@ -322,39 +333,53 @@ bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, 
   in->w = in->mem.get<int>(m);
   in->part = in->mem.get<int>(n);
   in->pos = in->mem.get<int>(n);
-  const int64_t nb = text_blocks(ids_size) + text_blocks(arcs_size) + 2;
-  ws.reserve((size_t)(ids_size + arcs_size + 4 * (m + n) + 12 * nb + 32 * (nb / kScanTile + 2)) + (64 << 10));
-  LoadFlags *flags = ws.get<LoadFlags>(1);
-  int *tail = ws.get<int>(m), *parent = ws.get<int>(n);
-  int64_t *id_first, *first;
-  const char *id_text = number_lines(ids, ids_size, ws, q.s, &id_first);
-  const char *text = number_lines(arcs, arcs_size, ws, q.s, &first);
-  GH_CUDA(cudaMemsetAsync(flags, 0, sizeof(LoadFlags), q.s));
-  GH_CUDA(cudaMemsetAsync(in->part, 0xff, sizeof(int) * (size_t)n, q.s));  // -1
-  GH_CUDA(cudaMemsetAsync(in->pos, 0xff, sizeof(int) * (size_t)n, q.s));
-  parse_lines_kernel<false><<<(unsigned)text_blocks(ids_size), kTextThreads, 0, q.s>>>(id_text, ids_size, id_first, n, n,
-                                                                                       in->part, in->pos, nullptr, flags);
-  parse_lines_kernel<true><<<(unsigned)text_blocks(arcs_size), kTextThreads, 0, q.s>>>(text, arcs_size, first, m, n, tail,
-                                                                                       in->v, in->w, flags);
-  sorted_kernel<<<blocks_for(m), 256, 0, q.s>>>(tail, m, flags);
+  const int64_t nb = (ids_size + kTextBlock - 1) / kTextBlock + (arcs_size + kTextBlock - 1) / kTextBlock;
+  ws.reserve((size_t)(ids_size + arcs_size + 4 * (m + n) + 12 * (nb + 1) + 32 * (nb / kScanTile + 2)) + (64 << 10));
+  LoadArgs A{};
+  A.flags = ws.get<LoadFlags>(1);
+  A.tail = ws.get<int>(m);
+  A.parent = ws.get<int>(n);
+  char *text[2] = {ws.get<char>(ids_size), ws.get<char>(arcs_size)};
+  A.count = ws.get<int>(nb + 1);
+  int64_t *first = ws.get<int64_t>(nb + 1);
+  GH_CUDA(cudaMemcpyAsync(text[0], ids, ids_size, cudaMemcpyHostToDevice, q.s));
+  GH_CUDA(cudaMemcpyAsync(text[1], arcs, arcs_size, cudaMemcpyHostToDevice, q.s));
+  A.text[0] = text[0];
+  A.text[1] = text[1];
+  A.size[0] = ids_size;
+  A.size[1] = arcs_size;
+  A.blocks[0] = (unsigned)((ids_size + kTextBlock - 1) / kTextBlock);
+  A.blocks[1] = (unsigned)(nb - A.blocks[0]);
+  A.first = first;
+  A.n = n;
+  A.m = m;
+  A.part = in->part;
+  A.pos = in->pos;
+  A.v = in->v;
+  A.w = in->w;
+  count_lines_kernel<<<(unsigned)nb, kTextThreads, 0, q.s>>>(A);
   GH_CUDA(cudaGetLastError());
-  check_arcs(*in, tail, m, n, parent, flags, q.s);
+  exclusive_scan<int>(A.count, first, nb + 1, ws, q.s);
+  parse_lines_kernel<<<(unsigned)nb, kTextThreads, 0, q.s>>>(A);
+  sorted_kernel<<<blocks_for(std::max<int64_t>(m, n)), 256, 0, q.s>>>(A);
+  GH_CUDA(cudaGetLastError());
+  check_arcs(*in, A, q.s);
   LoadFlags f{};
-  q.read(&f, flags, sizeof(f));
+  q.read(&f, A.flags, sizeof(f));
   if (f.odd) return false;
   if (f.unsorted) {  // the arcs of a vertex in file order: a stable sort by tail
     int *from = ws.get<int>(m), *v2 = in->mem.get<int>(m), *w2 = in->mem.get<int>(m);
     iota_kernel<<<blocks_for(m), 256, 0, q.s>>>(from, m);
     int bits = 1;
     while (bits < 32 && (int64_t(1) << bits) <= n) bits++;
-    radix_sort_pairs(reinterpret_cast<unsigned *>(tail), from, m, bits, ws, q.s);
+    radix_sort_pairs(reinterpret_cast<unsigned *>(A.tail), from, m, bits, ws, q.s);
     gather_arcs_kernel<<<blocks_for(m), 256, 0, q.s>>>(from, in->v, in->w, v2, w2, m);
     GH_CUDA(cudaGetLastError());
     in->v = v2;
     in->w = w2;
-    GH_CUDA(cudaMemsetAsync(flags, 0, sizeof(LoadFlags), q.s));
-    check_arcs(*in, tail, m, n, parent, flags, q.s);
-    q.read(&f, flags, sizeof(f));
+    GH_CUDA(cudaMemsetAsync(A.flags, 0, sizeof(LoadFlags), q.s));
+    check_arcs(*in, A, q.s);
+    q.read(&f, A.flags, sizeof(f));
   }
   if (f.odd || f.missing || f.split) return false;
   g.m = m;
