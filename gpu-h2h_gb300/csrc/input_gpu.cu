@@ -24,6 +24,7 @@
 #include <cstdlib>
 
 #include "graph.h"
+#include "quiet.h"
 #include "sort.h"
 
 namespace gh {
@@ -282,32 +283,6 @@ __global__ void check_connected_kernel(int *parent, int n, LoadFlags *flags) {
 }
 
 unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, (n + 255) / 256)); }
-
-// Loading and reading a graph back are host calls to their caller, who may be
-// capturing a graph: allocations must not count against the capture, and no
-// work goes to the legacy stream.
-struct RelaxedCapture {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  RelaxedCapture(const RelaxedCapture &) = delete;
-  RelaxedCapture &operator=(const RelaxedCapture &) = delete;
-};
-
-struct QuietStream {
-  cudaStream_t s = nullptr;
-  QuietStream() { GH_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
-  ~QuietStream() {
-    cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-  }
-  QuietStream(const QuietStream &) = delete;
-  QuietStream &operator=(const QuietStream &) = delete;
-  void read(void *to, const void *from, size_t bytes) {
-    GH_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, s));
-    GH_CUDA(cudaStreamSynchronize(s));
-  }
-};
 
 // Offsets and checks of arcs sorted by tail.
 void check_arcs(const DeviceInput &in, const LoadArgs &A, cudaStream_t s) {

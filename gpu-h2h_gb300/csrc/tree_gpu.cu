@@ -32,6 +32,7 @@
 #include <cstring>
 
 #include "graph.h"
+#include "quiet.h"
 #include "sort.h"
 
 namespace gh {
@@ -405,8 +406,10 @@ static void read_tree(const Graph &g, int *order, int *father, int *depth, int *
   const TreeStore &T = *g.tree;
   const int n = g.n, vb = g.dev.id_base;
   GH_CHECK(T.depth && g.dev.first, H2H_ERR_STATE, "tree not built");
+  RelaxedCapture relaxed;
+  QuietStream q;
   auto down = [&](auto *to, const auto *from, int64_t count) {
-    if (to) GH_CUDA(cudaMemcpy(to, from, sizeof(*to) * (size_t)count, cudaMemcpyDeviceToHost));
+    if (to) q.read(to, from, sizeof(*to) * (size_t)count);
   };
   down(order, T.elim + vb, n);
   down(father, T.father + vb, n);
@@ -450,8 +453,11 @@ const Graph &host_tree(const Graph &gc) {
   g.x_off.resize((size_t)n + 1);
   g.drow_host.resize((size_t)n + 1);
   read_tree(g, order.data(), g.father.data(), g.depth.data(), g.first.data(), g.x_off.data());
-  GH_CUDA(cudaMemcpy(g.drow_host.data(), g.tree->drow + g.dev.id_base, sizeof(int64_t) * ((size_t)n + 1),
-                     cudaMemcpyDeviceToHost));
+  {
+    RelaxedCapture relaxed;
+    QuietStream q;
+    q.read(g.drow_host.data(), g.tree->drow + g.dev.id_base, sizeof(int64_t) * ((size_t)n + 1));
+  }
   g.pos_hash.resize((size_t)n + 1);
   g.dis_hash.assign((size_t)n + 1, 0);
   std::vector<int> pre(n);

@@ -113,3 +113,32 @@ def test_forms_match_host_reader(tmp_path, capfd, monkeypatch):
     for name in want:
         assert got[name] == want[name], name
     assert taken == sum(gpu for _, _, gpu in forms().values())
+
+
+def test_load_and_read_back_during_a_capture(tmp_path):
+    """Loading a graph and reading a built one back stay host calls: they run
+    beside a graph capture (global mode) and do not spoil it."""
+    import gpuh2h
+    import torch
+
+    from small_graphs import write
+    n, edges = grid(9, 9)
+    files = write(tmp_path, n, [(u, v, w, w) for u, v, w in edges], 2)
+    ref = gpuh2h.Graph("g", 2, 1, 2, 1, files=files)
+    arcs, built = ref.input_arcs(), ref.contraction_noHub(1)
+    order = ref.order()
+    other = gpuh2h.Graph("g", 2, 1, 2, 1, files=files).contraction_noHub(1)
+    x = torch.zeros(4, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        x += 1
+        g = gpuh2h.Graph("g", 2, 1, 2, 1, files=files)
+        got = g.input_arcs()
+        assert (other.order() == order).all()
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 4
+    assert all((a == b).all() for a, b in zip(arcs, got))
+    for h in (g, built, other):
+        h.close()
