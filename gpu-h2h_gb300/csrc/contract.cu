@@ -1670,7 +1670,8 @@ void ElimPlan::release() {
   mem.release();
   members = extra = nullptr;
   sym_cells = nullptr;
-  grows = nullptr;
+  grows = sym_arrived = nullptr;
+  sym_best = nullptr;
   grid_map = nullptr;
   hg_partial = nullptr;
   grid_bar = nullptr;

@@ -213,8 +213,9 @@ struct ElimPlan {
   // of cs CTAs with nw warps, rows of up to smax members
   struct SymLaunch {
     int step, level, ncell, kmax, smax, npow, cs, nw;
-    bool heap, global;
-    int64_t lo, smem, rows_off;
+    bool heap, global, grid;  // grid: cs CTAs per cell in one cooperative launch
+    int64_t lo, smem, rows_off, best_off;
+    int arrived_off;
   };
   // What the list kernels' launches need on the device
   struct ListLaunches {
@@ -234,7 +235,9 @@ struct ElimPlan {
   // own, freed once they are compacted
   int *pool = nullptr;
   bool own_pool = false;
-  unsigned *grows = nullptr;
+  unsigned *grows = nullptr, *sym_arrived = nullptr;
+  unsigned long long *sym_best = nullptr;
+  int grid_cells = 0;
   int N = 0, heap_total = 0;
   int64_t M = 0, lub = 0, slots_size = 0, pool_size = 0;
   std::vector<Launch> launches;  // in step order; launches of one step are independent

@@ -31,6 +31,14 @@
 // through distributed shared memory, one cluster barrier, then each CTA copies
 // v's row from its owner and updates the rows it owns, a warp per row.
 //
+// A cell whose rows outgrow a cluster's shared memory keeps them in global
+// memory (L2) and, where the launch has few enough cells, takes up to 128 CTAs
+// that meet at a counter in global memory instead of a cluster barrier (kGrid,
+// a cooperative launch; every wait is bounded).  Its picks are bound by the
+// neighbours' rows, of which a lane has eight words in flight: the global order of a
+// 6.26M-vertex graph (7,801 members) 141 ms on one cluster, 91 on 128 CTAs a
+// word at a time, 38 now; of a 3.6M-vertex one (5,940) 68, 50 and 28 ms.
+//
 // Rules kept from the reference: a cell's first pick uses the stale keys
 // (input degree, height 0), later picks live ones (kernel_functions.cu:462-476);
 // a neighbour's height becomes max(height, HeightNow + 1); the global order
@@ -54,6 +62,7 @@ namespace {
 
 constexpr int kErrOverflow = 1;  // a list outgrew its capacity
 constexpr int kErrEmpty = 2;     // eliminated a vertex without neighbours
+constexpr int kErrTimeout = 4;   // a grid barrier wait ran out
 constexpr int kErrPick = 5;      // no candidate left to pick, or a vertex outside its cell
 constexpr int kErrPool = 6;      // the list pool is full
 
@@ -78,6 +87,11 @@ struct SymArgs {
   unsigned long long *pool_next;
   int64_t pool_size;
   int smax, npow, heap;
+  // kGrid: CTAs per cell, their best keys [cell][2][cs], arrivals per cell
+  int cs;
+  unsigned long long *best;
+  unsigned *arrived;
+  long long spin_limit;
 };
 
 __device__ __forceinline__ unsigned long long pack_key(int deg, int height, int l) {
@@ -100,14 +114,44 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long k) {
   return ((unsigned long long)hi << 32) | lo;
 }
 
-template <bool kGlobal>
+// All cs CTAs of a cell meet; `target` arrivals end the wait.  Writes before it
+// are seen by all after it.  False once a wait has run out (A.err is set, and
+// every CTA of the launch gives up at its next barrier).
+__device__ bool grid_meet(unsigned *arrived, unsigned target, const SymArgs &A, int *s_ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1);
+    int ok = 1;
+    const long long t0 = clock64();
+    unsigned seen;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
+      if (seen >= target) break;
+      if (*(volatile int *)A.err == kErrTimeout || clock64() - t0 > A.spin_limit) {
+        atomicCAS(A.err, 0, kErrTimeout);
+        ok = 0;
+        break;
+      }
+    }
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+template <bool kGlobal, bool kGrid>
 __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
+  static_assert(kGlobal || !kGrid, "a grid's rows are in global memory");
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned long long s_gmin[2][kMaxGroups];  // best key of every group of rows
   __shared__ unsigned long long s_best[2][16];          // best key of every CTA
   cg::cluster_group cluster = cg::this_cluster();
-  const int CS = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int CS = kGrid ? A.cs : (int)cluster.num_blocks();
+  const int rank = kGrid ? (int)(blockIdx.x % CS) : (int)cluster.block_rank();
   const int ci = (int)(blockIdx.x / CS);
+  __shared__ int s_ok;
+  unsigned meets = 0;
   const SymCell c = A.cells[ci];
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
   const int S = c.size, k = c.count, W = (S + 31) >> 5;
@@ -190,7 +234,11 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
     }
   }
   __syncthreads();
-  if (CS > 1) cluster.sync();
+  if (kGrid) {
+    if (!grid_meet(A.arrived + ci, ++meets * CS, A, &s_ok)) return;
+  } else if (CS > 1) {
+    cluster.sync();
+  }
   // Row r belongs to group r mod G, a lane of the group's warp (neighbours
   // have close ids, so they spread over the groups).  Each group's best key is
   // kept, so a pick looks at the groups and an update at the groups it hits.
@@ -246,7 +294,20 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
       const unsigned long long x = s_gmin[par][lane], y = s_gmin[par][lane + 32];
       b = x < y ? x : y;
     }
-    if (CS == 1) {
+    if (kGrid) {
+      unsigned long long *best = A.best + ((int64_t)ci * 2 + par) * CS;
+      if (wid == 0) {
+        b = warp_min(b);
+        if (lane == 0) best[rank] = b;
+      }
+      if (!grid_meet(A.arrived + ci, ++meets * CS, A, &s_ok)) return;
+      b = kNoKey;
+      for (int i = lane; i < CS; i += 32) {
+        const unsigned long long x = __ldcg(best + i);
+        b = x < b ? x : b;
+      }
+      b = warp_min(b);
+    } else if (CS == 1) {
       b = warp_min(b);
     } else {
       if (wid == 0) {
@@ -294,12 +355,24 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
             todo &= todo - 1;
             unsigned *row = own_row(r);
             int pc = 0;
-            for (int w = lane; w < W; w += 32) {
-              unsigned x = (kGlobal ? __ldcg(row + w) : row[w]) | rv[w];
-              if (w == (l >> 5)) x &= ~(1u << (l & 31));
-              if (w == (lv >> 5)) x &= ~(1u << (lv & 31));
-              row[w] = x;
-              pc += __popc(x);
+            constexpr int kAhead = kGlobal ? 8 : 1;  // words of a lane in flight
+            for (int w0 = lane; w0 < W; w0 += 32 * kAhead) {
+              unsigned x[kAhead];
+#pragma unroll
+              for (int q = 0; q < kAhead; q++) {
+                const int w = w0 + 32 * q;
+                x[q] = kGlobal ? (w < W ? __ldcg(row + w) : 0) : row[w];
+              }
+#pragma unroll
+              for (int q = 0; q < kAhead; q++) {
+                const int w = w0 + 32 * q;
+                if (kGlobal && w >= W) break;
+                unsigned y = x[q] | rv[w];
+                if (w == (l >> 5)) y &= ~(1u << (l & 31));
+                if (w == (lv >> 5)) y &= ~(1u << (lv & 31));
+                row[w] = y;
+                pc += __popc(y);
+              }
             }
             pc = __reduce_add_sync(0xffffffffu, pc);
             if (lane == at) deg = pc;
@@ -415,7 +488,7 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
       A.height[u] = hgt[r];
     }
   }
-  if (CS > 1) cluster.sync();  // no CTA leaves while a peer may still read its rows
+  if (!kGrid && CS > 1) cluster.sync();  // no CTA leaves while a peer may still read its rows
 }
 
 // Distinct neighbours of every vertex's input list as ~id and the number of
@@ -558,11 +631,12 @@ bool ElimPlan::plan_bits() {
   // outnumber the SMs keep few warps (1,024 cells of 259 members: 0.54 ms with
   // 4 warps, 0.67 with 8; 2,048 cells of 489: 3.7 with 4, 2.8 with 8, 3.9 with 16).
   cudaFuncAttributes fa;
-  GH_CUDA(cudaFuncGetAttributes(&fa, symbolic_kernel<false>));
-  const int smem_dyn = enable_max_dynamic_smem(symbolic_kernel<false>);
-  enable_max_dynamic_smem(symbolic_kernel<true>);
-  GH_CUDA(cudaFuncSetAttribute(symbolic_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  GH_CUDA(cudaFuncSetAttribute(symbolic_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  GH_CUDA(cudaFuncGetAttributes(&fa, symbolic_kernel<false, false>));
+  const int smem_dyn = enable_max_dynamic_smem(symbolic_kernel<false, false>);
+  enable_max_dynamic_smem(symbolic_kernel<true, false>);
+  const int smem_grid = enable_max_dynamic_smem(symbolic_kernel<true, true>);
+  GH_CUDA(cudaFuncSetAttribute(symbolic_kernel<false, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  GH_CUDA(cudaFuncSetAttribute(symbolic_kernel<true, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   int dev = 0;
   GH_CUDA(cudaGetDevice(&dev));
   GH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -576,7 +650,8 @@ bool ElimPlan::plan_bits() {
     return own * (8 + 24) + 4LL * smax + 4LL * pow2(smax) + 8 * w + (global ? 0 : 4 * own * w);
   };
   std::vector<SymCell> table;
-  int64_t grow_words = 0;
+  int64_t grow_words = 0, grid_best = 0;
+  grid_cells = 0;
   for (int st = 0; st <= nsteps; st++) {
     std::vector<Host> &cells = steps[st];
     std::stable_sort(cells.begin(), cells.end(), [](const Host &a, const Host &b) { return a.c.size > b.c.size; });
@@ -619,8 +694,8 @@ bool ElimPlan::plan_bits() {
           cfg.blockDim = dim3(nw * 32);
           cfg.dynamicSmemBytes = (size_t)sm;
           cfg.gridDim = dim3(L.ncell * cs);
-          const cudaError_t e = global ? cudaOccupancyMaxActiveClusters(&fit, symbolic_kernel<true>, &cfg)
-                                       : cudaOccupancyMaxActiveClusters(&fit, symbolic_kernel<false>, &cfg);
+          const cudaError_t e = global ? cudaOccupancyMaxActiveClusters(&fit, symbolic_kernel<true, false>, &cfg)
+                                       : cudaOccupancyMaxActiveClusters(&fit, symbolic_kernel<false, false>, &cfg);
           if (e != cudaSuccess || fit < 1) {
             cudaGetLastError();
             continue;
@@ -636,7 +711,33 @@ bool ElimPlan::plan_bits() {
             L.global = global != 0;
           }
         }
+      // rows in global memory: a pick reads its neighbours' rows from L2, 11 us of
+      // it with 16 CTAs and 5,940 members, and more CTAs pay for the dearer
+      // barrier (4.8 us a pick with 128)
+      if (L.global || best > 1e299)
+        for (int cs = 32; cs <= 128 && cs * L.ncell <= nsm; cs <<= 1) {
+          const int64_t sm = smem_for(smax, cs, true);
+          const int own = (smax + cs - 1) / cs, w = (smax + 31) / 32, nw = 16;
+          int per_sm = 0;
+          if (sm > smem_grid || (own + 31) / 32 > kMaxGroups) continue;
+          GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, symbolic_kernel<true, true>, nw * 32, (size_t)sm));
+          if (per_sm < 1) continue;
+          const double cost = 3.8 + (1.0 + 4.5e-5 * smax * w) / cs;
+          if (cost < best * 0.99) {
+            best = cost;
+            L.cs = cs;
+            L.nw = nw;
+            L.smem = sm;
+            L.global = L.grid = true;
+          }
+        }
       if (best > 1e299) return false;
+      if (L.grid) {
+        L.best_off = grid_best;
+        L.arrived_off = grid_cells;
+        grid_best += 2 * (int64_t)L.ncell * L.cs;
+        grid_cells += L.ncell;
+      }
       if (L.global) {
         L.rows_off = step_words;
         step_words += (int64_t)L.ncell * smax * ((smax + 31) / 32 | 1);
@@ -658,6 +759,10 @@ bool ElimPlan::plan_bits() {
     extra = mem.get<int>(N);
     sym_cells = mem.get<unsigned char>(sizeof(SymCell) * table.size());
     if (grow_words) grows = mem.get<unsigned>(grow_words);
+    if (grid_cells) {
+      sym_best = mem.get<unsigned long long>(grid_best);
+      sym_arrived = mem.get<unsigned>(grid_cells);
+    }
     for (int i = 0; i < K; i++) {
       const int n = gs[i]->n;
       members_kernel<<<std::max(1, std::min(4096, (n + 255) / 256)), 256>>>(
@@ -678,6 +783,7 @@ void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
   GH_CUDA(cudaMemsetAsync(height, 0, sizeof(int) * N, s));
   GH_CUDA(cudaMemsetAsync(ljunk, 0, sizeof(int) * N, s));
   GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  if (grid_cells) GH_CUDA(cudaMemsetAsync(sym_arrived, 0, sizeof(unsigned) * grid_cells, s));
   distinct_lists_kernel<<<std::max(1, std::min(4096, (N + 255) / 256)), 256, 0, s>>>(adj_off, adj_v, slot_off, pool,
                                                                                      lsize, extra, N);
   GH_CUDA(cudaGetLastError());
@@ -703,12 +809,23 @@ void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
     A.smax = L.smax;
     A.npow = L.npow;
     A.heap = L.heap;
+    if (L.grid) {
+      A.cs = L.cs;
+      A.best = sym_best + L.best_off;
+      A.arrived = sym_arrived + L.arrived_off;
+      A.spin_limit = spin_limit_cycles();
+    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = L.cs;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    if (L.grid) {
+      attr[0].id = cudaLaunchAttributeCooperative;
+      attr[0].val.cooperative = 1;
+    } else {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = L.cs;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.blockDim = dim3(L.nw * 32);
@@ -717,8 +834,9 @@ void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
     cfg.stream = ls;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (trace) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, ls); }
-    if (L.global) GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<true>, A));
-    else GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<false>, A));
+    if (L.grid) GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<true, true>, A));
+    else if (L.global) GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<true, false>, A));
+    else GH_CUDA(cudaLaunchKernelEx(&cfg, symbolic_kernel<false, false>, A));
     if (trace) {
       cudaEventRecord(e1, ls);
       cudaEventSynchronize(e1);
@@ -726,7 +844,7 @@ void ElimPlan::enqueue_bits(cudaStream_t s, cudaEvent_t *heap_ev, bool trace) {
       cudaEventElapsedTime(&ms, e0, e1);
       std::fprintf(stderr, "[gpuh2h] elim bits %s %d: %d cells x %d CTAs x %d warps, kmax %d, members %d, smem %lld%s: %.3f ms\n",
                    L.heap ? "heap" : "level", L.level, L.ncell, L.cs, L.nw, L.kmax, L.smax, (long long)L.smem,
-                   L.global ? " (rows in global memory)" : "", ms);
+                   L.grid ? " (one grid)" : L.global ? " (rows in global memory)" : "", ms);
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
     }
