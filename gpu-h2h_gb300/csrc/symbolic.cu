@@ -881,7 +881,11 @@ bool ElimPlan::grow_pool() {
   pool_size = std::min(most, 4 * pool_size);
   if (std::getenv("GPUH2H_TRACE"))
     std::fprintf(stderr, "[gpuh2h] elim bits: list pool grown to %lld entries\n", (long long)pool_size);
-  GH_CUDA(cudaMalloc(&pool, sizeof(int) * (size_t)pool_size));
+  if (cudaMalloc(&pool, sizeof(int) * (size_t)pool_size) != cudaSuccess) {
+    cudaGetLastError();
+    pool = nullptr;
+    return false;
+  }
   own_pool = true;
   slot_bytes = 4 * pool_size;
   return true;
