@@ -367,11 +367,14 @@ __global__ void long_positions_kernel(PosArgs A, int room) {
 }  // namespace
 
 // A narrow level's blocks are the chain the fill waits for and are cut finely;
-// elsewhere a task is a whole row range, because a task's own start (tables,
-// members, ancestors) costs as much as several steps: 64 / 256-column tasks
-// there took the 1M-vertex fill from 14.8 to 17.4 ms.
+// elsewhere a task's own start (tables, members, ancestors) costs as much as two
+// or three steps, so small separators keep whole rows, but wide ones, whose
+// tasks of 512 columns ran for 200 us each on the critical path, are cut too.
+// Columns by separator up to 16 / 64 / 256 / more, 264k, 1M and 6.26M vertices: 4096 /
+// 4096 / 512 / 128 2.56, 12.2 and 118.8 ms; 4096 / 512 / 128 / 64 2.25, 11.4,
+// 120.3; 4096 / 768 / 192 / 128 2.27, 11.3, 118.3; 1024 / 512 / 128 / 64 2.36, 12.0.
 TilePolicy::TilePolicy() {
-  static const int cb[kWidth][kSep] = {{64, 64, 64, 64}, {4096, 4096, 512, 128}, {4096, 4096, 512, 128}};
+  static const int cb[kWidth][kSep] = {{64, 64, 64, 64}, {4096, 768, 192, 128}, {4096, 768, 192, 128}};
   for (int w = 0; w < kWidth; w++)
     for (int b = 0; b < kSep; b++) {
       small_work[w][b] = 1024;
