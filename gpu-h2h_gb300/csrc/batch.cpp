@@ -114,7 +114,10 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       clk.reset();
       GH_CUDA(cudaEventRecord(b->ev[0], b->stream));
       cudaEvent_t hev[2] = {b->ev[1], b->ev[2]};
-      if (!b->elim->run(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr)) continue;  // the list kernels
+      if (!b->elim->run(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr)) {  // the list kernels
+        b->elim.reset();
+        continue;
+      }
       b->info.t_contract_us = event_us(b->ev[0], b->ev[1]);
       b->info.t_global_us = event_us(b->ev[1], b->ev[2]);
       clk.reset();
@@ -143,6 +146,7 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       b->fill = std::make_unique<gh::FillPlan>(b->gs, b->elim->lists, b->elim.get());
       if (!b->fill->weights_fit) {  // very wide separators: the list kernels, which need no update triangles
         b->fill.reset();
+        b->elim.reset();
         continue;
       }
       b->fill->prepare(pol);
