@@ -32,6 +32,7 @@ struct ListStore {
 struct DeviceInput {
   DeviceArena mem;
   int *off = nullptr, *v = nullptr, *w = nullptr, *part = nullptr, *pos = nullptr;
+  int device = 0;
   ~DeviceInput();
 };
 

@@ -302,6 +302,7 @@ bool parse_input(Graph &g, const char *ids, int64_t ids_size, const char *arcs, 
   Workspace ws;
   QuietStream q;
   auto in = std::make_shared<DeviceInput>();
+  GH_CUDA(cudaGetDevice(&in->device));
   in->mem.reserve(4 * (3 * (size_t)n + 2 * (size_t)m) + 5 * 256 + 256);
   in->off = in->mem.get<int>((int64_t)n + 1);
   in->v = in->mem.get<int>(m);
@@ -396,11 +397,20 @@ bool load_input_gpu(Graph &g, const char *ids, int64_t ids_size, const char *arc
 }
 
 // The graph's input on the device, uploaded from the host reader's arrays if need be.
+// Loading names no device, so a graph may be built on another than it was
+// parsed on.
 const DeviceInput &input_device(Graph &g) {
+  int device = 0;
+  GH_CUDA(cudaGetDevice(&device));
+  if (g.input && g.input->device != device) {
+    input_host(g);
+    g.input.reset();
+  }
   if (!g.input) {
     GH_CHECK((int64_t)g.adj_off.size() == (int64_t)g.n + 1 && (int)g.part_ids.size() == g.n, H2H_ERR_STATE,
              "the input arcs are not loaded");
     auto in = std::make_shared<DeviceInput>();
+    in->device = device;
     in->off = in->mem.get<int>((int64_t)g.n + 1);
     in->v = in->mem.get<int>(g.m);
     in->w = in->mem.get<int>(g.m);
@@ -426,6 +436,7 @@ const HostInput &input_host(const Graph &g) {
   if (g.input && (int64_t)g.adj_off.size() != (int64_t)g.n + 1) {
     const DeviceInput &in = *g.input;
     RelaxedCapture relaxed;
+    OnDevice there(in.device);
     QuietStream q;
     h.adj_v.resize(g.m);
     h.adj_w.resize(g.m);

@@ -18,6 +18,18 @@ struct RelaxedCapture {
   RelaxedCapture &operator=(const RelaxedCapture &) = delete;
 };
 
+// The calling thread's device for a while.
+struct OnDevice {
+  int before = 0;
+  explicit OnDevice(int device) {
+    GH_CUDA(cudaGetDevice(&before));
+    if (device != before) GH_CUDA(cudaSetDevice(device));
+  }
+  ~OnDevice() { cudaSetDevice(before); }
+  OnDevice(const OnDevice &) = delete;
+  OnDevice &operator=(const OnDevice &) = delete;
+};
+
 struct QuietStream {
   cudaStream_t s = nullptr;
   QuietStream() { GH_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
