@@ -31,7 +31,7 @@
 // A fill that takes a warp per (node, column block, separator chunk) tile is
 // bound by one L2 load per update and 13 us per tree level of the narrow top.
 // On one GB300 the blocks took the fill of a 264k-vertex road graph (4.5e9
-// updates) from 28.4 to 2.4 ms and of a 1M-vertex one (3.8e10) from 104 to 12.1
+// updates) from 28.4 to 2.1 ms and of a 1M-vertex one (3.8e10) from 104 to 11.1
 // ms.  Narrow levels are a chain of blocks (about 22 us each, a step of 32
 // members 3,100 clocks); below them a term costs an ALU slot of half rate and the
 // kernel fills over half of those slots.
@@ -963,8 +963,8 @@ struct FillKernelArgs {
   unsigned long long *trace_t;  // non-null (GPUH2H_TRACE): each node's publish time, ns
 };
 
-// A CTA of four warps takes tasks (a block, a range of columns) in the order
-// of the blocks' depths, waits for the father block's flag, and sweeps its
+// A CTA of four warps takes tasks (a block, a range of columns) in block
+// order, waits for the father block's flag, and sweeps its
 // columns 64 at a time and the top's members 32 at a time: the second factor
 // E goes through registers into shared memory one step ahead (so a step's
 // loads overlap the product before it), every thread owns a 4 x 4 patch of
@@ -977,7 +977,8 @@ struct FillKernelArgs {
 // ancestor's row at neighbouring positions.  The product holds the next
 // member's operands while it sums: with 57 clocks a member for 32 of sums it
 // was the longest part of a narrow step.  1M-vertex graph: 12.9 ms with one
-// mapping of loads and without the operands ahead, 12.1 with both; each alone
+// mapping of loads and without the operands ahead, 12.1 with both (with the tasks
+// and the block order of the time); each alone
 // gains nothing.
 // Five CTAs per SM (four: 12.3 ms; six hold 80 registers and spill).  Loads two
 // or three steps ahead, with 128 registers, gain nothing: a step waits 270
