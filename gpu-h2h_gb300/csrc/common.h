@@ -53,11 +53,14 @@ inline int enable_max_dynamic_smem(K kernel) {
 
 // Bound on one spin-wait of a kernel (a dependency or a barrier), in SM clock
 // cycles: 2 s at 2 GHz, or GPUH2H_SPIN_LIMIT_MS (profilers replay
-// instrumented kernels much slower).
+// instrumented kernels much slower; a fraction lets a wait run out on purpose).
 inline long long spin_limit_cycles() {
-  long long ms = 2000;
-  if (const char *e = std::getenv("GPUH2H_SPIN_LIMIT_MS")) ms = std::max(1LL, std::atoll(e));
-  return ms * 2000000LL;
+  double ms = 2000;
+  if (const char *e = std::getenv("GPUH2H_SPIN_LIMIT_MS")) {
+    ms = std::atof(e);
+    ms = ms > 0 ? std::max(1e-3, std::min(ms, 1e12)) : 1;
+  }
+  return (long long)(ms * 2e6);
 }
 
 inline int ilog2_floor(int64_t x) {  // floor(log2(x)) for x >= 1; equals (int)log2((double)x)

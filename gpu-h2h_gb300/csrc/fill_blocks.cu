@@ -1470,7 +1470,7 @@ BlockArgs block_args(const FillPlan &P) {
   B.closed = P.closed;
   B.anc = P.blk_anc;
   B.nblk = P.nblk;
-  B.err = P.err;
+  B.err = P.werr;  // the fill's own word is set where it is launched
   return B;
 }
 
@@ -1504,7 +1504,7 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   GH_CHECK(wtasks < INT32_MAX, H2H_ERR_ARG, "too many weight tasks");
   wtask_blk = work.get<int>(wtasks);
   expand_tasks_kernel<<<gw, 256>>>(wtask0, wtask_blk, nblk);
-  GH_CUDA(cudaMemset(err, 0, sizeof(int)));
+  GH_CUDA(cudaMemset(werr, 0, sizeof(int)));
   GH_CUDA(cudaMemset(pend_init, 0, sizeof(int) * nblk));
   parent_columns_kernel<<<gw, 256>>>(B, wtask0, blk_up, bm_up, pend_init);
   update_sizes_kernel<<<gb, 256>>>(blk_mem, pend_init, ucells, nblk);
@@ -1523,13 +1523,13 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   }
   arc_cells_kernel<<<grid_for(N, nsm), 256>>>(B, from.adj_off, from.adj_v, global, arc_cell, N);
   GH_CUDA(cudaGetLastError());
-  GH_CHECK(read_one(err) == 0, H2H_ERR_STATE, "an upper neighbour is missing from its block's separator");
+  GH_CHECK(read_one(werr) == 0, H2H_ERR_STATE, "an upper neighbour is missing from its block's separator");
 }
 
 void FillPlan::enqueue_weights(cudaStream_t s) {
   const BlockArgs B = block_args(*this);
   const int gn = std::max(1, std::min(8192, (N + 7) / 8));  // a warp per vertex
-  GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  GH_CUDA(cudaMemsetAsync(werr, 0, sizeof(int), s));
   const int gi = (nblk + kClosureWarps - 1) / kClosureWarps;
   if (!arcs) {  // the lists carry the weights
     gather_pos_weights_kernel<<<gn, 256, 0, s>>>(pos_hash, pos_src, lists.off, lists.w, pos_w, N);
@@ -1637,6 +1637,7 @@ void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
   GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   FillKernelArgs A{};
   A.B = block_args(*this);
+  A.B.err = err;
   A.dis = dis;
   A.hld_row = hld_row;
   A.seg_off = seg_off;

@@ -332,7 +332,10 @@ struct FillPlan {
   int *hld = nullptr, *htop = nullptr, *hpos = nullptr, *seg_top = nullptr, *seg_pos = nullptr;
   int64_t *hld_row = nullptr;
   int64_t *seg_off = nullptr;
-  int *done = nullptr, *next = nullptr, *err = nullptr, *tasks = nullptr;  // tasks: task -> block
+  int *done = nullptr, *next = nullptr, *tasks = nullptr;  // tasks: task -> block
+  // error words of the fill and of the weights, side by side: a rebuild runs
+  // both and then looks once, so neither clears the other's
+  int *err = nullptr, *werr = nullptr;
   // the blocks (fill_blocks.cu): top, separator size, first node / member /
   // cell of the weight tables per block; node lists and places; members'
   // positions and row offsets; direct and closed weights; first task and
@@ -383,7 +386,7 @@ struct FillPlan {
   void enqueue_weights(cudaStream_t s);
   // Resets the flags and runs the fill on s.
   void enqueue(cudaStream_t s, cudaEvent_t *fill_ev = nullptr);
-  void check_error();            // synchronises; throws if a dependency wait ran out
+  void check_error();            // synchronises; throws if a wait of the weights or of the fill ran out
   void trace_report();           // GPUH2H_TRACE: the last fill's time per level class
   void attach(bool first);       // per-graph views; first: of new arrays
 };

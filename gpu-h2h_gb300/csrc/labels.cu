@@ -454,7 +454,9 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
     seg_top = work.get<int>(std::max<int64_t>(seg_total, 1));
     seg_pos = work.get<int>(std::max<int64_t>(seg_total, 1));
     next = work.get<int>(1);
-    err = work.get<int>(1);
+    err = work.get<int>(2);
+    werr = err + 1;
+    GH_CUDA(cudaMemset(err, 0, 2 * sizeof(int)));
     hld_row = work.get<int64_t>(N);
     hld_row_kernel<<<std::max(1, std::min(8192, (N + 255) / 256)), 256>>>(hld, drow, hld_row, N);
     GH_CUDA(cudaGetLastError());
@@ -467,7 +469,6 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
       DeviceArena ws;
       PosArgs A{lists.off, lists.id, from && from->bits ? nullptr : lists.w, depth, pos_hash, pos_pos, pos_id, pos_w,
                 pos_src, ws.get<int>(N), ws.get<int>(1), err};
-      GH_CUDA(cudaMemset(err, 0, sizeof(int)));
       GH_CUDA(cudaMemset(A.count, 0, sizeof(int)));
       short_positions_kernel<<<std::max(1, std::min(nsm * 8, (N + 7) / 8)), 256>>>(A, N);
       if (max_m > 31) long_positions_kernel<<<std::max(1, std::min(N, nsm * 16)), 128, ksmem>>>(A, room);
@@ -506,7 +507,7 @@ void FillPlan::release_work() {
   for (void *p : {(void *)tasks, (void *)mbuf, (void *)trace_t}) cudaFree(p);
   grown_bytes = tasks_cap = mslots_cap = 0;
   trace_t = nullptr;
-  pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = tasks = nullptr;
+  pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = werr = tasks = nullptr;
   blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;
   hld_row = seg_off = blk_boff = blk_moff = blk_soff = bm_row = task0 = nullptr;
   loc_of = nullptr;
@@ -559,9 +560,10 @@ void FillPlan::trace_report() {
 
 void FillPlan::check_error() {
   GH_CUDA(cudaDeviceSynchronize());
-  int kerr = 0;
-  GH_CUDA(cudaMemcpy(&kerr, err, sizeof(int), cudaMemcpyDeviceToHost));
-  GH_CHECK(kerr == 0, H2H_ERR_DEVICE, "label fill: a dependency wait ran out (error code " + std::to_string(kerr) + ")");
+  int e[2] = {0, 0};  // err, werr
+  GH_CUDA(cudaMemcpy(e, err, sizeof(e), cudaMemcpyDeviceToHost));
+  GH_CHECK(e[1] == 0, H2H_ERR_DEVICE, "block weights: a dependency wait ran out (error code " + std::to_string(e[1]) + ")");
+  GH_CHECK(e[0] == 0, H2H_ERR_DEVICE, "label fill: a dependency wait ran out (error code " + std::to_string(e[0]) + ")");
 }
 
 void FillPlan::attach(bool first) {
