@@ -14,6 +14,19 @@
 
 namespace gh {
 
+// One allocation of n elements.  Without room the CUDA error is cleared before
+// the exception leaves, so that no later check trips over it.
+template <typename T>
+T *device_array(int64_t n) {
+  void *p = nullptr;
+  const cudaError_t e = cudaMalloc(&p, (size_t)std::max<int64_t>(n, 1) * sizeof(T));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
+  return static_cast<T *>(p);
+}
+
 class DeviceArena {
  public:
   DeviceArena() = default;
@@ -62,14 +75,9 @@ class DeviceArena {
 
  private:
   char *chunk(size_t size) {
-    void *p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, size);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    }
+    char *p = device_array<char>((int64_t)size);
     chunks_.push_back(p);
-    return static_cast<char *>(p);
+    return p;
   }
   std::vector<void *> chunks_;
   char *cur_ = nullptr;

@@ -1240,16 +1240,6 @@ struct ListArrays {
   DeviceArena mem;
 };
 
-template <typename T>
-T *dalloc(size_t n) {
-  T *p = nullptr;
-  if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) cudaGetLastError();
-  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  return p;
-}
-
 }  // namespace
 
 namespace {
@@ -1326,7 +1316,7 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
       // have took 4 GB there, and their cudaMalloc and cudaFree 3.5 ms.)
       pool_size = std::min<int64_t>(2 * (slots_size + 4), M + 192 * (int64_t)N + (1 << 16));
       own_pool = pool_size >= (int64_t(2) << 20);
-      pool = own_pool ? dalloc<int>(pool_size) : mem.get<int>(pool_size);
+      pool = own_pool ? device_array<int>(pool_size) : mem.get<int>(pool_size);
       slot_bytes = own_pool ? 4 * pool_size : 0;
     } else {
       pool_size = slots_size;

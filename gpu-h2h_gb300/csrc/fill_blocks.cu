@@ -39,6 +39,7 @@
 #include <climits>
 #include <cstdio>
 #include <cstdlib>
+#include <utility>
 
 #include "graph.h"
 #include "scan.h"
@@ -57,16 +58,6 @@ constexpr unsigned kInf = 0x7fffffffu;
 
 constexpr int kErrWait = 4;    // a dependency wait ran out
 constexpr int kErrNested = 6;  // an upper neighbour is missing from the block top's separator
-
-template <typename T>
-T *dalloc(size_t n, int64_t &bytes) {
-  T *p = nullptr;
-  if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  bytes += (int64_t)(n * sizeof(T));
-  return p;
-}
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *global) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global)
@@ -1582,56 +1573,66 @@ std::vector<int> FillPlan::level_classes() const {
   return cls;
 }
 
-// Tasks in block order, cut as the policy says.
+// Tasks in block order, cut as the policy says.  The new tables are made beside
+// the old ones and take their place once nothing can fail any more: without room
+// the plan keeps its policy and its tasks.
 void FillPlan::build_tiles(const TilePolicy &pol) {
-  policy = pol;
   Workspace ws;
   int *ntask = ws.get<int>(nblk + 1), *pieces = ws.get<int>(nblk + 1), *several = ws.get<int>(nblk + 1);
-  int64_t *piece0 = ws.get<int64_t>(nblk + 1), *slot0 = ws.get<int64_t>(nblk + 1);
-  if (!task0) {
-    task0 = work.get<int64_t>(nblk + 1);
-    tcols = work.get<int>(nblk + 1);
-    mslot = work.get<int>(nblk + 1);
-  }
+  int64_t *piece0 = ws.get<int64_t>(nblk + 1), *slot0 = ws.get<int64_t>(nblk + 1), *new_task0 = ws.get<int64_t>(nblk + 1);
+  int *new_tcols = ws.get<int>(nblk + 1);
   block_tasks_kernel<<<grid_for(nblk + 1, nsm), 256>>>(blk_top, depth, blk_mem, blk_boff, lvl_cls, pol, ntask, pieces,
-                                                            tcols, several, nblk);
+                                                            new_tcols, several, nblk);
   GH_CUDA(cudaGetLastError());
-  exclusive_scan<int>(ntask, task0, nblk + 1, ws, 0);
+  exclusive_scan<int>(ntask, new_task0, nblk + 1, ws, 0);
   exclusive_scan<int>(pieces, piece0, nblk + 1, ws, 0);
   exclusive_scan<int>(several, slot0, nblk + 1, ws, 0);
+  const int64_t new_ntasks = read_one(new_task0 + nblk), new_mslots = read_one(slot0 + nblk),
+                new_ntiles = read_one(piece0 + nblk);
+  GH_CHECK(new_ntasks >= nblk && new_ntasks < INT32_MAX, H2H_ERR_ARG, "too many fill tasks");
+  const int smem_dyn = enable_max_dynamic_smem(block_fill_kernel);
+  const size_t new_smem = 2 * sizeof(int) * (size_t)std::max(max_segs, 1);
+  GH_CHECK(new_smem <= (size_t)smem_dyn, H2H_ERR_DEVICE, "tree too large for the fill staging");
+  int per_sm = 0;
+  GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_fill_kernel, 128, new_smem));
+  if (!task0) {
+    int64_t *t0 = work.get<int64_t>(nblk + 1);
+    tcols = work.get<int>(nblk + 1);
+    mslot = work.get<int>(nblk + 1);
+    task0 = t0;
+  }
+  // the buffers that grow: all of them before any is replaced
+  struct Grown {
+    void *p = nullptr;
+    ~Grown() { cudaFree(p); }
+  } new_mbuf, new_tasks;
+  if (new_mslots > mslots_cap) new_mbuf.p = device_array<unsigned>(new_mslots * kRows * kRows);
+  if (new_ntasks > tasks_cap) new_tasks.p = device_array<int>(new_ntasks);
+  if (new_mbuf.p) {
+    grown_bytes += (new_mslots - mslots_cap) * kRows * kRows * 4;
+    mslots_cap = new_mslots;
+    new_mbuf.p = std::exchange(mbuf, static_cast<unsigned *>(new_mbuf.p));
+  }
+  if (new_tasks.p) {
+    grown_bytes += (new_ntasks - tasks_cap) * 4;
+    tasks_cap = new_ntasks;
+    new_tasks.p = std::exchange(tasks, static_cast<int *>(new_tasks.p));
+  }
+  GH_CUDA(cudaMemcpyAsync(task0, new_task0, sizeof(int64_t) * (nblk + 1), cudaMemcpyDeviceToDevice));
+  GH_CUDA(cudaMemcpyAsync(tcols, new_tcols, sizeof(int) * (nblk + 1), cudaMemcpyDeviceToDevice));
   narrow_kernel<<<grid_for(nblk + 1, nsm), 256>>>(slot0, mslot, nblk + 1);
-  GH_CUDA(cudaGetLastError());
-  ntasks = read_one(task0 + nblk);
-  mslots = read_one(slot0 + nblk);
-  if (mslots > mslots_cap) {
-    cudaFree(mbuf);
-    mbuf = nullptr;
-    grown_bytes -= mslots_cap * kRows * kRows * 4;
-    mslots_cap = 0;
-    mbuf = dalloc<unsigned>(mslots * kRows * kRows, grown_bytes);
-    mslots_cap = mslots;
-  }
-  ntiles = read_one(piece0 + nblk);
-  GH_CHECK(ntasks >= nblk && ntasks < INT32_MAX, H2H_ERR_ARG, "too many fill tasks");
-  if (ntasks > tasks_cap) {
-    cudaFree(tasks);
-    tasks = nullptr;
-    grown_bytes -= tasks_cap * 4;
-    tasks_cap = 0;
-    tasks = dalloc<int>(ntasks, grown_bytes);
-    tasks_cap = ntasks;
-  }
   expand_tasks_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(task0, tasks, nblk);
   GH_CUDA(cudaGetLastError());
-  const int smem_dyn = enable_max_dynamic_smem(block_fill_kernel);
-  smem = 2 * sizeof(int) * (size_t)std::max(max_segs, 1);
-  GH_CHECK(smem <= (size_t)smem_dyn, H2H_ERR_DEVICE, "tree too large for the fill staging");
-  int per_sm = 0;
-  GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_fill_kernel, 128, smem));
+  policy = pol;
+  ntasks = new_ntasks;
+  mslots = new_mslots;
+  ntiles = new_ntiles;
+  smem = new_smem;
   blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * std::max(1, per_sm), ntasks));
 }
 
 void FillPlan::enqueue(cudaStream_t s, cudaEvent_t *fill_ev) {
+  GH_CHECK(ntasks > 0 && tasks && (mbuf || !mslots), H2H_ERR_STATE, "the fill's tasks are not laid out");
   GH_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * 2 * (int64_t)nblk, s));
   GH_CUDA(cudaMemsetAsync(next, 0, sizeof(int), s));
   GH_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));

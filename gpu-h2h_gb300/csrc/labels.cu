@@ -57,11 +57,8 @@ namespace {
 
 template <typename T>
 T *dalloc(size_t n, int64_t &bytes) {
-  T *p = nullptr;
-  if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) throw Error(H2H_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  bytes += (int64_t)(n * sizeof(T));
+  T *p = device_array<T>((int64_t)n);
+  bytes += (int64_t)(std::max<size_t>(n, 1) * sizeof(T));
   return p;
 }
 
@@ -505,7 +502,7 @@ void FillPlan::release_work() {
   work.release();
   layout.reset();
   for (void *p : {(void *)tasks, (void *)mbuf, (void *)trace_t}) cudaFree(p);
-  grown_bytes = tasks_cap = mslots_cap = 0;
+  grown_bytes = tasks_cap = mslots_cap = ntasks = mslots = 0;
   trace_t = nullptr;
   pos_w = pos_src = hld = htop = hpos = seg_top = seg_pos = done = next = err = werr = tasks = nullptr;
   blk_top = blk_mem = bnode = blk_of = lvl_cls = bm_p = tcols = nullptr;
@@ -638,12 +635,7 @@ std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
   cudaEvent_t ev[2];
   GH_CUDA(cudaEventCreate(&ev[0]));
   GH_CUDA(cudaEventCreate(&ev[1]));
-  auto time_policy = [&](const TilePolicy &p) -> float {
-    try {
-      plan.build_tiles(p);
-    } catch (const Error &) {
-      return 1e30f;  // staging does not fit: not a candidate
-    }
+  auto time_fill = [&]() -> float {
     float best = 1e30f;
     for (int rep = 0; rep < 2; rep++) {
       plan.enqueue(s, ev);
@@ -654,12 +646,21 @@ std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
     }
     return best;
   };
+  auto time_policy = [&](const TilePolicy &p) -> float {
+    try {
+      plan.build_tiles(p);
+    } catch (const Error &) {
+      return 1e30f;  // no room for its tasks: not a candidate
+    }
+    return time_fill();
+  };
   static const int kSmall[] = {0, 1 << 10, 1 << 12, 1 << 14, 1 << 16, 1 << 20};
   static const int kCols[] = {64, 128, 256, 512, 1024, 4096};
   TilePolicy best = plan.policy;
   float best_ms = 0;
   try {
-    best_ms = time_policy(best);
+    plan.build_tiles(best);
+    best_ms = time_fill();
     for (int r = 0; r < rounds; r++)
       for (int wb = 0; wb < TilePolicy::kWidth; wb++)
         for (int sb = 0; sb < TilePolicy::kSep; sb++) {
@@ -679,7 +680,8 @@ std::string tile_policy_tune(FillPlan &plan, cudaStream_t s, int rounds) {
             if (t < best_ms * 0.98f) { best = p; best_ms = t; }
           }
         }
-    time_policy(best);  // leaves the tiles and the labels of the chosen policy
+    plan.build_tiles(best);  // leaves the tasks and the labels of the chosen policy
+    time_fill();
   } catch (...) {
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
