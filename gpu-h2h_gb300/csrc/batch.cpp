@@ -74,6 +74,15 @@ long long event_us(cudaEvent_t a, cudaEvent_t b) {
   return (long long)(ms * 1000.0f);
 }
 
+// A batch that fails on the way leaves its graphs as they were loaded: without
+// weights, lists and tree are no contraction to go on from.
+struct Unfinished {
+  std::vector<gh::Graph *> gs;
+  ~Unfinished() {
+    for (gh::Graph *g : gs) g->drop_build();
+  }
+};
+
 void copy_policy(const std::string &p, char *out, int cap) {
   if (!out || cap <= 0) return;
   const size_t n = std::min<size_t>(p.size(), (size_t)cap - 1);
@@ -102,6 +111,7 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       b->gs.push_back(&g);
     }
     gh::Clock total, clk;
+    Unfinished unfinished{b->gs};
     gh::build_elimination_sets(b->gs);
     b->info.t_sets_us = clk.us();
     clk.reset();
@@ -132,7 +142,6 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       gh::build_tree_gpu(b->gs);
       gh::build_rmq_gpu(b->gs);
       for (gh::Graph *g : b->gs) {
-        g->contracted = true;
         g->parallel_fine = 2;
         g->construct_device = 1;
         g->label_mode = H2H_LABEL_L4;
@@ -167,11 +176,12 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       for (gh::Graph *g : b->gs) {
         gh::upload_query_index(*g);
         g->sets.reset();
-        g->labelled = true;
       }
       b->info.t_attach_us = clk.us();
       break;
     }
+    unfinished.gs.clear();
+    for (gh::Graph *g : b->gs) g->contracted = g->labelled = true;
     b->info.t_total_us = total.us();
     b->fill_info();
     *out = b.release();

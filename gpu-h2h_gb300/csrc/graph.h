@@ -173,6 +173,9 @@ struct Graph : HostInput {
   std::shared_ptr<struct FillPlan> plan;  // blocks and weights made by the contraction, until the labels are built
   Timings t;
 
+  // After a contraction or a batch that failed on the way: what it had made is
+  // freed, and the graph is as it was loaded.
+  void drop_build();
   ~Graph() { dev.release(); }
 };
 

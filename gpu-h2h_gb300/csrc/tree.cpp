@@ -10,6 +10,20 @@
 
 namespace gh {
 
+void Graph::drop_build() {
+  plan.reset();
+  tree.reset();
+  sets.reset();
+  dev.release();
+  for (std::vector<int> *v : {&elim, &x_id, &x_w, &father, &depth, &first, &pos_id, &pos_pos, &pos_w, &tree_bfs, &tree_hash})
+    std::vector<int>().swap(*v);
+  for (std::vector<int64_t> *v : {&x_off, &dis_hash, &pos_hash, &drow_host}) std::vector<int64_t>().swap(*v);
+  head = -1;
+  tree_height = n_levels = gpu_vertices = 0;
+  x_total = decomposition_size = euler_n = h2h_size = rmq_total = pos_n = updates = row0 = row1 = 0;
+  contracted = labelled = false;
+}
+
 void allocate_labels_and_bfs(Graph &g) {
   Clock clk;
   const int n = g.n;

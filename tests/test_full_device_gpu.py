@@ -39,3 +39,34 @@ def test_policy_without_room_keeps_the_tasks(tmp_path):
     assert np.array_equal(g.labels()["dis"], want)
     b.close()
     g.close()
+
+
+@pytest.mark.parametrize("room_mb", (100, 220, 400))
+def test_failed_batch_leaves_loaded_graphs(tmp_path, room_mb):
+    """The batch fails in its elimination, with its lists made but not their
+    weights, and at its label rows."""
+    import gpuh2h
+    files = _road(tmp_path, 70000, 9)
+    ref = gpuh2h.Graph("r", 9, 2, 2, 1, files=files).contraction_noHub(1).constructLabel_noHub()
+    want, adj = ref.labels()["dis"], ref.adj()
+    ref.close()
+    gs = [gpuh2h.Graph("r", 9, 2, 2, 1, files=files) for _ in range(2)]
+    with device_room(room_mb << 20):
+        with pytest.raises(gpuh2h.H2HError) as e:
+            gpuh2h.Batch(gs)
+        assert e.value.code == -6
+    for g in gs:
+        for call in (g.order, g.adj, g.constructLabel_noHub):
+            with pytest.raises(gpuh2h.H2HError) as e:
+                call()
+            assert e.value.code == -4
+        assert g.info()["pos_size"] == 0 and g.info()["device_bytes"] == 0
+    gs[0].contraction_noHub(1)
+    assert all(np.array_equal(a, b) for a, b in zip(gs[0].adj(), adj))
+    gs[0].constructLabel_noHub()
+    assert np.array_equal(gs[0].labels()["dis"], want)
+    b = gpuh2h.Batch(gs[1:])
+    assert np.array_equal(gs[1].labels()["dis"], want)
+    b.close()
+    for g in gs:
+        g.close()
