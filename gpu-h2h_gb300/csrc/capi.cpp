@@ -1,6 +1,8 @@
 // capi.cpp -- the extern "C" entry points of include/gpuh2h.h and
 // include/gpuh2h_tools.h.  Every call converts internal exceptions into a
 // status code and a per-thread message; nothing exits the process.
+#include <cuda.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -11,6 +13,7 @@
 #include "gpuh2h_tools.h"
 #include "handle.h"
 #include "pool.h"
+#include "span.h"
 
 namespace gh {
 void write_partition_rate(const Graph &g, const std::string &dir);
@@ -22,6 +25,32 @@ const char *partition_file_prefix(int method);
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
 const std::string &last_error() { return g_last_error; }
+
+int *mapped_ints(const int *p, int64_t n, cudaMemoryType *type) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    *type = cudaMemoryTypeUnregistered;
+    return nullptr;
+  }
+  *type = a.type;
+  if (n <= 0 || a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+  // the range p belongs to: the runtime tells the kind of its first byte only
+  using Attributes = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+  static const Attributes attributes = [] {
+    void *f = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault) != cudaSuccess)
+      cudaGetLastError();
+    return reinterpret_cast<Attributes>(f);
+  }();
+  unsigned long long start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *to[2] = {&start, &size};
+  const auto at = reinterpret_cast<uintptr_t>(p);
+  if (!attributes || attributes(2, what, to, (CUdeviceptr)at) != CUDA_SUCCESS) return nullptr;
+  return ints_inside(at, n, start, size) ? static_cast<int *>(a.devicePointer) : nullptr;
+}
 
 }  // namespace gh
 
@@ -189,16 +218,6 @@ int h2h_build_labels(h2h_graph *h, int parallel_fine, int use_gpu_construct, int
   });
 }
 
-// Device address of page-locked host memory, nullptr for any other memory.
-static int *mapped_address(const int *p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return a.type == cudaMemoryTypeHost ? static_cast<int *>(a.devicePointer) : nullptr;
-}
-
 // Whether the answers may be written while pairs are still read: a query reads
 // its own pair before it writes its own answer, so only a shifted overlap is
 // a conflict.
@@ -280,9 +299,10 @@ int h2h_query_batch_host(const h2h_graph *hc, const int *x, const int *y, int *o
     const bool small = n <= kSmall;
     int *mx = nullptr, *my = nullptr, *mo = nullptr;
     if (!small && in_place_safe(x, out, n) && in_place_safe(y, out, n)) {
-      mx = mapped_address(x);
-      my = mx ? mapped_address(y) : nullptr;
-      mo = my ? mapped_address(out) : nullptr;
+      cudaMemoryType type;
+      mx = gh::mapped_ints(x, n, &type);
+      my = mx ? gh::mapped_ints(y, n, &type) : nullptr;
+      mo = my ? gh::mapped_ints(out, n, &type) : nullptr;
     }
     if (small || mo) {
       if (!s.pin) {

@@ -12,6 +12,12 @@ namespace gh {
 void set_last_error(const std::string &msg);
 const std::string &last_error();
 
+// Device address of the n ints at p when one page-locked allocation or
+// registration holds all of them and they are aligned, so that a kernel may use
+// them in place; nullptr otherwise, or for n = 0.  *type: what kind of memory p
+// points to.
+int *mapped_ints(const int *p, int64_t n, cudaMemoryType *type);
+
 // Host-buffer query staging owned by a handle.
 struct HostQueryStage {
   std::mutex mu;

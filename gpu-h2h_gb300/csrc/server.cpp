@@ -35,20 +35,6 @@ double now_us() {
   return duration<double, std::micro>(steady_clock::now().time_since_epoch()).count();
 }
 
-// cudaMemoryTypeHost for page-locked memory, Unregistered for pageable
-// memory, Device / Managed for memory the server does not take; *dev receives
-// the device address of page-locked memory.
-cudaMemoryType memory_type(const void *p, int **dev) {
-  *dev = nullptr;
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return cudaMemoryTypeUnregistered;
-  }
-  if (a.type == cudaMemoryTypeHost) *dev = static_cast<int *>(a.devicePointer);
-  return a.type;
-}
-
 // A piece of at least this many pairs in page-locked buffers is a launch of
 // its own on them; smaller ones are gathered in the slot's staging.
 constexpr int64_t kDirectPairs = 4096;
@@ -61,7 +47,7 @@ struct Request {
   int64_t n = 0;
   int64_t next = 0;      // first pair not yet placed in a batch
   int64_t remaining = 0; // pairs not yet answered
-  int *dx = nullptr, *dy = nullptr, *dout = nullptr;  // device addresses when all three buffers are page-locked
+  int *dx = nullptr, *dy = nullptr, *dout = nullptr;  // device addresses when all three buffers can be used in place
   double t_submit = 0, t_done = 0;
   bool done = false;
 };
@@ -337,8 +323,10 @@ int h2h_server_submit(h2h_server *s, int graph_id, const int *x, const int *y, i
     GH_CHECK(mode == H2H_QUERY_LCA || mode == H2H_QUERY_NOLCA, H2H_ERR_ARG, "mode must be 0 (LCA) or 1 (noLCA)");
     GH_CHECK(n >= 1, H2H_ERR_ARG, "a request holds at least one pair");
     GH_CHECK(x && y && out, H2H_ERR_ARG, "null buffer");
-    int *dx, *dy, *dout;
-    const cudaMemoryType tx = memory_type(x, &dx), ty = memory_type(y, &dy), to = memory_type(out, &dout);
+    cudaMemoryType tx, ty, to;  // Device / Managed: memory the server does not take
+    const int64_t direct = n >= kDirectPairs ? n : 0;
+    int *dx = gh::mapped_ints(x, direct, &tx), *dy = gh::mapped_ints(y, direct, &ty);
+    int *dout = gh::mapped_ints(out, direct, &to);
     for (cudaMemoryType t : {tx, ty, to})
       GH_CHECK(t == cudaMemoryTypeHost || t == cudaMemoryTypeUnregistered, H2H_ERR_ARG,
                "the server takes host buffers (pageable or page-locked)");
