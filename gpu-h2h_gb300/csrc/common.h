@@ -22,9 +22,11 @@ void set_last_error(const std::string &msg);
 #define GH_CUDA(call)                                                                              \
   do {                                                                                             \
     cudaError_t e_ = (call);                                                                       \
-    if (e_ != cudaSuccess)                                                                         \
+    if (e_ != cudaSuccess) {                                                                       \
+      cudaGetLastError(); /* reported here, not once more by the next check */                     \
       throw ::gh::Error(H2H_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_) + " (" + \
                                           __FILE__ + ":" + std::to_string(__LINE__) + ")");        \
+    }                                                                                              \
   } while (0)
 
 struct Clock {

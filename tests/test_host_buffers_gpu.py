@@ -85,3 +85,4 @@ def test_page_locked_in_part(graph):
     finally:
         for p in base:
             rt.cudaHostUnregister(p)
+    assert np.array_equal(g.query(x, y), want)  # a refused copy is no error of the next call
