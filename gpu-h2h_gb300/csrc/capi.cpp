@@ -225,58 +225,8 @@ static bool in_place_safe(const int *in, const int *out, int64_t n) {
   return in == out || in + n <= out || out + n <= in;
 }
 
-static int single_query(const h2h_graph *h, int x, int y, int mode) {
-  if (!h) { gh::set_last_error("null handle"); return -1; }
-  int res = -1;
-  int rc = guarded([&] {
-    const gh::Graph &g = h->g;
-    GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
-    GH_CHECK(x >= 0 && x < g.n && y >= 0 && y < g.n, H2H_ERR_ARG, "vertex out of range");
-    int out = 0;
-    GH_CHECK(h2h_query_batch_host(h, &x, &y, &out, 1, mode) == H2H_OK, H2H_ERR_CUDA, gh::last_error());
-    res = out;
-  });
-  return rc == H2H_OK ? res : -1;
-}
-
-int h2h_query_lca_nohub(const h2h_graph *h, int x, int y) { return single_query(h, x, y, H2H_QUERY_LCA); }
-int h2h_query_nolca_nohub(const h2h_graph *h, int x, int y) { return single_query(h, x, y, H2H_QUERY_NOLCA); }
-
-int h2h_query_batch(const h2h_graph *h, const int *x_dev, const int *y_dev, int *out_dev, int64_t n, int mode,
-                    void *stream) {
-  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
-  return guarded([&] {
-    const gh::Graph &g = h->g;
-    GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
-    GH_CHECK(mode == H2H_QUERY_LCA || mode == H2H_QUERY_NOLCA, H2H_ERR_ARG, "mode must be 0 (LCA) or 1 (noLCA)");
-    GH_CHECK(n >= 0, H2H_ERR_ARG, "negative batch size");
-    GH_CHECK(n == 0 || (x_dev && y_dev && out_dev), H2H_ERR_ARG, "null buffer");
-    gh::run_query_batch(g, x_dev, y_dev, out_dev, n, mode, (cudaStream_t)stream);
-  });
-}
-
-int h2h_query_batch_plain(const h2h_graph *h, const int *x_dev, const int *y_dev, int *out_dev, int64_t n, int mode,
-                          void *stream) {
-  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
-  return guarded([&] {
-    GH_CHECK(h->g.labelled, H2H_ERR_STATE, "labels not built");
-    GH_CHECK(mode == H2H_QUERY_LCA || mode == H2H_QUERY_NOLCA, H2H_ERR_ARG, "mode must be 0 (LCA) or 1 (noLCA)");
-    GH_CHECK(n == 0 || (x_dev && y_dev && out_dev), H2H_ERR_ARG, "null buffer");
-    gh::run_query_batch_plain(h->g, x_dev, y_dev, out_dev, n, mode, (cudaStream_t)stream);
-  });
-}
-
-int h2h_fill_labels_plain(const h2h_graph *h, double *ms, int64_t *mismatches) {
-  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
-  return guarded([&] { gh::fill_labels_plain(h->g, 0, ms, mismatches); });
-}
-
-int h2h_fill_labels_plain_node(const h2h_graph *h, double *ms, int64_t *mismatches) {
-  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
-  return guarded([&] { gh::fill_labels_plain(h->g, 1, ms, mismatches); });
-}
-
-int h2h_query_batch_host(const h2h_graph *hc, const int *x, const int *y, int *out, int64_t n, int mode) {
+// own: the buffers are this library's, not the caller's.
+static int host_batch(const h2h_graph *hc, const int *x, const int *y, int *out, int64_t n, int mode, bool own) {
   if (!hc) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
   h2h_graph *h = const_cast<h2h_graph *>(hc);
   return guarded([&] {
@@ -296,7 +246,12 @@ int h2h_query_batch_host(const h2h_graph *hc, const int *x, const int *y, int *o
     // the kernel streams 12 bytes a pair over the host link while it runs (2e6
     // pairs on a 264k-vertex graph 975 us, 1,050 with overlapped copies).
     constexpr int64_t kSmall = gh::HostQueryStage::kSmall;
-    const bool small = n <= kSmall;
+    auto on_host = [](const int *p) {  // device memory is the copies' below to refuse
+      cudaMemoryType type;
+      gh::mapped_ints(p, 0, &type);
+      return type != cudaMemoryTypeDevice;
+    };
+    const bool small = n <= kSmall && (own || (on_host(x) && on_host(y) && on_host(out)));
     int *mx = nullptr, *my = nullptr, *mo = nullptr;
     if (!small && in_place_safe(x, out, n) && in_place_safe(y, out, n)) {
       cudaMemoryType type;
@@ -374,6 +329,61 @@ int h2h_query_batch_host(const h2h_graph *hc, const int *x, const int *y, int *o
       throw gh::Error(H2H_ERR_ARG, "vertex id out of range in batch (those pairs answered -1)");
     }
   });
+}
+
+static int single_query(const h2h_graph *h, int x, int y, int mode) {
+  if (!h) { gh::set_last_error("null handle"); return -1; }
+  int res = -1;
+  int rc = guarded([&] {
+    const gh::Graph &g = h->g;
+    GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
+    GH_CHECK(x >= 0 && x < g.n && y >= 0 && y < g.n, H2H_ERR_ARG, "vertex out of range");
+    int out = 0;
+    GH_CHECK(host_batch(h, &x, &y, &out, 1, mode, true) == H2H_OK, H2H_ERR_CUDA, gh::last_error());
+    res = out;
+  });
+  return rc == H2H_OK ? res : -1;
+}
+
+int h2h_query_lca_nohub(const h2h_graph *h, int x, int y) { return single_query(h, x, y, H2H_QUERY_LCA); }
+int h2h_query_nolca_nohub(const h2h_graph *h, int x, int y) { return single_query(h, x, y, H2H_QUERY_NOLCA); }
+
+int h2h_query_batch(const h2h_graph *h, const int *x_dev, const int *y_dev, int *out_dev, int64_t n, int mode,
+                    void *stream) {
+  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
+  return guarded([&] {
+    const gh::Graph &g = h->g;
+    GH_CHECK(g.labelled, H2H_ERR_STATE, "labels not built");
+    GH_CHECK(mode == H2H_QUERY_LCA || mode == H2H_QUERY_NOLCA, H2H_ERR_ARG, "mode must be 0 (LCA) or 1 (noLCA)");
+    GH_CHECK(n >= 0, H2H_ERR_ARG, "negative batch size");
+    GH_CHECK(n == 0 || (x_dev && y_dev && out_dev), H2H_ERR_ARG, "null buffer");
+    gh::run_query_batch(g, x_dev, y_dev, out_dev, n, mode, (cudaStream_t)stream);
+  });
+}
+
+int h2h_query_batch_plain(const h2h_graph *h, const int *x_dev, const int *y_dev, int *out_dev, int64_t n, int mode,
+                          void *stream) {
+  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
+  return guarded([&] {
+    GH_CHECK(h->g.labelled, H2H_ERR_STATE, "labels not built");
+    GH_CHECK(mode == H2H_QUERY_LCA || mode == H2H_QUERY_NOLCA, H2H_ERR_ARG, "mode must be 0 (LCA) or 1 (noLCA)");
+    GH_CHECK(n == 0 || (x_dev && y_dev && out_dev), H2H_ERR_ARG, "null buffer");
+    gh::run_query_batch_plain(h->g, x_dev, y_dev, out_dev, n, mode, (cudaStream_t)stream);
+  });
+}
+
+int h2h_fill_labels_plain(const h2h_graph *h, double *ms, int64_t *mismatches) {
+  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
+  return guarded([&] { gh::fill_labels_plain(h->g, 0, ms, mismatches); });
+}
+
+int h2h_fill_labels_plain_node(const h2h_graph *h, double *ms, int64_t *mismatches) {
+  if (!h) { gh::set_last_error("null handle"); return H2H_ERR_ARG; }
+  return guarded([&] { gh::fill_labels_plain(h->g, 1, ms, mismatches); });
+}
+
+int h2h_query_batch_host(const h2h_graph *h, const int *x, const int *y, int *out, int64_t n, int mode) {
+  return host_batch(h, x, y, out, n, mode, false);
 }
 
 int h2h_get_info(const h2h_graph *h, h2h_info *info) {

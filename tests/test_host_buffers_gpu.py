@@ -86,3 +86,23 @@ def test_page_locked_in_part(graph):
         for p in base:
             rt.cudaHostUnregister(p)
     assert np.array_equal(g.query(x, y), want)  # a refused copy is no error of the next call
+
+
+@pytest.mark.parametrize("which", range(3))
+def test_small_batch_in_device_memory(graph, which):
+    """Device memory given for host memory is the copies' to refuse, in small
+    batches as in large ones; the library does not touch it from the host."""
+    import gpuh2h
+    import torch
+    g, x, y, want = graph
+    host = [np.ascontiguousarray(x[:100]), np.ascontiguousarray(y[:100]), np.zeros(100, np.int32)]
+    p = [a.ctypes.data for a in host]
+    on_device = torch.from_numpy(host[which]).cuda()
+    p[which] = on_device.data_ptr()
+    try:
+        g.query_host_ptr(*p, 100)
+        torch.cuda.synchronize()
+        assert np.array_equal(on_device.cpu().numpy() if which == 2 else host[2], want[:100])
+    except gpuh2h.H2HError as e:
+        assert e.code == -5
+    assert np.array_equal(g.query(x[:100], y[:100]), want[:100])
