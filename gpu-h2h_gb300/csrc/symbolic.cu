@@ -491,23 +491,56 @@ __global__ void __launch_bounds__(512, 2) symbolic_kernel(SymArgs A) {
   if (!kGrid && CS > 1) cluster.sync();  // no CTA leaves while a peer may still read its rows
 }
 
-// Distinct neighbours of every vertex's input list as ~id and the number of
-// repeated entries.
+// Distinct neighbours of every vertex's input list as ~id, in the list's order,
+// and the number of repeated entries.  A thread takes a list of up to 32
+// entries, its warp the longer ones: comparing every pair in one thread took
+// 3.7 s for a vertex of 16,000 neighbours (the whole contraction takes 0.2 s).
 __global__ void distinct_lists_kernel(const int *adj_off, const int *adj_v, int64_t *slot_off, int *pool, int *lsize,
                                       int *extra, int n) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const int b = adj_off[v], e = adj_off[v + 1];
-    int *list = pool + b;  // the pool starts with the input lists' places
-    slot_off[v] = b;
-    int c = 0;
-    for (int i = b; i < e; i++) {
-      const int x = ~adj_v[i];
-      bool seen = false;
-      for (int q = 0; q < c && !seen; q++) seen = list[q] == x;
-      if (!seen) list[c++] = x;
+  const int lane = threadIdx.x & 31;
+  for (int64_t v0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~int64_t(31); v0 < n;
+       v0 += (int64_t)gridDim.x * blockDim.x) {
+    const int v = (int)v0 + lane;
+    const int b = v < n ? adj_off[v] : 0, e = v < n ? adj_off[v + 1] : 0;
+    if (v < n) slot_off[v] = b;  // the pool starts with the input lists' places
+    if (v < n && e - b <= 32) {
+      int *list = pool + b;
+      int c = 0;
+      for (int i = b; i < e; i++) {
+        const int x = ~adj_v[i];
+        bool seen = false;
+        for (int q = 0; q < c && !seen; q++) seen = list[q] == x;
+        if (!seen) list[c++] = x;
+      }
+      lsize[v] = c;
+      extra[v] = e - b - c;
     }
-    lsize[v] = c;
-    extra[v] = e - b - c;
+    for (unsigned todo = __ballot_sync(0xffffffffu, e - b > 32); todo; todo &= todo - 1) {
+      const int from = __ffs(todo) - 1;
+      const int lb = __shfl_sync(0xffffffffu, b, from), le = __shfl_sync(0xffffffffu, e, from);
+      int c = 0;
+      for (int i0 = lb; i0 < le; i0 += 32) {
+        const int i = i0 + lane, x = i < le ? adj_v[i] : -1;
+        bool fresh = i < le;
+        for (int q0 = lb; q0 < i0; q0 += 32) {  // a lane per earlier entry, handed round
+          const int y = adj_v[q0 + lane];
+#pragma unroll
+          for (int q = 0; q < 32; q++) fresh &= __shfl_sync(0xffffffffu, y, q) != x;
+        }
+#pragma unroll
+        for (int q = 0; q < 31; q++) {
+          const int y = __shfl_sync(0xffffffffu, x, q);
+          if (q < lane) fresh &= y != x;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, fresh);
+        if (fresh) pool[lb + c + __popc(bal & ((1u << lane) - 1u))] = ~x;
+        c += __popc(bal);
+      }
+      if (lane == 0) {
+        lsize[v0 + from] = c;
+        extra[v0 + from] = le - lb - c;
+      }
+    }
   }
 }
 

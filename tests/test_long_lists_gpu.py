@@ -1,0 +1,42 @@
+"""Vertices of many neighbours on bit rows: input lists around a warp's 32
+entries and longer, with repeated entries near and far, give the oracle's order
+and lists; one list of 16,000 entries is not compared pair by pair in one
+thread."""
+import time
+
+import numpy as np
+import pytest
+
+from small_graphs import star, write
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("leaves", (31, 32, 33, 63, 64, 65, 400))
+@pytest.mark.parametrize("C", (1, 2))
+def test_repeated_entries_of_a_long_list(tmp_path, leaves, C):
+    import gpuh2h
+    from oracle import oracle
+    n, edges = star(leaves)
+    edges = edges + [(a, b, w + 2) for a, b, w in edges[::3]] + [(a, b, max(1, w - 1)) for a, b, w in edges[::-5]]
+    ring = [(k, (k + 1) % leaves, 4) for k in range(0, leaves, 2)]  # not all leaves alike
+    files = write(tmp_path, n, [(u, v, w, 1 + (3 * w + u) % 17) for u, v, w in edges + ring], 2)
+    want = oracle.OracleGraph(*files, 2, C, 2).contract()
+    g = gpuh2h.Graph("t", 2, C, 2, 1, files=files).contraction_noHub(1)
+    assert np.array_equal(g.order(), want.order())
+    assert all(np.array_equal(a, b) for a, b in zip(g.adj(), want.adj()))
+    g.close()
+
+
+def test_one_very_long_list(tmp_path):
+    """0.2 s; every pair in one thread took 3.9."""
+    import gpuh2h
+    n, edges = star(16000)
+    files = write(tmp_path, n, [(u, v, w, w) for u, v, w in edges], 1)
+    gpuh2h.Graph("t", 1, 1, 2, 1, files=files).contraction_noHub(1).close()
+    g = gpuh2h.Graph("t", 1, 1, 2, 1, files=files)
+    t0 = time.perf_counter()
+    g.contraction_noHub(1)
+    assert time.perf_counter() - t0 < 2
+    assert np.array_equal(np.sort(g.order()), np.arange(n))
+    g.close()
