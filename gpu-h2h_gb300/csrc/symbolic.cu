@@ -663,6 +663,13 @@ bool ElimPlan::plan_bits() {
   // of 469 members 0.44 ms with one CTA each, 0.62 with 2, 0.59 with 4, 0.70 with 16.  Cells that
   // outnumber the SMs keep few warps (1,024 cells of 259 members: 0.54 ms with
   // 4 warps, 0.67 with 8; 2,048 cells of 489: 3.7 with 4, 2.8 with 8, 3.9 with 16).
+  // A shallow partition has many bottom cells of thousands of members, whose rows
+  // fill a cluster's shared memory, so that only a dozen cells run at a time.
+  // With the rows in global memory a cell takes as few CTAs as its other tables
+  // need, a pick 2.2 us + 0.4 ns per owned member + 0.1 ns per member:
+  // 256 cells of 3,907 members 221 ms in shared memory on 16 CTAs each, 27 in
+  // global memory on 2 (71 on the list kernels); 64 of 4,131 65.6 -> 11.9 (46.7);
+  // 128 of 7,813 187 on 16 CTAs -> 89 on 8 (77.6); 512 of 1,954 41.6 -> 11.4 (49.9).
   cudaFuncAttributes fa;
   GH_CUDA(cudaFuncGetAttributes(&fa, symbolic_kernel<false, false>));
   const int smem_dyn = enable_max_dynamic_smem(symbolic_kernel<false, false>);
@@ -681,6 +688,15 @@ bool ElimPlan::plan_bits() {
   auto smem_for = [&](int smax, int cs, bool global) -> int64_t {
     const int64_t own = (smax + cs - 1) / cs, w = (smax + 31) / 32 | 1;
     return own * (8 + 24) + 4LL * smax + 4LL * pow2(smax) + 8 * w + (global ? 0 : 4 * own * w);
+  };
+  // room for the rows of a launch's cells in global memory; asked only where
+  // they take more than 64 MB
+  auto rows_fit = [&](int ncell, int smax) {
+    const int64_t bytes = 4LL * ncell * smax * ((smax + 31) / 32 | 1);
+    if (bytes <= (int64_t(64) << 20)) return true;
+    size_t fr = 0, tot = 0;
+    GH_CUDA(cudaMemGetInfo(&fr, &tot));
+    return (uint64_t)bytes <= fr / 4;
   };
   std::vector<SymCell> table;
   int64_t grow_words = 0, grid_best = 0;
@@ -708,10 +724,12 @@ bool ElimPlan::plan_bits() {
         L.kmax = std::max(L.kmax, cells[c].c.count);
       }
       double best = 1e300;
-      for (int global = 0; global < 2 && best > 1e299; global++)  // rows in global memory only where nothing else fits
+      const bool bottom = st == 0 && nsteps > 0;
+      // rows in global memory only for bottom cells, or where nothing else fits
+      for (int global = 0; global < 2 && (best > 1e299 || (bottom && rows_fit(L.ncell, smax))); global++)
         for (int cs = 1; cs <= 16; cs <<= 1) {
           const int64_t sm = smem_for(smax, cs, global);
-          if (sm > smem_dyn || (global && cs < 16)) continue;
+          if (sm > smem_dyn || (global && cs < 16 && !bottom)) continue;
           const int own = (smax + cs - 1) / cs, w = (smax + 31) / 32;
           int nw = cs > 1 ? (own >= 64 ? 16 : 8) : L.ncell > 4 * nsm ? (own >= 384 ? 8 : 4) : own >= 300 ? 16 : 8;
           if ((own + 31) / 32 > kMaxGroups) continue;
@@ -734,8 +752,8 @@ bool ElimPlan::plan_bits() {
             continue;
           }
           const double waves = std::ceil((double)L.ncell / fit);
-          const double rows = (st == 0 && nsteps > 0 ? 0.1 : 1.0) * (1.0 + 4.5e-5 * smax * w);
-          const double cost = waves * ((cs == 1 ? 1.1 : 1.5) + rows / cs);
+          const double rows = (bottom ? 0.1 : 1.0) * (1.0 + 4.5e-5 * smax * w);
+          const double cost = waves * (global && bottom ? 2.2 + 4e-4 * own + 1e-4 * smax : (cs == 1 ? 1.1 : 1.5) + rows / cs);
           if (cost < best * 0.99) {
             best = cost;
             L.cs = cs;
