@@ -589,43 +589,74 @@ __global__ void mark_kernel(const int *verts, int n, unsigned char *flag) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) flag[verts[i]] = 1;
 }
 
-// The cell every arc v -> x with x an upper neighbour of v starts from; -1
-// for the other direction and for repeated arcs of the global order.
+constexpr int64_t kOnce = int64_t(1) << 62;  // of a cell that only the first of its arcs may enter
+
+// The cell every arc v -> x with x an upper neighbour of v starts from; -1 for
+// the other direction.  A thread per arc (a thread per vertex is as slow as its
+// longest list): a warp finds the tails of its first and last arc, its lanes
+// theirs between the two.
 __global__ void arc_cells_kernel(BlockArgs B, const int *adj_off, const int *adj_v, const unsigned char *global,
-                                 int64_t *arc_cell, int n) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const int d = B.depth[v], b = B.blk_of[v], i = B.loc_of[v];
-    const int64_t m0 = B.moff[b], so = B.soff[b];
-    const int m = (int)(B.moff[b + 1] - m0), Rp = ((int)(B.boff[b + 1] - B.boff[b]) + 3) & ~3;
-    const int dt = B.depth[B.blk_top[b]] - 1;
-    const int a0 = adj_off[v], a1 = adj_off[v + 1];
-    for (int e = a0; e < a1; e++) {
-      const int x = adj_v[e];
-      int64_t cell = -1;
-      const int p = B.depth[x] - 1;
-      bool use = p < d - 1;
-      if (use && global[v])
-        for (int q = a0; q < e && use; q++) use = adj_v[q] != x;
-      if (use) {
-        int c;
-        if (p >= dt) {
-          c = m + B.loc_of[x];
-        } else {
-          int lo = 0, hi = m;
-          while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (B.bm_p[m0 + mid] < p) lo = mid + 1; else hi = mid;
-          }
-          c = lo;
-          if (lo >= m || B.bm_p[m0 + lo] != p) {
-            atomicCAS(B.err, 0, kErrNested);
-            c = -1;
-          }
-        }
-        if (c >= 0) cell = so + (int64_t)c * Rp + i;
-      }
-      arc_cell[e] = cell;
+                                 int64_t *arc_cell, unsigned *first, int n, int64_t m) {
+  const int lane = threadIdx.x & 31;
+  auto tail = [&](int64_t e, int lo, int hi) {  // the last list that starts at or before e
+    while (lo < hi) {
+      const int mid = lo + (hi - lo + 1) / 2;
+      if (adj_off[mid] <= e) lo = mid; else hi = mid - 1;
     }
+    return lo;
+  };
+  for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~int64_t(31); base < m;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int end = tail(lane == 0 ? base : min(base + 31, m - 1), 0, n - 1);
+    const int v0 = __shfl_sync(0xffffffffu, end, 0), v1 = __shfl_sync(0xffffffffu, end, 31);
+    const int64_t e = base + lane;
+    if (e >= m) continue;
+    const int v = tail(e, v0, v1), x = adj_v[e], p = B.depth[x] - 1;
+    int64_t cell = -1;
+    if (p < B.depth[v] - 1) {
+      const int b = B.blk_of[v];
+      const int64_t m0 = B.moff[b];
+      const int mem = (int)(B.moff[b + 1] - m0), Rp = ((int)(B.boff[b + 1] - B.boff[b]) + 3) & ~3;
+      int c;
+      if (p >= B.depth[B.blk_top[b]] - 1) {
+        c = mem + B.loc_of[x];
+      } else {
+        int lo = 0, hi = mem;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (B.bm_p[m0 + mid] < p) lo = mid + 1; else hi = mid;
+        }
+        c = lo;
+        if (lo >= mem || B.bm_p[m0 + lo] != p) {
+          atomicCAS(B.err, 0, kErrNested);
+          c = -1;
+        }
+      }
+      if (c >= 0) {
+        cell = B.soff[b] + (int64_t)c * Rp + B.loc_of[v];
+        if (global[v]) {
+          first[cell] = kInf;
+          cell |= kOnce;
+        }
+      }
+    }
+    arc_cell[e] = cell;
+  }
+}
+
+// Of the repeated arcs of the global order the first one stays: `first` takes
+// the smallest place per cell, then the others are dropped.
+__global__ void first_arcs_kernel(const int64_t *arc_cell, unsigned *first, int64_t m) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = arc_cell[e];
+    if (c >= 0 && (c & kOnce)) atomicMin(first + (c & ~kOnce), (unsigned)e);
+  }
+}
+
+__global__ void drop_arcs_kernel(int64_t *arc_cell, const unsigned *first, int64_t m) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = arc_cell[e];
+    if (c >= 0 && (c & kOnce)) arc_cell[e] = first[c & ~kOnce] == (unsigned)e ? c & ~kOnce : -1;
   }
 }
 
@@ -1512,8 +1543,15 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
     mark_kernel<<<grid_for(from.heap_total, nsm), 256>>>(from.heap_verts, from.heap_total, global);
     GH_CUDA(cudaGetLastError());
   }
-  arc_cells_kernel<<<grid_for(N, nsm), 256>>>(B, from.adj_off, from.adj_v, global, arc_cell, N);
-  GH_CUDA(cudaGetLastError());
+  if (from.M) {
+    const int ga = grid_for(from.M, nsm);
+    arc_cells_kernel<<<ga, 256>>>(B, from.adj_off, from.adj_v, global, arc_cell, direct, N, from.M);
+    if (from.heap_total) {  // the weights' cells are not in use yet
+      first_arcs_kernel<<<ga, 256>>>(arc_cell, direct, from.M);
+      drop_arcs_kernel<<<ga, 256>>>(arc_cell, direct, from.M);
+    }
+    GH_CUDA(cudaGetLastError());
+  }
   GH_CHECK(read_one(werr) == 0, H2H_ERR_STATE, "an upper neighbour is missing from its block's separator");
 }
 
