@@ -733,6 +733,10 @@ bool ElimPlan::plan_bits() {
           const int own = (smax + cs - 1) / cs, w = (smax + 31) / 32;
           int nw = cs > 1 ? (own >= 64 ? 16 : 8) : L.ncell > 4 * nsm ? (own >= 384 ? 8 : 4) : own >= 300 ? 16 : 8;
           if ((own + 31) / 32 > kMaxGroups) continue;
+          const double rows = (bottom ? 0.1 : 1.0) * (1.0 + 4.5e-5 * smax * w);
+          const double pick = global && bottom ? 2.2 + 4e-4 * own + 1e-4 * smax : (cs == 1 ? 1.1 : 1.5) + rows / cs;
+          // with an SM's 64 warps full it would not be better: the occupancy need not be asked
+          if (std::ceil((double)L.ncell * cs * nw / (64.0 * nsm)) * pick >= best * 0.99) continue;
           int fit = 0;
           cudaLaunchConfig_t cfg = {};
           cudaLaunchAttribute attr[1];
@@ -752,8 +756,7 @@ bool ElimPlan::plan_bits() {
             continue;
           }
           const double waves = std::ceil((double)L.ncell / fit);
-          const double rows = (bottom ? 0.1 : 1.0) * (1.0 + 4.5e-5 * smax * w);
-          const double cost = waves * (global && bottom ? 2.2 + 4e-4 * own + 1e-4 * smax : (cs == 1 ? 1.1 : 1.5) + rows / cs);
+          const double cost = waves * pick;
           if (cost < best * 0.99) {
             best = cost;
             L.cs = cs;
