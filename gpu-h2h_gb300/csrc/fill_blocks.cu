@@ -1617,8 +1617,17 @@ std::vector<int> FillPlan::level_classes() const {
 void FillPlan::build_tiles(const TilePolicy &pol) {
   Workspace ws;
   int *ntask = ws.get<int>(nblk + 1), *pieces = ws.get<int>(nblk + 1), *several = ws.get<int>(nblk + 1);
-  int64_t *piece0 = ws.get<int64_t>(nblk + 1), *slot0 = ws.get<int64_t>(nblk + 1), *new_task0 = ws.get<int64_t>(nblk + 1);
-  int *new_tcols = ws.get<int>(nblk + 1);
+  int64_t *piece0 = ws.get<int64_t>(nblk + 1), *slot0 = ws.get<int64_t>(nblk + 1);
+  // the first table is made in place: there is none to keep
+  const bool again = ntasks > 0;
+  if (!task0) {
+    int64_t *t0 = work.get<int64_t>(nblk + 1);
+    tcols = work.get<int>(nblk + 1);
+    mslot = work.get<int>(nblk + 1);
+    task0 = t0;
+  }
+  int64_t *new_task0 = again ? ws.get<int64_t>(nblk + 1) : task0;
+  int *new_tcols = again ? ws.get<int>(nblk + 1) : tcols;
   block_tasks_kernel<<<grid_for(nblk + 1, nsm), 256>>>(blk_top, depth, blk_mem, blk_boff, lvl_cls, pol, ntask, pieces,
                                                             new_tcols, several, nblk);
   GH_CUDA(cudaGetLastError());
@@ -1633,12 +1642,6 @@ void FillPlan::build_tiles(const TilePolicy &pol) {
   GH_CHECK(new_smem <= (size_t)smem_dyn, H2H_ERR_DEVICE, "tree too large for the fill staging");
   int per_sm = 0;
   GH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_fill_kernel, 128, new_smem));
-  if (!task0) {
-    int64_t *t0 = work.get<int64_t>(nblk + 1);
-    tcols = work.get<int>(nblk + 1);
-    mslot = work.get<int>(nblk + 1);
-    task0 = t0;
-  }
   // the buffers that grow: all of them before any is replaced
   struct Grown {
     void *p = nullptr;
@@ -1656,8 +1659,10 @@ void FillPlan::build_tiles(const TilePolicy &pol) {
     tasks_cap = new_ntasks;
     new_tasks.p = std::exchange(tasks, static_cast<int *>(new_tasks.p));
   }
-  GH_CUDA(cudaMemcpyAsync(task0, new_task0, sizeof(int64_t) * (nblk + 1), cudaMemcpyDeviceToDevice));
-  GH_CUDA(cudaMemcpyAsync(tcols, new_tcols, sizeof(int) * (nblk + 1), cudaMemcpyDeviceToDevice));
+  if (again) {
+    GH_CUDA(cudaMemcpyAsync(task0, new_task0, sizeof(int64_t) * (nblk + 1), cudaMemcpyDeviceToDevice));
+    GH_CUDA(cudaMemcpyAsync(tcols, new_tcols, sizeof(int) * (nblk + 1), cudaMemcpyDeviceToDevice));
+  }
   narrow_kernel<<<grid_for(nblk + 1, nsm), 256>>>(slot0, mslot, nblk + 1);
   expand_tasks_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(task0, tasks, nblk);
   GH_CUDA(cudaGetLastError());
