@@ -45,6 +45,7 @@ struct h2h_batch {
     elim.reset();
     if (stream) cudaStreamDestroy(stream);
   }
+  bool build_once(bool allow_bits, gh::Clock &clk);
   void drop_graph() {
     if (exec) cudaGraphExecDestroy(exec);
     exec = nullptr;
@@ -92,6 +93,65 @@ void copy_policy(const std::string &p, char *out, int cap) {
 
 }  // namespace
 
+// One attempt at the batch's graphs, whose elimination sets are made.  False:
+// the list kernels are to make another.
+bool h2h_batch::build_once(bool allow_bits, gh::Clock &clk) {
+  elim = std::make_unique<gh::ElimPlan>(gs, allow_bits);
+  GH_CUDA(cudaDeviceSynchronize());
+  info.t_plan_us = clk.us();
+  clk.reset();
+  GH_CUDA(cudaEventRecord(ev[0], stream));
+  cudaEvent_t hev[2] = {ev[1], ev[2]};
+  if (!elim->run(stream, hev, std::getenv("GPUH2H_TRACE") != nullptr)) return false;  // the list kernels
+  info.t_contract_us = event_us(ev[0], ev[1]);
+  info.t_global_us = event_us(ev[1], ev[2]);
+  clk.reset();
+  elim->build_lists();
+  for (gh::Graph *g : gs) {
+    g->contract_device = 1;
+    g->t.td_gpu = 0;
+    g->t.td_cpu = 0;
+  }
+  info.t_download_us = clk.us();
+  clk.reset();
+  gh::build_tree_gpu(gs);
+  gh::build_rmq_gpu(gs);
+  for (gh::Graph *g : gs) {
+    g->parallel_fine = 2;
+    g->construct_device = 1;
+    g->label_mode = H2H_LABEL_L4;
+    gh::allocate_labels_and_bfs(*g);
+  }
+  info.t_tree_us = clk.us();
+  clk.reset();
+  gh::TilePolicy pol;
+  if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
+    GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
+  fill = std::make_unique<gh::FillPlan>(gs, elim->lists, elim.get(), true);
+  if (!fill->weights_fit) return false;  // very wide separators: the list kernels need no update triangles
+  fill->prepare(pol);
+  GH_CUDA(cudaDeviceSynchronize());
+  info.t_fill_plan_us = clk.us();
+  clk.reset();
+  fill->enqueue_weights(stream);
+  fill->check_error();
+  info.t_contract_us += clk.us();  // the weights are the contraction's
+  clk.reset();
+  cudaEvent_t fev[2] = {ev[0], ev[3]};
+  fill->enqueue(stream, fev);
+  fill->check_error();
+  info.t_fill_us = event_us(ev[0], ev[3]);
+  fill->trace_report();
+  clk.reset();
+  fill->attach(true);
+  for (gh::Graph *g : gs) {
+    gh::upload_query_index(*g);
+    g->sets.reset();
+  }
+  info.t_attach_us = clk.us();
+  return true;
+}
+
 extern "C" {
 
 int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_batch **out) {
@@ -118,67 +178,17 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
     GH_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     for (auto &e : b->ev) GH_CUDA(cudaEventCreate(&e));
     for (bool allow_bits = true;; allow_bits = false) {
-      b->elim = std::make_unique<gh::ElimPlan>(b->gs, allow_bits);
-      GH_CUDA(cudaDeviceSynchronize());
-      b->info.t_plan_us = clk.us();
-      clk.reset();
-      GH_CUDA(cudaEventRecord(b->ev[0], b->stream));
-      cudaEvent_t hev[2] = {b->ev[1], b->ev[2]};
-      if (!b->elim->run(b->stream, hev, std::getenv("GPUH2H_TRACE") != nullptr)) {  // the list kernels
-        b->elim.reset();
-        continue;
+      try {
+        if (b->build_once(allow_bits, clk)) break;
+      } catch (const gh::Error &e) {  // no room on bit rows: the list kernels' needs are others
+        if (e.code != H2H_ERR_NOMEM || !b->elim || !b->elim->bits) throw;
       }
-      b->info.t_contract_us = event_us(b->ev[0], b->ev[1]);
-      b->info.t_global_us = event_us(b->ev[1], b->ev[2]);
-      clk.reset();
-      b->elim->build_lists();
+      b->fill.reset();
+      b->elim.reset();
       for (gh::Graph *g : b->gs) {
-        g->contract_device = 1;
-        g->t.td_gpu = 0;
-        g->t.td_cpu = 0;
+        g->tree.reset();
+        g->dev.release();
       }
-      b->info.t_download_us = clk.us();
-      clk.reset();
-      gh::build_tree_gpu(b->gs);
-      gh::build_rmq_gpu(b->gs);
-      for (gh::Graph *g : b->gs) {
-        g->parallel_fine = 2;
-        g->construct_device = 1;
-        g->label_mode = H2H_LABEL_L4;
-        gh::allocate_labels_and_bfs(*g);
-      }
-      b->info.t_tree_us = clk.us();
-      clk.reset();
-      gh::TilePolicy pol;
-      if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
-        GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
-      b->fill = std::make_unique<gh::FillPlan>(b->gs, b->elim->lists, b->elim.get());
-      if (!b->fill->weights_fit) {  // very wide separators: the list kernels, which need no update triangles
-        b->fill.reset();
-        b->elim.reset();
-        continue;
-      }
-      b->fill->prepare(pol);
-      GH_CUDA(cudaDeviceSynchronize());
-      b->info.t_fill_plan_us = clk.us();
-      clk.reset();
-      b->fill->enqueue_weights(b->stream);
-      b->fill->check_error();
-      b->info.t_contract_us += clk.us();  // the weights are the contraction's
-      clk.reset();
-      cudaEvent_t fev[2] = {b->ev[0], b->ev[3]};
-      b->fill->enqueue(b->stream, fev);
-      b->fill->check_error();
-      b->info.t_fill_us = event_us(b->ev[0], b->ev[3]);
-      b->fill->trace_report();
-      clk.reset();
-      b->fill->attach(true);
-      for (gh::Graph *g : b->gs) {
-        gh::upload_query_index(*g);
-        g->sets.reset();
-      }
-      b->info.t_attach_us = clk.us();
-      break;
     }
     unfinished.gs.clear();
     for (gh::Graph *g : b->gs) g->contracted = g->labelled = true;

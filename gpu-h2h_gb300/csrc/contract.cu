@@ -1921,65 +1921,78 @@ void download_lists(Graph &g) {
     for (int64_t k = 0; k < t; k++) g.x_id[k] -= g.dev.id_base;
 }
 
+// One attempt at contract_gpu.  False: the list kernels are to make another.
+// *bits: whether this one runs on bit rows.
+static bool contract_once(Graph &g, bool allow_bits, bool *bits) {
+  Clock clk;
+  const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
+  auto owned = std::make_unique<ElimPlan>(std::vector<Graph *>{&g}, allow_bits);
+  ElimPlan &plan = *owned;
+  *bits = plan.bits;
+  GH_CUDA(cudaDeviceSynchronize());
+  g.t.translate_lub = clk.us();
+  clk.reset();
+  cudaEvent_t ev[2];
+  GH_CUDA(cudaEventCreate(&ev[0]));
+  GH_CUDA(cudaEventCreate(&ev[1]));
+  long long heap_us = 0;
+  try {
+    if (!plan.run(0, ev, trace)) {  // lists longer than the list kernels' slots in all
+      cudaEventDestroy(ev[0]);
+      cudaEventDestroy(ev[1]);
+      return false;
+    }
+    float hms = 0;
+    GH_CUDA(cudaEventElapsedTime(&hms, ev[0], ev[1]));
+    heap_us = (long long)(hms * 1000.0f);
+  } catch (...) {
+    cudaEventDestroy(ev[0]);
+    cudaEventDestroy(ev[1]);
+    throw;
+  }
+  cudaEventDestroy(ev[0]);
+  cudaEventDestroy(ev[1]);
+  g.t.td_gpu = clk.us() - heap_us;  // partition levels
+  g.t.td_cpu = heap_us;             // global order over levels <= C (TDInCPUTime in the reference, on the GPU here)
+  clk.reset();
+  plan.build_lists();
+  g.t.translate_back = clk.us();
+  build_tree_gpu({&g});
+  build_rmq_gpu({&g});
+  clk.reset();
+  if (plan.bits) {
+    g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, plan.lists, &plan, false);
+    if (!g.plan->weights_fit) return false;  // very wide separators: the list kernels need no update triangles
+    g.plan->enqueue_weights(0);
+    g.plan->check_error();
+    g.plan->drop_weights();
+    if (trace) std::fprintf(stderr, "[gpuh2h] weights plan and weights: %.3f ms\n", clk.us() / 1e3);
+    g.t.td_gpu += clk.us();  // the weights
+    clk.reset();
+  }
+  owned.reset();  // the elimination's device state is freed here, inside the timed phase
+  g.sets.reset();
+  g.t.translate_back += clk.us();
+  return true;
+}
+
 // Whole contraction of one graph on the GPU: partition levels H..C+1, then
 // the global order over the vertices of levels <= C, the tree and the sparse
 // table.  The order, the fathers and the lists X(v)\{v} (sorted by id, the
 // lists at elimination time) stay on the device.  On bit rows the lists' weights follow from the
-// tree's blocks, which g.plan keeps for the label fill.
+// tree's blocks, which g.plan keeps for the label fill; where they find no room
+// the list kernels are tried, whose needs are others.
 void contract_gpu(Graph &g) {
-  Clock clk;
-  const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
   for (bool allow_bits = true;; allow_bits = false) {
-    auto owned = std::make_unique<ElimPlan>(std::vector<Graph *>{&g}, allow_bits);
-    ElimPlan &plan = *owned;
-    GH_CUDA(cudaDeviceSynchronize());
-    g.t.translate_lub = clk.us();
-    clk.reset();
-    cudaEvent_t ev[2];
-    GH_CUDA(cudaEventCreate(&ev[0]));
-    GH_CUDA(cudaEventCreate(&ev[1]));
-    long long heap_us = 0;
+    bool bits = false;
     try {
-      if (!plan.run(0, ev, trace)) {  // lists longer than the list kernels' slots in all
-        cudaEventDestroy(ev[0]);
-        cudaEventDestroy(ev[1]);
-        continue;
-      }
-      float hms = 0;
-      GH_CUDA(cudaEventElapsedTime(&hms, ev[0], ev[1]));
-      heap_us = (long long)(hms * 1000.0f);
-    } catch (...) {
-      cudaEventDestroy(ev[0]);
-      cudaEventDestroy(ev[1]);
-      throw;
+      if (contract_once(g, allow_bits, &bits)) return;
+    } catch (const Error &e) {
+      if (!bits || e.code != H2H_ERR_NOMEM) throw;
     }
-    cudaEventDestroy(ev[0]);
-    cudaEventDestroy(ev[1]);
-    g.t.td_gpu = clk.us() - heap_us;  // partition levels
-    g.t.td_cpu = heap_us;             // global order over levels <= C (TDInCPUTime in the reference, on the GPU here)
-    clk.reset();
-    plan.build_lists();
-    g.t.translate_back = clk.us();
-    build_tree_gpu({&g});
-    build_rmq_gpu({&g});
-    clk.reset();
-    if (plan.bits) {
-      g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, plan.lists, &plan);
-      if (!g.plan->weights_fit) {  // very wide separators: the list kernels, which need no update triangles
-        g.plan.reset();
-        continue;
-      }
-      g.plan->enqueue_weights(0);
-      g.plan->check_error();
-      g.plan->arcs = nullptr;
-      if (trace) std::fprintf(stderr, "[gpuh2h] weights plan and weights: %.3f ms\n", clk.us() / 1e3);
-      g.t.td_gpu += clk.us();  // the weights
-      clk.reset();
-    }
-    owned.reset();  // the elimination's device state is freed here, inside the timed phase
-    g.sets.reset();
-    g.t.translate_back += clk.us();
-    return;
+    g.plan.reset();
+    g.tree.reset();
+    g.dev.release();
   }
 }
 

@@ -1459,7 +1459,6 @@ void FillPlan::build_blocks() {
   cell_total = read_one(blk_soff + nblk);
   bm_p = work.get<int>(members);
   bm_row = work.get<int64_t>(members);
-  direct = work.get<unsigned>(cell_total);
   closed = work.get<unsigned>(cell_total);
   scatter_nodes_kernel<<<grid, 256>>>(top_of, blk_of_top, blk_boff, filled, bnode, N);
   block_nodes_kernel<<<grid_for((int64_t)nblk * 32, nsm), 256>>>(blk_top, blk_boff, blk_moff, hpos, pos_hash, pos_pos,
@@ -1502,21 +1501,27 @@ BlockArgs block_args(const FillPlan &P) {
 // arc's cell, the tasks of the block elimination and the blocks' places in
 // their parents.  The update triangles of very wide separators (a dense graph
 // of many thousand vertices) can outgrow the memory; weights_fit then tells
-// the caller to use the list kernels.
-void FillPlan::build_weights_plan(const ElimPlan &from) {
+// the caller to use the list kernels.  A plan that keeps its weights for
+// rebuilds has the label rows beside them; otherwise drop_weights frees what
+// only the weights need before the rows are allocated (of a 1M-vertex graph
+// 0.81 GB; small tables share the plan's memory and stay).
+void FillPlan::build_weights_plan(const ElimPlan &from, bool keep) {
   arcs = &from;
   Workspace ws;
   int *ntask = ws.get<int>(nblk + 1);
   int64_t *ucells = ws.get<int64_t>(nblk + 1);
   unsigned char *global = ws.get<unsigned char>(N);
+  const int64_t members = read_one(blk_moff + nblk);
+  // arrays of 8 MiB or more, which are allocations of their own in any arena
+  auto own = [&](int64_t bytes) -> DeviceArena & { return bytes >= (int64_t(8) << 20) ? weights_mem : work; };
+  direct = own(4 * cell_total).get<unsigned>(cell_total);
   wtask0 = work.get<int64_t>(nblk + 1);
   blk_up = work.get<int>(nblk);
   blk_uoff = work.get<int64_t>(nblk + 1);
   pending = work.get<int>(nblk);
   pend_init = work.get<int>(nblk);
-  const int64_t members = read_one(blk_moff + nblk);
-  bm_up = work.get<int>(members);
-  arc_cell = work.get<int64_t>(from.M);
+  bm_up = own(4 * members).get<int>(members);
+  arc_cell = own(8 * from.M).get<int64_t>(from.M);
   const BlockArgs B = block_args(*this);
   const int gb = grid_for(nblk + 1, nsm), gw = grid_for((int64_t)nblk * 32, nsm);
   weight_tasks_kernel<<<gb, 256>>>(blk_mem, ntask, nblk);
@@ -1524,7 +1529,7 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   exclusive_scan<int>(ntask, wtask0, nblk + 1, ws, 0);
   wtasks = read_one(wtask0 + nblk);
   GH_CHECK(wtasks < INT32_MAX, H2H_ERR_ARG, "too many weight tasks");
-  wtask_blk = work.get<int>(wtasks);
+  wtask_blk = own(4 * wtasks).get<int>(wtasks);
   expand_tasks_kernel<<<gw, 256>>>(wtask0, wtask_blk, nblk);
   GH_CUDA(cudaMemset(werr, 0, sizeof(int)));
   GH_CUDA(cudaMemset(pend_init, 0, sizeof(int) * nblk));
@@ -1535,9 +1540,16 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
   upd_total = read_one(blk_uoff + nblk);
   size_t fr = 0, tot = 0;
   GH_CUDA(cudaMemGetInfo(&fr, &tot));
-  weights_fit = (uint64_t)upd_total * 4 <= fr / 2;
+  const int64_t rows = keep ? dis_total + (int64_t)nblk * kRows * kRows : 0;  // label rows, in-block matrices
+  weights_fit = (uint64_t)(upd_total + rows) * 4 <= fr;
   if (!weights_fit) return;
-  upd = work.get<unsigned>(upd_total);
+  try {
+    upd = own(4 * upd_total).get<unsigned>(upd_total);
+  } catch (const Error &e) {
+    if (e.code != H2H_ERR_NOMEM) throw;
+    weights_fit = false;
+    return;
+  }
   GH_CUDA(cudaMemset(global, 0, N));
   if (from.heap_total) {
     mark_kernel<<<grid_for(from.heap_total, nsm), 256>>>(from.heap_verts, from.heap_total, global);
@@ -1553,6 +1565,14 @@ void FillPlan::build_weights_plan(const ElimPlan &from) {
     GH_CUDA(cudaGetLastError());
   }
   GH_CHECK(read_one(werr) == 0, H2H_ERR_STATE, "an upper neighbour is missing from its block's separator");
+}
+
+void FillPlan::drop_weights() {
+  arcs = nullptr;
+  weights_mem.release();
+  direct = upd = nullptr;
+  blk_up = bm_up = wtask_blk = pending = pend_init = nullptr;
+  blk_uoff = wtask0 = arc_cell = nullptr;
 }
 
 void FillPlan::enqueue_weights(cudaStream_t s) {

@@ -353,7 +353,7 @@ struct FillPlan {
   // weights from arcs: parent block and the members' places in it, update
   // triangles, task tables, arrivals a block waits for, each arc's cell
   const ElimPlan *arcs = nullptr;
-  bool weights_fit = true;  // false: the update triangles would take over half of the free memory
+  bool weights_fit = true;  // false: no room for the update triangles
   int *blk_up = nullptr, *bm_up = nullptr, *wtask_blk = nullptr, *pending = nullptr, *pend_init = nullptr;
   int64_t *blk_uoff = nullptr, *wtask0 = nullptr, *arc_cell = nullptr;
   unsigned *upd = nullptr;
@@ -368,19 +368,21 @@ struct FillPlan {
   size_t smem = 0;
   int nsm = 0;
   DeviceArena work;       // the plan's arrays but tasks and mbuf, which grow with the policy
+  DeviceArena weights_mem;  // those that only enqueue_weights reads, where they are large
   std::shared_ptr<DeviceArena> layout;  // the tree's heavy paths and segment offsets
   int64_t grown_bytes = 0;
-  int64_t work_bytes() const { return work.bytes + (layout ? layout->bytes : 0) + grown_bytes; }
+  int64_t work_bytes() const { return work.bytes + weights_mem.bytes + (layout ? layout->bytes : 0) + grown_bytes; }
   // The blocks and, when `arcs` made the order on bit rows, where each of its
   // arcs enters the blocks' weights.  lists: the graphs' X lists in the same
-  // forest numbering.
-  FillPlan(const std::vector<Graph *> &graphs, const ListStore &lists, const ElimPlan *arcs);
+  // forest numbering.  keep: the weights are made again after the labels (rebuilds).
+  FillPlan(const std::vector<Graph *> &graphs, const ListStore &lists, const ElimPlan *arcs, bool keep);
   ~FillPlan();
   void release_work();
   FillPlan(const FillPlan &) = delete;
   FillPlan &operator=(const FillPlan &) = delete;
   void build_blocks();
-  void build_weights_plan(const ElimPlan &arcs);
+  void build_weights_plan(const ElimPlan &arcs, bool keep);
+  void drop_weights();  // after the weights of a plan that makes them once
   void prepare(const TilePolicy &pol);  // label rows and tasks
   void build_tiles(const TilePolicy &pol);
   std::vector<int> level_classes() const;  // TilePolicy class per forest level

@@ -407,7 +407,7 @@ bool TilePolicy::parse(const std::string &text) {
   return true;
 }
 
-FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, const ElimPlan *from)
+FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, const ElimPlan *from, bool keep)
     : gs(graphs), lists(lst) {
   const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
   Clock tclk;
@@ -482,7 +482,7 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
     build_blocks();
     mark("blocks");
     if (from && from->bits) {
-      build_weights_plan(*from);
+      build_weights_plan(*from, keep);
       mark("weights plan");
     }
   } catch (...) {
@@ -500,6 +500,7 @@ void FillPlan::prepare(const TilePolicy &pol) {
 
 void FillPlan::release_work() {
   work.release();
+  weights_mem.release();
   layout.reset();
   for (void *p : {(void *)tasks, (void *)mbuf, (void *)trace_t}) cudaFree(p);
   grown_bytes = tasks_cap = mslots_cap = ntasks = mslots = 0;
@@ -704,7 +705,7 @@ void fill_labels_gpu(Graph &g) {
     if (const char *e = std::getenv("GPUH2H_TILE_POLICY"))
       GH_CHECK(pol.parse(e), H2H_ERR_ARG, "GPUH2H_TILE_POLICY: expected 12 entries small_work/col_block/sep_chunk");
     if (!g.plan) {  // contracted by the list kernels
-      g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, D.lists, nullptr);
+      g.plan = std::make_shared<FillPlan>(std::vector<Graph *>{&g}, D.lists, nullptr, false);
       g.plan->enqueue_weights(0);
     }
     FillPlan &plan = *g.plan;

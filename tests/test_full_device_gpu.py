@@ -70,3 +70,49 @@ def test_failed_batch_leaves_loaded_graphs(tmp_path, room_mb):
     b.close()
     for g in gs:
         g.close()
+
+
+def test_weights_leave_room_for_labels(tmp_path):
+    """A single build's highest use is 1.54 GB here, 1.69 when what only the weights
+    need stays until the labels are filled."""
+    import gpuh2h
+    gpuh2h.generate_road(str(tmp_path), "r", n=264346, target_arcs=int(264346 * 2.776), aspect_milli=1300,
+                         jitter_milli=300, diag_permille=50, hw_tiers=1, hw_permille10=50, hw_k=3, hw_scale_milli=400,
+                         partition_height=11, seed=5, cols=0, drop_permille=0)
+    files = gpuh2h.files_for(str(tmp_path), "r")
+    gpuh2h.Graph("r", 11, 2, 8, 1, files=files).contraction_noHub(1).constructLabel_noHub().close()
+    with device_room(1600 << 20):
+        g = gpuh2h.Graph("r", 11, 2, 8, 1, files=files).contraction_noHub(1).constructLabel_noHub()
+    assert g.info()["label_size"] > 0
+    g.close()
+
+
+@pytest.mark.parametrize("batch", (False, True))
+def test_triangles_without_room_use_the_list_kernels(tmp_path, monkeypatch, capfd, batch):
+    """The update triangles of a clique take 64 MB, its lists 9."""
+    import gpuh2h
+    from small_graphs import clique, write
+    n, edges = clique(1500)
+    files = write(tmp_path, n, [(u, v, w, w) for u, v, w in edges], 1)
+
+    def build():
+        b = gpuh2h.Batch([g]) if batch else g.contraction_noHub(1).constructLabel_noHub()
+        out = [g.order(), *g.adj(), g.labels()["dis"]]
+        if batch:
+            b.rebuild()
+            assert np.array_equal(g.labels()["dis"], out[-1])
+            b.close()
+        return out
+
+    g = gpuh2h.Graph("g", 1, 1, 2, 1, files=files)
+    want = build()
+    g.close()
+    g = gpuh2h.Graph("g", 1, 1, 2, 1, files=files)
+    monkeypatch.setenv("GPUH2H_TRACE", "1")
+    capfd.readouterr()
+    with device_room((180 if batch else 150) << 20):
+        got = build()
+    err = capfd.readouterr().err
+    assert "elim bits heap" in err and "elim heap" in err
+    assert all(np.array_equal(a, b) for a, b in zip(want, got))
+    g.close()
