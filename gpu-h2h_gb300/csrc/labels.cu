@@ -494,7 +494,7 @@ FillPlan::FillPlan(const std::vector<Graph *> &graphs, const ListStore &lst, con
 FillPlan::~FillPlan() { release_work(); }
 
 void FillPlan::prepare(const TilePolicy &pol) {
-  dis = storage->mem.get<int>(dis_total);
+  if (!dis) dis = storage->mem.get<int>(dis_total);  // a second attempt has them already
   build_tiles(pol);
 }
 
@@ -737,8 +737,13 @@ void fill_labels_gpu(Graph &g) {
     return;
   }
   g.plan.reset();
-  g.tree.reset();  // its host copies are made (allocate_labels_and_bfs)
   D.release_labels();
+  struct Undo {  // what a fill that fails had allocated; the tree stays for another
+    DeviceIndex *d;
+    ~Undo() {
+      if (d) d->release_labels();
+    }
+  } undo{&D};
   D.n = n;
   D.pos_base = 0;
   // padded row offsets
@@ -834,6 +839,8 @@ void fill_labels_gpu(Graph &g) {
     throw;
   }
   cleanup();
+  undo.d = nullptr;
+  g.tree.reset();  // its host copies are made (allocate_labels_and_bfs)
   g.drow_host.swap(drow);
   g.row0 = 0;
   g.row1 = D.dis_padded;

@@ -116,3 +116,26 @@ def test_triangles_without_room_use_the_list_kernels(tmp_path, monkeypatch, capf
     assert "elim bits heap" in err and "elim heap" in err
     assert all(np.array_equal(a, b) for a, b in zip(want, got))
     g.close()
+
+
+def test_labels_after_a_fill_without_room(tmp_path):
+    """A label fill of either kind that finds no room can be followed by either."""
+    import gpuh2h
+    files = _road(tmp_path, 70000, 9)
+    want = {}
+    for mode in (gpuh2h.LABEL_L3, gpuh2h.LABEL_L4):
+        ref = gpuh2h.Graph("r", 9, 2, 2, 1, files=files).contraction_noHub(1).constructLabel_noHub(2, 1, mode)
+        want[mode] = ref.labels()["dis"]
+        ref.close()
+    for modes in ((3, 4), (4, 4), (4, 3), (3, 3), (3, 4, 3)):
+        g = gpuh2h.Graph("r", 9, 2, 2, 1, files=files).contraction_noHub(1)
+        adj = g.adj()
+        with device_room(20 << 20):
+            for mode in modes[:-1]:
+                with pytest.raises(gpuh2h.H2HError) as e:
+                    g.constructLabel_noHub(2, 1, mode)
+                assert e.value.code == -6
+        g.constructLabel_noHub(2, 1, modes[-1])
+        assert np.array_equal(g.labels()["dis"], want[modes[-1]])
+        assert all(np.array_equal(a, b) for a, b in zip(g.adj(), adj))
+        g.close()
