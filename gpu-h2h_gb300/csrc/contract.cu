@@ -1323,24 +1323,24 @@ ElimPlan::ElimPlan(const std::vector<Graph *> &graphs, bool allow_bits) : gs(gra
       slot_nbr = mem.get<int>(pool_size + 4);  // + 4: a list's last 128-bit load stays inside
       slot_w = mem.get<int>(pool_size + 4);
       slot_off_init = mem.get<int64_t>(N);
+      cap = mem.get<int>(N);
+      deg0 = mem.get<int>(N);
+      h0 = mem.get<int>(N);
+      cpos = mem.get<int>(N);
+      cell_start = mem.get<int>(fcs.size());
+      cell_count = mem.get<int>(fcc.size());
     }
     pool_next = mem.get<unsigned long long>(1);
     pool_first = mem.get<unsigned long long>(1);
     slot_off = mem.get<int64_t>(N);
     lsize = mem.get<int>((int64_t)N + 1);  // + 1: the end of a scan
-    cap = mem.get<int>(N);
     cap_init = mem.get<int>(N);
     height = mem.get<int>(N);
     elim = mem.get<int>(N);
     elim_init = mem.get<int>(N);
-    deg0 = mem.get<int>(N);
     deg_init = mem.get<int>(N);
-    h0 = mem.get<int>(N);
-    cpos = mem.get<int>(N);
     err = mem.get<int>(1);
     ljunk = mem.get<int>(N);
-    cell_start = mem.get<int>(fcs.size());
-    cell_count = mem.get<int>(fcc.size());
     adj_off = mem.get<int>(N + 1);
     adj_v = mem.get<int>(std::max<int64_t>(M, 1));
     adj_w = mem.get<int>(std::max<int64_t>(M, 1));

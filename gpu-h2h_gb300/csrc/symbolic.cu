@@ -670,8 +670,6 @@ bool ElimPlan::plan_bits() {
   // 256 cells of 3,907 members 221 ms in shared memory on 16 CTAs each, 27 in
   // global memory on 2 (71 on the list kernels); 64 of 4,131 65.6 -> 11.9 (46.7);
   // 128 of 7,813 187 on 16 CTAs -> 89 on 8 (77.6); 512 of 1,954 41.6 -> 11.4 (49.9).
-  cudaFuncAttributes fa;
-  GH_CUDA(cudaFuncGetAttributes(&fa, symbolic_kernel<false, false>));
   const int smem_dyn = enable_max_dynamic_smem(symbolic_kernel<false, false>);
   enable_max_dynamic_smem(symbolic_kernel<true, false>);
   const int smem_grid = enable_max_dynamic_smem(symbolic_kernel<true, true>);
