@@ -2,6 +2,7 @@
 // include/gpuh2h_tools.h.  Every call converts internal exceptions into a
 // status code and a per-thread message; nothing exits the process.
 #include <cuda.h>
+#include <dlfcn.h>
 
 #include <algorithm>
 #include <atomic>
@@ -37,10 +38,9 @@ int *mapped_ints(const int *p, int64_t n, cudaMemoryType *type) {
   if (n <= 0 || a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
   // the range p belongs to: the runtime tells the kind of its first byte only
   using Attributes = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
-  static const Attributes attributes = [] {
-    void *f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault) != cudaSuccess)
-      cudaGetLastError();
+  static const Attributes attributes = [] {  // of the driver the runtime has loaded, which stays so
+    void *lib = dlopen("libcuda.so.1", RTLD_LAZY | RTLD_NOLOAD);
+    void *f = lib ? dlsym(lib, "cuPointerGetAttributes") : nullptr;
     return reinterpret_cast<Attributes>(f);
   }();
   unsigned long long start = 0;
