@@ -12,9 +12,9 @@
 //
 // The list structure, the elimination order, the tree and the label layout
 // depend only on the arcs, never on their weights, so a rebuild after new
-// weights replays the device work alone: the reset of the lists, every
-// elimination launch, the gather of shortcut weights into the pos entries
-// and the fill, captured once as a CUDA graph.
+// weights replays the block elimination of the weights and the fill, captured
+// once as a CUDA graph (with the list kernels also the reset of the lists, every
+// elimination launch and the gather of the shortcut weights).
 #include <algorithm>
 #include <cstdlib>
 #include <cstdio>

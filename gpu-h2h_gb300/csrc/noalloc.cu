@@ -14,7 +14,7 @@
 // A first kernel checks every caller-passed offset, id and depth against the
 // declared sizes and sets the error word before anything else is written;
 // the fill kernel does no work once that word is set.  The fill itself is
-// the dataflow form of the L4 label fill (labels.cu):
+// node by node, not over blocks of the tree, whose tables outgrow the scratch:
 // persistent CTAs take nodes in the caller's order, wait for the father's
 // flag (bounded spin with an error exit), stage the node's separator and
 // ancestor rows in shared memory and compute each label column as the exact

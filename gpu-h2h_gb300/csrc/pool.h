@@ -1,6 +1,6 @@
 // pool.h -- a fixed set of worker threads with a blocking parallel_for, used
-// by the host phases (elimination fill-in merges, sparse table, label
-// allocation).  The reference spawns fresh std::threads per level instead.
+// by the host phases (reading and checking files, the L3 fill's position
+// lists).  The reference spawns fresh std::threads per level instead.
 #pragma once
 
 #include <algorithm>

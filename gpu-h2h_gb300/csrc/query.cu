@@ -103,9 +103,9 @@ __device__ __forceinline__ int64_t rmq_row(const QArgs &A, int i) {
 //
 // Bound: HBM on large batches, the chain of dependent loads on small ones.  On
 // one GB300, against loading positions and entries of one query in turn: 2e6
-// pairs on a 264k-vertex road graph 800 -> 690 us (0.91 of HBM), 1e5 pairs 73
+// pairs on a 264k-vertex road graph 812 -> 692 us (0.91 of HBM), 1e5 pairs 72
 // -> 61 us, 1e5 pairs in noLCA mode on a 70k-vertex graph 66 -> 45 us, 1e3
-// pairs 9.6 -> 7.8 us.  Spreading a warp over several queries (8 lanes each)
+// pairs 8 us either way.  Spreading a warp over several queries (8 lanes each)
 // took 2,200 us: a row is then read in 128-byte pieces at different times,
 // which DRAM serves at a third of its rate.
 template <bool LCA_MODE, int TILE>

@@ -1,6 +1,6 @@
 // scan.h -- exclusive prefix sums on the GPU and the scratch memory they take,
-// shared by the tree build (tree_gpu.cu) and the label fill's plan
-// (fill_blocks.cu).
+// shared by the loader, the elimination sets, the tree build and the label
+// fill's plan.
 #pragma once
 
 #include <algorithm>

@@ -101,8 +101,9 @@ int h2h_query_batch(const h2h_graph *g, const int *x_dev, const int *y_dev, int 
 
 /* The same from host buffers, the answers in `out` on return (the Query_noHub
  * flow, main.cu:218-240: translateQuery, kernel, translateQueryResultBack).
- * Page-locked buffers and batches of up to 4,096 pairs are read and written
- * by the kernel over the host link; larger pageable ones are copied.
+ * Batches of up to 4,096 pairs, and larger ones in page-locked buffers (each
+ * wholly inside one page-locked range, aligned to an int), are read and written
+ * by the kernel over the host link; others are copied.
  * Returns H2H_ERR_ARG when a pair holds an id outside [0, n) (those pairs
  * answer -1); the flag it reads belongs to this call path alone. */
 int h2h_query_batch_host(const h2h_graph *g, const int *x, const int *y, int *out, int64_t n, int mode);
@@ -192,7 +193,7 @@ typedef struct {
 
 /* Builds `count` graphs loaded by h2h_load / h2h_load_files and not yet
  * contracted.  threads: kept for callers; every phase runs on the GPU over all
- * graphs. */
+ * graphs.  A batch that fails leaves its graphs as they were loaded. */
 int h2h_batch_build(h2h_graph *const *graphs, int count, int threads, h2h_batch **out);
 /* Replaces the arc weights of graph `index` for the next h2h_batch_rebuild:
  * w holds one weight per stored arc in h2h_copy_input_arcs order. */
