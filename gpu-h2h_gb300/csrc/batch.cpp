@@ -181,7 +181,7 @@ int h2h_batch_build(h2h_graph *const *graphs, int count, int /*threads*/, h2h_ba
       try {
         if (b->build_once(allow_bits, clk)) break;
       } catch (const gh::Error &e) {  // no room on bit rows: the list kernels' needs are others
-        if (e.code != H2H_ERR_NOMEM || !b->elim || !b->elim->bits) throw;
+        if (e.code != H2H_ERR_NOMEM || !allow_bits || (b->elim && !b->elim->bits)) throw;
       }
       b->fill.reset();
       b->elim.reset();

@@ -1922,7 +1922,7 @@ void download_lists(Graph &g) {
 }
 
 // One attempt at contract_gpu.  False: the list kernels are to make another.
-// *bits: whether this one runs on bit rows.
+// *bits: whether this one runs on bit rows, as far as is known.
 static bool contract_once(Graph &g, bool allow_bits, bool *bits) {
   Clock clk;
   const bool trace = std::getenv("GPUH2H_TRACE") != nullptr;
@@ -1984,7 +1984,7 @@ static bool contract_once(Graph &g, bool allow_bits, bool *bits) {
 // the list kernels are tried, whose needs are others.
 void contract_gpu(Graph &g) {
   for (bool allow_bits = true;; allow_bits = false) {
-    bool bits = false;
+    bool bits = allow_bits;  // its own tables may already find no room
     try {
       if (contract_once(g, allow_bits, &bits)) return;
     } catch (const Error &e) {
